@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kAThreads, 1) mla_sparse_decode_kernel(const A
         reinterpret_cast<volatile uint32_t*>(base_ptr + kABarOffset + 8 * kABarriers);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(slot_ptr + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
     const int split = blockIdx.x;
     const int hg = blockIdx.y;
     const int b = blockIdx.z;
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kAThreads, 1) mla_sparse_decode_kernel(const A
     const uint32_t tmem_base = *slot_ptr;
 
     if (warp == 0) {
-        if (lane == 0 && n_tiles > 0) {
+        if (n_tiles > 0 && elect_one()) {
             bool ok = mbar_wait(qfull, 0, abort_flag, 61);
             // Scores of tile q are issued as soon as its rows have landed and a score buffer is
             // free (q - v < 2), P V of tile v as soon as its probabilities are written: whichever
@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(kFThreads, 1) attn_prefill_kernel(
     volatile uint32_t* slot_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + kFBarOff + 8 * (kFBars + 2));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(slot_ptr + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
     const int qb = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);   // heaviest first
     const int h = blockIdx.y;
     const int q0 = qb * 256;
@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(kFThreads, 1) attn_prefill_kernel(
     const uint32_t tmem_base = *slot_ptr;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // one operand: `chunks` 64-dim blocks of 128 rows starting at `row`, as one box or one per chunk
             auto load = [&](const CUtensorMap* m, bool one, int chunks, uint32_t dst, int row, int head,
                             uint32_t bar) {
@@ -707,7 +707,7 @@ __global__ void __launch_bounds__(kFThreads, 1) attn_prefill_kernel(
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // fp32 accumulate, bf16 x bf16, M = 128; S: both K-major, N = 128; O: B MN-major, N = 64 * cv
             const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (16u << 17) | (8u << 24);
             const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
@@ -964,7 +964,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFThreads, 1) attn_p
     volatile uint32_t* slot_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + kGBarOff + 8 * kGBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(slot_ptr + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
     const int rank = static_cast<int>(cluster_ctarank());
     const int qb = static_cast<int>(gridDim.x >> 1) - 1 - static_cast<int>(blockIdx.x >> 1);   // heaviest first
     const int h = blockIdx.y;
@@ -1013,7 +1013,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFThreads, 1) attn_p
 
     // The u-th use of a two-stage barrier (key tile 2 u + st) completes its phase u.
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             const int pe_head = a.pe_shared ? 0 : h;
             bool ok = true;
             auto load_k = [&](int j) {                         // this CTA's 128 keys of key tile j
@@ -1040,7 +1040,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFThreads, 1) attn_p
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (rank == 0 && lane == 0) {
+        if (rank == 0 && elect_one()) {
             // fp32 accumulate, bf16 x bf16, M = 256 over the pair; S: N = 256, both K-major; O: N = 128, B MN-major
             const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (32u << 17) | (16u << 24);
             const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (16u << 17) | (16u << 24);
@@ -1097,7 +1097,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFThreads, 1) attn_p
                 issue_pv(j);
                 RT_FTRACE(5, j);
             }
-        } else if (rank == 1 && lane == 0) {
+        } else if (rank == 1 && elect_one()) {
             // Relay: tells the leader that this CTA's tiles have landed, in the producer's order.
             bool ok = mbar_wait(q_full, 0, abort_flag, 88);
             if (ok) mbar_arrive_cluster(map_to_cta(q_full, 0));

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(
         reinterpret_cast<volatile uint32_t*>(base_ptr + Cfg::kBarOffset + 8 * (2 * Cfg::kStages + 4));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(slot_ptr + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
     const int num_m = (M + kBM - 1) / kBM, num_n = (N + BN - 1) / BN;
     const int k_splits = SPLITK ? k_splits_arg : 1;
     const int tiles_per_batch = num_m * num_n;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(
     const uint32_t tmem_base = *slot_ptr;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             int acc = 0;
@@ -281,7 +281,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBPThreads, 1) gemm_
         reinterpret_cast<volatile uint32_t*>(base_ptr + kBPBarOffset + 8 * (2 * kBPStages + 4));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(slot_ptr + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
     const int num_m = (M + 255) / 256, num_n = (N + 255) / 256;
@@ -314,7 +314,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBPThreads, 1) gemm_
     const uint32_t tmem_base = *slot_ptr;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -338,7 +338,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBPThreads, 1) gemm_
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (rank == 0 && lane == 0) {
+        if (rank == 0 && elect_one()) {
             const uint32_t peer_cempty0 = map_to_cta(cempty_bar(0), 1);
             const uint32_t peer_tfull0 = map_to_cta(tfull_bar(0), 1);
             int stage = 0, acc = 0;
@@ -379,7 +379,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBPThreads, 1) gemm_
                     acc_phase ^= 1u;
                 }
             }
-        } else if (rank == 1 && lane == 0) {
+        } else if (rank == 1 && elect_one()) {
             const uint32_t leader_cfull0 = map_to_cta(cfull_bar(0), 0);
             int stage = 0;
             uint32_t phase = 0;
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(kFThreads, 1) gemm_nvfp4_kernel(
         reinterpret_cast<volatile uint32_t*>(base_ptr + kFBarOffset + 8 * (3 * kFStages + 4));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(slot_ptr + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
     const int num_n = (N + kFBN - 1) / kFBN;
     const int num_m = __ldg(tile_count);
     const int num_tiles = num_m * num_n;
@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(kFThreads, 1) gemm_nvfp4_kernel(
     const uint32_t tmem_base = *slot_ptr;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(kFThreads, 1) gemm_nvfp4_kernel(
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             int acc = 0;
@@ -822,7 +822,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) gemm_n
         reinterpret_cast<volatile uint32_t*>(base_ptr + kPBarOffset + 8 * kPBarriers);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(slot_ptr + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
     const int num_w = (N + 255) / 256;              // weight tiles of 256 rows
@@ -863,7 +863,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) gemm_n
     if (warp == 0) {
         // Operand producer: per stage one load of this CTA's 128 weight rows and one of its
         // half of the token rows, two K blocks each.
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0, it = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -901,7 +901,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) gemm_n
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (rank == 0 && lane == 0) {
+        if (rank == 0 && elect_one()) {
             int stage = 0, it = 0;
             uint32_t phase = 0, acc_phase = 0, sf_par = 0;     // sf_par: which two-stage scale slot
             bool ok = true;
@@ -959,7 +959,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1) gemm_n
                 ++tile_i;
 #endif
             }
-        } else if (rank == 1 && lane == 0) {
+        } else if (rank == 1 && elect_one()) {
             // Relay: tells the leader that this CTA's operands of a stage have landed.
             const uint32_t leader_cfull0 = map_to_cta(cfull_bar(0), 0);
             int stage = 0;
@@ -1293,7 +1293,7 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
         reinterpret_cast<volatile uint32_t*>(base_ptr + kQBarOffset + 8 * (2 * kQStages + 4));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(slot_ptr + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
     const int num_m = (M + kBM - 1) / kBM, num_n = (N + kQBN - 1) / kQBN;
     const int num_tiles = num_m * num_n;
     const int num_kb = K / kQBK;
@@ -1322,7 +1322,7 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
     const uint32_t tmem_base = *slot_ptr;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -1344,7 +1344,7 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             int buf = 0;
@@ -1502,7 +1502,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) index_score_kernel(
         reinterpret_cast<volatile uint32_t*>(base_ptr + kIdxBarOffset + 8 * kIdxBarriers);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(slot_ptr + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
     const int q_rows = queries * heads;
     const int num_qb = (q_rows + 255) / 256;
     const int num_kt = (keys + 127) / 128;
@@ -1536,7 +1536,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) index_score_kernel(
     const uint32_t tmem_base = *slot_ptr;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0, qs = 0;
             uint32_t phase = 0, qphase = 0;
             bool ok = true;
@@ -1565,7 +1565,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) index_score_kernel(
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0, qs = 0, buf = 0;
             uint32_t phase = 0, qphase = 0, buf_phase = 0;
             bool ok = true;
