@@ -17,42 +17,36 @@ namespace rt {
 constexpr int kItem = 16;         // columns per work item
 constexpr int kActThreads = 256;  // threads per CTA for the streaming kernels
 
-// Loads the 16 values of one work item. With UP, the values are
-// bf16(silu(gate) * up), i.e. what the unfused torch path would hand to the quantiser.
-template <bool UP>
+// Loads the 16 values of one work item as eight bf16 pairs. With UP, the values are
+// bf16(silu(gate) * up), i.e. what the unfused torch path would hand to the quantiser. NEG
+// delivers their negatives, which is what quotient_e4m3x4 divides.
+template <bool UP, bool NEG = false>
 __device__ __forceinline__ void load_item(const __nv_bfloat16* __restrict__ x,
                                           const __nv_bfloat16* __restrict__ up, int64_t row,
                                           int64_t col, int64_t xstride, int64_t ustride,
-                                          float (&v)[16]) {
+                                          uint32_t (&v)[8]) {
     const uint4* px = reinterpret_cast<const uint4*>(x + row * xstride + col);
-    const uint4 a0 = ld_stream16(px), a1 = ld_stream16(px + 1);
-    float lo[8], hi[8];
-    unpack_bf16x8(a0, lo);
-    unpack_bf16x8(a1, hi);
+    uint4 a0 = ld_stream16(px), a1 = ld_stream16(px + 1);
     if constexpr (UP) {
         const uint4* pu = reinterpret_cast<const uint4*>(up + row * ustride + col);
         const uint4 b0 = ld_stream16(pu), b1 = ld_stream16(pu + 1);
-        float ulo[8], uhi[8];
-        unpack_bf16x8(b0, ulo);
-        unpack_bf16x8(b1, uhi);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            lo[k] = round_bf16(swiglu_f32(lo[k], ulo[k]));
-            hi[k] = round_bf16(swiglu_f32(hi[k], uhi[k]));
-        }
+        a0 = swiglu8<NEG>(a0, b0);
+        a1 = swiglu8<NEG>(a1, b1);
     }
+    v[0] = a0.x; v[1] = a0.y; v[2] = a0.z; v[3] = a0.w;
+    v[4] = a1.x; v[5] = a1.y; v[6] = a1.z; v[7] = a1.w;
+    if constexpr (NEG && !UP) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        v[k] = lo[k];
-        v[8 + k] = hi[k];
+        for (int k = 0; k < 8; ++k) v[k] ^= 0x80008000u;
     }
 }
 
-__device__ __forceinline__ float absmax16(const float (&v)[16]) {
-    float m = 0.f;
+__device__ __forceinline__ float absmax16(const uint32_t (&v)[8]) {
+    uint32_t m = absmax_bf16x2(v[0], v[1]);
 #pragma unroll
-    for (int k = 0; k < 16; ++k) m = fmaxf(m, fabsf(v[k]));
-    return m;
+    for (int k = 2; k < 8; ++k) m = absmax_bf16x2(m, v[k]);
+    // a group of NaNs only: no maximum
+    return fmaxf(0.f, fmaxf(bf16_lo(m), bf16_hi(m)));
 }
 
 // Two fp32 -> two e4m3 (RNE, saturating), `lo` in the low byte.
@@ -60,6 +54,26 @@ __device__ __forceinline__ uint32_t cvt_e4m3x2(float lo, float hi) {
     uint16_t d;
     asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(d) : "f"(hi), "f"(lo));
     return d;
+}
+
+// e4m3 codes of a / b for four values given as the NEGATED bf16 pairs na0, na1: `b` and its
+// correctly rounded reciprocal with the sign flipped, `nrb`, both twice in a register pair. The
+// arithmetic of div_shared, two quotients per instruction; carried negated, a zero comes out with
+// the sign of a.
+__device__ __forceinline__ uint32_t quotient_e4m3x4(uint32_t na0, uint32_t na1, uint64_t b, uint64_t nrb) {
+    uint32_t out[2];
+    const uint32_t na[2] = {na0, na1};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint64_t a = pack_f32x2(bf16_lo(na[i]), bf16_hi(na[i]));
+        const uint64_t nq = mul_f32x2(a, nrb);
+        float lo, hi;
+        unpack_f32x2(fma_f32x2(fma_f32x2(nq, b, a), nrb, nq), lo, hi);
+        // no explicit clamp: the saturating conversion maps |q| > 448 to +-448,
+        // which is what clamp(-448, 448) followed by a cast yields
+        out[i] = cvt_e4m3x2(lo, hi);
+    }
+    return out[0] | (out[1] << 16);
 }
 
 // e4m3 byte -> fp32 (exact).
@@ -82,12 +96,7 @@ __global__ void __launch_bounds__(kActThreads) swiglu_kernel(
     const int64_t col = static_cast<int64_t>(id - row * items_per_row) * 8;
     const uint4 g = ld_stream16(gate + row * gstride + col);
     const uint4 u = ld_stream16(up + row * ustride + col);
-    float gf[8], uf[8], o[8];
-    unpack_bf16x8(g, gf);
-    unpack_bf16x8(u, uf);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = swiglu_f32(gf[k], uf[k]);
-    st_stream16(out + row * cols + col, pack_bf16x8(o));
+    st_stream16(out + row * cols + col, swiglu8<false>(g, u));
 }
 
 // ---------------------------------------------------------------------------
@@ -105,8 +114,8 @@ __global__ void __launch_bounds__(kActThreads) quant_fp8_kernel(
     const uint32_t row = id / items_per_row;
     const uint32_t item = id - row * items_per_row;
     const int64_t col = static_cast<int64_t>(item) * kItem;
-    float v[16];
-    load_item<UP>(x, up, row, col, xstride, ustride, v);
+    uint32_t v[8];
+    load_item<UP, true>(x, up, row, col, xstride, ustride, v);
     float amax = absmax16(v);
     // the 8 lanes of a group share one shuffle mask segment
     const uint32_t lane = threadIdx.x & 31u;
@@ -116,19 +125,11 @@ __global__ void __launch_bounds__(kActThreads) quant_fp8_kernel(
     amax = fmaxf(amax, __shfl_xor_sync(gmask, amax, 4));
     amax = fmaxf(amax, 1.0e-4f);
     const float scale = __fdiv_rn(amax, 448.0f);
-    const float rscale = __frcp_rn(scale);
+    const float nrscale = -__frcp_rn(scale);
+    const uint64_t b2 = pack_f32x2(scale, scale), nrb2 = pack_f32x2(nrscale, nrscale);
     uint32_t w[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        float q[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            // no explicit clamp: the saturating conversion maps |q| > 448 to +-448,
-            // which is what clamp(-448, 448) followed by a cast yields
-            q[j] = div_shared(v[4 * k + j], scale, rscale);
-        }
-        w[k] = cvt_e4m3x2(q[0], q[1]) | (cvt_e4m3x2(q[2], q[3]) << 16);
-    }
+    for (int k = 0; k < 4; ++k) w[k] = quotient_e4m3x4(v[2 * k], v[2 * k + 1], b2, nrb2);
     st_stream16(codes + static_cast<int64_t>(row) * cols + col, make_uint4(w[0], w[1], w[2], w[3]));
     if ((item & 7u) == 0) scales[static_cast<int64_t>(row) * (cols >> 7) + (item >> 3)] = scale;
 }
@@ -250,19 +251,13 @@ __global__ void __launch_bounds__(kActThreads) absmax_kernel(
         const uint32_t row = id / items_per_row;
         if (row < r_lo || row >= r_hi) continue;
         const int64_t col = static_cast<int64_t>(id - row * items_per_row) * kItem;
-        float v[16];
+        uint32_t v[8];
         load_item<UP>(x, up, row, col, xstride, ustride, v);
         m = fmaxf(m, absmax16(v));
         if constexpr (STORE) {
-            float lo[8], hi[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                lo[k] = v[k];
-                hi[k] = v[8 + k];
-            }
             uint4* ph = reinterpret_cast<uint4*>(h + static_cast<int64_t>(row) * hstride + col);
-            st_stream16(ph, pack_bf16x8(lo));
-            st_stream16(ph + 1, pack_bf16x8(hi));
+            ph[0] = make_uint4(v[0], v[1], v[2], v[3]);
+            ph[1] = make_uint4(v[4], v[5], v[6], v[7]);
         }
     }
     m = warp_max(m);
@@ -290,6 +285,25 @@ __device__ __forceinline__ uint32_t cvt_e2m1x2(float lo, float hi) {
     return d;
 }
 
+// The sixteen e2m1 codes and the block scale of one work item under the global scale gs.
+__device__ __forceinline__ uint2 quant_item_nvfp4(const uint32_t (&v)[8], float gs, float six_gs, uint32_t& bs) {
+    const float t = fminf(__fdiv_rn(absmax16(v), six_gs), 448.0f);
+    bs = cvt_e4m3x2(t, 0.f) & 0xffu;
+    const float denom = __fmul_rn(gs, e4m3_to_f32(bs));
+    uint32_t c[2] = {0u, 0u};
+    if (denom > 0.f) {
+        const float inv = __frcp_rn(denom);
+        const uint64_t inv2 = pack_f32x2(inv, inv);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            float a, b;
+            unpack_f32x2(mul_f32x2(pack_f32x2(bf16_lo(v[k]), bf16_hi(v[k])), inv2), a, b);
+            c[k >> 2] |= cvt_e2m1x2(a, b) << (8 * (k & 3));
+        }
+    }
+    return make_uint2(c[0], c[1]);
+}
+
 __device__ __forceinline__ int64_t sf_offset(int layout, int64_t row, int64_t blk,
                                              int64_t nblk) {
     if (layout == RT_SF_ROWMAJOR) return row * nblk + blk;
@@ -304,7 +318,9 @@ __global__ void __launch_bounds__(kActThreads) quant_nvfp4_kernel(
     const float* __restrict__ amax_in, uint8_t* __restrict__ codes, uint8_t* __restrict__ sf,
     float* __restrict__ gs_out, uint32_t items, uint32_t items_per_row, int64_t xstride,
     int64_t ustride, int64_t cols, int layout) {
-    const uint32_t id = blockIdx.x * kActThreads + threadIdx.x;
+    // last rows first: the pass that found amax went over the same tensor (or wrote it) front to
+    // back, so its end is what L2 still holds
+    const uint32_t id = (gridDim.x - 1u - blockIdx.x) * kActThreads + threadIdx.x;
     const float amax = __ldg(amax_in);
     const float gs = amax > 0.f ? __fdiv_rn(amax, 2688.0f) : 1.0f;
     if (id == 0 && gs_out) *gs_out = gs;
@@ -312,22 +328,10 @@ __global__ void __launch_bounds__(kActThreads) quant_nvfp4_kernel(
     const uint32_t row = id / items_per_row;
     const uint32_t blk = id - row * items_per_row;
     const int64_t col = static_cast<int64_t>(blk) * kItem;
-    float v[16];
+    uint32_t v[8], bs;
     load_item<UP>(x, up, row, col, xstride, ustride, v);
-    const float bmax = absmax16(v);
-    const float t = fminf(__fdiv_rn(bmax, __fmul_rn(6.0f, gs)), 448.0f);
-    const uint32_t bs = cvt_e4m3x2(t, 0.f) & 0xffu;
-    const float denom = __fmul_rn(gs, e4m3_to_f32(bs));
-    uint32_t lo = 0, hi = 0;
-    if (denom > 0.f) {
-        const float inv = __frcp_rn(denom);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            lo |= cvt_e2m1x2(__fmul_rn(v[2 * k], inv), __fmul_rn(v[2 * k + 1], inv)) << (8 * k);
-            hi |= cvt_e2m1x2(__fmul_rn(v[8 + 2 * k], inv), __fmul_rn(v[9 + 2 * k], inv)) << (8 * k);
-        }
-    }
-    st_stream8(codes + static_cast<int64_t>(row) * (cols >> 1) + (col >> 1), make_uint2(lo, hi));
+    const uint2 c = quant_item_nvfp4(v, gs, __fmul_rn(6.0f, gs), bs);
+    st_stream8(codes + static_cast<int64_t>(row) * (cols >> 1) + (col >> 1), c);
     sf[sf_offset(layout, row, blk, items_per_row)] = static_cast<uint8_t>(bs);
 }
 
@@ -344,7 +348,9 @@ __global__ void __launch_bounds__(kActThreads) quant_nvfp4_tiles_kernel(
     uint8_t* __restrict__ codes, uint8_t* __restrict__ sf, float* __restrict__ gs_out,
     const int4* __restrict__ tile_map, const int32_t* __restrict__ tile_count,
     uint32_t items_per_row, int64_t xstride, int64_t ustride, int64_t cols) {
-    const int tile = blockIdx.x >> 4, sub = blockIdx.x & 15;
+    // last tiles first: what the pass before this one wrote last is still in L2
+    const unsigned unit = gridDim.x - 1u - blockIdx.x;
+    const int tile = static_cast<int>(unit >> 4), sub = static_cast<int>(unit & 15u);
     const float amax = __ldg(amax_in);
     const float gs = amax > 0.f ? __fdiv_rn(amax, 2688.0f) : 1.0f;
     if (blockIdx.x == 0 && threadIdx.x == 0 && gs_out) *gs_out = gs;
@@ -366,22 +372,9 @@ __global__ void __launch_bounds__(kActThreads) quant_nvfp4_tiles_kernel(
         const int64_t dst_row = tm.y + r_local;
         const int64_t src_row = sorted_pairs ? (__ldg(sorted_pairs + dst_row) / topk) : dst_row;
         const int64_t col = static_cast<int64_t>(blk) * kItem;
-        float v[16];
+        uint32_t v[8], bs;
         load_item<UP>(x, up, src_row, col, xstride, ustride, v);
-        const float bmax = absmax16(v);
-        const float t = fminf(__fdiv_rn(bmax, six_gs), 448.0f);
-        const uint32_t bs = cvt_e4m3x2(t, 0.f) & 0xffu;
-        const float denom = __fmul_rn(gs, e4m3_to_f32(bs));
-        uint32_t lo = 0, hi = 0;
-        if (denom > 0.f) {
-            const float inv = __frcp_rn(denom);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                lo |= cvt_e2m1x2(__fmul_rn(v[2 * k], inv), __fmul_rn(v[2 * k + 1], inv)) << (8 * k);
-                hi |= cvt_e2m1x2(__fmul_rn(v[8 + 2 * k], inv), __fmul_rn(v[9 + 2 * k], inv)) << (8 * k);
-            }
-        }
-        st_stream8(codes + dst_row * (cols >> 1) + (col >> 1), make_uint2(lo, hi));
+        st_stream8(codes + dst_row * (cols >> 1) + (col >> 1), quant_item_nvfp4(v, gs, six_gs, bs));
         *sf_dst = static_cast<uint8_t>(bs);
     }
 }

@@ -95,20 +95,7 @@ def moe_gather_nvfp4(codes: torch.Tensor, sf: torch.Tensor, sorted_pairs: torch.
     return out, sf_out
 
 
-def swiglu_absmax_rows(gate: torch.Tensor, up: torch.Tensor, window):
-    """(h, amax): h = bf16(silu(gate) * up) and max |h| over the rows of `window` (a pair of
-    one-element device tensors [begin], [end], or None for all rows); rows outside the window
-    are not written (rt_swiglu_absmax_rows)."""
-    h = torch.empty(gate.shape, dtype=torch.bfloat16, device=gate.device)
-    out = torch.empty(1, dtype=torch.float32, device=gate.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_swiglu_absmax_rows(
-        gate.data_ptr(), up.data_ptr(), h.data_ptr(), out.data_ptr(), gate.shape[0], gate.shape[1],
-        gate.stride(0), up.stride(0), h.stride(0),
-        window[0].data_ptr() if window is not None else None,
-        window[1].data_ptr() if window is not None else None, _lib.RT_BF16, ops._stream()),
-        "rt_swiglu_absmax_rows")
-    return h, out
+swiglu_absmax_rows = ops.swiglu_absmax
 
 
 def moe_quant_nvfp4(x: torch.Tensor, tile_map: torch.Tensor, tile_count: torch.Tensor,

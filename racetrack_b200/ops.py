@@ -354,6 +354,22 @@ def tensor_absmax(x: torch.Tensor, up: Optional[torch.Tensor] = None) -> torch.T
     return out
 
 
+def swiglu_absmax(gate: torch.Tensor, up: torch.Tensor, window=None):
+    """(h, amax): h = bf16(silu(gate) * up) and max |h| over the rows of `window` (a pair of
+    one-element int32 device tensors [begin], [end], or None for all rows) of 2-D gate and up with
+    16-byte aligned rows; rows outside the window are not written (rt_swiglu_absmax_rows)."""
+    h = torch.empty(gate.shape, dtype=torch.bfloat16, device=gate.device)
+    out = torch.empty(1, dtype=torch.float32, device=gate.device)
+    lib = _lib.load()
+    _lib.check(lib.rt_swiglu_absmax_rows(
+        gate.data_ptr(), up.data_ptr(), h.data_ptr(), out.data_ptr(), gate.shape[0], gate.shape[1],
+        gate.stride(0), up.stride(0), h.stride(0),
+        window[0].data_ptr() if window is not None else None,
+        window[1].data_ptr() if window is not None else None, _lib.RT_BF16, _stream()),
+        "rt_swiglu_absmax_rows")
+    return h, out
+
+
 def sf_tiled_bytes(rows: int, cols: int) -> int:
     """Size of a 128x4-tiled NVFP4 block-scale buffer for a [rows, cols] tensor."""
     return ((rows + 127) // 128) * ((cols // 16 + 3) // 4) * 512
@@ -382,7 +398,13 @@ def fused_nvfp4_quant(x: torch.Tensor, *, up: Optional[torch.Tensor] = None,
     u2 = None
     if up is not None:
         x2, u2 = _gate_up(x, up, "fused_nvfp4_quant")
-    if amax is None:
+    if amax is None and up is not None and x2.shape[0] > 0:
+        # one evaluation of SwiGLU: the abs-max pass writes its bf16 result and the quantiser reads
+        # that (4 + 2 + 2 + 0.56 bytes an element, as many as two passes over gate and up move, at
+        # half the instructions; 4096 x 18432 on one B200: 120 us against 161)
+        x2, amax = swiglu_absmax(x2, u2)
+        u2 = None
+    elif amax is None:
         amax = tensor_absmax(x, up)
     rows = x2.shape[0]
     if out is not None:

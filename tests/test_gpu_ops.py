@@ -242,6 +242,26 @@ def test_act_quant_fp8_edge_values(ops):
         ops.fused_act_quant(cu(torch.zeros(2, 100, dtype=torch.bfloat16)))
 
 
+def test_swiglu_of_every_bf16_gate(ops):
+    """The written-out division of the SwiGLU kernels is the IEEE one: every bf16 gate (zeros of both
+    signs, subnormals, the magnitudes beyond 80 that take the general form, infinities) against
+    several ups, bit for bit against torch on the same device; NaN exactly where torch has NaN."""
+    gate = torch.arange(-32768, 32768, device="cuda").to(torch.int16).view(torch.bfloat16).view(256, 256)
+    for up in (1.0, -1.0, 0.0, 1.0078125, -0.333984375, 3.0e38, 1.0e-38):
+        u = torch.full_like(gate, up)
+        want = (torch.nn.functional.silu(gate.float()) * u.float()).to(torch.bfloat16)
+        got = ops.fused_swiglu(gate, u)
+        nan = torch.isnan(want)
+        assert torch.equal(torch.isnan(got), nan)
+        assert torch.equal(got.view(torch.int16)[~nan], want.view(torch.int16)[~nan]), f"up = {up}"
+
+
+def test_swiglu_nvfp4_quant_without_rows(ops):
+    x = torch.empty(0, 256, device="cuda", dtype=torch.bfloat16)
+    codes, sf, _ = ops.fused_swiglu_nvfp4_quant(x, x)
+    assert codes.shape == (0, 128) and sf.shape == (0, 16)
+
+
 @pytest.mark.parametrize("tokens,inter", [(16, 512), (64, I.DENSE_INTER)])
 def test_swiglu_quant_fp8(ops, tokens, inter, golden_small):
     d = I.swiglu_quant_inputs(tokens, inter)
