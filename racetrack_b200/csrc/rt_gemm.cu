@@ -54,6 +54,11 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
 // slabs in split order, so the result does not depend on which SM finished first. A projection
 // of a few dozen decode tokens has too few output tiles to occupy the GPU, while its weight
 // matrix is what has to be streamed.
+// a_bytes: what the A box of a stage brings in. With fewer than 128 rows in all (decode) the box is
+// cut to the rows there are (in steps of 8, a swizzle atom): a full box is mostly zero fill, which
+// takes shared-memory bandwidth like data and halved the rate at which the weights came in. The
+// rows of the stage that are never written hold whatever was there; an output row depends on its
+// own A row only and theirs are not stored.
 // BATCHED: `batch` independent products of the same shape in one launch (the per-head absorbed
 // projections of MLA: q_nope . W_UK and latent . W_UV, racetrack/models/deepseek.py:799,810): the
 // tensor maps are 3-D {K, rows, batch}, a work item is (batch, m-tile, n-tile) and c advances
@@ -61,7 +66,7 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
 template <int BN, bool F32OUT, bool SPLITK = false, bool BATCHED = false>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(
     const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-    void* __restrict__ c_out, int M, int N, int K, int64_t ldc, int k_splits_arg = 1,
+    void* __restrict__ c_out, int M, int N, int K, int64_t ldc, uint32_t a_bytes, int k_splits_arg = 1,
     int64_t split_stride = 0, int batch = 1, int64_t c_batch_stride = 0) {
     static_assert(!SPLITK || F32OUT, "split-K accumulates into an fp32 output");
     static_assert(!(SPLITK && BATCHED), "one or the other");
@@ -123,7 +128,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(
                 for (int kb = kb0; kb < kb1; ++kb) {
                     if (!(ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, 1))) break;
                     const uint32_t sa = base + stage * Cfg::kStageBytes;
-                    mbar_arrive_expect_tx(full_bar(stage), Cfg::kStageBytes);
+                    mbar_arrive_expect_tx(full_bar(stage), a_bytes + Cfg::kBBytes);
                     if constexpr (BATCHED) {
                         tma_load_3d(sa, &tmap_a, kb * kBK, tm * kBM, bidx, full_bar(stage));
                         tma_load_3d(sa + Cfg::kABytes, &tmap_b, kb * kBK, tn * BN, bidx, full_bar(stage));
@@ -1805,12 +1810,16 @@ int sm_count() {
     return n;
 }
 
+// Rows of the A box of a stage: a tile's 128, or the rows there are, whole swizzle atoms.
+static uint32_t a_box_rows(int64_t m) { return static_cast<uint32_t>(m >= kBM ? kBM : (m + 7) / 8 * 8); }
+static uint32_t a_box_bytes(int64_t m) { return a_box_rows(m) * kBK * 2; }
+
 template <int BN, bool F32OUT>
 static int launch_bf16(const void* a, const void* b, void* c, int64_t M, int64_t N, int64_t K,
                        int64_t lda, int64_t ldb, int64_t ldc, cudaStream_t st) {
     using Cfg = GemmCfg<BN>;
     CUtensorMap ta, tb;
-    if (int rc = make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a, K, M, lda * 2, kBK, kBM))
+    if (int rc = make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a, K, M, lda * 2, kBK, a_box_rows(M)))
         return rc;
     if (int rc = make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, b, K, N, ldb * 2, kBK, BN))
         return rc;
@@ -1820,9 +1829,33 @@ static int launch_bf16(const void* a, const void* b, void* c, int64_t M, int64_t
     const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + BN - 1) / BN);
     const int grid = static_cast<int>(tiles < sm_count() ? tiles : sm_count());
     gemm_bf16_kernel<BN, F32OUT><<<grid, kGemmThreads, Cfg::kSmemBytes, st>>>(
-        ta, tb, c, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), ldc);
+        ta, tb, c, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), ldc, a_box_bytes(M));
     count_launch();
     return check_launch("gemm_bf16_kernel");
+}
+
+// How many ranges the K blocks of a product with `tiles` output tiles are cut into: the count with
+// the smallest estimate of ((rounds of work items over the SMs) x (K blocks of an item, half a block
+// for the change of tile) + 4 for the first loads and the last epilogue) x (time of a K block) + the
+// pass that adds the slabs (a launch, then slab_bytes written and read per range). One item per SM
+// and round, so 56 tiles take 5 ranges (280 items, two rounds of 148), not 6 (336, a third round
+// for a quarter of the SMs). 64 x 7168 x 16384 on one B200: 52 -> 44 us, 4096 x 256 x 7168 (32 whole
+// tiles before) 47 -> 23, 2048 x 128 x 7168 28 -> 15.
+static int64_t pick_splits(int64_t tiles, int64_t num_kb, int64_t min_kb, double kb_us, double slab_bytes) {
+    const int64_t sms = sm_count();
+    int64_t best = 1;
+    double best_us = (static_cast<double>((tiles + sms - 1) / sms) * (num_kb + 0.5) + 4) * kb_us;
+    for (int64_t s = 2; s <= num_kb / min_kb && s <= 64; ++s) {
+        const int64_t per = (num_kb + s - 1) / s;
+        if ((num_kb + per - 1) / per != s) continue;             // a range would be empty
+        const double us = (static_cast<double>((tiles * s + sms - 1) / sms) * (per + 0.5) + 4) * kb_us + 2.0 +
+                          s * slab_bytes / 3.0e6;
+        if (us < best_us) {
+            best_us = us;
+            best = s;
+        }
+    }
+    return best;
 }
 
 // out[m, n] = part[0][m, n] + part[1][m, n] + ... in split order (fp32), rounded to bf16 or kept.
@@ -1874,7 +1907,7 @@ static int launch_bf16_batched(const void* a, const void* b, void* c, int64_t ba
                                int64_t c_bs, cudaStream_t st) {
     using Cfg = GemmCfg<128>;
     CUtensorMap ta, tb;
-    if (int rc = make_tmap_bf16_batched(&ta, a, K, M, batch, lda * 2, a_bs * 2, kBM)) return rc;
+    if (int rc = make_tmap_bf16_batched(&ta, a, K, M, batch, lda * 2, a_bs * 2, a_box_rows(M))) return rc;
     if (int rc = make_tmap_bf16_batched(&tb, b, K, N, batch, ldb * 2, b_bs * 2, 128)) return rc;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&gemm_bf16_kernel<128, false, false, true>),
                                      static_cast<int>(Cfg::kSmemBytes), "rt_gemm_bf16_batched"))
@@ -1882,8 +1915,8 @@ static int launch_bf16_batched(const void* a, const void* b, void* c, int64_t ba
     const int64_t items = ((M + kBM - 1) / kBM) * ((N + 127) / 128) * batch;
     const int grid = static_cast<int>(items < sm_count() ? items : sm_count());
     gemm_bf16_kernel<128, false, false, true><<<grid, kGemmThreads, Cfg::kSmemBytes, st>>>(
-        ta, tb, c, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), ldc, 1, 0,
-        static_cast<int>(batch), c_bs);
+        ta, tb, c, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), ldc,
+        a_box_bytes(M), 1, 0, static_cast<int>(batch), c_bs);
     count_launch();
     return check_launch("gemm_bf16_kernel<batched>");
 }
@@ -1895,7 +1928,7 @@ static int launch_bf16_splitk(const void* a, const void* b, float* c, void* out,
                               int64_t ldo, int splits, cudaStream_t st) {
     using Cfg = GemmCfg<128>;
     CUtensorMap ta, tb;
-    if (int rc = make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a, K, M, lda * 2, kBK, kBM))
+    if (int rc = make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a, K, M, lda * 2, kBK, a_box_rows(M)))
         return rc;
     if (int rc = make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, b, K, N, ldb * 2, kBK, 128))
         return rc;
@@ -1905,7 +1938,8 @@ static int launch_bf16_splitk(const void* a, const void* b, float* c, void* out,
     const int64_t items = ((M + kBM - 1) / kBM) * ((N + 127) / 128) * splits;
     const int grid = static_cast<int>(items < sm_count() ? items : sm_count());
     gemm_bf16_kernel<128, true, true><<<grid, kGemmThreads, Cfg::kSmemBytes, st>>>(
-        ta, tb, c, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), ldc, splits, M * ldc);
+        ta, tb, c, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), ldc,
+        a_box_bytes(M), splits, M * ldc);
     count_launch();
     if (int rc = check_launch("gemm_bf16_kernel<split-K>")) return rc;
     const int64_t total4 = M * (N / 4);
@@ -2215,6 +2249,12 @@ extern "C" int rt_gemm_nvfp4_schedule(int schedule) {
     return previous;
 }
 
+// Whether the CTA-pair schedule (256 x 256 tiles, whole 64-element K blocks) takes a bf16 product:
+// once its tiles fill the machine and more than half of a tile's rows exist.
+static bool bf16_pair_pays(int64_t m, int64_t n, int64_t k) {
+    return k % 64 == 0 && m > 128 && ((m + 255) / 256) * ((n + 255) / 256) >= tc::sm_count() / 2;
+}
+
 extern "C" int rt_gemm_bf16(const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k,
                             int64_t lda, int64_t ldb, int64_t ldc, int out_dtype, void* stream) {
     RT_REQUIRE(out_dtype == RT_BF16 || out_dtype == RT_F32, RT_ERR_UNSUPPORTED,
@@ -2230,17 +2270,22 @@ extern "C" int rt_gemm_bf16(const void* a, const void* b, void* c, int64_t m, in
                "rt_gemm_bf16: dimension too large");
     cudaStream_t st = as_stream(stream);
     // CTA pairs (256 x 256 tiles) once they fill the machine; they need whole 64-element K blocks
-    const bool pair_ok = k % 64 == 0;
-    const bool pair_pays = ((m + 255) / 256) * ((n + 255) / 256) >= tc::sm_count() / 2;
-    if (pair_ok && (tc::g_bf16_schedule == 2 || (tc::g_bf16_schedule == 0 && pair_pays))) {
+    if ((tc::g_bf16_schedule == 2 && k % 64 == 0) || (tc::g_bf16_schedule == 0 && bf16_pair_pays(m, n, k))) {
         if (out_dtype == RT_F32) return tc::launch_bf16_pair<true>(a, b, c, m, n, k, lda, ldb, ldc, st);
         return tc::launch_bf16_pair<false>(a, b, c, m, n, k, lda, ldb, ldc, st);
     }
+    // a K block of a 128 x 256 tile takes 1.6 times as long as one of 128 x 128: narrow tiles where
+    // they need less than that many more rounds over the SMs (777 x 2112 x 7168: 119 tiles against
+    // 63, both one round)
+    const int64_t m_tiles = (m + 127) / 128, sms = tc::sm_count();
+    const int64_t rounds_narrow = (m_tiles * ((n + 127) / 128) + sms - 1) / sms;
+    const int64_t rounds_wide = (m_tiles * ((n + 255) / 256) + sms - 1) / sms;
+    const bool narrow = n <= 128 || 5 * rounds_narrow < 8 * rounds_wide;
     if (out_dtype == RT_F32) {
-        if (n <= 128) return tc::launch_bf16<128, true>(a, b, c, m, n, k, lda, ldb, ldc, st);
+        if (narrow) return tc::launch_bf16<128, true>(a, b, c, m, n, k, lda, ldb, ldc, st);
         return tc::launch_bf16<256, true>(a, b, c, m, n, k, lda, ldb, ldc, st);
     }
-    if (n <= 128) return tc::launch_bf16<128, false>(a, b, c, m, n, k, lda, ldb, ldc, st);
+    if (narrow) return tc::launch_bf16<128, false>(a, b, c, m, n, k, lda, ldb, ldc, st);
     return tc::launch_bf16<256, false>(a, b, c, m, n, k, lda, ldb, ldc, st);
 }
 
@@ -2263,15 +2308,9 @@ extern "C" int rt_gemm_bf16_batched(const void* a, const void* b, void* c, int64
 }
 
 extern "C" int64_t rt_gemm_bf16_splitk_splits(int64_t m, int64_t n, int64_t k) {
-    if (m <= 0 || n <= 0 || k <= 0) return 1;
-    const int64_t tiles = ((m + 127) / 128) * ((n + 127) / 128);
-    const int64_t num_kb = (k + 63) / 64;
-    // enough work items for two per SM, at least 4 K blocks each
-    int64_t splits = (2 * tc::sm_count() + tiles - 1) / tiles;
-    if (splits > num_kb / 4) splits = num_kb / 4;
-    if (splits < 1) splits = 1;
-    const int64_t per = (num_kb + splits - 1) / splits;
-    return (num_kb + per - 1) / per;          // no split is empty
+    if (m <= 0 || n <= 0 || k <= 0 || tc::g_bf16_schedule != 0 || bf16_pair_pays(m, n, k)) return 1;
+    // a K block of 64 of a 128 x 128 tile: 0.25 us of its CTA
+    return tc::pick_splits(((m + 127) / 128) * ((n + 127) / 128), (k + 63) / 64, 4, 0.25, 4.0 * m * n);
 }
 
 extern "C" int rt_gemm_bf16_splitk(const void* a, const void* b, float* workspace, void* out,

@@ -269,3 +269,28 @@ def test_linear_bf16_split_k_for_few_rows(ops, m, n, k, out_dtype):
     finally:
         ops.SPLITK_MAX_ROWS = saved
     assert float((out.float() - one.float()).abs().max()) <= 2.0 ** -6 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("m,n,k,out_dtype,splits", [
+    (777, 256, 7168, torch.float32, True),     # router logits of a prefill: 14 tiles, split
+    (2048, 128, 7168, torch.bfloat16, True),   # the indexer's key projection: one column of tiles
+    (129, 136, 1096, torch.float32, True),     # second row and column tile nearly empty, partial K block
+    (1000, 2112, 7168, torch.bfloat16, False), # narrow tiles instead of split ones
+    (64, 24576, 1536, torch.bfloat16, None),   # few rows against many columns: never CTA pairs
+    (3, 40, 264, torch.bfloat16, False),       # a box of 8 rows, 3 of them there
+])
+def test_linear_bf16_tile_and_split_choice(ops, m, n, k, out_dtype, splits):
+    """The products the tile-width, split-K and row-box rules decide, against fp64. fp32 sums of K
+    products of magnitude <= |x||w|: K * 2^-24 of the sum of magnitudes, plus bf16's half ulp."""
+    from racetrack_b200 import _lib
+    got = int(_lib.load().rt_gemm_bf16_splitk_splits(m, n, k))
+    assert splits is None or (got > 1) == splits
+    x = I.randn((m, k), 500 + m).cuda()
+    w = I.randn((n, k), 600 + n, std=0.05).cuda()
+    out = ops.linear_bf16(x, w, out_dtype=out_dtype)
+    ops.tc_error_state()
+    ref = x.double() @ w.double().t()
+    bound = k * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    if out_dtype == torch.bfloat16:
+        bound += 2.0 ** -8 * ref.abs()
+    assert bool(((out.double() - ref).abs() <= bound).all())
