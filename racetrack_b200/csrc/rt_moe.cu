@@ -319,17 +319,149 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(
 // ---------------------------------------------------------------------------
 // Top-k selection of the sparse indexer: the k largest scores of every query row
 // ---------------------------------------------------------------------------
-// One CTA per row. fp32 scores become order-preserving 32-bit keys; four 8-bit radix passes
-// (shared-memory histograms, most significant digit first) find the k-th largest key exactly
-// and how many elements equal to it still belong to the selection; a last pass writes the
-// indices of all larger keys and of the first of the equal ones, in ascending index order
-// (ballot-based ordered compaction, 1024 elements per sweep).
+// fp32 scores become order-preserving 32-bit keys; equal keys are taken in index order; the
+// indices are written in ascending order. Two forms, by the length of a row:
+//   up to 8192 keys   index_topk_reg_kernel: the row's keys stay in registers (256 threads, up to
+//                     32 keys each), a bisection between the row's smallest and largest key finds
+//                     the k-th: a step is one compare and add per key, one warp reduction and one
+//                     block barrier, and it stops as soon as exactly k keys lie above the middle
+//                     (about 20 steps for scores without ties). Nothing collides: histogram atomics
+//                     of scores, whose exponents hardly differ, serialise on a few bins.
+//                     2048 rows x 4096 keys on one B200: 183 -> 38 us (that radix form before), 64 rows 30 -> 9.
+//   longer rows       index_topk_kernel: four 8-bit radix passes over the row in memory.
 constexpr int kTopkThreads = 1024;
 
 __device__ __forceinline__ uint32_t order_key(float v) {
     uint32_t u = __float_as_uint(v);
     if (u == 0x80000000u) u = 0u;                           // -0.0 compares equal to +0.0
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);      // larger float <=> larger key
+}
+
+constexpr int kTopkRegThreads = 256;
+
+// Key of slot j of a thread: element j * 256 + threadIdx.x, so loads and stores are coalesced.
+template <int ITEMS>
+__global__ void __launch_bounds__(kTopkRegThreads) index_topk_reg_kernel(
+    const float* __restrict__ scores, int32_t* __restrict__ indices, int keys, int64_t ld,
+    int topk) {
+    constexpr int kWarps = kTopkRegThreads / 32;
+    __shared__ uint32_t s_lo[kWarps], s_hi[kWarps];
+    __shared__ int s_count[2][kWarps];
+    __shared__ int s_slot[ITEMS * kWarps];       // selected elements before (slot, warp)
+    __shared__ int s_scan[kWarps];
+    const float* row = scores + static_cast<int64_t>(blockIdx.x) * ld;
+    int32_t* out = indices + static_cast<int64_t>(blockIdx.x) * topk;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (topk == keys) {                          // every key is selected
+        for (int i = tid; i < keys; i += kTopkRegThreads) out[i] = i;
+        return;
+    }
+    uint32_t key[ITEMS];
+    uint32_t lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const int i = j * kTopkRegThreads + tid;
+        // slots past the row hold 0: smaller than or equal to every key, never counted because the
+        // middle of a bisection step is always above the row's smallest key
+        key[j] = i < keys ? order_key(row[i]) : 0u;
+        if (i < keys) {
+            lo = min(lo, key[j]);
+            hi = max(hi, key[j]);
+        }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) {
+        s_lo[warp] = lo;
+        s_hi[warp] = hi;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+        lo = min(lo, s_lo[w]);
+        hi = max(hi, s_hi[w]);
+    }
+    // the k-th largest key lies in [lo, hi]; `above` keys are known to be larger than hi
+    int above = 0;
+    bool exact = false;                          // exactly topk keys are >= lo
+    for (int step = 0; lo < hi; step ^= 1) {
+        const uint32_t mid = lo + ((hi - lo) >> 1) + ((hi - lo) & 1u);
+        int c = 0;
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) c += key[j] >= mid ? 1 : 0;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) s_count[step][warp] = c;
+        __syncthreads();
+        c = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) c += s_count[step][w];
+        if (c >= topk) {
+            lo = mid;
+            if (c == topk) {
+                exact = true;
+                break;
+            }
+        } else {
+            hi = mid - 1u;
+            above = c;
+        }
+    }
+    const uint32_t kth = lo;
+    int take_eq = exact ? keys : topk - above;   // how many elements equal to kth are selected
+
+    // exclusive prefix, over (slot, warp) in index order, of the counts in s_slot
+    auto scan_slots = [&]() {
+        __syncthreads();
+        int v = 0;
+        if (tid < ITEMS * kWarps) v = s_slot[tid];
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) s_scan[warp] = incl;
+        __syncthreads();
+        int before = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) before += w < warp ? s_scan[w] : 0;
+        if (tid < ITEMS * kWarps) s_slot[tid] = before + incl - v;
+        __syncthreads();
+    };
+
+    uint32_t sel = 0u;                           // bit j: element of slot j is selected
+    if (exact) {
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) sel |= (key[j] >= kth ? 1u : 0u) << j;
+    } else {
+        // rank of every element equal to kth among the equal ones of the row
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            const uint32_t b = __ballot_sync(0xffffffffu, key[j] == kth && j * kTopkRegThreads + tid < keys);
+            if (lane == 0) s_slot[j * kWarps + warp] = __popc(b);
+        }
+        scan_slots();
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            const bool eq = key[j] == kth && j * kTopkRegThreads + tid < keys;
+            const uint32_t b = __ballot_sync(0xffffffffu, eq);
+            const int rank = s_slot[j * kWarps + warp] + __popc(b & ((1u << lane) - 1u));
+            sel |= (key[j] > kth || (eq && rank < take_eq) ? 1u : 0u) << j;
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const uint32_t b = __ballot_sync(0xffffffffu, (sel >> j) & 1u);
+        if (lane == 0) s_slot[j * kWarps + warp] = __popc(b);
+    }
+    scan_slots();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const uint32_t b = __ballot_sync(0xffffffffu, (sel >> j) & 1u);
+        const int pos = s_slot[j * kWarps + warp] + __popc(b & ((1u << lane) - 1u));
+        if (((sel >> j) & 1u) && pos < topk) out[pos] = j * kTopkRegThreads + tid;
+    }
 }
 
 __global__ void __launch_bounds__(kTopkThreads) index_topk_kernel(
@@ -359,14 +491,26 @@ __global__ void __launch_bounds__(kTopkThreads) index_topk_kernel(
             if ((key & mask_hi) == prefix) atomicAdd(&hist[(key >> shift) & 0xffu], 1);
         }
         __syncthreads();
-        if (tid == 0) {
-            int remaining = s_remaining, bin = 255;
-            for (; bin > 0; --bin) {
-                if (hist[bin] >= remaining) break;
-                remaining -= hist[bin];
+        if (warp == 0) {
+            // lane l owns bins [8 * (31 - l), 8 * (31 - l) + 8): a prefix sum over lanes counts the
+            // elements of all larger bins; the lane in whose bins the k-th falls walks its eight
+            int own = 0;
+#pragma unroll
+            for (int b = 0; b < 8; ++b) own += hist[8 * (31 - lane) + b];
+            int incl = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += u;
             }
-            s_prefix = prefix | (static_cast<uint32_t>(bin) << shift);
-            s_remaining = remaining;
+            const int want = s_remaining;
+            __syncwarp();
+            if (incl - own < want && incl >= want) {
+                int remaining = want - (incl - own), bin = 8 * (31 - lane) + 7;
+                while (hist[bin] < remaining) remaining -= hist[bin--];
+                s_prefix = prefix | (static_cast<uint32_t>(bin) << shift);
+                s_remaining = remaining;
+            }
         }
         __syncthreads();
     }
@@ -604,8 +748,20 @@ extern "C" int rt_index_topk(const float* scores, int32_t* indices, int64_t quer
                (long long)topk, (long long)keys);
     RT_REQUIRE(keys < (1LL << 31) && queries < (1LL << 31) && score_stride >= keys,
                RT_ERR_UNSUPPORTED, "rt_index_topk: dimension too large or stride below keys");
-    index_topk_kernel<<<static_cast<unsigned>(queries), kTopkThreads, 0, as_stream(stream)>>>(
-        scores, indices, static_cast<int>(keys), score_stride, static_cast<int>(topk));
+    // the row in registers as long as it fits (the line lies where 32 keys a thread end)
+    const unsigned grid = static_cast<unsigned>(queries);
+    const int n = static_cast<int>(keys), k = static_cast<int>(topk);
+    cudaStream_t st = as_stream(stream);
+    if (keys <= 4 * kTopkRegThreads)
+        index_topk_reg_kernel<4><<<grid, kTopkRegThreads, 0, st>>>(scores, indices, n, score_stride, k);
+    else if (keys <= 8 * kTopkRegThreads)
+        index_topk_reg_kernel<8><<<grid, kTopkRegThreads, 0, st>>>(scores, indices, n, score_stride, k);
+    else if (keys <= 16 * kTopkRegThreads)
+        index_topk_reg_kernel<16><<<grid, kTopkRegThreads, 0, st>>>(scores, indices, n, score_stride, k);
+    else if (keys <= 32 * kTopkRegThreads)
+        index_topk_reg_kernel<32><<<grid, kTopkRegThreads, 0, st>>>(scores, indices, n, score_stride, k);
+    else
+        index_topk_kernel<<<grid, kTopkThreads, 0, st>>>(scores, indices, n, score_stride, k);
     count_launch();
     return check_launch("index_topk_kernel");
 }

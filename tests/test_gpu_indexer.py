@@ -99,6 +99,27 @@ def test_index_topk_selects_the_largest(ops, rows, keys, topk):
     _check_selection(scores, idx, topk)
 
 
+@pytest.mark.parametrize("keys", [1, 31, 256, 257, 1024, 1025, 2048, 2049, 4096, 4097, 8192, 8193, 20000])
+@pytest.mark.parametrize("kind", ["random", "few values", "masked", "constant", "specials"])
+def test_index_topk_equals_a_stable_sort(ops, keys, kind):
+    """Every row length class (keys in registers up to 8192, radix passes beyond) against a stable
+    descending sort: equal scores are taken in index order, -0 ranks as +0, indices ascend."""
+    g = torch.Generator().manual_seed(keys)
+    s = torch.randn(5, keys, generator=g)
+    if kind == "few values":
+        s = torch.randint(-2, 3, (5, keys), generator=g).float()
+    elif kind == "masked":
+        s[:, keys // 3:] = float("-inf")
+    elif kind == "constant":
+        s = torch.full((5, keys), -3.5)
+    elif kind == "specials":
+        s[:, ::3], s[:, 1::7], s[:, 2::5], s[0] = 0.0, -0.0, float("inf"), float("-inf")
+    for topk in sorted({1, max(1, keys // 2), max(1, keys - 1), keys}):
+        idx = ops.index_topk(s.cuda(), topk).cpu()
+        order = torch.sort(s + 0.0, dim=1, descending=True, stable=True)[1][:, :topk]
+        assert torch.equal(idx.long(), order.sort(dim=1)[0]), (keys, kind, topk)
+
+
 def test_index_topk_ties_and_masked_scores(ops):
     """Quantised scores (many equal values) and -inf entries: the selection is still exactly
     the k largest, ties at the k-th place going to the lower indices."""
