@@ -6,10 +6,12 @@ object is missing or a call returns a non-zero status, a RuntimeError is raised.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 from ctypes import c_char_p, c_float, c_int, c_int64, c_void_p
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "librt_b200.so"
+TORCH_PATH = LIB_PATH.with_name("_rt_torch.so")
 
 RT_BF16, RT_F32, RT_F16 = 0, 1, 2
 RT_ROPE_HALF, RT_ROPE_INTERLEAVED = 0, 1
@@ -96,6 +98,28 @@ def load() -> ctypes.CDLL:
         fn.argtypes = argtypes
     _lib = lib
     return lib
+
+
+_native = None
+
+
+def native():
+    """The tensor-level entry points (csrc/rt_torch.cpp) over the loaded library: imported once,
+    handed the addresses of the C functions they call."""
+    global _native
+    if _native is not None:
+        return _native
+    lib = load()
+    if not TORCH_PATH.exists():
+        raise RuntimeError(
+            f"_rt_torch.so not found at {TORCH_PATH}; build it with `python -m racetrack_b200.build`")
+    import torch  # noqa: F401  (its libraries resolve the module's symbols)
+    spec = importlib.util.spec_from_file_location("_rt_torch", TORCH_PATH)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    mod.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in mod.table()})
+    _native = mod
+    return mod
 
 
 def available() -> bool:

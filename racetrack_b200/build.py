@@ -1,22 +1,26 @@
-"""Builds librt_b200.so (the C-ABI kernel library) in-tree with nvcc for sm_100a.
+"""Builds librt_b200.so (the C-ABI kernel library, nvcc for sm_100a) and _rt_torch.so (the
+tensor-level entry points over it, g++ against the installed torch) in-tree.
 
 Usage: python -m racetrack_b200.build [--force] [--verbose]
 
-The library is written next to this file as ``lib/librt_b200.so``; it is the only
-binary the package loads. nvcc cross-compiles, so no GPU is needed to build.
+Both are written next to this file under ``lib/``; they are the only binaries the package
+loads. nvcc cross-compiles, so no GPU is needed to build.
 """
 from __future__ import annotations
 
 import hashlib
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_DIR = PKG_DIR / "lib"
 LIB_PATH = LIB_DIR / "librt_b200.so"
+TORCH_PATH = LIB_DIR / "_rt_torch.so"
 STAMP = LIB_DIR / "librt_b200.stamp"
 
 # Flags per source. The element-wise kernels are built without FMA contraction so
@@ -47,18 +51,30 @@ def _nvcc() -> str:
 
 def _fingerprint() -> str:
     h = hashlib.sha256()
-    for path in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh"))
+    for path in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.cpp"))
                        + [PKG_DIR.parent / "include" / "rt_b200.h", Path(__file__)]):
         h.update(path.name.encode())
         h.update(path.read_bytes())
     return h.hexdigest()
 
 
+def _torch_command() -> list[str]:
+    torch_dir = Path(importlib.util.find_spec("torch").origin).parent
+    cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    includes = [torch_dir / "include", torch_dir / "include/torch/csrc/api/include",
+                sysconfig.get_paths()["include"], f"{cuda_home}/include"]
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+            "-DTORCH_EXTENSION_NAME=_rt_torch", *[f"-I{d}" for d in includes],
+            str(CSRC / "rt_torch.cpp"), "-o", str(TORCH_PATH), f"-L{torch_dir / 'lib'}",
+            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python",
+            f"-Wl,-rpath,{torch_dir / 'lib'}"]
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every source and link the shared library; no-op when up to date."""
+    """Compile every source and link the shared libraries; no-op when up to date."""
     LIB_DIR.mkdir(exist_ok=True)
     fp = _fingerprint()
-    if not force and LIB_PATH.exists() and STAMP.exists() and STAMP.read_text() == fp:
+    if not force and LIB_PATH.exists() and TORCH_PATH.exists() and STAMP.exists() and STAMP.read_text() == fp:
         return LIB_PATH
     nvcc = _nvcc()
     objs = []
@@ -71,12 +87,14 @@ def build(force: bool = False, verbose: bool = False) -> Path:
             print(" ".join(cmd), flush=True)
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
         objs.append(str(obj))
+    procs.append(("rt_torch.cpp", subprocess.Popen(_torch_command(), stdout=subprocess.PIPE,
+                                                   stderr=subprocess.STDOUT, text=True)))
     failed = False
     for src, proc in procs:
         out, _ = proc.communicate()
         if proc.returncode != 0:
             failed = True
-            sys.stderr.write(f"nvcc failed on {src}:\n{out}\n")
+            sys.stderr.write(f"compilation of {src} failed:\n{out}\n")
         elif verbose or out.strip():
             sys.stderr.write(out)
     if failed:

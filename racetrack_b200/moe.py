@@ -82,17 +82,7 @@ def moe_gather_nvfp4(codes: torch.Tensor, sf: torch.Tensor, sorted_pairs: torch.
     """MoE dispatch of token rows quantised once (codes [T, cols/2], row-major scales
     [T, cols/16] from ops.fused_nvfp4_quant): (codes [total_rows, cols/2] in expert order,
     tile-aligned scales) for the rows of a tile map (rt_moe_gather_nvfp4)."""
-    cols = codes.shape[1] * 2
-    max_tiles = tile_map.shape[0] // 2
-    dev = codes.device
-    out = torch.empty(total_rows, cols // 2, dtype=torch.uint8, device=dev)
-    sf_out = torch.empty(max_tiles * (cols // 64) * 512, dtype=torch.uint8, device=dev)
-    lib = _lib.load()
-    _lib.check(lib.rt_moe_gather_nvfp4(
-        codes.data_ptr(), sf.data_ptr(), sorted_pairs.data_ptr(), topk, out.data_ptr(),
-        sf_out.data_ptr(), tile_map.data_ptr(), tile_count.data_ptr(), max_tiles, cols,
-        ops._stream()), "rt_moe_gather_nvfp4")
-    return out, sf_out
+    return _lib.native().moe_gather_nvfp4(codes, sf, sorted_pairs, topk, tile_map, tile_count, total_rows)
 
 
 swiglu_absmax_rows = ops.swiglu_absmax
@@ -104,20 +94,7 @@ def moe_quant_nvfp4(x: torch.Tensor, tile_map: torch.Tensor, tile_count: torch.T
     """NVFP4 codes [total_rows, cols/2] + tile-aligned block scales for the rows of a tile map
     (rt_moe_quant_nvfp4): gathers token rows when sorted_pairs is given, applies SwiGLU when
     `up` is given. Rows outside every tile are left unwritten."""
-    cols = x.shape[-1]
-    max_tiles = tile_map.shape[0] // 2
-    dev = x.device
-    codes = torch.empty(total_rows, cols // 2, dtype=torch.uint8, device=dev)
-    sf = torch.empty(max_tiles * (cols // 64) * 512, dtype=torch.uint8, device=dev)
-    gs = torch.empty(1, dtype=torch.float32, device=dev)
-    lib = _lib.load()
-    _lib.check(lib.rt_moe_quant_nvfp4(
-        x.data_ptr(), up.data_ptr() if up is not None else None,
-        sorted_pairs.data_ptr() if sorted_pairs is not None else None, topk, amax.data_ptr(),
-        codes.data_ptr(), sf.data_ptr(), gs.data_ptr(), tile_map.data_ptr(), tile_count.data_ptr(),
-        max_tiles, cols, x.stride(0), up.stride(0) if up is not None else 0, _lib.RT_BF16,
-        ops._stream()), "rt_moe_quant_nvfp4")
-    return codes, sf, gs
+    return _lib.native().moe_quant_nvfp4(x, tile_map, tile_count, total_rows, amax, sorted_pairs, topk, up)
 
 
 def fused_moe_experts(x: Optional[torch.Tensor], weights: torch.Tensor, indices: torch.Tensor,
@@ -139,44 +116,17 @@ def fused_moe_experts(x: Optional[torch.Tensor], weights: torch.Tensor, indices:
     A dict passed as `parts` receives the intermediates (expert offsets, permutation, the two
     tensor-wide amax values, gate_up, h and the per-pair expert outputs) for stage-wise checks.
     """
-    if x_quant is not None:
-        tokens, hidden = x_quant[0].shape[0], x_quant[0].shape[1] * 2
-    else:
-        tokens, hidden = x.shape
-    topk = indices.shape[1]
-    pairs = tokens * topk
-    count = experts.count
-    offsets, sorted_pairs, pair_pos = ops.fused_moe_permute(indices, n_experts)
-    max_tiles = (pairs + 127) // 128 + count
-    tile_map, _tile_base, tile_count = ops.moe_tile_map(offsets, expert_begin, expert_begin + count,
-                                                        max_tiles)
-    local = count != n_experts
-    window = (offsets[expert_begin:expert_begin + 1], offsets[expert_begin + count:expert_begin + count + 1]) \
-        if local else None
-    # dispatch: every token row is quantised once, then its codes and scales are copied into
-    # expert order (the bf16 rows are not read topk times)
-    if x_quant is not None:
-        x_codes, x_sf, a_gs = x_quant
-        x_amax = None
-    else:
-        x_amax = ops.tensor_absmax(x)
-        x_codes, x_sf, a_gs = ops.fused_nvfp4_quant(x, amax=x_amax)
-    a_codes, a_sf = moe_gather_nvfp4(x_codes, x_sf.view(torch.uint8), sorted_pairs, topk, tile_map,
-                                     tile_count, pairs)
-    gate_up = ops.gemm_nvfp4_grouped(a_codes, a_sf, a_gs, experts.w13_codes, experts.w13_sf,
-                                     experts.w13_gs, tile_map, tile_count, n=2 * experts.inter,
-                                     groups=count)
-    gate, up = gate_up[:, :experts.inter], gate_up[:, experts.inter:]
-    # SwiGLU once: this pass writes h and finds the tensor-wide amax its quantisation needs
-    h, h_amax = swiglu_absmax_rows(gate, up, window)
-    h_codes, h_sf, h_gs = moe_quant_nvfp4(h, tile_map, tile_count, pairs, amax=h_amax)
-    expert_out = ops.gemm_nvfp4_grouped(h_codes, h_sf, h_gs, experts.w2_codes, experts.w2_sf,
-                                        experts.w2_gs, tile_map, tile_count, n=hidden, groups=count)
+    q_codes, q_sf, q_gs = x_quant if x_quant is not None else (None, None, None)
+    if out_dtype not in (torch.bfloat16, torch.float32):
+        raise RuntimeError("fused_moe_experts: out_dtype must be bfloat16 or float32")
+    y, *stages = _lib.native().moe_experts(
+        x, weights, indices, experts.w13_codes, experts.w13_sf, experts.w13_gs, experts.w2_codes,
+        experts.w2_sf, experts.w2_gs, experts.count, experts.inter, n_experts, expert_begin, shared,
+        out_dtype == torch.float32, q_codes, q_sf, q_gs, out)
     if parts is not None:
-        parts.update(offsets=offsets, sorted_pairs=sorted_pairs, pair_pos=pair_pos, x_gs=a_gs, x_amax=x_amax,
-                     gate_up=gate_up, h=h, h_amax=h_amax, expert_out=expert_out)
-    return ops.fused_moe_combine(expert_out, pair_pos, weights, shared, pos_window=window,
-                                 out_dtype=out_dtype, out=out)
+        parts.update(zip(("offsets", "sorted_pairs", "pair_pos", "x_gs", "x_amax", "gate_up", "h", "h_amax",
+                          "expert_out"), stages))
+    return y
 
 
 def fused_moe_forward(x: torch.Tensor, gate_weight: torch.Tensor, gate_bias: Optional[torch.Tensor],

@@ -2,7 +2,9 @@
 
 Every function here takes CUDA tensors, allocates its outputs with torch's caching
 allocator, and enqueues hand-written sm_100a kernels from librt_b200.so on the
-current CUDA stream through the C ABI (include/rt_b200.h). Signatures and argument
+current CUDA stream through the C ABI (include/rt_b200.h). Checks, allocations and the call
+itself are native (csrc/rt_torch.cpp): in Python they took 20 - 36 us a call, more than the
+kernels of a decode step. Signatures and argument
 meaning follow racetrack's own kernel contracts (the file:line each one mirrors is
 given in its docstring); the ``fallback`` keyword every racetrack kernel receives is
 accepted and ignored - there is no torch or CPU fallback, unsupported inputs raise.
@@ -16,6 +18,9 @@ import torch
 from . import _lib
 
 _BF16 = torch.bfloat16
+
+
+_native = _lib.native
 
 
 def _stream() -> int:
@@ -69,24 +74,7 @@ def fused_residual_norm(update: torch.Tensor, residual: torch.Tensor, weight: to
     ``_kernel_call("fused_residual_norm", ...)``).
     """
     del fallback
-    _require_cuda(update, residual, weight)
-    _require_bf16("fused_residual_norm", update)
-    _require_bf16("fused_residual_norm", residual)
-    if update.shape != residual.shape:
-        raise RuntimeError("fused_residual_norm: update and residual shapes differ")
-    cols = update.shape[-1]
-    if weight.numel() != cols:
-        raise RuntimeError("fused_residual_norm: weight length does not match the last dimension")
-    u2, r2 = _rows_view(update), _rows_view(residual)
-    w = weight.contiguous()
-    normed = torch.empty(update.shape, dtype=update.dtype, device=update.device)
-    hidden = torch.empty(update.shape, dtype=update.dtype, device=update.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_residual_norm(u2.data_ptr(), r2.data_ptr(), w.data_ptr(), _weight_tag(w),
-                                    normed.data_ptr(), hidden.data_ptr(), u2.shape[0], cols,
-                                    u2.stride(0), r2.stride(0), float(eps), _lib.RT_BF16,
-                                    _stream()), "rt_residual_norm")
-    return normed, hidden
+    return _native().residual_norm(update, residual, weight, eps)
 
 
 def fused_residual_norm_legacy(residual: torch.Tensor, update: torch.Tensor, weight: torch.Tensor,
@@ -101,17 +89,7 @@ def fused_rms_norm(x: torch.Tensor, weight: torch.Tensor, *, eps: float,
                    fallback: Optional[Callable] = None) -> torch.Tensor:
     """rms_norm(x) * weight; partitions/_base.py:24-28, racetrack/models/deepseek.py:478-483."""
     del fallback
-    _require_cuda(x, weight)
-    _require_bf16("fused_rms_norm", x)
-    cols = x.shape[-1]
-    x2 = _rows_view(x)
-    w = weight.contiguous()
-    out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_rms_norm(x2.data_ptr(), w.data_ptr(), _weight_tag(w), out.data_ptr(),
-                               x2.shape[0], cols, x2.stride(0), cols, float(eps), _lib.RT_BF16,
-                               _stream()), "rt_rms_norm")
-    return out
+    return _native().rms_norm(x, weight, eps)
 
 
 # ---------------------------------------------------------------------------
@@ -135,44 +113,6 @@ def _inv_freq(half: int, base: float, device: torch.device) -> torch.Tensor:
     return t
 
 
-def _freqs_table(freqs_cis: torch.Tensor, half: int) -> torch.Tensor:
-    """[rows, half, 2] fp32 view of a complex64 freqs_cis tensor (no copy when contiguous)."""
-    if not freqs_cis.is_complex():
-        raise RuntimeError("freqs_cis must be a complex tensor")
-    table = torch.view_as_real(freqs_cis.reshape(-1, half).contiguous())
-    if table.dtype != torch.float32:
-        table = table.float()
-    return table
-
-
-def _norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, positions, table, table_rows, eps, mode):
-    _require_cuda(q_c, kv_c, k_pe, q_weight, kv_weight)
-    for name, t in (("q_c", q_c), ("kv_c", kv_c), ("k_pe", k_pe)):
-        _require_bf16(f"fused_norm_rope {name}", t)
-    q2, kv2, k2 = _rows_view(q_c), _rows_view(kv_c), k_pe.reshape(-1, k_pe.shape[-1])
-    if k2.stride(-1) != 1:
-        k2 = k2.contiguous()
-    tokens = q2.shape[0]
-    if kv2.shape[0] != tokens or k2.shape[0] != tokens:
-        raise RuntimeError("fused_norm_rope: q_c, kv_c and k_pe disagree on the token count")
-    qw, kvw = q_weight.contiguous(), kv_weight.contiguous()
-    if qw.dtype != kvw.dtype:
-        kvw = kvw.to(qw.dtype)
-    q_out = torch.empty(q_c.shape, dtype=q_c.dtype, device=q_c.device)
-    kv_out = torch.empty(kv_c.shape, dtype=kv_c.dtype, device=kv_c.device)
-    k_out = torch.empty(k_pe.shape, dtype=k_pe.dtype, device=k_pe.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_norm_rope(q2.data_ptr(), qw.data_ptr(), kv2.data_ptr(), kvw.data_ptr(),
-                                _weight_tag(qw), k2.data_ptr(),
-                                positions.data_ptr() if positions is not None else None,
-                                table.data_ptr(), table_rows,
-                                q_out.data_ptr(), kv_out.data_ptr(), k_out.data_ptr(),
-                                tokens, q2.shape[1], kv2.shape[1], k2.shape[1],
-                                q2.stride(0), kv2.stride(0), k2.stride(0),
-                                float(eps), mode, _lib.RT_BF16, _stream()), "rt_norm_rope")
-    return q_out, kv_out, k_out
-
-
 def fused_norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, positions, *, eps: float,
                     rope_base: float, fallback: Optional[Callable] = None):
     """(rms_norm(q_c), rms_norm(kv_c), apply_rope(k_pe)) with half-split RoPE.
@@ -181,13 +121,8 @@ def fused_norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, positions, *, eps: flo
     inputs are normally column slices of one [T, q_lora+kv_lora+rope] projection output.
     """
     del fallback
-    half = k_pe.shape[-1] // 2
-    pos = positions.reshape(-1)
-    if pos.dtype != torch.int64:
-        pos = pos.to(torch.int64)
-    pos = pos.contiguous()
-    table = _inv_freq(half, rope_base, k_pe.device)
-    return _norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, pos, table, 0, eps, _lib.RT_ROPE_HALF)
+    table = _inv_freq(k_pe.shape[-1] // 2, rope_base, k_pe.device)
+    return _native().norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, positions, table, None, eps)
 
 
 def fused_norm_rope_interleaved(q_c, q_weight, kv_c, kv_weight, k_pe, freqs_cis, *, eps: float,
@@ -196,34 +131,7 @@ def fused_norm_rope_interleaved(q_c, q_weight, kv_c, kv_weight, k_pe, freqs_cis,
     (racetrack/models/deepseek.py:766-776). ``freqs_cis`` is the complex64
     [seqlen, rope_dim/2] slice for the tokens; rows wrap around per batch element."""
     del fallback
-    half = k_pe.shape[-1] // 2
-    table = _freqs_table(freqs_cis, half)
-    return _norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, None, table, table.shape[0], eps,
-                      _lib.RT_ROPE_INTERLEAVED)
-
-
-def _rope_heads(x: torch.Tensor, positions, table, table_rows, mode, inplace: bool):
-    _require_cuda(x)
-    _require_bf16("fused_rope", x)
-    if x.dim() < 2:
-        raise RuntimeError("fused_rope: expected [..., heads, rope_dim]")
-    d = x.shape[-1]
-    heads = x.shape[-2]
-    x3 = x.reshape(-1, heads, d) if x.dim() != 3 else x
-    ok = (x3.stride(2) == 1 and x3.stride(0) % 8 == 0 and x3.stride(1) % 8 == 0
-          and x3.data_ptr() % 16 == 0)
-    if not ok:
-        if inplace:
-            raise RuntimeError("fused_rope: in-place rotation needs a 16-byte aligned strided view")
-        x3 = x3.contiguous()
-    out3 = x3 if inplace else torch.empty((x3.shape[0], heads, d), dtype=x.dtype, device=x.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_rope(x3.data_ptr(), positions.data_ptr() if positions is not None else None,
-                           table.data_ptr(), table_rows, out3.data_ptr(),
-                           x3.shape[0], heads, d, x3.stride(0), x3.stride(1),
-                           out3.stride(0), out3.stride(1), mode, _lib.RT_BF16, _stream()),
-               "rt_rope")
-    return x if inplace else out3.view(x.shape)
+    return _native().norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, None, None, freqs_cis, eps)
 
 
 def fused_rope(x: torch.Tensor, freqs_cis: torch.Tensor, *, inplace: bool = False,
@@ -232,9 +140,7 @@ def fused_rope(x: torch.Tensor, freqs_cis: torch.Tensor, *, inplace: bool = Fals
     by freqs_cis [seq, rope_dim/2]; racetrack/models/deepseek.py:604-624 with interleaved=True
     (kernel name as in partitions/dsv3_2/3336cdbd/kernels/triton/rope.py:57-62)."""
     del fallback
-    half = x.shape[-1] // 2
-    table = _freqs_table(freqs_cis, half)
-    return _rope_heads(x, None, table, table.shape[0], _lib.RT_ROPE_INTERLEAVED, inplace)
+    return _native().rope(x, None, None, freqs_cis, inplace)
 
 
 def fused_rope_half(x: torch.Tensor, positions: torch.Tensor, *, rope_base: float = 10000.0,
@@ -242,9 +148,8 @@ def fused_rope_half(x: torch.Tensor, positions: torch.Tensor, *, rope_base: floa
     """Half-split RoPE of x [tokens, heads, rope_dim] at integer positions;
     partitions/dsv3_2/model.py:55-81 (apply_rope), racetrack/realistic_bench.py:297-302."""
     del fallback
-    half = x.shape[-1] // 2
-    pos = positions.reshape(-1).to(torch.int64).contiguous()
-    return _rope_heads(x, pos, _inv_freq(half, rope_base, x.device), 0, _lib.RT_ROPE_HALF, inplace)
+    table = _inv_freq(x.shape[-1] // 2, rope_base, x.device)
+    return _native().rope(x, positions, table, None, inplace)
 
 
 def head_broadcast_(dst: torch.Tensor, src: torch.Tensor) -> torch.Tensor:
@@ -268,26 +173,11 @@ def head_broadcast_(dst: torch.Tensor, src: torch.Tensor) -> torch.Tensor:
 # SwiGLU and activation quantisation
 # ---------------------------------------------------------------------------
 
-def _gate_up(gate: torch.Tensor, up: torch.Tensor, who: str):
-    _require_cuda(gate, up)
-    _require_bf16(who, gate)
-    _require_bf16(who, up)
-    if gate.shape != up.shape:
-        raise RuntimeError(f"{who}: gate and up shapes differ")
-    return _rows_view(gate), _rows_view(up)
-
-
 def fused_swiglu(gate: torch.Tensor, up: torch.Tensor, *,
                  fallback: Optional[Callable] = None) -> torch.Tensor:
     """(silu(gate.float()) * up.float()).type_as(gate); racetrack/models/deepseek.py:850-853."""
     del fallback
-    g2, u2 = _gate_up(gate, up, "fused_swiglu")
-    out = torch.empty(gate.shape, dtype=gate.dtype, device=gate.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_swiglu(g2.data_ptr(), u2.data_ptr(), out.data_ptr(), g2.shape[0],
-                             g2.shape[1], g2.stride(0), u2.stride(0), _lib.RT_BF16, _stream()),
-               "rt_swiglu")
-    return out
+    return _native().swiglu(gate, up)
 
 
 def fused_act_quant(x: torch.Tensor, *, out: Optional[tuple] = None, fallback: Optional[Callable] = None):
@@ -295,26 +185,8 @@ def fused_act_quant(x: torch.Tensor, *, out: Optional[tuple] = None, fallback: O
     ``out`` = (codes, scales) contiguous tensors of those shapes to write into (codes as
     float8_e4m3fn or uint8)."""
     del fallback
-    _require_cuda(x)
-    _require_bf16("fused_act_quant", x)
-    n = x.shape[-1]
-    if n % 128 != 0:
-        raise RuntimeError(f"fused_act_quant: last dim ({n}) must be a multiple of 128")
-    x2 = _rows_view(x)
-    if out is not None:
-        codes, scales = out
-        if (codes.element_size() != 1 or scales.dtype != torch.float32 or not codes.is_contiguous()
-                or not scales.is_contiguous() or tuple(codes.shape) != tuple(x.shape)
-                or tuple(scales.shape) != (*x.shape[:-1], n // 128)):
-            raise RuntimeError("fused_act_quant: out must be contiguous (1-byte codes [..., N], fp32 scales [..., N/128])")
-    else:
-        codes = torch.empty(x.shape, dtype=torch.float8_e4m3fn, device=x.device)
-        scales = torch.empty(*x.shape[:-1], n // 128, dtype=torch.float32, device=x.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_act_quant_fp8(x2.data_ptr(), codes.data_ptr(), scales.data_ptr(),
-                                    x2.shape[0], n, x2.stride(0), _lib.RT_BF16, _stream()),
-               "rt_act_quant_fp8")
-    return codes, scales
+    codes, scales = out if out is not None else (None, None)
+    return _native().act_quant(x, codes, scales)
 
 
 def fused_swiglu_quant(gate: torch.Tensor, up: torch.Tensor, *,
@@ -322,52 +194,21 @@ def fused_swiglu_quant(gate: torch.Tensor, up: torch.Tensor, *,
     """act_quant(swiglu(gate, up)) without materialising the bf16 product;
     benchmarks/gsm8k/flat_decode.py:132-136."""
     del fallback
-    g2, u2 = _gate_up(gate, up, "fused_swiglu_quant")
-    n = gate.shape[-1]
-    if n % 128 != 0:
-        raise RuntimeError(f"fused_swiglu_quant: last dim ({n}) must be a multiple of 128")
-    codes = torch.empty(gate.shape, dtype=torch.float8_e4m3fn, device=gate.device)
-    scales = torch.empty(*gate.shape[:-1], n // 128, dtype=torch.float32, device=gate.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_swiglu_quant_fp8(g2.data_ptr(), u2.data_ptr(), codes.data_ptr(),
-                                       scales.data_ptr(), g2.shape[0], n, g2.stride(0),
-                                       u2.stride(0), _lib.RT_BF16, _stream()),
-               "rt_swiglu_quant_fp8")
-    return codes, scales
+    return _native().swiglu_quant(gate, up)
 
 
 def tensor_absmax(x: torch.Tensor, up: Optional[torch.Tensor] = None) -> torch.Tensor:
     """max(|x|) over the whole tensor as a 1-element fp32 CUDA tensor (of swiglu(x, up)
     when ``up`` is given). Feeds the NVFP4 global scale."""
-    _require_cuda(x)
-    _require_bf16("tensor_absmax", x)
-    if x.shape[-1] % 16 != 0:
-        raise RuntimeError("tensor_absmax: last dim must be a multiple of 16")
-    x2 = _rows_view(x)
-    u2 = _rows_view(up) if up is not None else None
-    out = torch.empty(1, dtype=torch.float32, device=x.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_absmax(x2.data_ptr(), u2.data_ptr() if u2 is not None else None,
-                             out.data_ptr(), x2.shape[0], x2.shape[1], x2.stride(0),
-                             u2.stride(0) if u2 is not None else 0, _lib.RT_BF16, _stream()),
-               "rt_absmax")
-    return out
+    return _native().tensor_absmax(x, up)
 
 
 def swiglu_absmax(gate: torch.Tensor, up: torch.Tensor, window=None):
     """(h, amax): h = bf16(silu(gate) * up) and max |h| over the rows of `window` (a pair of
     one-element int32 device tensors [begin], [end], or None for all rows) of 2-D gate and up with
     16-byte aligned rows; rows outside the window are not written (rt_swiglu_absmax_rows)."""
-    h = torch.empty(gate.shape, dtype=torch.bfloat16, device=gate.device)
-    out = torch.empty(1, dtype=torch.float32, device=gate.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_swiglu_absmax_rows(
-        gate.data_ptr(), up.data_ptr(), h.data_ptr(), out.data_ptr(), gate.shape[0], gate.shape[1],
-        gate.stride(0), up.stride(0), h.stride(0),
-        window[0].data_ptr() if window is not None else None,
-        window[1].data_ptr() if window is not None else None, _lib.RT_BF16, _stream()),
-        "rt_swiglu_absmax_rows")
-    return h, out
+    begin, end = window if window is not None else (None, None)
+    return _native().swiglu_absmax(gate, up, begin, end)
 
 
 def sf_tiled_bytes(rows: int, cols: int) -> int:
@@ -389,45 +230,8 @@ def fused_nvfp4_quant(x: torch.Tensor, *, up: Optional[torch.Tensor] = None,
     racetrack has no NVFP4 arithmetic; the format follows the build's stated configuration.
     """
     del fallback
-    _require_cuda(x)
-    _require_bf16("fused_nvfp4_quant", x)
-    n = x.shape[-1]
-    if n % 16 != 0:
-        raise RuntimeError(f"fused_nvfp4_quant: last dim ({n}) must be a multiple of 16")
-    x2 = _rows_view(x)
-    u2 = None
-    if up is not None:
-        x2, u2 = _gate_up(x, up, "fused_nvfp4_quant")
-    if amax is None and up is not None and x2.shape[0] > 0:
-        # one evaluation of SwiGLU: the abs-max pass writes its bf16 result and the quantiser reads
-        # that (4 + 2 + 2 + 0.56 bytes an element, as many as two passes over gate and up move, at
-        # half the instructions; 4096 x 18432 on one B200: 120 us against 161)
-        x2, amax = swiglu_absmax(x2, u2)
-        u2 = None
-    elif amax is None:
-        amax = tensor_absmax(x, up)
-    rows = x2.shape[0]
-    if out is not None:
-        codes, sf = out
-        want_sf = (sf_tiled_bytes(rows, n),) if tiled_scales else (*x.shape[:-1], n // 16)
-        if (codes.dtype != torch.uint8 or sf.dtype != torch.uint8 or not codes.is_contiguous()
-                or not sf.is_contiguous() or tuple(codes.shape) != (*x.shape[:-1], n // 2)
-                or tuple(sf.shape) != tuple(want_sf)):
-            raise RuntimeError("fused_nvfp4_quant: out must be contiguous uint8 (codes [..., N/2], scales)")
-    else:
-        codes = torch.empty(*x.shape[:-1], n // 2, dtype=torch.uint8, device=x.device)
-        if tiled_scales:
-            sf = torch.empty(sf_tiled_bytes(rows, n), dtype=torch.uint8, device=x.device)
-        else:
-            sf = torch.empty(*x.shape[:-1], n // 16, dtype=torch.uint8, device=x.device)
-    gs = torch.empty(1, dtype=torch.float32, device=x.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_nvfp4_quant(x2.data_ptr(), u2.data_ptr() if u2 is not None else None,
-                                  amax.data_ptr(), codes.data_ptr(), sf.data_ptr(), gs.data_ptr(),
-                                  rows, n, x2.stride(0), u2.stride(0) if u2 is not None else 0,
-                                  _lib.RT_SF_TILED128x4 if tiled_scales else _lib.RT_SF_ROWMAJOR,
-                                  _lib.RT_BF16, _stream()), "rt_nvfp4_quant")
-    return codes, sf.view(torch.float8_e4m3fn), gs
+    codes, sf = out if out is not None else (None, None)
+    return _native().nvfp4_quant(x, up, amax, tiled_scales, codes, sf)
 
 
 def fused_swiglu_nvfp4_quant(gate: torch.Tensor, up: torch.Tensor, **kw):
@@ -447,53 +251,17 @@ def fused_moe_route(logits: torch.Tensor, bias: Optional[torch.Tensor], *, n_gro
     everything in Gate.forward after the logits GEMM (racetrack/models/deepseek.py:899-920).
     ``out`` = (weights, indices) contiguous tensors of those shapes to write into."""
     del fallback
-    _require_cuda(logits)
-    if logits.dtype != torch.float32 or logits.dim() != 2:
-        raise RuntimeError("fused_moe_route: logits must be a 2-D float32 tensor")
-    if logits.stride(1) != 1:
-        logits = logits.contiguous()
-    if bias is not None:
-        bias = bias.to(torch.float32).contiguous()
-    tokens, n_experts = logits.shape
-    if out is not None:
-        weights, indices = out
-        if (weights.dtype != torch.float32 or indices.dtype != torch.int64 or not weights.is_contiguous()
-                or not indices.is_contiguous() or tuple(weights.shape) != (tokens, topk)
-                or tuple(indices.shape) != (tokens, topk)):
-            raise RuntimeError("fused_moe_route: out must be contiguous (fp32 [T, topk], int64 [T, topk])")
-    else:
-        weights = torch.empty(tokens, topk, dtype=torch.float32, device=logits.device)
-        indices = torch.empty(tokens, topk, dtype=torch.int64, device=logits.device)
     func = {"sigmoid": _lib.RT_SCORE_SIGMOID, "softmax": _lib.RT_SCORE_SOFTMAX,
             "topk_softmax": _lib.RT_SCORE_TOPK_SOFTMAX}[score_func]
-    lib = _lib.load()
-    _lib.check(lib.rt_moe_route(logits.data_ptr(), bias.data_ptr() if bias is not None else None,
-                                weights.data_ptr(), indices.data_ptr(), tokens, n_experts,
-                                logits.stride(0), n_groups, topk_groups, topk, float(route_scale),
-                                func, _stream()), "rt_moe_route")
-    return weights, indices
+    weights, indices = out if out is not None else (None, None)
+    return _native().moe_route(logits, bias, n_groups, topk_groups, topk, route_scale, func, weights, indices)
 
 
 def fused_moe_permute(indices: torch.Tensor, n_experts: int):
     """Stable sort of (token, slot) pairs by expert ->
     (expert_offsets int32 [E+1], sorted_pairs int32 [T*topk], pair_pos int32 [T*topk]);
     replaces bincount + per-expert torch.where of racetrack/models/deepseek.py:1011-1017."""
-    _require_cuda(indices)
-    if indices.dtype != torch.int64 or indices.dim() != 2:
-        raise RuntimeError("fused_moe_permute: indices must be a 2-D int64 tensor")
-    indices = indices.contiguous()
-    tokens, topk = indices.shape
-    dev = indices.device
-    lib = _lib.load()
-    ws_bytes = int(lib.rt_moe_permute_workspace_bytes(tokens, topk, n_experts))
-    workspace = torch.empty(max(ws_bytes, 4), dtype=torch.uint8, device=dev)
-    offsets = torch.empty(n_experts + 1, dtype=torch.int32, device=dev)
-    sorted_pairs = torch.empty(tokens * topk, dtype=torch.int32, device=dev)
-    pair_pos = torch.empty(tokens * topk, dtype=torch.int32, device=dev)
-    _lib.check(lib.rt_moe_permute(indices.data_ptr(), offsets.data_ptr(), sorted_pairs.data_ptr(),
-                                  pair_pos.data_ptr(), workspace.data_ptr(), tokens, topk,
-                                  n_experts, _stream()), "rt_moe_permute")
-    return offsets, sorted_pairs, pair_pos
+    return _native().moe_permute(indices, n_experts)
 
 
 def fused_moe_gather(x: torch.Tensor, sorted_pairs: torch.Tensor, topk: int) -> torch.Tensor:
@@ -521,30 +289,11 @@ def fused_moe_combine(expert_out: torch.Tensor, pair_pos: torch.Tensor, weights:
     CUDA tensors (entries of expert_offsets) restricts the sum to an expert-parallel rank's
     slice of the sorted range without a host read-back. ``out_dtype=torch.float32`` returns the
     fp32 sums (what the reference all-reduces across expert-parallel ranks before its cast)."""
-    _require_cuda(expert_out, pair_pos, weights)
-    _require_bf16("fused_moe_combine", expert_out)
-    tokens, topk = weights.shape
-    cols = expert_out.shape[-1]
-    expert_out = expert_out.contiguous()
-    weights = weights.to(torch.float32).contiguous()
-    if shared is not None:
-        _require_bf16("fused_moe_combine", shared)
-        shared = shared.reshape(tokens, cols).contiguous()
-    if pos_end is None:
-        pos_end = tokens * topk
     if out_dtype not in (torch.bfloat16, torch.float32):
         raise RuntimeError("fused_moe_combine: out_dtype must be bfloat16 or float32")
-    y = _out_buffer(out, (tokens, cols), out_dtype, expert_out.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_moe_combine(expert_out.data_ptr(), pair_pos.data_ptr(), weights.data_ptr(),
-                                  shared.data_ptr() if shared is not None else None, y.data_ptr(),
-                                  tokens, topk, cols, pos_begin, pos_end,
-                                  pos_window[0].data_ptr() if pos_window is not None else None,
-                                  pos_window[1].data_ptr() if pos_window is not None else None,
-                                  _lib.RT_F32 if out_dtype == torch.float32 else _lib.RT_BF16,
-                                  _stream()),
-               "rt_moe_combine")
-    return y
+    begin, end = pos_window if pos_window is not None else (None, None)
+    return _native().moe_combine(expert_out, pair_pos, weights, shared, pos_begin, pos_end, begin, end,
+                                 out_dtype == torch.float32, out)
 
 
 # ---------------------------------------------------------------------------
@@ -560,57 +309,15 @@ def tc_error_state() -> None:
 SPLITK_MAX_ROWS = 65536   # linear_bf16 never splits K for more rows than this
 
 
-def _out_buffer(out: Optional[torch.Tensor], shape: tuple, dtype: torch.dtype, device) -> torch.Tensor:
-    """The caller's output buffer when it fits (contiguous, right shape and type: e.g. a buffer
-    other ranks read over NVLink), else a fresh tensor."""
-    if out is None:
-        return torch.empty(shape, dtype=dtype, device=device)
-    if tuple(out.shape) != tuple(shape) or out.dtype != dtype or not out.is_contiguous():
-        raise RuntimeError(f"out must be a contiguous {dtype} tensor of shape {tuple(shape)}")
-    return out
-
-
 def linear_bf16(x: torch.Tensor, weight: torch.Tensor, *,
                 out_dtype: torch.dtype = torch.bfloat16,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """F.linear(x, weight) for bf16 x [..., K] and weight [N, K] on the tcgen05 tensor cores
     (the bf16 branch of racetrack/models/deepseek.py:316-345 `linear`). out_dtype=torch.float32
     returns the fp32 accumulators (router logits, racetrack/models/deepseek.py:898)."""
-    _require_cuda(x, weight)
-    _require_bf16("linear_bf16 x", x)
-    _require_bf16("linear_bf16 weight", weight)
-    k = x.shape[-1]
-    if weight.dim() != 2 or weight.shape[1] != k:
-        raise RuntimeError("linear_bf16: weight must be [N, K] with K matching x")
-    x2 = _rows_view(x)
-    w = weight if (weight.stride(1) == 1 and weight.stride(0) % 8 == 0
-                   and weight.data_ptr() % 16 == 0) else weight.contiguous()
-    n = w.shape[0]
     if out_dtype not in (torch.bfloat16, torch.float32):
         raise RuntimeError("linear_bf16: out_dtype must be bfloat16 or float32")
-    lib = _lib.load()
-    rows = x2.shape[0]
-    # too few output tiles to occupy the GPU (a few decode tokens, the 128 - 256 columns of a router
-    # or an index projection): the library says into how many ranges to cut K. 4096 x 256 x 7168 on
-    # one B200: 23 us against 47 as 32 whole tiles
-    splits = int(lib.rt_gemm_bf16_splitk_splits(rows, n, k)) if 0 < rows <= SPLITK_MAX_ROWS else 1
-    if splits > 1:
-        # partial products per K range, then their sum in a fixed order: bit-reproducible, and
-        # identical on every rank that forms the same replicated projection
-        part = torch.empty(splits, rows, n, dtype=torch.float32, device=x.device)
-        out = _out_buffer(out, (*x.shape[:-1], n), out_dtype, x.device)
-        _lib.check(lib.rt_gemm_bf16_splitk(
-            x2.data_ptr(), w.data_ptr(), part.data_ptr(), out.data_ptr(), rows, n, k,
-            x2.stride(0), w.stride(0), n, n, splits,
-            _lib.RT_F32 if out_dtype == torch.float32 else _lib.RT_BF16, _stream()),
-            "rt_gemm_bf16_splitk")
-        return out
-    out = _out_buffer(out, (*x.shape[:-1], n), out_dtype, x.device)
-    _lib.check(lib.rt_gemm_bf16(x2.data_ptr(), w.data_ptr(), out.data_ptr(), x2.shape[0], n, k,
-                                x2.stride(0), w.stride(0), n,
-                                _lib.RT_F32 if out_dtype == torch.float32 else _lib.RT_BF16,
-                                _stream()), "rt_gemm_bf16")
-    return out
+    return _native().linear_bf16(x, weight, out_dtype == torch.float32, out, SPLITK_MAX_ROWS)
 
 
 def linear_bf16_batched(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
@@ -618,23 +325,7 @@ def linear_bf16_batched(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     a column slice of a projection output) and weight bf16 [H, N, K] -> bf16 [T, H, N], one launch
     for all heads. The absorbed projections of the MLA decode branch
     (racetrack/models/deepseek.py:799,810)."""
-    _require_cuda(x, weight)
-    _require_bf16("linear_bf16_batched x", x)
-    _require_bf16("linear_bf16_batched weight", weight)
-    if x.dim() != 3 or weight.dim() != 3 or weight.shape[0] != x.shape[1] or weight.shape[2] != x.shape[2]:
-        raise RuntimeError("linear_bf16_batched: expected x [T, H, K] and weight [H, N, K]")
-    if x.stride(2) != 1 or x.stride(0) % 8 or x.stride(1) % 8 or x.data_ptr() % 16:
-        x = x.contiguous()
-    if weight.stride(2) != 1 or weight.stride(0) % 8 or weight.stride(1) % 8 or weight.data_ptr() % 16:
-        weight = weight.contiguous()
-    tokens, heads, k = x.shape
-    n = weight.shape[1]
-    out = torch.empty(tokens, heads, n, dtype=torch.bfloat16, device=x.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_gemm_bf16_batched(x.data_ptr(), weight.data_ptr(), out.data_ptr(), heads, tokens, n, k,
-                                        x.stride(0), x.stride(1), weight.stride(1), weight.stride(0),
-                                        out.stride(0), out.stride(1), _stream()), "rt_gemm_bf16_batched")
-    return out
+    return _native().linear_bf16_batched(x, weight)
 
 
 _SPLIT_WEIGHTS: dict[tuple, tuple] = {}     # key -> (hi | lo halves, the weight itself)
@@ -718,32 +409,14 @@ def linear_fp8(x_codes: torch.Tensor, x_scales: torch.Tensor, w_codes: torch.Ten
                w_scales: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """FP8 block-scaled linear: fp8_gemm(a, a_s, b, b_s) of racetrack/models/deepseek.py:110-145
     -> bf16 [..., N]. x_codes / x_scales as fused_act_quant returns them."""
-    _require_cuda(x_codes, x_scales, w_codes, w_scales)
-    k = x_codes.shape[-1]
-    n = w_codes.shape[0]
-    if w_codes.shape[1] != k or x_codes.dtype != torch.float8_e4m3fn or w_codes.dtype != torch.float8_e4m3fn:
-        raise RuntimeError("linear_fp8: expected e4m3fn codes with matching K")
-    xc = x_codes.reshape(-1, k)
-    xs = x_scales.reshape(-1, k // 128)
-    if not (xc.is_contiguous() and xs.is_contiguous() and w_codes.is_contiguous()
-            and w_scales.is_contiguous()):
-        raise RuntimeError("linear_fp8: operands must be contiguous")
-    if xs.dtype != torch.float32 or w_scales.dtype != torch.float32 \
-            or w_scales.shape != ((n + 127) // 128, k // 128):
-        raise RuntimeError("linear_fp8: scales must be fp32 [M, K/128] and [ceil(N/128), K/128]")
-    out = _out_buffer(out, (*x_codes.shape[:-1], n), torch.bfloat16, x_codes.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_gemm_fp8(xc.data_ptr(), xs.data_ptr(), w_codes.data_ptr(), w_scales.data_ptr(),
-                               out.data_ptr(), xc.shape[0], n, k, k, k, n, _stream()), "rt_gemm_fp8")
-    return out
+    return _native().linear_fp8(x_codes, x_scales, w_codes, w_scales, out)
 
 
 def linear_fp8_act(x: torch.Tensor, w_codes: torch.Tensor, w_scales: torch.Tensor,
                    out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """`linear(x, weight)` with an FP8 weight as racetrack/models/deepseek.py:343-345 runs it:
     act_quant(x) then the FP8 block-scaled GEMM."""
-    codes, scales = fused_act_quant(x)
-    return linear_fp8(codes, scales, w_codes, w_scales, out=out)
+    return _native().linear_fp8_act(x, w_codes, w_scales, out)
 
 
 def moe_tile_map(offsets: torch.Tensor, g_begin: int, g_end: int, max_tiles: int):
@@ -753,18 +426,7 @@ def moe_tile_map(offsets: torch.Tensor, g_begin: int, g_end: int, max_tiles: int
     128-row tiles (one scale row tile each); rows [max_tiles, max_tiles + tile_count[1]) cut
     the same rows into tiles of up to 256 rows for the CTA-pair GEMM. No host
     synchronisation."""
-    _require_cuda(offsets)
-    if offsets.dtype != torch.int32:
-        raise RuntimeError("moe_tile_map: offsets must be int32")
-    dev = offsets.device
-    tile_map = torch.empty(2 * max_tiles, 4, dtype=torch.int32, device=dev)
-    tile_base = torch.empty(g_end - g_begin + 1, dtype=torch.int32, device=dev)
-    tile_count = torch.empty(2, dtype=torch.int32, device=dev)
-    lib = _lib.load()
-    _lib.check(lib.rt_moe_tile_map(offsets.data_ptr(), g_begin, g_end, tile_map.data_ptr(),
-                                   tile_base.data_ptr(), tile_count.data_ptr(), max_tiles,
-                                   _stream()), "rt_moe_tile_map")
-    return tile_map, tile_base, tile_count
+    return _native().moe_tile_map(offsets, g_begin, g_end, max_tiles)
 
 
 def gemm_nvfp4_grouped(a_codes: torch.Tensor, a_sf: torch.Tensor, a_gs: torch.Tensor,
@@ -777,23 +439,8 @@ def gemm_nvfp4_grouped(a_codes: torch.Tensor, a_sf: torch.Tensor, a_gs: torch.Te
     b_codes uint8 [groups * n, K/2]; b_sf tiled scales per group; b_gs fp32 [groups];
     tile_map / tile_count as moe_tile_map returns them.
     Returns bf16 [rows, n]; rows outside every tile are left untouched."""
-    _require_cuda(a_codes, a_sf, a_gs, b_codes, b_sf, b_gs, tile_map, tile_count)
-    rows, kh = a_codes.shape
-    if b_codes.shape != (groups * n, kh):
-        raise RuntimeError("gemm_nvfp4_grouped: b_codes must be [groups * n, K/2]")
-    if not (a_codes.is_contiguous() and b_codes.is_contiguous()):
-        raise RuntimeError("gemm_nvfp4_grouped: code tensors must be contiguous")
-    if out is None:
-        out = torch.empty(rows, n, dtype=torch.bfloat16, device=a_codes.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_gemm_nvfp4_grouped(a_codes.data_ptr(), a_sf.data_ptr(), a_gs.data_ptr(),
-                                         b_codes.data_ptr(), b_sf.data_ptr(), b_gs.data_ptr(),
-                                         out.data_ptr(), tile_map.data_ptr(),
-                                         tile_count.data_ptr(), tile_map.shape[0] // 2, rows,
-                                         groups,
-                                         n, 2 * kh, out.stride(0), _stream()),
-               "rt_gemm_nvfp4_grouped")
-    return out
+    return _native().gemm_nvfp4_grouped(a_codes, a_sf, a_gs, b_codes, b_sf, b_gs, tile_map, tile_count,
+                                        n, groups, out)
 
 
 def index_prep(x: torch.Tensor, freqs_cis: torch.Tensor, *, positions: Optional[torch.Tensor] = None,
@@ -806,32 +453,7 @@ def index_prep(x: torch.Tensor, freqs_cis: torch.Tensor, *, positions: Optional[
     x bf16 [S, H, 128] (H = 1 for keys); freqs_cis complex64 [table, 32]; positions int64 [S]
     (default 0..S-1). Returns (codes float8_e4m3fn [S, H, 128], scales fp32 [S, H]) and, on
     request, the rotated bf16 tensor that was quantised."""
-    _require_cuda(x, freqs_cis)
-    _require_bf16("index_prep", x)
-    if x.dim() != 3 or x.shape[-1] != 128:
-        raise RuntimeError("index_prep: x must be [S, H, 128]")
-    s_len, heads, dim = x.shape
-    x2 = x.reshape(s_len * heads, dim)
-    if x2.stride(1) != 1:
-        x2 = x2.contiguous()
-    fr = torch.view_as_real(freqs_cis).to(torch.float32).contiguous()
-    if fr.shape[-2:] != (32, 2):
-        raise RuntimeError("index_prep: freqs_cis must be [table, 32] complex")
-    codes = torch.empty(s_len, heads, dim, dtype=torch.float8_e4m3fn, device=x.device)
-    scales = torch.empty(s_len, heads, dtype=torch.float32, device=x.device)
-    rotated = torch.empty(s_len, heads, dim, dtype=torch.bfloat16, device=x.device) \
-        if return_rotated else None
-    lw = ln_weight.to(torch.float32).contiguous() if ln_weight is not None else None
-    lb = ln_bias.to(torch.float32).contiguous() if ln_bias is not None else None
-    pos = positions.to(torch.int64).contiguous() if positions is not None else None
-    lib = _lib.load()
-    _lib.check(lib.rt_index_prep(
-        x2.data_ptr(), lw.data_ptr() if lw is not None else None,
-        lb.data_ptr() if lb is not None else None, pos.data_ptr() if pos is not None else None,
-        fr.data_ptr(), fr.shape[0], heads, codes.data_ptr(), scales.data_ptr(),
-        rotated.data_ptr() if rotated is not None else None, s_len * heads, dim, 64,
-        x2.stride(0), float(eps), _lib.RT_BF16, _stream()), "rt_index_prep")
-    return (codes, scales, rotated) if return_rotated else (codes, scales)
+    return _native().index_prep(x, freqs_cis, positions, ln_weight, ln_bias, eps, return_rotated)
 
 
 def fp8_index(q: torch.Tensor, weights: torch.Tensor, k: torch.Tensor, k_scale: torch.Tensor, *,
@@ -843,49 +465,13 @@ def fp8_index(q: torch.Tensor, weights: torch.Tensor, k: torch.Tensor, k_scale: 
     first N rows of longer per-sequence caches), k_scale fp32 [B, N] or [B, N, 1]; the batch
     dimension may be missing. With causal_offset = c, keys n > m + c get -inf (the mask the
     reference adds before top-k). One launch for all sequences. Returns fp32 [B, M, N]."""
-    _require_cuda(q, weights, k, k_scale)
-    if q.dtype != torch.float8_e4m3fn or k.dtype != torch.float8_e4m3fn:
-        raise RuntimeError("fp8_index: q and k must be float8_e4m3fn")
-    m, h, d = q.shape[-3:]
-    n = k.shape[-2]
-    lead = q.shape[:-3]
-    if k.shape[:-2] != lead or len(lead) > 1:
-        raise RuntimeError("fp8_index: q [B, M, H, D] and k [B, N, D] must share at most one batch dim")
-    batch = lead[0] if lead else 1
-    q3 = q.reshape(batch, m, h, d).contiguous()
-    k3 = k.reshape(batch, n, d)
-    if k3.stride(2) != 1 or k3.stride(1) != d or (batch > 1 and k3.stride(0) % d):
-        k3 = k3.contiguous()
-    w3 = weights.reshape(batch, m, h).to(torch.float32).contiguous()
-    ks = k_scale.reshape(batch, n).to(torch.float32)
-    if ks.stride(1) != 1:
-        ks = ks.contiguous()
-    scores = torch.empty(batch, m, n, dtype=torch.float32, device=q.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_fp8_index_batched(
-        q3.data_ptr(), w3.data_ptr(), k3.data_ptr(), ks.data_ptr(), scores.data_ptr(), batch, m, h,
-        n, d, scores.stride(1), -1 if causal_offset is None else int(causal_offset),
-        (k3.stride(0) // d) if batch > 1 else n, ks.stride(0) if batch > 1 else n, scores.stride(0),
-        _stream()), "rt_fp8_index_batched")
-    return scores.reshape(*lead, m, n)
+    return _native().fp8_index(q, weights, k, k_scale, causal_offset)
 
 
 def index_topk(scores: torch.Tensor, topk: int) -> torch.Tensor:
     """Indices (int32 [..., M, min(topk, N)], ascending) of the largest scores of every row
     (racetrack/models/deepseek.py:683; the reference uses them as a set)."""
-    _require_cuda(scores)
-    if scores.dtype != torch.float32:
-        raise RuntimeError("index_topk: scores must be float32")
-    n = scores.shape[-1]
-    s2 = scores.reshape(-1, n)
-    if s2.stride(1) != 1:
-        s2 = s2.contiguous()
-    kk = min(int(topk), n)
-    out = torch.empty(s2.shape[0], kk, dtype=torch.int32, device=scores.device)
-    lib = _lib.load()
-    _lib.check(lib.rt_index_topk(s2.data_ptr(), out.data_ptr(), s2.shape[0], n, s2.stride(0), kk,
-                                 _stream()), "rt_index_topk")
-    return out.reshape(*scores.shape[:-1], kk)
+    return _native().index_topk(scores, int(topk))
 
 
 def mla_sparse_decode(q_abs: torch.Tensor, q_pe: torch.Tensor, kv_cache: torch.Tensor,
@@ -896,37 +482,7 @@ def mla_sparse_decode(q_abs: torch.Tensor, q_pe: torch.Tensor, kv_cache: torch.T
     bf16 [B, S, 512], pe_cache bf16 [B, S, 64], indices int32 [B, n_sel] of the keys each sequence
     attends to (the indexer's top-k; None = all S keys) -> bf16 [B, H, 512], the softmax-weighted
     sum of the selected latent rows."""
-    _require_cuda(q_abs)
-    for name, t in (("q_abs", q_abs), ("q_pe", q_pe), ("kv_cache", kv_cache), ("pe_cache", pe_cache)):
-        if t.dtype != torch.bfloat16 or t.dim() != 3 or t.stride(2) != 1:
-            raise RuntimeError(f"mla_sparse_decode: {name} must be bf16 [*, *, d] with a contiguous last dim")
-    batch, heads, dim = q_abs.shape
-    keys = kv_cache.shape[1]
-    if dim != 512 or kv_cache.shape[2] != 512 or q_pe.shape != (batch, heads, 64) or \
-            pe_cache.shape != (batch, keys, 64) or kv_cache.shape[0] != batch:
-        raise RuntimeError("mla_sparse_decode: shapes must be [B,H,512], [B,H,64], [B,S,512], [B,S,64]")
-    if indices is not None:
-        if indices.dtype != torch.int32 or indices.dim() != 2 or indices.shape[0] != batch:
-            raise RuntimeError("mla_sparse_decode: indices must be int32 [B, n_sel]")
-        if indices.stride(1) != 1:
-            indices = indices.contiguous()
-        n_sel = indices.shape[1]
-    else:
-        n_sel = keys
-    lib = _lib.load()
-    splits = int(lib.rt_mla_sparse_decode_splits(batch, heads, n_sel))
-    dev = q_abs.device
-    out = torch.empty(batch, heads, 512, dtype=torch.bfloat16, device=dev)
-    part_o = torch.empty(batch * splits * heads * 512, dtype=torch.float32, device=dev)
-    part_ml = torch.empty(batch * splits * heads * 2, dtype=torch.float32, device=dev)
-    _lib.check(lib.rt_mla_sparse_decode(
-        q_abs.data_ptr(), q_pe.data_ptr(), kv_cache.data_ptr(), pe_cache.data_ptr(),
-        indices.data_ptr() if indices is not None else None, out.data_ptr(), part_o.data_ptr(),
-        part_ml.data_ptr(), batch, heads, keys, n_sel, q_abs.stride(0), q_abs.stride(1),
-        q_pe.stride(0), q_pe.stride(1), kv_cache.stride(0), kv_cache.stride(1), pe_cache.stride(0),
-        pe_cache.stride(1), indices.stride(0) if indices is not None else 0, splits,
-        float(softmax_scale), _stream()), "rt_mla_sparse_decode")
-    return out
+    return _native().mla_sparse_decode(q_abs, q_pe, kv_cache, pe_cache, indices, softmax_scale)
 
 
 def attention_prefill(q: torch.Tensor, k_nope: torch.Tensor, k_pe: Optional[torch.Tensor],
