@@ -602,9 +602,8 @@ int rt_mla_sparse_decode(const void* q_abs, const void* q_pe, const void* kv, co
  *      racetrack/models/deepseek.py:780-792 (MHA prefill of MLA.forward).
  */
 /* Selects the schedule of rt_attn_causal_prefill for this process and returns the previous
- * setting: 0 = by shape and length (default), 1 = one CTA per 256 query rows with key tiles of
- * 128, 2 = CTA pairs (tcgen05 cta_group::2, 256 query rows per pair, key tiles of 256) wherever
- * the head shape is 128 + 64 / 128. */
+ * setting: 0 (default), 1 or 2. One schedule is left (one CTA per 256 query rows with key tiles
+ * of 128), so every setting runs it. */
 int rt_attn_prefill_schedule(int schedule);
 int rt_attn_causal_prefill(const void* q, const void* k_nope, const void* k_pe, const void* v,
                            void* out, int64_t tokens, int64_t heads, int64_t nope_dim,
@@ -623,7 +622,7 @@ int rt_attn_causal_prefill(const void* q, const void* k_nope, const void* k_pe, 
  * quantisation group is one head's value dims), bit for bit what rt_act_quant_fp8 makes of the
  * bf16 output of rt_attn_causal_prefill: the input of an FP8 output projection
  * (racetrack/models/deepseek.py:343-345 applied to w_o) without the [tokens, heads * 128] bf16
- * round trip. Head shape 128 + 64 / 128 only (the CTA-pair schedule).
+ * round trip. Head shape 128 + 64 / 128 only.
  */
 int rt_attn_causal_prefill_fp8(const void* q, const void* k_nope, const void* k_pe, const void* v,
                                void* out_codes, float* out_scales, int64_t tokens, int64_t heads,

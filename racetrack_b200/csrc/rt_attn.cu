@@ -527,8 +527,11 @@ __device__ long long g_fa_trace[10 * 64];
 #define RT_FTRACE(ev, it) do { } while (0)
 #endif
 
-// 0: by shape and length, 1: the single-CTA kernel, 2: CTA pairs wherever the head shape allows
-// (rt_attn_prefill_schedule; for A/B measurements and tests).
+// What rt_attn_prefill_schedule was last given. There is one schedule: the CTA pairs with key tiles
+// of 256 keys that used to take the MLA head shape from 1024 tokens on only paid while every MMA
+// cost its issuing thread 60 - 70 cycles (28 large MMAs per 256 keys instead of 40). With
+// the issuing loops behind elect_one() one B200 gives, pairs against this schedule: 8192 tokens x 128
+// heads 2643 / 2438 us, 4096 731 / 645, 2048 259 / 219, 1024 106 / 85, 777 97 / 71.
 static int g_attn_schedule = 0;
 
 struct PrefillArgs {
@@ -540,7 +543,7 @@ struct PrefillArgs {
     int one_op;                  // bit i set: operand i (q_nope, q_pe, k_nope, k_pe, v) arrives as ONE box
     int pe_shared;               // k_pe has one row per token for all heads
     float scale_log2;
-    // optional (pair schedule, v_dim 128): the output as act_quant leaves it, FP8 e4m3 codes
+    // optional (v_dim 128): the output as act_quant leaves it, FP8 e4m3 codes
     // [tokens, heads * 128] and one fp32 scale per token and head (= per 128-wide group)
     uint8_t* out_codes;
     float* out_scales;
@@ -559,54 +562,58 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return y;
 }
 
-// 2^x for x <= 8 on the FMA pipe (the special-function unit evaluates only 4 exponentials per
-// clock and scheduler, which would bound the softmax): x = n + f with n = round(x), |f| <= 1/2,
-// 2^f by a degree-4 polynomial (relative error 4e-6, far below the bf16 rounding of P), 2^n by
-// adding n to the exponent field. Inputs below -125 give 0 like ex2.approx.ftz.
-__device__ __forceinline__ float ex2_poly(float x) {
-    x = fmaxf(x, -125.f);
-    const float t = x + 12582912.f;                       // 1.5 * 2^23: the integer part lands in the low bits
-    const float f = x - (t - 12582912.f);
-    float p = fmaf(f, 9.6181291e-3f, 5.5504109e-2f);
-    p = fmaf(p, f, 2.4022651e-1f);
-    p = fmaf(p, f, 6.9314718e-1f);
-    p = fmaf(p, f, 1.0f);
-    return __uint_as_float(__float_as_uint(p) + (__float_as_uint(t) << 23));
+// 2^x of a pair for x <= 8 on the FMA pipe, two elements per instruction: x = n + f with
+// n = round(x), |f| <= 1/2, 2^f by the degree-5 minimax polynomial (Remez; relative error 2.3e-7
+// evaluated in fp32, as much as ex2.approx), 2^n by adding n to the exponent field. Inputs below
+// -125 give 0 to within 2^-125.
+__device__ __forceinline__ void ex2_poly2(uint64_t x, float& p0, float& p1) {
+    float x0, x1;
+    unpack_f32x2(x, x0, x1);
+    x = pack_f32x2(fmaxf(x0, -125.f), fmaxf(x1, -125.f));
+    const uint64_t magic = pack_f32x2(12582912.f, 12582912.f);    // 1.5 * 2^23: the integer part lands in the low bits
+    const uint64_t nmagic = pack_f32x2(-12582912.f, -12582912.f);
+    const uint64_t t = add_f32x2(x, magic);
+    const uint64_t f = fma_f32x2(add_f32x2(t, nmagic), pack_f32x2(-1.f, -1.f), x);
+    uint64_t p = fma_f32x2(f, pack_f32x2(1.3276472e-3f, 1.3276472e-3f), pack_f32x2(9.67554133e-3f, 9.67554133e-3f));
+    p = fma_f32x2(p, f, pack_f32x2(5.55071327e-2f, 5.55071327e-2f));
+    p = fma_f32x2(p, f, pack_f32x2(2.40221197e-1f, 2.40221197e-1f));
+    p = fma_f32x2(p, f, pack_f32x2(6.93146967e-1f, 6.93146967e-1f));
+    p = fma_f32x2(p, f, pack_f32x2(1.00000007f, 1.00000007f));
+    float t0, t1;
+    unpack_f32x2(t, t0, t1);
+    unpack_f32x2(p, p0, p1);
+    p0 = __uint_as_float(__float_as_uint(p0) + (__float_as_uint(t0) << 23));
+    p1 = __uint_as_float(__float_as_uint(p1) + (__float_as_uint(t1) << 23));
 }
 
-// 32 scores of one row -> 32 probabilities as 16 bf16 pairs, and their fp32 sum. One pair in
-// kFPolyEvery takes the polynomial route, the rest the special-function unit (0: none).
+// 32 scores of one row -> 32 probabilities as 16 bf16 pairs, and their fp32 sum (in two pairs of
+// partial sums). One pair in kPolyEvery takes the polynomial, the rest the special-function unit
+// (0: none take it).
+// The softmax of a tile is a chain between two MMAs, so its instructions count although neither the
+// issue slots nor the special-function unit are full: two elements per FMA and an eighth of the
+// exponentials off the special-function unit, 4096 tokens x 128 heads 717 -> 673 us, 2048 226 -> 218
+// (one pair in 4: the same; one in 2: 731; no polynomial: 709).
 #ifndef RT_FA_POLY_EVERY
-#define RT_FA_POLY_EVERY 0
+#define RT_FA_POLY_EVERY 6
 #endif
-#ifndef RT_FA_PAIR_POLY_EVERY
-#define RT_FA_PAIR_POLY_EVERY 0
-#endif
-template <int kFPolyEvery>
-__device__ __forceinline__ void softmax_chunk(const uint32_t (&r)[32], uint32_t (&pk)[16], float scale,
-                                              float m, float& sum) {
-    float acc0 = 0.f, acc1 = 0.f;
+template <int kPolyEvery>
+__device__ __forceinline__ void softmax_chunk(const uint32_t (&r)[32], uint32_t (&pk)[16], uint64_t scale,
+                                              uint64_t neg_m, uint64_t (&sum)[2]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-        const float x0 = fmaf(__uint_as_float(r[2 * i]), scale, -m);
-        const float x1 = fmaf(__uint_as_float(r[2 * i + 1]), scale, -m);
+        const uint64_t x =
+            fma_f32x2(pack_f32x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), scale, neg_m);
         float p0, p1;
-        if (kFPolyEvery > 0 && (i % (kFPolyEvery > 0 ? kFPolyEvery : 1)) == kFPolyEvery - 1) {
-            p0 = ex2_poly(x0);
-            p1 = ex2_poly(x1);
+        if (kPolyEvery > 0 && (i % (kPolyEvery > 0 ? kPolyEvery : 1)) == kPolyEvery - 1) {
+            ex2_poly2(x, p0, p1);
         } else {
-            p0 = ex2_approx(x0);
-            p1 = ex2_approx(x1);
+            unpack_f32x2(x, p0, p1);
+            p0 = ex2_approx(p0);
+            p1 = ex2_approx(p1);
         }
-#if defined(RT_FA_DIAG) && RT_FA_DIAG == 2      // diagnostic build only: no exponentials
-        p0 = x0;
-        p1 = x1;
-#endif
-        acc0 += p0;
-        acc1 += p1;
+        sum[i & 1] = add_f32x2(sum[i & 1], pack_f32x2(p0, p1));
         pk[i] = pack_bf16x2(p0, p1);
     }
-    sum += acc0 + acc1;
 }
 
 __global__ void __launch_bounds__(kFThreads, 1) attn_prefill_kernel(
@@ -849,12 +856,15 @@ __global__ void __launch_bounds__(kFThreads, 1) attn_prefill_kernel(
             }
             m_ref = m_new;
             // P = exp2(s * scale - m) as bf16 pairs into columns [32 hh, 32 hh + 32) of S_t
-            float s0 = 0.f, s1 = 0.f;
+            const uint64_t scale2 = pack_f32x2(a.scale_log2, a.scale_log2), neg_m2 = pack_f32x2(-m_new, -m_new);
+            uint64_t sums[2] = {0u, 0u};
             uint32_t pk[16];
-            softmax_chunk<RT_FA_POLY_EVERY>(r0, pk, a.scale_log2, m_new, s0);
+            softmax_chunk<RT_FA_POLY_EVERY>(r0, pk, scale2, neg_m2, sums);
             tmem_st_32x16(ts + 32u * hh, pk);
-            softmax_chunk<RT_FA_POLY_EVERY>(r1, pk, a.scale_log2, m_new, s1);
+            softmax_chunk<RT_FA_POLY_EVERY>(r1, pk, scale2, neg_m2, sums);
             tmem_st_32x16(ts + 32u * hh + 16u, pk);
+            float s0, s1;
+            unpack_f32x2(add_f32x2(sums[0], sums[1]), s0, s1);
             l += s0 + s1;
             tmem_st_wait();
             tc_fence_before();
@@ -874,6 +884,48 @@ __global__ void __launch_bounds__(kFThreads, 1) attn_prefill_kernel(
             asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
             const float inv = 1.f / (l + xl[hh ^ 1]);
             const int token = q0 + 128 * t + row;
+            if (a.out_codes != nullptr) {
+                // act_quant of the bf16 output (racetrack/models/deepseek.py:85-107) without writing
+                // it: the 128 values of this row and head (value dims of 128) are one quantisation
+                // group; its amax is the maximum of the two threads' 64 values, rounded to bf16 as
+                // the tensor would be
+                uint32_t xb[32];
+                uint32_t big = 0u;
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t o[32];
+                    tmem_ld_32x32(to + 32u * (2 * hh + c), o);
+                    tmem_ld_wait(o);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const uint32_t w = pack_bf16x2(__uint_as_float(o[2 * i]) * inv, __uint_as_float(o[2 * i + 1]) * inv);
+                        xb[16 * c + i] = w;
+                        big = absmax_bf16x2(big, w);
+                    }
+                }
+                float amax = fmaxf(0.f, fmaxf(bf16_lo(big), bf16_hi(big)));
+                float* xa = reinterpret_cast<float*>(base_ptr + kFQOff) + 512 + (t * 128 + row) * 2;   // behind the denominators
+                xa[hh] = amax;
+                asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
+                amax = fmaxf(fmaxf(amax, xa[hh ^ 1]), 1.0e-4f);
+                const float scale = __fdiv_rn(amax, 448.0f);
+                const float rscale = __frcp_rn(scale);
+                if (token < a.tokens) {
+                    uint8_t* crow = a.out_codes + (static_cast<int64_t>(token) * a.heads + h) * 128 + 64 * hh;
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const uint32_t x0 = xb[8 * v + 2 * k], x1 = xb[8 * v + 2 * k + 1];
+                            w[k] = attn_cvt_e4m3x2(div_shared(bf16_lo(x0), scale, rscale), div_shared(bf16_hi(x0), scale, rscale)) |
+                                   (attn_cvt_e4m3x2(div_shared(bf16_lo(x1), scale, rscale), div_shared(bf16_hi(x1), scale, rscale)) << 16);
+                        }
+                        *reinterpret_cast<uint4*>(crow + 16 * v) = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                    if (hh == 0) a.out_scales[static_cast<int64_t>(token) * a.heads + h] = scale;
+                }
+            } else {
             __nv_bfloat16* orow = a.out + static_cast<int64_t>(token) * a.o_ts + static_cast<int64_t>(h) * a.o_hs;
 #pragma unroll 1
             for (int c = o_half * hh; c < o_half * (hh + 1); ++c) {
@@ -895,6 +947,7 @@ __global__ void __launch_bounds__(kFThreads, 1) attn_prefill_kernel(
                     }
                 }
             }
+            }
         }
     }
     tc_fence_before();
@@ -902,384 +955,6 @@ __global__ void __launch_bounds__(kFThreads, 1) attn_prefill_kernel(
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, 512);
-    }
-}
-
-
-// ---------------------------------------------------------------------------
-// The same attention on CTA PAIRS (tcgen05 cta_group::2) with key tiles of 256 keys, for the
-// MLA head shape (128 nope + 64 rope dims, values of 128)
-// ---------------------------------------------------------------------------
-// What paces the kernel above is the thread that issues its MMAs: every tcgen05.mma costs that
-// thread about 65 cycles, every commit as much and every barrier wait about 100, whatever the
-// shape of the MMA, and a 128 x 128 x 16 MMA keeps the tensor core busy for just 64. So this
-// schedule issues larger MMAs: a pair of CTAs covers 256 query rows of one head (128 per CTA)
-// and walks key tiles of 256 keys,
-//   S = Q K^T     12 MMAs of 256 x 256 x 16 (each CTA brings its own 128 query rows as A and 128
-//                 of the tile's keys as B), 128 cycles of tensor core each;
-//   O += P V      16 MMAs of 256 x 128 x 16 (A = P from tensor memory, B = the values MN-major,
-//                 each CTA bringing 64 of the 128 value dims for all 256 keys), 64 cycles each;
-// 28 MMAs, two commits and four waits (about 2400 cycles of the issuing thread) for 2560 cycles
-// of tensor-core work per key tile, where the single-CTA schedule spends 40 MMAs on the same
-// work. Tensor memory per CTA: S 256 columns | P 128 (bf16 pairs) | O 128. P has its own columns,
-// so S(j + 1) is issued as soon as the softmax threads hold the scores of tile j in registers
-// and runs under their exponentials; O += P(j) V(j) follows when P(j) is complete. Softmax: 16
-// warps, four threads per query row with 64 scores each; the four partial maxima of a row meet
-// in shared memory as bf16. A thread writes P(j) only after O += P(j - 1) V(j - 1) has completed
-// (the same barrier tells it that O is at rest for a rescale). Shared memory per CTA: Q 48 KB,
-// two stages of its 128 keys (96 KB), two stages of its 64 value dims of 256 keys (64 KB).
-// One thread of the leader CTA (cluster rank 0) issues every MMA and commits to the barriers of
-// both CTAs; the peer's warp 1 relays "my tiles have landed" to the leader; the softmax warps of
-// both CTAs arrive on the leader's s_free and p_full. Loads never use multicast.
-constexpr uint32_t kGQOff = 0;                              // [3 chunks][128 rows][128 B]
-constexpr uint32_t kGKOff = 3 * kFChunk;                    // key stages: 2 x 3 chunks of this CTA's 128 keys
-constexpr uint32_t kGKStage = 3 * kFChunk;
-constexpr uint32_t kGVOff = kGKOff + 2 * kGKStage;          // value stages: 2 x [256 keys][64 dims]
-constexpr uint32_t kGVStage = 2 * kFChunk;
-constexpr uint32_t kGBarOff = kGVOff + 2 * kGVStage;
-constexpr int kGBars = 15;     // q_full k_full[2] v_full[2] s_done[2] pv_done[2] s_free p_full row_sync[4]
-constexpr uint32_t kGXmOff = kGBarOff + kGBars * 8 + 16;    // row maxima as bf16 [2 steps][128 rows][4]
-constexpr uint32_t kGSmemBytes = kGXmOff + 2 * 128 * 4 * 2 + 1024;
-constexpr uint32_t kGTmemP = 256, kGTmemO = 384;            // first column of P and of O
-static_assert(kGSmemBytes <= 232448, "shared memory budget");
-
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFThreads, 1) attn_prefill_pair_kernel(
-    const __grid_constant__ CUtensorMap tm_qn, const __grid_constant__ CUtensorMap tm_qp,
-    const __grid_constant__ CUtensorMap tm_kn, const __grid_constant__ CUtensorMap tm_kp,
-    const __grid_constant__ CUtensorMap tm_v, const PrefillArgs a) {
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-    const uint32_t bars = base + kGBarOff;
-    const uint32_t q_full = bars;
-    auto k_full = [&](int st) { return bars + 8u * (1 + st); };
-    auto v_full = [&](int st) { return bars + 8u * (3 + st); };
-    auto s_done = [&](int st) { return bars + 8u * (5 + st); };     // S of a key tile complete: scores
-                                                                    // readable, its key stage free
-    auto pv_done = [&](int st) { return bars + 8u * (7 + st); };    // O += P V of a key tile complete: its
-                                                                    // value stage and P free, O at rest
-    const uint32_t s_free = bars + 8u * 9, p_full = bars + 8u * 10; // used in the leader only
-    auto row_sync = [&](int quad) { return bars + 8u * (11 + quad); };  // the four warps that share query rows
-    const uint32_t slot = bars + 8u * kGBars;
-    volatile uint32_t* slot_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + kGBarOff + 8 * kGBars);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(slot_ptr + 1);
-
-    const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
-    const int rank = static_cast<int>(cluster_ctarank());
-    const int qb = static_cast<int>(gridDim.x >> 1) - 1 - static_cast<int>(blockIdx.x >> 1);   // heaviest first
-    const int h = blockIdx.y;
-    const int q0 = qb * 256;                 // first query row of the pair
-    const int n = qb + 1;                    // key tiles 0 .. qb of 256 keys; the last one is diagonal
-
-    if (threadIdx.x == 0) {
-        *abort_flag = 0;
-        const uint32_t landed = rank == 0 ? 2 : 1;          // own producer (+ the peer's relay)
-        mbar_init(q_full, landed);
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(k_full(i), landed);
-            mbar_init(v_full(i), landed);
-            mbar_init(s_done(i), 1);
-            mbar_init(pv_done(i), 1);
-        }
-        mbar_init(s_free, 32);                              // lane 0 of the 16 softmax warps of both CTAs
-        mbar_init(p_full, 32);
-        for (int i = 0; i < 4; ++i) mbar_init(row_sync(i), 4);
-        fence_mbar_init();
-        // The queries and the first two key tiles are requested here, by the thread that has just
-        // initialised the barriers they complete on (this CTA's own), so that their latency runs
-        // under the tensor-memory allocation and the cluster-wide synchronisation below instead
-        // of after them: a work item lasts some tens of microseconds and there are thousands.
-        const int pe_head0 = a.pe_shared ? 0 : h;
-        mbar_arrive_expect_tx(q_full, 3 * kFChunk);
-        tma_load_4d(base + kGQOff, &tm_qn, 0, q0 + 128 * rank, 0, h, q_full);
-        tma_load_4d(base + kGQOff + 2 * kFChunk, &tm_qp, 0, q0 + 128 * rank, 0, h, q_full);
-        for (int j = 0; j < 2 && j < n; ++j) {
-            const uint32_t dst = base + kGKOff + j * kGKStage;
-            mbar_arrive_expect_tx(k_full(j), kGKStage);
-            tma_load_4d(dst, &tm_kn, 0, 256 * j + 128 * rank, 0, h, k_full(j));
-            tma_load_4d(dst + 2 * kFChunk, &tm_kp, 0, 256 * j + 128 * rank, 0, pe_head0, k_full(j));
-        }
-        tma_prefetch_desc(&tm_v);
-    }
-    if (warp == 1) {
-        tmem_alloc_pair(slot, 512);
-        tmem_relinquish_pair();
-    }
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync();                          // the peer's barriers exist before anyone signals them
-    tc_fence_after();
-    const uint32_t tmem_base = *slot_ptr;
-
-    // The u-th use of a two-stage barrier (key tile 2 u + st) completes its phase u.
-    if (warp == 0) {
-        if (elect_one()) {
-            const int pe_head = a.pe_shared ? 0 : h;
-            bool ok = true;
-            auto load_k = [&](int j) {                         // this CTA's 128 keys of key tile j
-                const int st = j & 1;
-                if (j >= 2 && !(ok = mbar_wait(s_done(st), ((j >> 1) & 1) ^ 1u, abort_flag, 81))) return;
-                const uint32_t dst = base + kGKOff + st * kGKStage;
-                const int row = 256 * j + 128 * rank;
-                mbar_arrive_expect_tx(k_full(st), kGKStage);
-                tma_load_4d(dst, &tm_kn, 0, row, 0, h, k_full(st));
-                tma_load_4d(dst + 2 * kFChunk, &tm_kp, 0, row, 0, pe_head, k_full(st));
-            };
-            auto load_v = [&](int j) {                         // this CTA's 64 value dims of key tile j
-                const int st = j & 1;
-                if (j >= 2 && !(ok = mbar_wait(pv_done(st), ((j >> 1) & 1) ^ 1u, abort_flag, 82))) return;
-                mbar_arrive_expect_tx(v_full(st), kGVStage);
-                tma_load_4d(base + kGVOff + st * kGVStage, &tm_v, 0, 256 * j, rank, h, v_full(st));
-            };
-            // in the order the stages become free: S(j) completes after O += P(j - 2) V(j - 2)
-            // (the queries and key tiles 0 and 1 were requested before the cluster-wide set-up)
-            for (int j = 0; ok && j < n; ++j) {
-                load_v(j);
-                if (ok && j + 2 < n) load_k(j + 2);
-            }
-        }
-        __syncwarp();
-    } else if (warp == 1) {
-        if (rank == 0 && elect_one()) {
-            // fp32 accumulate, bf16 x bf16, M = 256 over the pair; S: N = 256, both K-major; O: N = 128, B MN-major
-            const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (32u << 17) | (16u << 24);
-            const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (16u << 17) | (16u << 24);
-            auto issue_s = [&](int j) {
-                const uint32_t kb = base + kGKOff + (j & 1) * kGKStage;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const uint64_t adesc = smem_desc_sw128(base + kGQOff + c * kFChunk);
-                    const uint64_t bdesc = smem_desc_sw128(kb + c * kFChunk);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        mma_f16_pair(tmem_base, adesc + 2u * k, bdesc + 2u * k, idesc_s, (c | k) != 0 ? 1u : 0u);
-                }
-                mma_commit_pair_both(s_done(j & 1));
-            };
-            auto issue_pv = [&](int j) {
-                const uint32_t vb = base + kGVOff + (j & 1) * kGVStage;
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-#if defined(RT_FA_DIAG) && RT_FA_DIAG == 3      // diagnostic build only (wrong results): B read K-major
-                    mma_f16_ts_pair(tmem_base + kGTmemO, tmem_base + kGTmemP + 8u * k,
-                                    smem_desc_sw128(vb + (k >> 2) * 8192) + 2u * (k & 3), idesc_o & ~(1u << 16),
-                                    (j | k) != 0 ? 1u : 0u);
-#elif defined(RT_FA_DIAG) && RT_FA_DIAG == 4    // diagnostic build only (wrong results): A read from shared memory
-                    mma_f16_pair(tmem_base + kGTmemO, smem_desc_sw128(base + kGQOff) + 2u * (k & 3),
-                                 smem_desc_sw128_mn(vb + k * 2048, kGVStage), idesc_o, (j | k) != 0 ? 1u : 0u);
-#else
-                    mma_f16_ts_pair(tmem_base + kGTmemO, tmem_base + kGTmemP + 8u * k,
-                                    smem_desc_sw128_mn(vb + k * 2048, kGVStage), idesc_o, (j | k) != 0 ? 1u : 0u);
-#endif
-                }
-                mma_commit_pair_both(pv_done(j & 1));
-            };
-            bool ok = mbar_wait(q_full, 0, abort_flag, 83) && mbar_wait(k_full(0), 0, abort_flag, 84);
-            if (ok) {
-                tc_fence_after();
-                issue_s(0);
-            }
-            for (int j = 0; ok && j < n; ++j) {
-                if (j + 1 < n) {
-                    RT_FTRACE(0, j);
-                    if (!(ok = mbar_wait(s_free, j & 1, abort_flag, 85))) break;
-                    if (!(ok = mbar_wait(k_full((j + 1) & 1), ((j + 1) >> 1) & 1, abort_flag, 84))) break;
-                    RT_FTRACE(1, j);
-                    tc_fence_after();
-                    issue_s(j + 1);
-                    RT_FTRACE(2, j);
-                }
-                if (!(ok = mbar_wait(p_full, j & 1, abort_flag, 86))) break;
-                RT_FTRACE(3, j);
-                if (!(ok = mbar_wait(v_full(j & 1), (j >> 1) & 1, abort_flag, 87))) break;
-                RT_FTRACE(4, j);
-                tc_fence_after();
-                issue_pv(j);
-                RT_FTRACE(5, j);
-            }
-        } else if (rank == 1 && elect_one()) {
-            // Relay: tells the leader that this CTA's tiles have landed, in the producer's order.
-            bool ok = mbar_wait(q_full, 0, abort_flag, 88);
-            if (ok) mbar_arrive_cluster(map_to_cta(q_full, 0));
-            auto relay = [&](uint32_t bar, int j) {
-                if ((ok = mbar_wait(bar, (j >> 1) & 1, abort_flag, 89))) mbar_arrive_cluster(map_to_cta(bar, 0));
-            };
-            if (ok) relay(k_full(0), 0);
-            if (ok && n > 1) relay(k_full(1), 1);
-            for (int j = 0; ok && j < n; ++j) {
-                relay(v_full(j & 1), j);
-                if (ok && j + 2 < n) relay(k_full(j & 1), j + 2);
-            }
-        }
-        __syncwarp();
-    } else {
-        const int quad = warp & 3;                            // the tensor-memory lane quarter it may touch
-        const int cq = (warp - 2) >> 2;                       // which 64 key columns of the tile
-        const int row = quad * 32 + lane;                     // query row within this CTA's tile
-        const int prow = 128 * rank + row;                    // query row within the pair's 256
-        const uint32_t row_bar = row_sync(quad);              // barrier of the four warps of these rows (a
-                                                              // bounded wait, unlike a named barrier)
-        const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
-        const uint32_t ts = tmem_base + lane_base + static_cast<uint32_t>(64 * cq);
-        const uint32_t tp = tmem_base + lane_base + kGTmemP + static_cast<uint32_t>(32 * cq);
-        const uint32_t to = tmem_base + lane_base + kGTmemO + static_cast<uint32_t>(32 * cq);
-        const uint32_t s_free_leader = map_to_cta(s_free, 0), p_leader = map_to_cta(p_full, 0);
-        const float ninf = __int_as_float(0xff800000);
-        __nv_bfloat16* xm_base = reinterpret_cast<__nv_bfloat16*>(base_ptr + kGXmOff) + row * 4;
-        float m_ref = ninf, l = 0.f;
-        bool ok = true;
-        for (int j = 0; ok && j < n; ++j) {
-            if (!(ok = mbar_wait(s_done(j & 1), (j >> 1) & 1, abort_flag, 90))) break;
-            if (threadIdx.x == 64) RT_FTRACE(6, j);
-            tc_fence_after();
-            // this thread's 64 scores in registers; then the score columns are free for the next tile
-            uint32_t r0[32], r1[32];
-            tmem_ld_32x32(ts, r0);
-            tmem_ld_32x32(ts + 32u, r1);
-            tmem_ld_wait(r0);
-            tmem_ld_wait(r1);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(s_free_leader);
-            if (threadIdx.x == 64) RT_FTRACE(7, j);
-            if (j == n - 1) {                                 // diagonal tile: keys beyond the row's own are masked
-                const int c0 = 64 * cq;
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    if (c0 + i > prow) r0[i] = 0xff800000u;
-                    if (c0 + 32 + i > prow) r1[i] = 0xff800000u;
-                }
-            }
-            float mx0 = ninf, mx1 = ninf, mx2 = ninf, mx3 = ninf;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                mx0 = fmaxf(mx0, __uint_as_float(r0[i]));
-                mx1 = fmaxf(mx1, __uint_as_float(r0[16 + i]));
-                mx2 = fmaxf(mx2, __uint_as_float(r1[i]));
-                mx3 = fmaxf(mx3, __uint_as_float(r1[16 + i]));
-            }
-            // the four threads of a row exchange their maxima as bf16, so all use the same value;
-            // the slots alternate with the step, so a fast warp cannot overwrite one still being read
-            __nv_bfloat16* xm = xm_base + (j & 1) * 512;
-            xm[cq] = __float2bfloat16_rn(fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * a.scale_log2);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(row_bar);
-            if (!(ok = mbar_wait(row_bar, j & 1, abort_flag, 93))) break;
-            const uint2 all = *reinterpret_cast<const uint2*>(xm_base + (j & 1) * 512);
-            const __nv_bfloat162 p01 = *reinterpret_cast<const __nv_bfloat162*>(&all.x);
-            const __nv_bfloat162 p23 = *reinterpret_cast<const __nv_bfloat162*>(&all.y);
-            const float mt = fmaxf(fmaxf(__low2float(p01), __high2float(p01)),
-                                   fmaxf(__low2float(p23), __high2float(p23)));
-            const bool grow = mt > m_ref + 8.f;
-            const float m_new = grow ? mt : m_ref;
-            // the probabilities first, in registers: P(j - 1) still occupies the P columns
-            float s0 = 0.f, s1 = 0.f;
-            uint32_t pk0[16], pk1[16];
-#if defined(RT_FA_DIAG) && RT_FA_DIAG == 1      // diagnostic build only (wrong results): no exponentials
-#pragma unroll
-            for (int i = 0; i < 16; ++i) { pk0[i] = r0[i]; pk1[i] = r1[i]; }
-#else
-            softmax_chunk<RT_FA_PAIR_POLY_EVERY>(r0, pk0, a.scale_log2, m_new, s0);
-            softmax_chunk<RT_FA_PAIR_POLY_EVERY>(r1, pk1, a.scale_log2, m_new, s1);
-#endif
-            if (threadIdx.x == 64) RT_FTRACE(8, j);
-            // P(j - 1) has been consumed and O is at rest once O += P(j - 1) V(j - 1) has completed
-            if (j > 0) {
-                if (!(ok = mbar_wait(pv_done((j - 1) & 1), ((j - 1) >> 1) & 1, abort_flag, 91))) break;
-                tc_fence_after();
-                if (__any_sync(0xffffffffu, grow)) {
-                    const float alpha = grow ? ex2_approx(m_ref - m_new) : 1.f;
-                    l *= alpha;
-#pragma unroll 1
-                    for (int c = 0; c < 4; ++c) {             // this thread's 32 output columns, 8 at a time
-                        uint32_t o[8];
-                        tmem_ld_32x8(to + 8u * c, o);
-                        tmem_ld_wait(o);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                        tmem_st_32x8(to + 8u * c, o);
-                    }
-                }
-            }
-            m_ref = m_new;
-            tmem_st_32x16(tp, pk0);
-            tmem_st_32x16(tp + 16u, pk1);
-            l += s0 + s1;
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(p_leader);
-            if (threadIdx.x == 64) RT_FTRACE(9, j);
-        }
-        if (ok && (ok = mbar_wait(pv_done((n - 1) & 1), ((n - 1) >> 1) & 1, abort_flag, 92))) {
-            tc_fence_after();
-            // the row's denominator is the sum of its four threads' partial sums: exchanged through
-            // the query tile's shared memory, which no MMA reads any more
-            float* xl = reinterpret_cast<float*>(base_ptr + kGQOff) + row * 4;
-            xl[cq] = l;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(row_bar);
-            ok = mbar_wait(row_bar, n & 1, abort_flag, 93);
-            const float4 ls = *reinterpret_cast<const float4*>(xl);
-            const float inv = 1.f / ((ls.x + ls.y) + (ls.z + ls.w));
-            const int token = q0 + prow;
-            uint32_t o[32];
-            tmem_ld_32x32(to, o);
-            tmem_ld_wait(o);
-            if (a.out_codes != nullptr) {
-                // act_quant of the bf16 output (racetrack/models/deepseek.py:85-107) without writing
-                // it: the 128 values of this row and head are one quantisation group; its amax is
-                // the maximum of the four threads' 32 values, rounded to bf16 as the tensor would be
-                float xb[32];
-                float amax = 0.f;
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    xb[i] = __bfloat162float(__float2bfloat16_rn(__uint_as_float(o[i]) * inv));
-                    amax = fmaxf(amax, fabsf(xb[i]));
-                }
-                float* xa = xl + 512;                         // [128 rows][4], behind the denominators
-                xa[cq] = amax;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(row_bar);
-                ok = ok && mbar_wait(row_bar, (n + 1) & 1, abort_flag, 93);
-                const float4 am = *reinterpret_cast<const float4*>(xa);
-                amax = fmaxf(fmaxf(fmaxf(am.x, am.y), fmaxf(am.z, am.w)), 1.0e-4f);
-                const float scale = __fdiv_rn(amax, 448.0f);
-                const float rscale = __frcp_rn(scale);
-                if (ok && token < a.tokens) {
-                    uint32_t w[8];
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        w[k] = attn_cvt_e4m3x2(div_shared(xb[4 * k], scale, rscale),
-                                               div_shared(xb[4 * k + 1], scale, rscale)) |
-                               (attn_cvt_e4m3x2(div_shared(xb[4 * k + 2], scale, rscale),
-                                                div_shared(xb[4 * k + 3], scale, rscale)) << 16);
-                    uint8_t* crow = a.out_codes + (static_cast<int64_t>(token) * a.heads + h) * 128 + 32 * cq;
-                    *reinterpret_cast<uint4*>(crow) = make_uint4(w[0], w[1], w[2], w[3]);
-                    *reinterpret_cast<uint4*>(crow + 16) = make_uint4(w[4], w[5], w[6], w[7]);
-                    if (cq == 0) a.out_scales[static_cast<int64_t>(token) * a.heads + h] = scale;
-                }
-            } else if (ok && token < a.tokens) {
-                __nv_bfloat16* orow = a.out + static_cast<int64_t>(token) * a.o_ts +
-                                      static_cast<int64_t>(h) * a.o_hs + 32 * cq;
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    uint4 w;
-                    w.x = pack_bf16x2(__uint_as_float(o[8 * v + 0]) * inv, __uint_as_float(o[8 * v + 1]) * inv);
-                    w.y = pack_bf16x2(__uint_as_float(o[8 * v + 2]) * inv, __uint_as_float(o[8 * v + 3]) * inv);
-                    w.z = pack_bf16x2(__uint_as_float(o[8 * v + 4]) * inv, __uint_as_float(o[8 * v + 5]) * inv);
-                    w.w = pack_bf16x2(__uint_as_float(o[8 * v + 6]) * inv, __uint_as_float(o[8 * v + 7]) * inv);
-                    *reinterpret_cast<uint4*>(orow + 8 * v) = w;
-                }
-            }
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync();     // no CTA leaves, or frees tensor memory, while its peer may still signal it
-    if (warp == 1) {
-        tc_fence_after();
-        tmem_dealloc_pair(tmem_base, 512);
     }
 }
 
@@ -1291,13 +966,13 @@ int make_tmap_bf16_4d(CUtensorMap* map, const void* ptr, const uint64_t dims[4],
 // (an SM retires about one tiled load per 500 cycles whatever its size); otherwise the row is
 // the fastest dimension and one box per chunk is issued, the part beyond dim reading as zero.
 static int make_attn_tmap(CUtensorMap* map, const void* ptr, int64_t dim, int64_t tokens, int64_t heads,
-                          int64_t ts, int64_t hs, bool* one_op, uint32_t box_rows = 128, uint32_t box_chunks = 0) {
+                          int64_t ts, int64_t hs, bool* one_op) {
     *one_op = dim % 64 == 0;
     if (*one_op) {
         const uint64_t dims[4] = {64, static_cast<uint64_t>(tokens), static_cast<uint64_t>(dim / 64),
                                   static_cast<uint64_t>(heads)};
         const uint64_t strides[3] = {static_cast<uint64_t>(ts) * 2, 128, static_cast<uint64_t>(hs) * 2};
-        const uint32_t box[4] = {64, box_rows, box_chunks ? box_chunks : static_cast<uint32_t>(dim / 64), 1};
+        const uint32_t box[4] = {64, 128, static_cast<uint32_t>(dim / 64), 1};
         return make_tmap_bf16_4d(map, ptr, dims, strides, box);
     }
     const uint64_t dims[4] = {static_cast<uint64_t>(dim), static_cast<uint64_t>(tokens), 1,
@@ -1541,23 +1216,6 @@ static int attn_causal_prefill(const void* q, const void* k_nope, const void* k_
         tm_kp = tm_kn;
     }
     a.one_op = (one[0] ? 1 : 0) | (one[1] ? 2 : 0) | (one[2] ? 4 : 0) | (one[3] ? 8 : 0) | (one[4] ? 16 : 0);
-    const bool mla_shape = nope_dim == 128 && rope_dim == 64 && v_dim == 128;
-    if (mla_shape && (out_codes || tc::g_attn_schedule == 2 || (tc::g_attn_schedule == 0 && tokens >= 1024))) {
-        // the MLA head shape on CTA pairs with key tiles of 256 keys: a CTA brings 128 keys of a
-        // tile (the boxes above) and 64 of the value dims for all of its 256 keys
-        bool ignore;
-        if (int rc = tc::make_attn_tmap(&tm_v, v, v_dim, tokens, heads, v_token_stride, v_head_stride, &ignore,
-                                        256, 1))
-            return rc;
-        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&tc::attn_prefill_pair_kernel),
-                                         static_cast<int>(tc::kGSmemBytes), "rt_attn_causal_prefill"))
-            return rc;
-        dim3 pgrid(static_cast<unsigned>(2 * ((tokens + 255) / 256)), static_cast<unsigned>(heads));
-        tc::attn_prefill_pair_kernel<<<pgrid, tc::kFThreads, tc::kGSmemBytes, as_stream(stream)>>>(
-            tm_qn, tm_qp, tm_kn, tm_kp, tm_v, a);
-        count_launch();
-        return check_launch("attn_prefill_pair_kernel");
-    }
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&tc::attn_prefill_kernel),
                                      static_cast<int>(tc::kFSmemBytes), "rt_attn_causal_prefill"))
         return rc;
