@@ -1281,10 +1281,28 @@ constexpr uint32_t kQTmemCols = 512;
 constexpr uint32_t kQIdesc = (1u << 4) | (static_cast<uint32_t>(kQBN >> 3) << 17) |
                              (static_cast<uint32_t>(kBM >> 4) << 24);
 
+// Work items: the first full_tiles output tiles whole, the tiles behind them cut along K into
+// k_splits ranges of kb_per blocks, one item each. A cut item leaves its fp32 sums in slab
+// (tile - full_tiles) * k_splits + range of the workspace (a 128 x 256 block as [64 column
+// quads][128 rows] float4, so that a warp's stores are contiguous) and fp8_tail_reduce_kernel adds
+// the ranges in order. SPLIT = false: no such tiles.
+// a_bytes: what the A box of a stage brings in (the rows there are, when fewer than 128).
+struct Fp8Item {
+    int tile, kb0, kb1;      // K blocks [kb0, kb1)
+    int slab;                // -1: a whole tile
+};
+__device__ __forceinline__ Fp8Item fp8_item(int item, int full_tiles, int k_splits, int kb_per, int num_kb) {
+    if (item < full_tiles) return {item, 0, num_kb, -1};
+    const int rel = item - full_tiles, range = rel % k_splits;
+    return {full_tiles + rel / k_splits, range * kb_per, min(num_kb, (range + 1) * kb_per), rel};
+}
+
+template <bool SPLIT>
 __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
     const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
     const float* __restrict__ a_s, const float* __restrict__ b_s, __nv_bfloat16* __restrict__ c,
-    int M, int N, int K, int64_t ldc) {
+    int M, int N, int K, int64_t ldc, uint32_t a_bytes, int num_items, int full_tiles_arg, int k_splits,
+    int kb_per, float4* __restrict__ slabs) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -1300,8 +1318,8 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
 
     const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
     const int num_m = (M + kBM - 1) / kBM, num_n = (N + kQBN - 1) / kQBN;
-    const int num_tiles = num_m * num_n;
     const int num_kb = K / kQBK;
+    const int full_tiles = SPLIT ? full_tiles_arg : num_items;
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
@@ -1331,13 +1349,14 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
+            for (int item = blockIdx.x; ok && item < num_items; item += gridDim.x) {
+                const Fp8Item it = fp8_item(item, full_tiles, k_splits, kb_per, num_kb);
                 int tm, tn;
-                tile_coords(tile, num_m, num_n, tm, tn);
-                for (int kb = 0; kb < num_kb; ++kb) {
+                tile_coords(it.tile, num_m, num_n, tm, tn);
+                for (int kb = it.kb0; kb < it.kb1; ++kb) {
                     if (!(ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, 21))) break;
                     const uint32_t sa = base + stage * kQStageBytes;
-                    mbar_arrive_expect_tx(full_bar(stage), kQStageBytes);
+                    mbar_arrive_expect_tx(full_bar(stage), a_bytes + kQBBytes);
                     tma_load_2d(sa, &tmap_a, kb * kQBK, tm * kBM, full_bar(stage));
                     tma_load_2d(sa + kQABytes, &tmap_b, kb * kQBK, tn * kQBN, full_bar(stage));
                     if (++stage == kQStages) {
@@ -1355,8 +1374,9 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
             int buf = 0;
             uint32_t buf_phase = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-                for (int kb = 0; kb < num_kb; ++kb) {
+            for (int item = blockIdx.x; ok && item < num_items; item += gridDim.x) {
+                const Fp8Item it = fp8_item(item, full_tiles, k_splits, kb_per, num_kb);
+                for (int kb = it.kb0; kb < it.kb1; ++kb) {
                     if (!(ok = mbar_wait(pempty_bar(buf), buf_phase ^ 1u, abort_flag, 22))) break;
                     if (!(ok = mbar_wait(full_bar(stage), phase, abort_flag, 23))) break;
                     tc_fence_after();
@@ -1390,9 +1410,10 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
         int buf = 0;
         uint32_t buf_phase = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
+        for (int item = blockIdx.x; ok && item < num_items; item += gridDim.x) {
+            const Fp8Item it = fp8_item(item, full_tiles, k_splits, kb_per, num_kb);
             int tm, tn;
-            tile_coords(tile, num_m, num_n, tm, tn);
+            tile_coords(it.tile, num_m, num_n, tm, tn);
             const int row = tm * kBM + quad * 32 + lane;
             const int col_base = tn * kQBN + half * 128;
             const bool live = col_base < N;                       // whole half outside the matrix?
@@ -1401,7 +1422,7 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
             float acc[128];
 #pragma unroll
             for (int i = 0; i < 128; ++i) acc[i] = 0.f;
-            for (int kb = 0; kb < num_kb; ++kb) {
+            for (int kb = it.kb0; kb < it.kb1; ++kb) {
                 const float scale = __ldg(as_row + kb) * __ldg(bs_row + kb);
                 if (!(ok = mbar_wait(pfull_bar(buf), buf_phase, abort_flag, 24))) break;
                 tc_fence_after();
@@ -1435,6 +1456,15 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
                 }
             }
             if (!ok) break;
+            if (SPLIT && it.slab >= 0) {
+                if (row < M && live) {
+                    float4* dst = slabs + (static_cast<int64_t>(it.slab) * 64 + half * 32) * 128 + quad * 32 + lane;
+#pragma unroll
+                    for (int v = 0; v < 32; ++v)
+                        dst[v * 128] = make_float4(acc[4 * v], acc[4 * v + 1], acc[4 * v + 2], acc[4 * v + 3]);
+                }
+                continue;
+            }
             if (row < M && live) {
                 __nv_bfloat16* crow = c + static_cast<int64_t>(row) * ldc + col_base;
 #pragma unroll
@@ -1455,6 +1485,28 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
         tc_fence_after();
         tmem_dealloc(tmem_base, kQTmemCols);
     }
+}
+
+// The tiles gemm_fp8_kernel<true> cut along K: c = bf16(range 0 + range 1 + ...). One CTA per 16
+// columns of a tile, one thread per row and 8 columns.
+__global__ void __launch_bounds__(256) fp8_tail_reduce_kernel(const float4* __restrict__ slabs,
+                                                              __nv_bfloat16* __restrict__ c, int M, int N,
+                                                              int64_t ldc, int full_tiles, int k_splits) {
+    const int num_m = (M + kBM - 1) / kBM, num_n = (N + kQBN - 1) / kQBN;
+    const int rel = blockIdx.x >> 4, cols = ((blockIdx.x & 15) * 2 + (threadIdx.x >> 7)) * 8;
+    int tm, tn;
+    tile_coords(full_tiles + rel, num_m, num_n, tm, tn);
+    const int row = tm * kBM + (threadIdx.x & 127), col = tn * kQBN + cols;
+    if (row >= M || col >= N) return;              // N % 8 == 0: a started vector is complete
+    const float4* src = slabs + (static_cast<int64_t>(rel) * k_splits * 64 + cols / 4) * 128 + (threadIdx.x & 127);
+    float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int s = 0; s < k_splits; ++s, src += 64 * 128) {
+        const float4 lo = __ldg(src), hi = __ldg(src + 128);
+        f[0] += lo.x; f[1] += lo.y; f[2] += lo.z; f[3] += lo.w;
+        f[4] += hi.x; f[5] += hi.y; f[6] += hi.z; f[7] += hi.w;
+    }
+    *reinterpret_cast<uint4*>(c + static_cast<int64_t>(row) * ldc + col) = pack_bf16x8(f);
 }
 
 // ---------------------------------------------------------------------------
@@ -2025,22 +2077,57 @@ static int launch_index_score(const void* q, const float* weights, const void* k
     return check_launch("index_score_kernel");
 }
 
-static int launch_fp8(const void* a, const float* a_s, const void* b, const float* b_s, void* c,
+// How rt_gemm_fp8_ws cuts a product: whole tiles for the full rounds over the SMs, the tiles of the
+// last, partial round along K, so that it takes a fraction of a round instead of a whole one with
+// most SMs idle (2048 x 7168: 448 tiles are three rounds of 148 and four tiles; a decode projection
+// is a partial round only). `splits` == 1: not cut, because half the SMs or more have a tile of the
+// round anyway or the ranges and the pass that adds them would cost what they save (0.5 us a K
+// block; a launch and the slabs, written and read at L2's pace).
+struct Fp8Plan {
+    int64_t full, splits, per;
+};
+static Fp8Plan fp8_plan(int64_t m, int64_t n, int64_t k) {
+    const int64_t tiles = ((m + kBM - 1) / kBM) * ((n + kQBN - 1) / kQBN), num_kb = k / kQBK, sms = sm_count();
+    const int64_t tail = tiles % sms;
+    Fp8Plan whole = {tiles, 1, num_kb};
+    if (tail == 0) return whole;
+    int64_t splits = std::min(sms / tail, num_kb / 3);
+    if (splits < 2) return whole;
+    const int64_t per = (num_kb + splits - 1) / splits;
+    splits = (num_kb + per - 1) / per;
+    const double slab_us = 2.0 * tail * splits * kBM * kQBN * 4 * std::min<int64_t>(m, kBM) / kBM / 6.0e6;
+    if (0.5 * per + 5.0 + slab_us >= 0.5 * num_kb) return whole;
+    return {tiles - tail, splits, per};
+}
+
+static int launch_fp8(const void* a, const float* a_s, const void* b, const float* b_s, void* c, void* workspace,
                       int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc,
                       cudaStream_t st) {
     CUtensorMap ta, tb;
-    if (int rc = make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, a, K, M, lda, kQBK, kBM)) return rc;
+    const uint32_t a_rows = a_box_rows(M);
+    if (int rc = make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, a, K, M, lda, kQBK, a_rows)) return rc;
     if (int rc = make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, b, K, N, ldb, kQBK, kQBN)) return rc;
-    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&gemm_fp8_kernel),
-                                     static_cast<int>(kQSmemBytes), "rt_gemm_fp8"))
-        return rc;
     const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + kQBN - 1) / kQBN);
-    const int grid = static_cast<int>(tiles < sm_count() ? tiles : sm_count());
-    gemm_fp8_kernel<<<grid, kQThreads, kQSmemBytes, st>>>(
+    const Fp8Plan plan = workspace ? fp8_plan(M, N, K) : Fp8Plan{tiles, 1, K / kQBK};
+    const bool split = plan.splits > 1;
+    const int64_t items = plan.full + (tiles - plan.full) * plan.splits;
+    auto kernel = split ? &gemm_fp8_kernel<true> : &gemm_fp8_kernel<false>;
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(kQSmemBytes),
+                                     "rt_gemm_fp8"))
+        return rc;
+    const int grid = static_cast<int>(items < sm_count() ? items : sm_count());
+    kernel<<<grid, kQThreads, kQSmemBytes, st>>>(
         ta, tb, a_s, b_s, static_cast<__nv_bfloat16*>(c), static_cast<int>(M), static_cast<int>(N),
-        static_cast<int>(K), ldc);
+        static_cast<int>(K), ldc, a_rows * kQBK, static_cast<int>(items), static_cast<int>(plan.full),
+        static_cast<int>(plan.splits), static_cast<int>(plan.per), static_cast<float4*>(workspace));
     count_launch();
-    return check_launch("gemm_fp8_kernel");
+    if (int rc = check_launch("gemm_fp8_kernel")) return rc;
+    if (!split) return RT_OK;
+    fp8_tail_reduce_kernel<<<static_cast<unsigned>(16 * (tiles - plan.full)), 256, 0, st>>>(
+        static_cast<const float4*>(workspace), static_cast<__nv_bfloat16*>(c), static_cast<int>(M),
+        static_cast<int>(N), ldc, static_cast<int>(plan.full), static_cast<int>(plan.splits));
+    count_launch();
+    return check_launch("fp8_tail_reduce_kernel");
 }
 
 // Schedule of the NVFP4 GEMM: 0 = by size (CTA pairs unless the work list is too short to
@@ -2105,20 +2192,39 @@ static int launch_nvfp4_pair(const void* a_codes, const void* a_sf, const float*
 
 using namespace rt;
 
-extern "C" int rt_gemm_fp8(const void* a, const float* a_scales, const void* b,
-                           const float* b_scales, void* c, int64_t m, int64_t n, int64_t k,
-                           int64_t lda, int64_t ldb, int64_t ldc, void* stream) {
+static int gemm_fp8_checked(const void* a, const float* a_scales, const void* b, const float* b_scales, void* c,
+                            void* workspace, int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb,
+                            int64_t ldc, void* stream) {
     RT_REQUIRE(m >= 0 && n > 0 && k > 0, RT_ERR_BAD_ARG, "rt_gemm_fp8: bad shape");
     if (m == 0) return RT_OK;
     RT_REQUIRE(a && a_scales && b && b_scales && c, RT_ERR_BAD_ARG, "rt_gemm_fp8: null pointer");
     RT_REQUIRE(k % 128 == 0, RT_ERR_UNSUPPORTED, "rt_gemm_fp8: k must be a multiple of 128");
     RT_REQUIRE(n % 8 == 0 && lda % 16 == 0 && ldb % 16 == 0 && ldc % 8 == 0, RT_ERR_UNSUPPORTED,
                "rt_gemm_fp8: n %% 8, lda/ldb %% 16 and ldc %% 8 are required");
-    RT_REQUIRE(aligned16(a) && aligned16(b) && aligned16(c), RT_ERR_UNSUPPORTED,
+    RT_REQUIRE(aligned16(a) && aligned16(b) && aligned16(c) && aligned16(workspace), RT_ERR_UNSUPPORTED,
                "rt_gemm_fp8: pointers must be 16-byte aligned");
     RT_REQUIRE(m < (1LL << 31) && n < (1LL << 31) && k < (1LL << 31), RT_ERR_UNSUPPORTED,
                "rt_gemm_fp8: dimension too large");
-    return tc::launch_fp8(a, a_scales, b, b_scales, c, m, n, k, lda, ldb, ldc, as_stream(stream));
+    return tc::launch_fp8(a, a_scales, b, b_scales, c, workspace, m, n, k, lda, ldb, ldc, as_stream(stream));
+}
+
+extern "C" int rt_gemm_fp8(const void* a, const float* a_scales, const void* b, const float* b_scales, void* c,
+                           int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb, int64_t ldc, void* stream) {
+    return gemm_fp8_checked(a, a_scales, b, b_scales, c, nullptr, m, n, k, lda, ldb, ldc, stream);
+}
+
+extern "C" int64_t rt_gemm_fp8_workspace_bytes(int64_t m, int64_t n, int64_t k) {
+    if (m <= 0 || n <= 0 || k <= 0 || k % 128) return 0;
+    const tc::Fp8Plan plan = tc::fp8_plan(m, n, k);
+    if (plan.splits < 2) return 0;
+    const int64_t tiles = ((m + 127) / 128) * ((n + 255) / 256);
+    return (tiles - plan.full) * plan.splits * 128 * 256 * 4;
+}
+
+extern "C" int rt_gemm_fp8_ws(const void* a, const float* a_scales, const void* b, const float* b_scales, void* c,
+                              void* workspace, int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb,
+                              int64_t ldc, void* stream) {
+    return gemm_fp8_checked(a, a_scales, b, b_scales, c, workspace, m, n, k, lda, ldb, ldc, stream);
 }
 
 static int fp8_index_checked(const void* q, const float* weights, const void* k,

@@ -294,3 +294,37 @@ def test_linear_bf16_tile_and_split_choice(ops, m, n, k, out_dtype, splits):
     if out_dtype == torch.bfloat16:
         bound += 2.0 ** -8 * ref.abs()
     assert bool(((out.double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (13, 2112, 7168),       # a decode projection: nine tiles, all of them cut, the last one narrow
+    (1, 7168, 2048),        # a box of 8 rows, one of them there
+    (129, 264, 1664),       # two row and two column tiles, nearly empty, 13 K blocks
+    (2048, 7168, 2304),     # three full rounds and four tiles, cut
+    (300, 4096, 384),       # three K blocks: whole tiles
+])
+def test_linear_fp8_tail_tiles_cut_along_k(ops, m, n, k):
+    """Tiles of a partial round over the SMs are summed in K ranges: against fp64 of the dequantised
+    operands. Per K block of 128 the products are exact in fp32 to 128 * 2^-24 of their magnitudes,
+    the scaled sums add k / 128 + ranges roundings more, bf16 rounds once."""
+    from racetrack_b200 import _lib
+    lib = _lib.load()
+    x = I.randn((m, k), 700 + m).cuda()
+    w = I.randn((n, k), 800 + n, std=0.05).cuda()
+    xc, xs = ops.fused_act_quant(x)
+    wc, ws = ops.quantize_weight_fp8(w)
+    out = ops.linear_fp8(xc, xs, wc, ws)
+    ops.tc_error_state()
+    assert torch.equal(out, ops.linear_fp8(xc, xs, wc, ws)), "must be bit-reproducible"
+    a = xc.double() * xs.double().repeat_interleave(128, dim=1)
+    b = wc.double() * ws.double().repeat_interleave(128, dim=0)[:n].repeat_interleave(128, dim=1)
+    bound = (256 + k // 64) * 2.0 ** -24 * (a.abs() @ b.abs().t()) + 2.0 ** -8 * (a @ b.t()).abs()
+    assert bool(((out.double() - a @ b.t()).abs() <= bound).all())
+    # whole tiles only: the same sums in one range
+    whole = torch.empty_like(out)
+    _lib.check(lib.rt_gemm_fp8(xc.data_ptr(), xs.data_ptr(), wc.data_ptr(), ws.data_ptr(), whole.data_ptr(), m, n,
+                               k, k, k, n, torch.cuda.current_stream().cuda_stream), "rt_gemm_fp8")
+    if int(lib.rt_gemm_fp8_workspace_bytes(m, n, k)) == 0:
+        assert torch.equal(out, whole)
+    else:
+        assert bool(((out.double() - whole.double()).abs() <= 2 * bound).all())
