@@ -484,6 +484,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBPThreads, 1) gemm_
 // tcgen05.st per warp and stage; every smem stage owns 32 scale columns, so the copy of stage
 // s+1 runs while the MMAs of stage s execute. (Issuing the eight tcgen05.cp per stage from the
 // MMA thread instead serialised with the MMAs and cost a third of the kernel time.)
+// The A box of a tile has the smallest of 8, 16, ... 128 rows that covers the tile's valid ones: with
+// few rows per group the kernel streams weights, and a box of 128 rows that are mostly zero fill
+// (past the last row of all) held the copies back. The rows of the stage behind the box hold old
+// codes; their scales are zero and they have no output row. 256 experts, w2 / w13 on one B200:
+// 13 tokens 219 -> 120 / 229 -> 228 us, 4 tokens 68 -> 46 / 124 -> 83, 1 token 21 -> 15 / 42 -> 28.
+// (Two K blocks per copy and stage, 3 stages: 2 - 3 % slower where HBM is the bound.)
 // Warps: 0 TMA producer, 1 MMA issuer, 2-5 epilogue, 6-9 scale loaders.
 constexpr int kFBN = 128;                          // tile columns
 constexpr int kFBK = 256;                          // K elements per stage
@@ -500,8 +506,14 @@ constexpr uint32_t kFTmemSf = 256;                 // first scale column
 constexpr uint32_t kFIdesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kFBN >> 3) << 17) |
                              (static_cast<uint32_t>(kBM >> 4) << 24);
 
+// Token-row tensor maps with boxes of 8 << b rows: the kernels pick the smallest that covers
+// the rows (this one) or half the rows (the CTA pairs) of a tile.
+struct TokenMaps {
+    CUtensorMap box[5];
+};
+
 __global__ void __launch_bounds__(kFThreads, 1) gemm_nvfp4_kernel(
-    const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+    const __grid_constant__ TokenMaps tmaps_a, const __grid_constant__ CUtensorMap tmap_b,
     const uint8_t* __restrict__ sfa, const uint8_t* __restrict__ sfb,
     const float* __restrict__ a_gs, const float* __restrict__ b_gs, __nv_bfloat16* __restrict__ c,
     const int4* __restrict__ tile_map, const int* __restrict__ tile_count, int N, int K,
@@ -540,7 +552,7 @@ __global__ void __launch_bounds__(kFThreads, 1) gemm_nvfp4_kernel(
             mbar_init(tempty_bar(a), 128);
         }
         fence_mbar_init();
-        tma_prefetch_desc(&tmap_a);
+        tma_prefetch_desc(&tmaps_a.box[0]);
         tma_prefetch_desc(&tmap_b);
     }
     if (warp == 1) {
@@ -563,11 +575,14 @@ __global__ void __launch_bounds__(kFThreads, 1) gemm_nvfp4_kernel(
                 const uint8_t* sfa_t = sfa + static_cast<int64_t>(tm.w) * kt * 512;
                 const uint8_t* sfb_t =
                     sfb + (static_cast<int64_t>(tm.x) * n_row_tiles + tn) * kt * 512;
+                int b = 0;                                  // box of 8 << b rows
+                while ((8 << b) < tm.z) ++b;
+                const uint32_t tx = (1024u << b) + kFTileBytes + 2 * kFSfBytes;
                 for (int kb = 0; kb < num_kb; ++kb) {
                     if (!(ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, 11))) break;
                     const uint32_t sa = base + stage * kFStageBytes;
-                    mbar_arrive_expect_tx(full_bar(stage), kFStageBytes);
-                    tma_load_2d(sa, &tmap_a, kb * 128, tm.y, full_bar(stage));
+                    mbar_arrive_expect_tx(full_bar(stage), tx);
+                    tma_load_2d(sa, &tmaps_a.box[b], kb * 128, tm.y, full_bar(stage));
                     tma_load_2d(sa + kFTileBytes, &tmap_b, kb * 128, tm.x * N + tn * kFBN,
                                 full_bar(stage));
                     bulk_load(sa + 2 * kFTileBytes, sfa_t + static_cast<int64_t>(kb) * kFSfBytes,
@@ -766,10 +781,6 @@ constexpr uint32_t kPSfStageCols = 2 * kPSfCols;   // per operand stage (two K b
 static_assert(kPStageBytes % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
 static_assert(kPTmemSf + 2 * kPSfStageCols <= kPTmemCols, "tensor memory budget");
 static_assert(kPSmemBytes <= 232448, "shared memory budget");
-
-struct TokenMaps {
-    CUtensorMap box[5];     // the token operand with boxes of 8, 16, 32, 64 and 128 rows
-};
 
 // Optional pipeline trace (never compiled into the library): with -DRT_PAIR_TRACE the leader
 // CTA of pair 0 stamps clock64() at eight points of its first 128 K blocks.
@@ -2141,10 +2152,13 @@ static int launch_nvfp4_single(const void* a_codes, const void* a_sf, const floa
                                const int32_t* tile_map, const int32_t* tile_count,
                                int64_t max_m_tiles, int64_t total_rows, int64_t groups, int64_t N,
                                int64_t K, int64_t ldc, cudaStream_t st) {
-    CUtensorMap ta, tb;
-    if (int rc = make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, a_codes, K / 2, total_rows,
-                              K / 2, 128, kBM))
-        return rc;
+    CUtensorMap tb;
+    TokenMaps ta;
+    for (int b = 0; b < 5; ++b) {
+        if (int rc = make_tmap_2d(&ta.box[b], CU_TENSOR_MAP_DATA_TYPE_UINT8, a_codes, K / 2, total_rows,
+                                  K / 2, 128, 8u << b))
+            return rc;
+    }
     if (int rc = make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, b_codes, K / 2, groups * N, K / 2,
                               128, kFBN))
         return rc;

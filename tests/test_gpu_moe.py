@@ -159,3 +159,44 @@ def test_moe_gather_nvfp4_equals_gather_fused_quantiser(mods, tokens, hidden, n_
     assert_bit_exact(codes, ref_codes, "codes")
     used = int(tile_count[0]) * (hidden // 64) * 512
     assert_bit_exact(sf[:used], ref_sf[:used], "tiled scales")
+
+
+@pytest.mark.parametrize("rows", [[1], [8, 9], [16, 0, 17], [64, 65, 33], [128, 129, 1], [3, 255]])
+def test_grouped_gemm_token_box_fits_the_rows(mods, rows):
+    """Groups around the sizes of the token box (8, 16, ... 128 rows) on the single-CTA schedule, with
+    other groups' rows behind each: against fp64 of the dequantised operands. Sums of K exact e2m1
+    products times two e4m3 scales: K * 2^-24 of their magnitudes, bf16 rounds once."""
+    ops, moe = mods
+    groups, n, k = len(rows), 128, 512
+    g = torch.Generator().manual_seed(sum(rows))
+    total = sum(rows)
+    x = torch.randn(total, k, generator=g).bfloat16().cuda()
+    w = (torch.randn(groups, n, k, generator=g) * 0.1).bfloat16().cuda()
+    offsets = torch.tensor([sum(rows[:i]) for i in range(groups + 1)], dtype=torch.int32, device="cuda")
+    max_tiles = (total + 127) // 128 + groups
+    tile_map, _, tile_count = ops.moe_tile_map(offsets, 0, groups, max_tiles)
+    a_codes, a_sf, a_gs = moe.moe_quant_nvfp4(x, tile_map, tile_count, total, amax=ops.tensor_absmax(x))
+    parts = [ops.fused_nvfp4_quant(w[i], tiled_scales=True) for i in range(groups)]
+    prev = ops.gemm_nvfp4_schedule(1)
+    try:
+        out = ops.gemm_nvfp4_grouped(a_codes, a_sf, a_gs, torch.cat([p[0] for p in parts]),
+                                     torch.cat([p[1].view(torch.uint8) for p in parts]),
+                                     torch.cat([p[2] for p in parts]), tile_map, tile_count, n=n, groups=groups)
+    finally:
+        ops.gemm_nvfp4_schedule(prev)
+    ops.tc_error_state()
+
+    def dequant(t, amax):
+        codes, sf, gs = (v.cpu() for v in ops.fused_nvfp4_quant(t, amax=amax))
+        table = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0])
+        table = torch.cat([table, -table]).double()
+        both = torch.stack([codes & 15, codes >> 4], dim=-1).reshape(t.shape[0], -1).long()
+        return table[both] * sf.double().repeat_interleave(16, dim=1) * gs.double()
+    a = dequant(x, ops.tensor_absmax(x))
+    lo = 0
+    for i, r in enumerate(rows):
+        b = dequant(w[i], ops.tensor_absmax(w[i]))
+        ref = a[lo:lo + r] @ b.t()
+        bound = 2 * k * 2.0 ** -24 * (a[lo:lo + r].abs() @ b.abs().t()) + 2.0 ** -8 * ref.abs()
+        assert bool(((out[lo:lo + r].cpu().double() - ref).abs() <= bound).all()), (i, r)
+        lo += r
