@@ -212,6 +212,14 @@ int rt_swiglu_absmax_rows(const void* gate, const void* up, void* h, float* amax
                           int64_t rows, int64_t cols, int64_t gate_stride, int64_t up_stride,
                           int64_t h_stride, const int32_t* row_begin, const int32_t* row_end,
                           int dtype, void* stream);
+/* rt_absmax of x, and rt_swiglu_absmax_rows, onto a start value: *amax = max(*amax, max |.|) of a
+ * non-negative *amax the caller has set (no launch of their own to clear it). */
+int rt_absmax_onto(const void* x, float* amax, int64_t rows, int64_t cols, int64_t x_stride,
+                   int dtype, void* stream);
+int rt_swiglu_absmax_rows_onto(const void* gate, const void* up, void* h, float* amax, int64_t rows,
+                               int64_t cols, int64_t gate_stride, int64_t up_stride,
+                               int64_t h_stride, const int32_t* row_begin, const int32_t* row_end,
+                               int dtype, void* stream);
 
 /* Block-scale layouts for NVFP4 */
 typedef enum rt_sf_layout {
@@ -318,6 +326,17 @@ int64_t rt_moe_permute_workspace_bytes(int64_t tokens, int64_t topk, int64_t n_e
 int rt_moe_permute(const int64_t* indices, int32_t* expert_offsets,
                    int32_t* sorted_pairs, int32_t* pair_pos, void* workspace,
                    int64_t tokens, int64_t topk, int64_t n_experts, void* stream);
+
+/*
+ * rt_moe_permute, then rt_moe_tile_map of the experts [g_begin, g_end) on its offsets, and zero into
+ * the two floats of amax2 (may be NULL; the start of rt_absmax_onto / rt_swiglu_absmax_rows_onto):
+ * what a routed expert MLP needs before its first GEMM, in one launch for up to 1024 pairs.
+ * ref: racetrack/models/deepseek.py:1011-1018.
+ */
+int rt_moe_plan(const int64_t* indices, int32_t* expert_offsets, int32_t* sorted_pairs,
+                int32_t* pair_pos, void* workspace, int32_t* tile_map, int32_t* tile_base,
+                int32_t* tile_count, float* amax2, int64_t max_tiles, int64_t g_begin,
+                int64_t g_end, int64_t tokens, int64_t topk, int64_t n_experts, void* stream);
 
 /*
  * rt_moe_permute for callers that have no scratch memory to hand over and must not trigger

@@ -39,6 +39,9 @@ SIGNATURES: dict[str, tuple] = {
     "rt_moe_route": (_I, [_P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _F, _I, _P]),
     "rt_moe_permute_workspace_bytes": (_L, [_L, _L, _L]),
     "rt_moe_permute": (_I, [_P, _P, _P, _P, _P, _L, _L, _L, _P]),
+    "rt_moe_plan": (_I, [_P] * 9 + [_L] * 6 + [_P]),
+    "rt_absmax_onto": (_I, [_P, _P, _L, _L, _L, _I, _P]),
+    "rt_swiglu_absmax_rows_onto": (_I, [_P, _P, _P, _P, _L, _L, _L, _L, _L, _P, _P, _I, _P]),
     "rt_moe_permute_static_max_ints": (_L, []),
     "rt_moe_permute_static": (_I, [_P, _P, _P, _P, _L, _L, _L, _P]),
     "rt_moe_gather": (_I, [_P, _P, _P, _L, _L, _L, _L, _I, _P]),

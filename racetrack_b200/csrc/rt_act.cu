@@ -340,7 +340,9 @@ __global__ void __launch_bounds__(kActThreads) quant_nvfp4_kernel(
 // tile's own 128-row scale tiles, rows of the tile beyond `valid rows` get zero scales.
 // With sorted_pairs the source row of destination row r is sorted_pairs[r] / topk (the
 // token gather of the MoE dispatch fused into the quantiser); otherwise source = destination.
-// Grid: 16 CTAs per tile, each doing 8 rows.
+// Grid: 16 CTAs per tile, each doing 8 rows and a sixteenth of the tile's scale tiles' zeros. With a
+// row or two per tile the zeros are most of the stores (13 tokens of 256 experts, 104 rows x 7168 on
+// one B200: 14 us as bytes or words of a row, 9 as 16 bytes a lane; h of 64 tokens 13 -> 7).
 template <bool UP>
 __global__ void __launch_bounds__(kActThreads) quant_nvfp4_tiles_kernel(
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ up,
@@ -359,23 +361,40 @@ __global__ void __launch_bounds__(kActThreads) quant_nvfp4_tiles_kernel(
     const float six_gs = __fmul_rn(6.0f, gs);
     const uint32_t kt = items_per_row >> 2;
     uint8_t* sf_tile = sf + static_cast<int64_t>(tm.w) * kt * 512;
-    for (uint32_t it = threadIdx.x; it < 8u * items_per_row; it += kActThreads) {
+    const uint32_t row0 = sub * 8u;
+    const uint32_t valid = static_cast<uint32_t>(min(8, max(0, tm.z - static_cast<int>(row0))));
+    for (uint32_t it = threadIdx.x; it < valid * items_per_row; it += kActThreads) {
         const uint32_t rr = it / items_per_row;
         const uint32_t blk = it - rr * items_per_row;
-        const uint32_t r_local = sub * 8u + rr;
-        uint8_t* sf_dst = sf_tile + static_cast<int64_t>(blk >> 2) * 512 + (r_local & 31u) * 16u +
-                          (r_local >> 5) * 4u + (blk & 3u);
-        if (static_cast<int>(r_local) >= tm.z) {
-            *sf_dst = 0;
-            continue;
-        }
+        const uint32_t r_local = row0 + rr;
         const int64_t dst_row = tm.y + r_local;
         const int64_t src_row = sorted_pairs ? (__ldg(sorted_pairs + dst_row) / topk) : dst_row;
         const int64_t col = static_cast<int64_t>(blk) * kItem;
         uint32_t v[8], bs;
         load_item<UP>(x, up, src_row, col, xstride, ustride, v);
         st_stream8(codes + dst_row * (cols >> 1) + (col >> 1), quant_item_nvfp4(v, gs, six_gs, bs));
-        *sf_dst = static_cast<uint8_t>(bs);
+        // four neighbouring lanes hold the four scales of one 64-column group of the row (a row has a
+        // multiple of four blocks): one 4-byte store
+        const uint32_t quad = 0xfu << (threadIdx.x & 28u);
+        bs <<= 8 * (blk & 3u);
+        bs |= __shfl_xor_sync(quad, bs, 1);
+        bs |= __shfl_xor_sync(quad, bs, 2);
+        if ((blk & 3u) == 0)
+            *reinterpret_cast<uint32_t*>(sf_tile + static_cast<int64_t>(blk >> 2) * 512 + (r_local & 31u) * 16u +
+                                         (r_local >> 5) * 4u) = bs;
+    }
+    // rows past the tile's valid ones: zero scales. A warp per 512-byte scale tile, lane l the 16 bytes
+    // of rows l, l + 32, l + 64, l + 96.
+    const int lane = threadIdx.x & 31;
+    for (uint32_t k = sub * (kActThreads / 32) + (threadIdx.x >> 5); k < kt; k += 16 * (kActThreads / 32)) {
+        uint32_t* dst = reinterpret_cast<uint32_t*>(sf_tile + static_cast<int64_t>(k) * 512 + lane * 16);
+        if (lane >= tm.z) {
+            *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+        } else {
+#pragma unroll
+            for (int j = 1; j < 4; ++j)
+                if (lane + 32 * j >= tm.z) dst[j] = 0u;
+        }
     }
 }
 
@@ -524,7 +543,7 @@ extern "C" int rt_swiglu_quant_fp8(const void* gate, const void* up, void* codes
 static int absmax_common(const void* x, const void* up, float* amax_out, int64_t rows,
                          int64_t cols, int64_t x_stride, int64_t up_stride,
                          const int32_t* row_begin, const int32_t* row_end, int dtype,
-                         void* stream, void* h = nullptr, int64_t h_stride = 0) {
+                         void* stream, bool clear, void* h = nullptr, int64_t h_stride = 0) {
     uint32_t items, per_row;
     if (int rc = check_stream_args("rt_absmax", x, rows, cols, x_stride, 16, dtype, items, per_row,
                                    kItem))
@@ -533,9 +552,12 @@ static int absmax_common(const void* x, const void* up, float* amax_out, int64_t
     if (up) RT_REQUIRE(up_stride % 8 == 0 && aligned16(up), RT_ERR_UNSUPPORTED,
                        "rt_absmax: up must be 16-byte aligned with stride %% 8 == 0");
     cudaStream_t st = as_stream(stream);
-    absmax_clear_kernel<<<1, 1, 0, st>>>(amax_out);
-    count_launch();
-    if (items == 0) return check_launch("absmax_clear_kernel");
+    if (clear) {
+        absmax_clear_kernel<<<1, 1, 0, st>>>(amax_out);
+        count_launch();
+        if (int rc = check_launch("absmax_clear_kernel")) return rc;
+    }
+    if (items == 0) return RT_OK;
     // persistent grid: 148 SMs x 8 resident CTAs, each thread loops over items
     unsigned grid = (items + kActThreads - 1) / kActThreads;
     if (grid > 148u * 8u) grid = 148u * 8u;
@@ -559,7 +581,7 @@ extern "C" int rt_absmax(const void* x, const void* up, float* amax_out, int64_t
                          int64_t cols, int64_t x_stride, int64_t up_stride, int dtype,
                          void* stream) {
     return absmax_common(x, up, amax_out, rows, cols, x_stride, up_stride, nullptr, nullptr, dtype,
-                         stream);
+                         stream, true);
 }
 
 extern "C" int rt_absmax_rows(const void* x, const void* up, float* amax_out, int64_t rows,
@@ -567,10 +589,10 @@ extern "C" int rt_absmax_rows(const void* x, const void* up, float* amax_out, in
                               const int32_t* row_begin, const int32_t* row_end, int dtype,
                               void* stream) {
     return absmax_common(x, up, amax_out, rows, cols, x_stride, up_stride, row_begin, row_end,
-                         dtype, stream);
+                         dtype, stream, true);
 }
 
-extern "C" int rt_swiglu_absmax_rows(const void* gate, const void* up, void* h, float* amax_out,
+static int swiglu_absmax_common(bool clear, const void* gate, const void* up, void* h, float* amax_out,
                                      int64_t rows, int64_t cols, int64_t gate_stride,
                                      int64_t up_stride, int64_t h_stride,
                                      const int32_t* row_begin, const int32_t* row_end, int dtype,
@@ -579,7 +601,27 @@ extern "C" int rt_swiglu_absmax_rows(const void* gate, const void* up, void* h, 
     RT_REQUIRE(h_stride % 8 == 0 && aligned16(h), RT_ERR_UNSUPPORTED,
                "rt_swiglu_absmax_rows: h must be 16-byte aligned with stride %% 8 == 0");
     return absmax_common(gate, up, amax_out, rows, cols, gate_stride, up_stride, row_begin, row_end,
-                         dtype, stream, h, h_stride);
+                         dtype, stream, clear, h, h_stride);
+}
+
+extern "C" int rt_swiglu_absmax_rows(const void* gate, const void* up, void* h, float* amax_out, int64_t rows,
+                                     int64_t cols, int64_t gate_stride, int64_t up_stride, int64_t h_stride,
+                                     const int32_t* row_begin, const int32_t* row_end, int dtype, void* stream) {
+    return swiglu_absmax_common(true, gate, up, h, amax_out, rows, cols, gate_stride, up_stride, h_stride,
+                                row_begin, row_end, dtype, stream);
+}
+
+extern "C" int rt_swiglu_absmax_rows_onto(const void* gate, const void* up, void* h, float* amax, int64_t rows,
+                                          int64_t cols, int64_t gate_stride, int64_t up_stride, int64_t h_stride,
+                                          const int32_t* row_begin, const int32_t* row_end, int dtype,
+                                          void* stream) {
+    return swiglu_absmax_common(false, gate, up, h, amax, rows, cols, gate_stride, up_stride, h_stride, row_begin,
+                                row_end, dtype, stream);
+}
+
+extern "C" int rt_absmax_onto(const void* x, float* amax, int64_t rows, int64_t cols, int64_t x_stride, int dtype,
+                              void* stream) {
+    return absmax_common(x, nullptr, amax, rows, cols, x_stride, 0, nullptr, nullptr, dtype, stream, false);
 }
 
 extern "C" int rt_moe_quant_nvfp4(const void* x, const void* up, const int32_t* sorted_pairs,
@@ -597,7 +639,8 @@ extern "C" int rt_moe_quant_nvfp4(const void* x, const void* up, const int32_t* 
     RT_REQUIRE(cols % 64 == 0, RT_ERR_UNSUPPORTED,
                "rt_moe_quant_nvfp4: cols must be a multiple of 64 (whole scale tiles)");
     RT_REQUIRE(x_stride % 8 == 0 && aligned16(x) && (!up || (up_stride % 8 == 0 && aligned16(up))) &&
-                   aligned16(tile_map) && (reinterpret_cast<uintptr_t>(codes) & 7u) == 0,
+                   aligned16(tile_map) && (reinterpret_cast<uintptr_t>(codes) & 7u) == 0 &&
+                   aligned16(block_scales),
                RT_ERR_UNSUPPORTED, "rt_moe_quant_nvfp4: alignment (16-byte inputs, stride %% 8)");
     RT_REQUIRE(max_tiles < (1LL << 27), RT_ERR_UNSUPPORTED, "rt_moe_quant_nvfp4: too many tiles");
     const unsigned grid = static_cast<unsigned>(max_tiles * 16);

@@ -8,6 +8,7 @@
 // Permutation: counting sort in three small launches (per-block histograms,
 // scan, stable scatter); positions are a pure function of the indices, so the
 // result is deterministic and equal to what a per-expert torch.where loop yields.
+#include <algorithm>
 #include <mutex>
 
 #include "rt_common.cuh"
@@ -257,6 +258,110 @@ __global__ void __launch_bounds__(kPermThreads) moe_scatter_kernel(
     }
 }
 
+// The three passes above and the work lists of the grouped GEMMs (moe_tile_map_kernel) for at most
+// one block's worth of pairs, in one launch: a decode step sorts 8 - 1024 pairs, four dependent
+// kernels of 2 - 4 us each before its experts may start. Also sets amax2[0..1] to zero, the start
+// of the two abs-max passes that follow. Same outputs as the separate kernels.
+__global__ void __launch_bounds__(kPermThreads) moe_plan_kernel(
+    const int64_t* __restrict__ indices, int32_t* __restrict__ expert_offsets,
+    int32_t* __restrict__ sorted_pairs, int32_t* __restrict__ pair_pos, int n_pairs, int n_experts,
+    int g_begin, int g_end, int4* __restrict__ tile_map, int32_t* __restrict__ tile_base,
+    int32_t* __restrict__ tile_count, int max_tiles, float* __restrict__ amax2) {
+    extern __shared__ int plan_smem[];
+    int* base = plan_smem;                                                       // [n_experts + 1]
+    unsigned short* wc = reinterpret_cast<unsigned short*>(plan_smem + n_experts + 1);   // [warps][n_experts]
+    __shared__ long long warp_tot[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // the block has a thread for every pair and every expert; `warps` hold pairs
+    const int block_warps = blockDim.x >> 5, warps = (n_pairs + 31) >> 5;
+    if (tid < 2 && amax2) amax2[tid] = 0.f;
+    for (int i = tid; i < warps * n_experts; i += blockDim.x) wc[i] = 0;
+    __syncthreads();
+    int e = -1;
+    if (tid < n_pairs) {
+        e = static_cast<int>(indices[tid]);
+        if (e < 0 || e >= n_experts) e = -1;
+    }
+    // invalid lanes get unique keys so they match nobody
+    const unsigned peers = __match_any_sync(0xffffffffu, e >= 0 ? e : n_experts + lane);
+    const int rank = __popc(peers & ((1u << lane) - 1u));
+    if (e >= 0 && rank == 0) wc[warp * n_experts + e] = static_cast<unsigned short>(__popc(peers));
+    __syncthreads();
+    // block-wide exclusive scan (one value per thread); returns the total through `all`
+    auto scan = [&](long long v, long long& all) {
+        long long incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) warp_tot[warp] = incl;
+        __syncthreads();
+        long long before = 0;
+        all = 0;
+        for (int w = 0; w < block_warps; ++w) {
+            before += w < warp ? warp_tot[w] : 0;
+            all += warp_tot[w];
+        }
+        __syncthreads();
+        return before + incl - v;
+    };
+    int total = 0;
+    if (tid < n_experts) {
+        for (int w = 0; w < warps; ++w) {
+            const int c = wc[w * n_experts + tid];
+            wc[w * n_experts + tid] = static_cast<unsigned short>(total);
+            total += c;
+        }
+    }
+    long long all;
+    const int excl = static_cast<int>(scan(total, all));
+    if (tid < n_experts) {
+        base[tid] = excl;
+        expert_offsets[tid] = excl;
+    }
+    if (tid == 0) {
+        base[n_experts] = static_cast<int>(all);
+        expert_offsets[n_experts] = static_cast<int>(all);
+    }
+    __syncthreads();
+    if (e >= 0) {
+        const int dest = base[e] + wc[warp * n_experts + e] + rank;
+        sorted_pairs[dest] = tid;
+        pair_pos[tid] = dest;
+    }
+    // tiles of the groups: 128-row ones counted in the low word, wide ones in the high word
+    const int groups = g_end - g_begin;
+    int row0 = 0, rows = 0;
+    if (tid < groups) {
+        row0 = base[g_begin + tid];
+        rows = base[g_begin + tid + 1] - row0;
+    }
+    const int ntile = (rows + 127) / 128, nwide = (rows + 255) / 256;
+    const long long first64 = scan(static_cast<long long>(ntile) | (static_cast<long long>(nwide) << 32), all);
+    if (tid < groups) {
+        const int first = static_cast<int>(first64 & 0xffffffffLL), wfirst = static_cast<int>(first64 >> 32);
+        tile_base[tid] = first;
+        for (int t = 0; t < ntile; ++t) {
+            if (first + t < max_tiles)
+                tile_map[first + t] = make_int4(tid, row0 + t * 128, min(128, rows - t * 128), first + t);
+        }
+        for (int t = 0; t < nwide; ++t) {
+            if (wfirst + t < max_tiles)
+                tile_map[max_tiles + wfirst + t] =
+                    make_int4(tid, row0 + t * 256, min(256, rows - t * 256), first + 2 * t);
+        }
+    }
+    if (tid == 0) {
+        const int tiles = static_cast<int>(all & 0xffffffffLL);
+        tile_base[groups] = tiles;
+        tile_count[0] = min(tiles, max_tiles);
+        tile_count[1] = min(static_cast<int>(all >> 32), max_tiles);
+    }
+}
+
+__global__ void zero2_kernel(float* v) { v[threadIdx.x] = 0.f; }
+
 // ---------------------------------------------------------------------------
 // Gather / combine
 // ---------------------------------------------------------------------------
@@ -282,19 +387,33 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(
     // a window given in device memory (expert offsets of this rank) overrides the host values
     if (pos_begin_ptr) pos_begin = __ldg(pos_begin_ptr);
     if (pos_end_ptr) pos_end = __ldg(pos_end_ptr);
-    for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
+    for (int v = blockIdx.y * blockDim.x + threadIdx.x; v < nvec; v += gridDim.y * blockDim.x) {
         float acc[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) acc[k] = 0.f;
-        for (int s = 0; s < topk; ++s) {
-            const int pos = __ldg(pair_pos + t * topk + s);
-            if (pos < pos_begin || pos >= pos_end) continue;
-            const float w = __ldg(weights + t * topk + s);
-            float f[8];
-            unpack_bf16x8(
-                ld_stream16(reinterpret_cast<const uint4*>(expert_out) + (int64_t)pos * nvec + v), f);
+        // eight slots at a time: their rows are asked for before the first is used, in slot order
+        for (int s0 = 0; s0 < topk; s0 += 8) {
+            uint4 raw[8];
+            float w[8];
+            bool mine[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) acc[k] = __fadd_rn(acc[k], __fmul_rn(f[k], w));
+            for (int i = 0; i < 8; ++i) {
+                mine[i] = false;
+                if (s0 + i < topk) {
+                    const int pos = __ldg(pair_pos + t * topk + s0 + i);
+                    w[i] = __ldg(weights + t * topk + s0 + i);
+                    mine[i] = pos >= pos_begin && pos < pos_end;
+                    if (mine[i]) raw[i] = ld_stream16(reinterpret_cast<const uint4*>(expert_out) + (int64_t)pos * nvec + v);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (!mine[i]) continue;
+                float f[8];
+                unpack_bf16x8(raw[i], f);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) acc[k] = __fadd_rn(acc[k], __fmul_rn(f[k], w[i]));
+            }
         }
         if (shared) {
             float f[8];
@@ -649,6 +768,42 @@ extern "C" int rt_moe_permute(const int64_t* indices, int32_t* expert_offsets,
     return RT_OK;
 }
 
+extern "C" int rt_moe_plan(const int64_t* indices, int32_t* expert_offsets, int32_t* sorted_pairs,
+                           int32_t* pair_pos, void* workspace, int32_t* tile_map, int32_t* tile_base,
+                           int32_t* tile_count, float* amax2, int64_t max_tiles, int64_t g_begin,
+                           int64_t g_end, int64_t tokens, int64_t topk, int64_t n_experts, void* stream) {
+    RT_REQUIRE(tokens >= 0 && topk > 0 && n_experts > 0, RT_ERR_BAD_ARG, "rt_moe_plan: bad shape");
+    cudaStream_t st = as_stream(stream);
+    // one launch while the pairs fit the block and the groups are experts of its scan
+    if (tokens * topk > 0 && tokens * topk <= kPermThreads && n_experts <= 1024 && g_begin >= 0 && g_end > g_begin &&
+        g_end <= n_experts && max_tiles > 0) {
+        RT_REQUIRE(indices && expert_offsets && sorted_pairs && pair_pos && tile_map && tile_base && tile_count,
+                   RT_ERR_BAD_ARG, "rt_moe_plan: null pointer");
+        RT_REQUIRE(aligned16(tile_map), RT_ERR_UNSUPPORTED, "rt_moe_plan: tile_map must be 16-byte aligned");
+        const int ne = static_cast<int>(n_experts);
+        const int np = static_cast<int>(tokens * topk), warps = (np + 31) / 32;
+        const int threads = std::max(warps, (ne + 31) / 32) * 32;
+        const int smem = (ne + 1) * 4 + warps * ne * 2;
+        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&moe_plan_kernel), smem, "rt_moe_plan"))
+            return rc;
+        moe_plan_kernel<<<1, threads, smem, st>>>(
+            indices, expert_offsets, sorted_pairs, pair_pos, np, ne,
+            static_cast<int>(g_begin), static_cast<int>(g_end), reinterpret_cast<int4*>(tile_map), tile_base,
+            tile_count, static_cast<int>(max_tiles), amax2);
+        count_launch();
+        return check_launch("moe_plan_kernel");
+    }
+    if (amax2) {
+        zero2_kernel<<<1, 2, 0, st>>>(amax2);
+        count_launch();
+        if (int rc = check_launch("zero2_kernel")) return rc;
+    }
+    if (int rc = rt_moe_permute(indices, expert_offsets, sorted_pairs, pair_pos, workspace, tokens, topk,
+                                n_experts, stream))
+        return rc;
+    return rt_moe_tile_map(expert_offsets, g_begin, g_end, tile_map, tile_base, tile_count, max_tiles, stream);
+}
+
 // ---------------------------------------------------------------------------
 // rt_moe_permute without a caller-provided workspace
 // ---------------------------------------------------------------------------
@@ -804,7 +959,9 @@ extern "C" int rt_moe_combine(const void* expert_out, const int32_t* pair_pos,
     int threads = (nvec + 31) / 32 * 32;
     if (threads > 256) threads = 256;
     auto kernel = dtype == RT_F32 ? moe_combine_kernel<true> : moe_combine_kernel<false>;
-    kernel<<<static_cast<unsigned>(tokens), threads, 0, as_stream(stream)>>>(
+    // few tokens: a token's columns over several CTAs (7168 columns of one token: 14 us as one)
+    const unsigned pieces = tokens < 256 ? static_cast<unsigned>((nvec + threads - 1) / threads) : 1u;
+    kernel<<<dim3(static_cast<unsigned>(tokens), pieces), threads, 0, as_stream(stream)>>>(
         (const __nv_bfloat16*)expert_out, pair_pos, weights, (const __nv_bfloat16*)shared, y, nvec,
         (int)topk, (int)pos_begin, (int)pos_end, pos_begin_ptr, pos_end_ptr);
     count_launch();

@@ -22,7 +22,7 @@ using OptTensor = std::optional<Tensor>;
     X(rt_last_error) X(rt_residual_norm) X(rt_rms_norm) X(rt_norm_rope) X(rt_rope) X(rt_swiglu)   \
     X(rt_act_quant_fp8) X(rt_swiglu_quant_fp8) X(rt_absmax) X(rt_swiglu_absmax_rows)              \
     X(rt_nvfp4_quant) X(rt_moe_route) X(rt_moe_permute_workspace_bytes) X(rt_moe_permute)         \
-    X(rt_moe_tile_map) X(rt_moe_gather_nvfp4) X(rt_moe_quant_nvfp4) X(rt_moe_combine)             \
+    X(rt_moe_tile_map) X(rt_moe_plan) X(rt_absmax_onto) X(rt_swiglu_absmax_rows_onto) X(rt_moe_gather_nvfp4) X(rt_moe_quant_nvfp4) X(rt_moe_combine)             \
     X(rt_gemm_bf16) X(rt_gemm_bf16_splitk_splits) X(rt_gemm_bf16_splitk) X(rt_gemm_bf16_batched)  \
     X(rt_gemm_fp8_workspace_bytes) X(rt_gemm_fp8_ws) X(rt_gemm_nvfp4_grouped) X(rt_index_prep) X(rt_fp8_index_batched)              \
     X(rt_index_topk) X(rt_mla_sparse_decode_splits) X(rt_mla_sparse_decode)
@@ -566,31 +566,63 @@ py::tuple moe_experts(const OptTensor& x, const Tensor& weights, const Tensor& i
     const int64_t tokens = q_codes ? q_codes->size(0) : x->size(0);
     const int64_t hidden = q_codes ? q_codes->size(1) * 2 : x->size(1);
     const int64_t topk = indices.size(1), pairs = tokens * topk;
-    auto [offsets, sorted_pairs, pair_pos] = moe_permute(indices, n_experts);
+    require_cuda({&indices});
+    if (indices.scalar_type() != at::kLong || indices.dim() != 2)
+        fail("fused_moe_permute: indices must be a 2-D int64 tensor");
+    const Tensor idx = indices.contiguous();
     const int64_t max_tiles = (pairs + 127) / 128 + count;
-    auto [tile_map, tile_base, tile_count] = moe_tile_map(offsets, expert_begin, expert_begin + count, max_tiles);
+    Tensor workspace = empty(
+        {std::max<int64_t>(p_rt_moe_permute_workspace_bytes(tokens, topk, n_experts), 4)}, at::kByte, idx);
+    Tensor offsets = empty({n_experts + 1}, at::kInt, idx), sorted_pairs = empty({pairs}, at::kInt, idx);
+    Tensor pair_pos = empty({pairs}, at::kInt, idx), tile_map = empty({2 * max_tiles, 4}, at::kInt, idx);
+    Tensor tile_base = empty({count + 1}, at::kInt, idx), tile_count = empty({2}, at::kInt, idx);
+    Tensor amax2 = empty({2}, at::kFloat, idx);           // of x and of h, zeroed by the plan
+    check(p_rt_moe_plan(data<int64_t>(idx), data<int32_t>(offsets), data<int32_t>(sorted_pairs),
+                        data<int32_t>(pair_pos), workspace.data_ptr(), data<int32_t>(tile_map),
+                        data<int32_t>(tile_base), data<int32_t>(tile_count), data<float>(amax2), max_tiles,
+                        expert_begin, expert_begin + count, tokens, topk, n_experts, stream()),
+          "rt_moe_plan");
     OptTensor begin, end;
     if (count != n_experts) {
         begin = offsets.slice(0, expert_begin, expert_begin + 1);
         end = offsets.slice(0, expert_begin + count, expert_begin + count + 1);
     }
-    // dispatch: every token row is quantised once, then its codes and scales are copied into
-    // expert order (the bf16 rows are not read topk times)
-    Tensor x_codes, x_sf, x_gs;
+    Tensor a_codes, a_sf, x_gs;
     OptTensor x_amax;
     if (q_codes) {
-        x_codes = *q_codes;
-        x_sf = *q_sf;
         x_gs = *q_gs;
+        std::tie(a_codes, a_sf) = moe_gather_nvfp4(*q_codes, *q_sf, sorted_pairs, topk, tile_map, tile_count, pairs);
     } else {
-        x_amax = tensor_absmax(*x, std::nullopt);
-        std::tie(x_codes, x_sf, x_gs) = nvfp4_quant(*x, std::nullopt, x_amax, false, std::nullopt, std::nullopt);
+        require_cuda({&*x});
+        require_bf16("tensor_absmax", *x);
+        if (hidden % 16 != 0) fail("tensor_absmax: last dim must be a multiple of 16");
+        const Tensor x2 = rows_view(*x);
+        x_amax = amax2.slice(0, 0, 1);
+        check(p_rt_absmax_onto(x2.data_ptr(), data<float>(amax2), tokens, hidden, x2.stride(0), RT_BF16, stream()),
+              "rt_absmax_onto");
+        if (pairs <= 256) {
+            // few rows: quantised straight into expert order, once per pair, instead of once per token
+            // and copied; the same bits (7168 columns, top 8, one B200: 1 token 6 us against 11 in two
+            // launches, 13 tokens 9 / 12; 64 tokens 17 / 14)
+            std::tie(a_codes, a_sf, x_gs) =
+                moe_quant_nvfp4(x2, tile_map, tile_count, pairs, *x_amax, sorted_pairs, topk, std::nullopt);
+        } else {
+            // every token row is quantised once, then its codes and scales are copied into expert
+            // order (the bf16 rows are not read topk times)
+            auto [x_codes, x_sf, gs] = nvfp4_quant(*x, std::nullopt, x_amax, false, std::nullopt, std::nullopt);
+            x_gs = gs;
+            std::tie(a_codes, a_sf) = moe_gather_nvfp4(x_codes, x_sf, sorted_pairs, topk, tile_map, tile_count, pairs);
+        }
     }
-    auto [a_codes, a_sf] = moe_gather_nvfp4(x_codes, x_sf, sorted_pairs, topk, tile_map, tile_count, pairs);
     Tensor gate_up_out = gemm_nvfp4_grouped(a_codes, a_sf, x_gs, w13_codes, w13_sf, w13_gs, tile_map, tile_count,
                                             2 * inter, count, std::nullopt);
     // SwiGLU once: this pass writes h and finds the tensor-wide amax its quantisation needs
-    auto [h, h_amax] = swiglu_absmax(gate_up_out.slice(1, 0, inter), gate_up_out.slice(1, inter, 2 * inter), begin, end);
+    const Tensor gate = gate_up_out.slice(1, 0, inter), up = gate_up_out.slice(1, inter, 2 * inter);
+    Tensor h = empty({pairs, inter}, at::kBFloat16, gate_up_out), h_amax = amax2.slice(0, 1, 2);
+    check(p_rt_swiglu_absmax_rows_onto(gate.data_ptr(), up.data_ptr(), h.data_ptr(), data<float>(h_amax), pairs, inter,
+                                       gate.stride(0), up.stride(0), inter, data<int32_t>(begin), data<int32_t>(end),
+                                       RT_BF16, stream()),
+          "rt_swiglu_absmax_rows_onto");
     auto [h_codes, h_sf, h_gs] = moe_quant_nvfp4(h, tile_map, tile_count, pairs, h_amax, std::nullopt, 1, std::nullopt);
     Tensor expert_out = gemm_nvfp4_grouped(h_codes, h_sf, h_gs, w2_codes, w2_sf, w2_gs, tile_map, tile_count, hidden,
                                            count, std::nullopt);

@@ -200,3 +200,51 @@ def test_grouped_gemm_token_box_fits_the_rows(mods, rows):
         bound = 2 * k * 2.0 ** -24 * (a[lo:lo + r].abs() @ b.abs().t()) + 2.0 ** -8 * ref.abs()
         assert bool(((out[lo:lo + r].cpu().double() - ref).abs() <= bound).all()), (i, r)
         lo += r
+
+
+@pytest.mark.parametrize("tokens,topk,n_experts,begin,count", [
+    (1, 8, 256, 0, 256), (13, 8, 256, 64, 128), (128, 8, 256, 0, 256),   # one launch: up to 1024 pairs
+    (31, 33, 40, 0, 40), (1024, 1, 3, 1, 2), (5, 2, 1024, 1000, 24),
+    (129, 8, 256, 0, 256), (341, 3, 7, 2, 5),                           # one block does not hold the pairs
+])
+def test_moe_plan_equals_permute_and_tile_map(mods, tokens, topk, n_experts, begin, count):
+    from racetrack_b200 import _lib
+    ops, _ = mods
+    lib = _lib.load()
+    g = torch.Generator().manual_seed(tokens)
+    idx = torch.randint(0, n_experts, (tokens, topk), generator=g).cuda()
+    want = ops.fused_moe_permute(idx, n_experts)
+    pairs = tokens * topk
+    max_tiles = (pairs + 127) // 128 + count
+    tm, tb, tc = ops.moe_tile_map(want[0], begin, begin + count, max_tiles)
+    new = [torch.full_like(t, -7) for t in (*want, tm, tb, tc)]
+    amax2 = torch.full((2,), 5.0, device="cuda")
+    ws = torch.empty(int(lib.rt_moe_permute_workspace_bytes(tokens, topk, n_experts)), dtype=torch.uint8, device="cuda")
+    o, sp, pp, m, b, c = (t.data_ptr() for t in new)
+    _lib.check(lib.rt_moe_plan(idx.data_ptr(), o, sp, pp, ws.data_ptr(), m, b, c, amax2.data_ptr(), max_tiles, begin,
+                               begin + count, tokens, topk, n_experts, torch.cuda.current_stream().cuda_stream), "plan")
+    for got, ref in zip((new[0], new[1], new[2], new[4], new[5]), (*want, tb, tc)):
+        assert torch.equal(got, ref)
+    n128, n256 = int(tc[0]), int(tc[1])
+    assert torch.equal(new[3][:n128], tm[:n128])
+    assert torch.equal(new[3][max_tiles:max_tiles + n256], tm[max_tiles:max_tiles + n256])
+    assert amax2.tolist() == [0.0, 0.0]
+
+
+@pytest.mark.parametrize("tokens", [1, 32, 33])
+def test_experts_quantise_few_rows_in_expert_order(mods, tokens):
+    """Up to 256 pairs the rows are quantised straight into expert order, beyond once per token and
+    copied: the same bits as handing the rows over already quantised."""
+    ops, moe = mods
+    g = torch.Generator().manual_seed(tokens)
+    x = torch.randn(tokens, 512, generator=g).bfloat16().cuda()
+    w13 = (torch.randn(16, 512, 512, generator=g) * 0.05).bfloat16().cuda()
+    w2 = (torch.randn(16, 512, 256, generator=g) * 0.05).bfloat16().cuda()
+    experts = moe.quantize_experts(w13, w2)
+    weights, indices = ops.fused_moe_route(torch.randn(tokens, 16, generator=g).cuda(), None, n_groups=1,
+                                           topk_groups=1, topk=8, route_scale=1.0, score_func="topk_softmax")
+    got = moe.fused_moe_experts(x, weights, indices, experts, n_experts=16)
+    codes, sf, gs = ops.fused_nvfp4_quant(x)
+    want = moe.fused_moe_experts(None, weights, indices, experts, n_experts=16,
+                                 x_quant=(codes, sf.view(torch.uint8), gs))
+    assert torch.equal(got, want)
