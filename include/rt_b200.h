@@ -119,6 +119,14 @@ int rt_norm_rope(const void* q_c, const void* q_weight,
                  int64_t tokens, int64_t q_cols, int64_t kv_cols, int64_t rope_dim,
                  int64_t q_stride, int64_t kv_stride, int64_t k_stride,
                  float eps, int rope_mode, int dtype, void* stream);
+/* The same with the rows of kv_out (kv_out_stride % 8 == 0) and k_out that far apart, in elements: a
+ * decode step writes the new token straight into its sequences' caches. */
+int rt_norm_rope_into(const void* q_c, const void* q_weight, const void* kv_c, const void* kv_weight,
+                      int weight_dtype, const void* k_pe, const int64_t* positions, const float* table,
+                      int64_t table_rows, void* q_out, void* kv_out, void* k_out, int64_t tokens,
+                      int64_t q_cols, int64_t kv_cols, int64_t rope_dim, int64_t q_stride,
+                      int64_t kv_stride, int64_t k_stride, int64_t kv_out_stride, int64_t k_out_stride,
+                      float eps, int rope_mode, int dtype, void* stream);
 
 /*
  * RoPE on a [tokens, heads, rope_dim] view: element (t, h, :) starts at
@@ -545,6 +553,20 @@ int rt_index_prep(const void* x, const float* ln_weight, const float* ln_bias,
                   int64_t rows_per_position, void* codes, float* scales, void* rotated,
                   int64_t rows, int64_t dim, int64_t rope_dim, int64_t x_stride, float eps,
                   int dtype, void* stream);
+/* The same with rows of codes (codes_stride bytes apart, % 4 == 0) and scales (scales_stride floats
+ * apart) placed by the caller, e.g. in a key cache. */
+int rt_index_prep_into(const void* x, const float* ln_weight, const float* ln_bias,
+                       const int64_t* positions, const float* freqs, int64_t table_rows,
+                       int64_t rows_per_position, void* codes, float* scales, void* rotated,
+                       int64_t rows, int64_t dim, int64_t rope_dim, int64_t x_stride,
+                       int64_t codes_stride, int64_t scales_stride, float eps, int dtype,
+                       void* stream);
+
+/* Head weights of the index scores: out[s, h] = ((both[s, h] + both[s, heads + h]) * c1 * q_scale[s, h])
+ * * c2 in fp32, `both` [rows, 2 * heads] the projection by an fp32 weight's two bf16 halves.
+ * ref: racetrack/models/deepseek.py:677-678. */
+int rt_index_head_weights(const float* both, const float* q_scale, float* out, int64_t rows,
+                          int64_t heads, float c1, float c2, void* stream);
 
 /*
  * Index scores of the sparse-attention indexer (tcgen05, FP8 x FP8, fp32 accumulate):

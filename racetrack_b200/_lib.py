@@ -29,6 +29,7 @@ SIGNATURES: dict[str, tuple] = {
     "rt_rms_norm": (_I, [_P, _P, _I, _P, _L, _L, _L, _L, _F, _I, _P]),
     "rt_norm_rope": (_I, [_P, _P, _P, _P, _I, _P, _P, _P, _L, _P, _P, _P,
                           _L, _L, _L, _L, _L, _L, _L, _F, _I, _I, _P]),
+    "rt_norm_rope_into": (_I, [_P, _P, _P, _P, _I, _P, _P, _P, _L, _P, _P, _P] + [_L] * 9 + [_F, _I, _I, _P]),
     "rt_rope": (_I, [_P, _P, _P, _L, _P, _L, _L, _L, _L, _L, _L, _L, _I, _I, _P]),
     "rt_head_broadcast": (_I, [_P, _P, _L, _L, _L, _L, _L, _L, _I, _P]),
     "rt_swiglu": (_I, [_P, _P, _P, _L, _L, _L, _L, _I, _P]),
@@ -61,6 +62,8 @@ SIGNATURES: dict[str, tuple] = {
     "rt_moe_tile_map": (_I, [_P, _L, _L, _P, _P, _P, _L, _P]),
     "rt_gemm_nvfp4_schedule": (_I, [_I]),
     "rt_index_prep": (_I, [_P, _P, _P, _P, _P, _L, _L, _P, _P, _P, _L, _L, _L, _L, _F, _I, _P]),
+    "rt_index_prep_into": (_I, [_P, _P, _P, _P, _P, _L, _L, _P, _P, _P] + [_L] * 6 + [_F, _I, _P]),
+    "rt_index_head_weights": (_I, [_P, _P, _P, _L, _L, _F, _F, _P]),
     "rt_fp8_index": (_I, [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _P]),
     "rt_fp8_index_batched": (_I, [_P, _P, _P, _P, _P] + [_L] * 10 + [_P]),
     "rt_index_topk": (_I, [_P, _P, _L, _L, _L, _L, _P]),

@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(256) index_prep_kernel(
     const float* __restrict__ ln_b, const int64_t* __restrict__ positions,
     const float2* __restrict__ freqs, int table_rows, int rows_per_pos,
     uint8_t* __restrict__ codes, float* __restrict__ scales, __nv_bfloat16* __restrict__ rotated,
-    int64_t rows, int64_t xstride, float eps) {
+    int64_t rows, int64_t xstride, int64_t cstride, int64_t sstride, float eps) {
     const int lane = threadIdx.x & 31;
     const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(256) index_prep_kernel(
     const float rscale = __frcp_rn(scale);
     const uint32_t packed = cvt_e4m3x2(div_shared(v[0], scale, rscale), div_shared(v[1], scale, rscale)) |
                             (cvt_e4m3x2(div_shared(v[2], scale, rscale), div_shared(v[3], scale, rscale)) << 16);
-    *reinterpret_cast<uint32_t*>(codes + row * 128 + 4 * lane) = packed;
-    if (lane == 0) scales[row] = scale;
+    *reinterpret_cast<uint32_t*>(codes + row * cstride + 4 * lane) = packed;
+    if (lane == 0) scales[row * sstride] = scale;
 }
 
 // ---------------------------------------------------------------------------
@@ -689,11 +689,11 @@ extern "C" int rt_moe_gather_nvfp4(const void* codes_in, const void* sf_in,
     return check_launch("moe_gather_nvfp4_kernel");
 }
 
-extern "C" int rt_index_prep(const void* x, const float* ln_weight, const float* ln_bias,
+static int index_prep_common(const void* x, const float* ln_weight, const float* ln_bias,
                              const int64_t* positions, const float* freqs, int64_t table_rows,
                              int64_t rows_per_position, void* codes, float* scales, void* rotated,
                              int64_t rows, int64_t dim, int64_t rope_dim, int64_t x_stride,
-                             float eps, int dtype, void* stream) {
+                             int64_t codes_stride, int64_t scales_stride, float eps, int dtype, void* stream) {
     RT_REQUIRE(rows >= 0 && rows_per_position > 0 && table_rows > 0, RT_ERR_BAD_ARG,
                "rt_index_prep: bad shape");
     if (rows == 0) return RT_OK;
@@ -703,7 +703,7 @@ extern "C" int rt_index_prep(const void* x, const float* ln_weight, const float*
     RT_REQUIRE(dtype == RT_BF16, RT_ERR_UNSUPPORTED, "rt_index_prep: only bf16 activations");
     RT_REQUIRE(dim == 128 && rope_dim == 64, RT_ERR_UNSUPPORTED,
                "rt_index_prep: index head dimension 128 with a 64-wide rope slice only");
-    RT_REQUIRE(x_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 7u) == 0 &&
+    RT_REQUIRE(x_stride % 4 == 0 && codes_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 7u) == 0 &&
                    (reinterpret_cast<uintptr_t>(codes) & 3u) == 0 &&
                    (!rotated || (reinterpret_cast<uintptr_t>(rotated) & 7u) == 0) &&
                    (!ln_weight || (aligned16(ln_weight) && aligned16(ln_bias))) &&
@@ -717,14 +717,61 @@ extern "C" int rt_index_prep(const void* x, const float* ln_weight, const float*
         index_prep_kernel<true><<<grid, 256, 0, st>>>(
             (const __nv_bfloat16*)x, ln_weight, ln_bias, positions, (const float2*)freqs,
             (int)table_rows, (int)rows_per_position, (uint8_t*)codes, scales,
-            (__nv_bfloat16*)rotated, rows, x_stride, eps);
+            (__nv_bfloat16*)rotated, rows, x_stride, codes_stride, scales_stride, eps);
     else
         index_prep_kernel<false><<<grid, 256, 0, st>>>(
             (const __nv_bfloat16*)x, nullptr, nullptr, positions, (const float2*)freqs,
             (int)table_rows, (int)rows_per_position, (uint8_t*)codes, scales,
-            (__nv_bfloat16*)rotated, rows, x_stride, eps);
+            (__nv_bfloat16*)rotated, rows, x_stride, codes_stride, scales_stride, eps);
     count_launch();
     return check_launch("index_prep_kernel");
+}
+
+extern "C" int rt_index_prep(const void* x, const float* ln_weight, const float* ln_bias, const int64_t* positions,
+                             const float* freqs, int64_t table_rows, int64_t rows_per_position, void* codes,
+                             float* scales, void* rotated, int64_t rows, int64_t dim, int64_t rope_dim,
+                             int64_t x_stride, float eps, int dtype, void* stream) {
+    return index_prep_common(x, ln_weight, ln_bias, positions, freqs, table_rows, rows_per_position, codes, scales,
+                             rotated, rows, dim, rope_dim, x_stride, 128, 1, eps, dtype, stream);
+}
+
+extern "C" int rt_index_prep_into(const void* x, const float* ln_weight, const float* ln_bias,
+                                  const int64_t* positions, const float* freqs, int64_t table_rows,
+                                  int64_t rows_per_position, void* codes, float* scales, void* rotated, int64_t rows,
+                                  int64_t dim, int64_t rope_dim, int64_t x_stride, int64_t codes_stride,
+                                  int64_t scales_stride, float eps, int dtype, void* stream) {
+    return index_prep_common(x, ln_weight, ln_bias, positions, freqs, table_rows, rows_per_position, codes, scales,
+                             rotated, rows, dim, rope_dim, x_stride, codes_stride, scales_stride, eps, dtype, stream);
+}
+
+namespace rt {
+// out[s, h] = ((hi[s, h] + lo[s, h]) * c1 * q_scale[s, h]) * c2, `both` = [s][hi | lo]: one fp32 rounding
+// per operation, as the four element-wise passes it replaces.
+__global__ void __launch_bounds__(256) index_head_weights_kernel(const float* __restrict__ both,
+                                                                 const float* __restrict__ q_scale,
+                                                                 float* __restrict__ out, int64_t total, int heads,
+                                                                 float c1, float c2) {
+    const int64_t i = blockIdx.x * 256LL + threadIdx.x;
+    if (i >= total) return;
+    const int64_t s = i / heads;
+    const int64_t at = i + s * heads;            // row s of `both` starts at 2 * s * heads
+    const float w = __fmul_rn(__fadd_rn(both[at], both[at + heads]), c1);
+    out[i] = __fmul_rn(__fmul_rn(w, q_scale[i]), c2);
+}
+}  // namespace rt
+
+extern "C" int rt_index_head_weights(const float* both, const float* q_scale, float* out, int64_t rows, int64_t heads,
+                                     float c1, float c2, void* stream) {
+    RT_REQUIRE(rows >= 0 && heads > 0, RT_ERR_BAD_ARG, "rt_index_head_weights: bad shape");
+    if (rows == 0) return RT_OK;
+    RT_REQUIRE(both && q_scale && out, RT_ERR_BAD_ARG, "rt_index_head_weights: null pointer");
+    RT_REQUIRE(rows * heads < (1LL << 38) && heads < (1LL << 31), RT_ERR_UNSUPPORTED,
+               "rt_index_head_weights: tensor too large");
+    const int64_t total = rows * heads;
+    index_head_weights_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, as_stream(stream)>>>(
+        both, q_scale, out, total, static_cast<int>(heads), c1, c2);
+    count_launch();
+    return check_launch("index_head_weights_kernel");
 }
 
 extern "C" int rt_nvfp4_quant(const void* x, const void* up, const float* amax_in, void* codes,

@@ -179,8 +179,8 @@ __global__ void __launch_bounds__(512) norm_rope_kernel(
     const __nv_bfloat16* __restrict__ k_pe, const int64_t* __restrict__ positions,
     const float* __restrict__ table, int64_t table_rows, __nv_bfloat16* __restrict__ q_out,
     __nv_bfloat16* __restrict__ kv_out, __nv_bfloat16* __restrict__ k_out, int nq, int nkv,
-    int rope_dim, int64_t q_stride, int64_t kv_stride, int64_t k_stride, float q_cols_f,
-    float kv_cols_f, float eps, int mode) {
+    int rope_dim, int64_t q_stride, int64_t kv_stride, int64_t k_stride, int64_t kvo_stride,
+    int64_t ko_stride, float q_cols_f, float kv_cols_f, float eps, int mode) {
     __shared__ float scratch[64];
     extern __shared__ float cs[];  // [2 * rope_dim/2]
     const int64_t t = blockIdx.x;
@@ -218,13 +218,13 @@ __global__ void __launch_bounds__(512) norm_rope_kernel(
 #pragma unroll
             for (int k = 0; k < 8; ++k) o[k] = (h[i][k] * rs) * w[k];
             uint4* dst = is_q ? (reinterpret_cast<uint4*>(q_out) + t * nq + v)
-                              : (reinterpret_cast<uint4*>(kv_out) + t * nkv + (v - nq));
+                              : (reinterpret_cast<uint4*>(kv_out + t * kvo_stride) + (v - nq));
             st_stream16(dst, pack_bf16x8(o));
         }
     }
     // k_pe rotation: rope_dim elements per token, scalar accesses are enough.
     const __nv_bfloat16* kin = k_pe + t * k_stride;
-    __nv_bfloat16* kout = k_out + t * rope_dim;
+    __nv_bfloat16* kout = k_out + t * ko_stride;
     for (int i = threadIdx.x; i < half; i += blockDim.x) {
         const float c = cs[i], s = cs[half + i];
         float o1, o2;
@@ -256,8 +256,8 @@ __global__ void __launch_bounds__(kNrWarps * 32) norm_rope_warp_kernel(
     const __nv_bfloat16* __restrict__ k_pe, const int64_t* __restrict__ positions,
     const float* __restrict__ table, int64_t table_rows, __nv_bfloat16* __restrict__ q_out,
     __nv_bfloat16* __restrict__ kv_out, __nv_bfloat16* __restrict__ k_out, int64_t tokens, int nq,
-    int nkv, int rope_dim, int64_t q_stride, int64_t kv_stride, int64_t k_stride, float q_cols_f,
-    float kv_cols_f, float eps, int mode) {
+    int nkv, int rope_dim, int64_t q_stride, int64_t kv_stride, int64_t k_stride, int64_t kvo_stride,
+    int64_t ko_stride, float q_cols_f, float kv_cols_f, float eps, int mode) {
     const int lane = threadIdx.x & 31;
     const int64_t t = static_cast<int64_t>(blockIdx.x) * kNrWarps + (threadIdx.x >> 5);
     if (t >= tokens) return;
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(kNrWarps * 32) norm_rope_warp_kernel(
     const float rq = rsqrtf(sq / q_cols_f + eps);
     const float rkv = rsqrtf(skv / kv_cols_f + eps);
     uint4* qo = reinterpret_cast<uint4*>(q_out) + t * nq;
-    uint4* kvo = reinterpret_cast<uint4*>(kv_out) + t * nkv;
+    uint4* kvo = reinterpret_cast<uint4*>(kv_out + t * kvo_stride);
 #pragma unroll
     for (int i = 0; i < kNrQMax; ++i)
         if (lane + 32 * i < nq) {
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kNrWarps * 32) norm_rope_warp_kernel(
         }
     const int half = rope_dim >> 1;
     const __nv_bfloat16* kin = k_pe + t * k_stride;
-    __nv_bfloat16* kout = k_out + t * rope_dim;
+    __nv_bfloat16* kout = k_out + t * ko_stride;
     for (int i = lane; i < half; i += 32) {
         float c, s, o1, o2;
         if (mode == RT_ROPE_HALF) {
@@ -511,12 +511,13 @@ static int check_rope_args(const char* who, const int64_t* positions, const floa
     return RT_OK;
 }
 
-extern "C" int rt_norm_rope(const void* q_c, const void* q_weight, const void* kv_c,
+static int norm_rope_common(const void* q_c, const void* q_weight, const void* kv_c,
                             const void* kv_weight, int weight_dtype, const void* k_pe,
                             const int64_t* positions, const float* table, int64_t table_rows,
                             void* q_out, void* kv_out, void* k_out, int64_t tokens, int64_t q_cols,
                             int64_t kv_cols, int64_t rope_dim, int64_t q_stride, int64_t kv_stride,
-                            int64_t k_stride, float eps, int rope_mode, int dtype, void* stream) {
+                            int64_t k_stride, int64_t kvo_stride, int64_t ko_stride, float eps, int rope_mode,
+                            int dtype, void* stream) {
     RT_REQUIRE(tokens >= 0 && q_cols > 0 && kv_cols > 0, RT_ERR_BAD_ARG, "rt_norm_rope: bad shape");
     if (tokens == 0) return RT_OK;
     RT_REQUIRE(q_c && q_weight && kv_c && kv_weight && k_pe && q_out && kv_out && k_out,
@@ -526,7 +527,8 @@ extern "C" int rt_norm_rope(const void* q_c, const void* q_weight, const void* k
                "rt_norm_rope: weight dtype must be bf16 or f32");
     if (int rc = check_rope_args("rt_norm_rope", positions, table, table_rows, rope_dim, rope_mode))
         return rc;
-    RT_REQUIRE(q_cols % 8 == 0 && kv_cols % 8 == 0 && q_stride % 8 == 0 && kv_stride % 8 == 0,
+    RT_REQUIRE(q_cols % 8 == 0 && kv_cols % 8 == 0 && q_stride % 8 == 0 && kv_stride % 8 == 0 &&
+                   kvo_stride % 8 == 0,
                RT_ERR_UNSUPPORTED, "rt_norm_rope: q/kv cols and strides must be multiples of 8");
     RT_REQUIRE(aligned16(q_c) && aligned16(kv_c) && aligned16(q_weight) && aligned16(kv_weight) &&
                    aligned16(q_out) && aligned16(kv_out),
@@ -548,13 +550,13 @@ extern "C" int rt_norm_rope(const void* q_c, const void* q_weight, const void* k
                 (const __nv_bfloat16*)q_c, q_weight, (const __nv_bfloat16*)kv_c, kv_weight,
                 (const __nv_bfloat16*)k_pe, positions, table, table_rows, (__nv_bfloat16*)q_out,
                 (__nv_bfloat16*)kv_out, (__nv_bfloat16*)k_out, tokens, nq, nkv, (int)rope_dim,
-                q_stride, kv_stride, k_stride, (float)q_cols, (float)kv_cols, eps, rope_mode);
+                q_stride, kv_stride, k_stride, kvo_stride, ko_stride, (float)q_cols, (float)kv_cols, eps, rope_mode);
         else
             norm_rope_warp_kernel<false><<<wgrid, kNrWarps * 32, 0, st>>>(
                 (const __nv_bfloat16*)q_c, q_weight, (const __nv_bfloat16*)kv_c, kv_weight,
                 (const __nv_bfloat16*)k_pe, positions, table, table_rows, (__nv_bfloat16*)q_out,
                 (__nv_bfloat16*)kv_out, (__nv_bfloat16*)k_out, tokens, nq, nkv, (int)rope_dim,
-                q_stride, kv_stride, k_stride, (float)q_cols, (float)kv_cols, eps, rope_mode);
+                q_stride, kv_stride, k_stride, kvo_stride, ko_stride, (float)q_cols, (float)kv_cols, eps, rope_mode);
         count_launch();
         return check_launch("norm_rope_warp_kernel");
     }
@@ -564,13 +566,13 @@ extern "C" int rt_norm_rope(const void* q_c, const void* q_weight, const void* k
             (const __nv_bfloat16*)q_c, q_weight, (const __nv_bfloat16*)kv_c, kv_weight,          \
             (const __nv_bfloat16*)k_pe, positions, table, table_rows, (__nv_bfloat16*)q_out,     \
             (__nv_bfloat16*)kv_out, (__nv_bfloat16*)k_out, nq, nkv, (int)rope_dim, q_stride,     \
-            kv_stride, k_stride, (float)q_cols, (float)kv_cols, eps, rope_mode);                 \
+            kv_stride, k_stride, kvo_stride, ko_stride, (float)q_cols, (float)kv_cols, eps, rope_mode);                 \
     else                                                                                         \
         norm_rope_kernel<V, false><<<grid, threads, smem, st>>>(                                 \
             (const __nv_bfloat16*)q_c, q_weight, (const __nv_bfloat16*)kv_c, kv_weight,          \
             (const __nv_bfloat16*)k_pe, positions, table, table_rows, (__nv_bfloat16*)q_out,     \
             (__nv_bfloat16*)kv_out, (__nv_bfloat16*)k_out, nq, nkv, (int)rope_dim, q_stride,     \
-            kv_stride, k_stride, (float)q_cols, (float)kv_cols, eps, rope_mode);
+            kv_stride, k_stride, kvo_stride, ko_stride, (float)q_cols, (float)kv_cols, eps, rope_mode);
     switch (vpt) {
         case 1: RT_LAUNCH_NR(1) break;
         case 2: RT_LAUNCH_NR(2) break;
@@ -580,6 +582,28 @@ extern "C" int rt_norm_rope(const void* q_c, const void* q_weight, const void* k
 #undef RT_LAUNCH_NR
     count_launch();
     return check_launch("norm_rope_kernel");
+}
+
+extern "C" int rt_norm_rope(const void* q_c, const void* q_weight, const void* kv_c, const void* kv_weight,
+                            int weight_dtype, const void* k_pe, const int64_t* positions, const float* table,
+                            int64_t table_rows, void* q_out, void* kv_out, void* k_out, int64_t tokens,
+                            int64_t q_cols, int64_t kv_cols, int64_t rope_dim, int64_t q_stride,
+                            int64_t kv_stride, int64_t k_stride, float eps, int rope_mode, int dtype,
+                            void* stream) {
+    return norm_rope_common(q_c, q_weight, kv_c, kv_weight, weight_dtype, k_pe, positions, table, table_rows, q_out,
+                            kv_out, k_out, tokens, q_cols, kv_cols, rope_dim, q_stride, kv_stride, k_stride, kv_cols,
+                            rope_dim, eps, rope_mode, dtype, stream);
+}
+
+extern "C" int rt_norm_rope_into(const void* q_c, const void* q_weight, const void* kv_c, const void* kv_weight,
+                                 int weight_dtype, const void* k_pe, const int64_t* positions, const float* table,
+                                 int64_t table_rows, void* q_out, void* kv_out, void* k_out, int64_t tokens,
+                                 int64_t q_cols, int64_t kv_cols, int64_t rope_dim, int64_t q_stride,
+                                 int64_t kv_stride, int64_t k_stride, int64_t kv_out_stride, int64_t k_out_stride,
+                                 float eps, int rope_mode, int dtype, void* stream) {
+    return norm_rope_common(q_c, q_weight, kv_c, kv_weight, weight_dtype, k_pe, positions, table, table_rows, q_out,
+                            kv_out, k_out, tokens, q_cols, kv_cols, rope_dim, q_stride, kv_stride, k_stride,
+                            kv_out_stride, k_out_stride, eps, rope_mode, dtype, stream);
 }
 
 extern "C" int rt_rope(const void* x, const int64_t* positions, const float* table,

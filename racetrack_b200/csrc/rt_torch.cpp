@@ -19,12 +19,12 @@ using at::Tensor;
 using OptTensor = std::optional<Tensor>;
 
 #define RT_TABLE(X)                                                                               \
-    X(rt_last_error) X(rt_residual_norm) X(rt_rms_norm) X(rt_norm_rope) X(rt_rope) X(rt_swiglu)   \
+    X(rt_last_error) X(rt_residual_norm) X(rt_rms_norm) X(rt_norm_rope_into) X(rt_rope) X(rt_swiglu)   \
     X(rt_act_quant_fp8) X(rt_swiglu_quant_fp8) X(rt_absmax) X(rt_swiglu_absmax_rows)              \
     X(rt_nvfp4_quant) X(rt_moe_route) X(rt_moe_permute_workspace_bytes) X(rt_moe_permute)         \
     X(rt_moe_tile_map) X(rt_moe_plan) X(rt_absmax_onto) X(rt_swiglu_absmax_rows_onto) X(rt_moe_gather_nvfp4) X(rt_moe_quant_nvfp4) X(rt_moe_combine)             \
     X(rt_gemm_bf16) X(rt_gemm_bf16_splitk_splits) X(rt_gemm_bf16_splitk) X(rt_gemm_bf16_batched)  \
-    X(rt_gemm_fp8_workspace_bytes) X(rt_gemm_fp8_ws) X(rt_gemm_nvfp4_grouped) X(rt_index_prep) X(rt_fp8_index_batched)              \
+    X(rt_gemm_fp8_workspace_bytes) X(rt_gemm_fp8_ws) X(rt_gemm_nvfp4_grouped) X(rt_index_prep_into) X(rt_index_head_weights) X(rt_fp8_index_batched)              \
     X(rt_index_topk) X(rt_mla_sparse_decode_splits) X(rt_mla_sparse_decode)
 
 #define RT_POINTER(name) decltype(&::name) p_##name = nullptr;
@@ -135,11 +135,20 @@ Tensor freqs_table(const Tensor& freqs_cis, int64_t half) {
     return table.scalar_type() == at::kFloat ? table : table.to(at::kFloat);
 }
 
+// Whether `out` can take [rows, cols] of `type` rows in place (a slice of a cache).
+bool row_slots(const Tensor& out, int64_t rows, int64_t cols, at::ScalarType type, int64_t align) {
+    return out.is_cuda() && out.scalar_type() == type && out.dim() == 2 && same_shape(out, {rows, cols}) &&
+           out.stride(1) == 1 && (rows <= 1 || out.stride(0) >= cols) &&
+           out.stride(0) * out.element_size() % align == 0 &&
+           reinterpret_cast<uintptr_t>(out.data_ptr()) % align == 0;
+}
+
 // positions + inverse frequencies (half-split pairs), or a complex table (interleaved pairs)
 std::tuple<Tensor, Tensor, Tensor> norm_rope(const Tensor& q_c, const Tensor& q_weight, const Tensor& kv_c,
                                              const Tensor& kv_weight, const Tensor& k_pe,
                                              const OptTensor& positions, const OptTensor& inv_freq,
-                                             const OptTensor& freqs_cis, double eps) {
+                                             const OptTensor& freqs_cis, double eps, const OptTensor& kv_into,
+                                             const OptTensor& k_into) {
     Tensor pos, table;
     int mode = RT_ROPE_INTERLEAVED;
     int64_t table_rows = 0;
@@ -165,14 +174,25 @@ std::tuple<Tensor, Tensor, Tensor> norm_rope(const Tensor& q_c, const Tensor& q_
     Tensor kvw = kv_weight.contiguous();
     if (qw.scalar_type() != kvw.scalar_type()) kvw = kvw.to(qw.scalar_type());
     Tensor q_out = empty(q_c.sizes(), at::kBFloat16, q_c);
-    Tensor kv_out = empty(kv_c.sizes(), at::kBFloat16, kv_c);
-    Tensor k_out = empty(k_pe.sizes(), at::kBFloat16, k_pe);
-    check(p_rt_norm_rope(q2.data_ptr(), qw.data_ptr(), kv2.data_ptr(), kvw.data_ptr(), weight_tag(qw),
+    // into the caller's rows where they can be written as they are, else a tensor and a copy
+    const bool into = kv_into && k_into && row_slots(*kv_into, tokens, kv2.size(1), at::kBFloat16, 16) &&
+                      row_slots(*k_into, tokens, k2.size(1), at::kBFloat16, 2);
+    Tensor kv_out = into ? *kv_into : empty(kv_c.sizes(), at::kBFloat16, kv_c);
+    Tensor k_out = into ? *k_into : empty(k_pe.sizes(), at::kBFloat16, k_pe);
+    check(p_rt_norm_rope_into(q2.data_ptr(), qw.data_ptr(), kv2.data_ptr(), kvw.data_ptr(), weight_tag(qw),
                          k2.data_ptr(), pos.defined() ? data<int64_t>(pos) : nullptr, data<float>(table),
                          table_rows, q_out.data_ptr(), kv_out.data_ptr(), k_out.data_ptr(), tokens, q2.size(1),
                          kv2.size(1), k2.size(1), q2.stride(0), kv2.stride(0), k2.stride(0),
+                         into ? kv_out.stride(0) : kv2.size(1), into ? k_out.stride(0) : k2.size(1),
                          static_cast<float>(eps), mode, RT_BF16, stream()),
           "rt_norm_rope");
+    if (into) {
+        kv_out.unsafeGetTensorImpl()->bump_version();
+        k_out.unsafeGetTensorImpl()->bump_version();
+    } else if (kv_into && k_into) {
+        kv_into->copy_(kv_out);
+        k_into->copy_(k_out);
+    }
     return {q_out, kv_out, k_out};
 }
 
@@ -425,11 +445,6 @@ Tensor linear_fp8(const Tensor& x_codes, const Tensor& x_scales, const Tensor& w
     return out;
 }
 
-Tensor linear_fp8_act(const Tensor& x, const Tensor& w_codes, const Tensor& w_scales, const OptTensor& out) {
-    const auto [codes, scales] = act_quant(x, std::nullopt, std::nullopt);
-    return linear_fp8(codes, scales, w_codes, w_scales, out);
-}
-
 Tensor gemm_nvfp4_grouped(const Tensor& a_codes, const Tensor& a_sf, const Tensor& a_gs, const Tensor& b_codes,
                           const Tensor& b_sf, const Tensor& b_gs, const Tensor& tile_map, const Tensor& tile_count,
                           int64_t n, int64_t groups, const OptTensor& out_in) {
@@ -562,7 +577,7 @@ py::tuple moe_experts(const OptTensor& x, const Tensor& weights, const Tensor& i
                       const Tensor& w13_sf, const Tensor& w13_gs, const Tensor& w2_codes, const Tensor& w2_sf,
                       const Tensor& w2_gs, int64_t count, int64_t inter, int64_t n_experts, int64_t expert_begin,
                       const OptTensor& shared, bool f32_out, const OptTensor& q_codes, const OptTensor& q_sf,
-                      const OptTensor& q_gs, const OptTensor& out) {
+                      const OptTensor& q_gs, const OptTensor& out, const std::optional<py::function>& around_w13) {
     const int64_t tokens = q_codes ? q_codes->size(0) : x->size(0);
     const int64_t hidden = q_codes ? q_codes->size(1) * 2 : x->size(1);
     const int64_t topk = indices.size(1), pairs = tokens * topk;
@@ -614,8 +629,10 @@ py::tuple moe_experts(const OptTensor& x, const Tensor& weights, const Tensor& i
             std::tie(a_codes, a_sf) = moe_gather_nvfp4(x_codes, x_sf, sorted_pairs, topk, tile_map, tile_count, pairs);
         }
     }
+    if (around_w13) (*around_w13)(true);
     Tensor gate_up_out = gemm_nvfp4_grouped(a_codes, a_sf, x_gs, w13_codes, w13_sf, w13_gs, tile_map, tile_count,
                                             2 * inter, count, std::nullopt);
+    if (around_w13) (*around_w13)(false);
     // SwiGLU once: this pass writes h and finds the tensor-wide amax its quantisation needs
     const Tensor gate = gate_up_out.slice(1, 0, inter), up = gate_up_out.slice(1, inter, 2 * inter);
     Tensor h = empty({pairs, inter}, at::kBFloat16, gate_up_out), h_amax = amax2.slice(0, 1, 2);
@@ -633,7 +650,8 @@ py::tuple moe_experts(const OptTensor& x, const Tensor& weights, const Tensor& i
 // ---- sparse indexer and decode attention -----------------------------------------------------------
 
 py::tuple index_prep(const Tensor& x, const Tensor& freqs_cis, const OptTensor& positions, const OptTensor& ln_weight,
-                     const OptTensor& ln_bias, double eps, bool return_rotated) {
+                     const OptTensor& ln_bias, double eps, bool return_rotated, const OptTensor& codes_into,
+                     const OptTensor& scales_into) {
     require_cuda({&x, &freqs_cis});
     require_bf16("index_prep", x);
     if (x.dim() != 3 || x.size(-1) != 128) fail("index_prep: x must be [S, H, 128]");
@@ -642,18 +660,45 @@ py::tuple index_prep(const Tensor& x, const Tensor& freqs_cis, const OptTensor& 
     if (x2.stride(1) != 1) x2 = x2.contiguous();
     const Tensor fr = at::view_as_real(freqs_cis).to(at::kFloat).contiguous();
     if (fr.dim() < 2 || fr.size(-2) != 32 || fr.size(-1) != 2) fail("index_prep: freqs_cis must be [table, 32] complex");
-    Tensor codes = empty({s_len, heads, dim}, at::kFloat8_e4m3fn, x), scales = empty({s_len, heads}, at::kFloat, x);
+    // one key per token: into the caller's cache rows where they can be written as they are
+    const bool into = codes_into && scales_into && heads == 1 &&
+                      row_slots(*codes_into, s_len, dim, at::kFloat8_e4m3fn, 4) && scales_into->is_cuda() &&
+                      scales_into->scalar_type() == at::kFloat && scales_into->dim() == 1 &&
+                      scales_into->size(0) == s_len && (s_len <= 1 || scales_into->stride(0) >= 1);
+    Tensor codes = into ? *codes_into : empty({s_len, heads, dim}, at::kFloat8_e4m3fn, x);
+    Tensor scales = into ? *scales_into : empty({s_len, heads}, at::kFloat, x);
     OptTensor rotated, lw, lb, pos;
     if (return_rotated) rotated = empty({s_len, heads, dim}, at::kBFloat16, x);
     if (ln_weight) lw = ln_weight->to(at::kFloat).contiguous();
     if (ln_bias) lb = ln_bias->to(at::kFloat).contiguous();
     if (positions) pos = positions->to(at::kLong).contiguous();
-    check(p_rt_index_prep(x2.data_ptr(), data<float>(lw), data<float>(lb), data<int64_t>(pos), data<float>(fr),
+    check(p_rt_index_prep_into(x2.data_ptr(), data<float>(lw), data<float>(lb), data<int64_t>(pos), data<float>(fr),
                           fr.size(0), heads, codes.data_ptr(), data<float>(scales),
                           rotated ? rotated->data_ptr() : nullptr, s_len * heads, dim, 64, x2.stride(0),
+                          into ? codes.stride(0) : dim, into ? scales.stride(0) : 1,
                           static_cast<float>(eps), RT_BF16, stream()),
           "rt_index_prep");
+    if (into) {
+        codes.unsafeGetTensorImpl()->bump_version();
+        scales.unsafeGetTensorImpl()->bump_version();
+    } else if (codes_into && scales_into) {
+        codes_into->copy_(codes.view({s_len, heads * dim}));
+        scales_into->copy_(scales.view({s_len * heads}));
+    }
     return return_rotated ? py::make_tuple(codes, scales, *rotated) : py::make_tuple(codes, scales);
+}
+
+Tensor index_head_weights(const Tensor& both, const Tensor& q_scale, double c1, double c2) {
+    require_cuda({&both, &q_scale});
+    const int64_t rows = q_scale.size(0), heads = q_scale.size(1);
+    if (both.scalar_type() != at::kFloat || q_scale.scalar_type() != at::kFloat || q_scale.dim() != 2 ||
+        !same_shape(both, {rows, 2 * heads}) || !both.is_contiguous() || !q_scale.is_contiguous())
+        fail("index_head_weights: expected contiguous fp32 [S, 2 * H] and [S, H]");
+    Tensor out = empty({rows, heads}, at::kFloat, both);
+    check(p_rt_index_head_weights(data<float>(both), data<float>(q_scale), data<float>(out), rows, heads,
+                                  static_cast<float>(c1), static_cast<float>(c2), stream()),
+          "rt_index_head_weights");
+    return out;
 }
 
 Tensor fp8_index(const Tensor& q, const Tensor& weights, const Tensor& k, const Tensor& k_scale,
@@ -754,7 +799,6 @@ PYBIND11_MODULE(_rt_torch, m) {
     RT_DEF(linear_bf16);
     RT_DEF(linear_bf16_batched);
     RT_DEF(linear_fp8);
-    RT_DEF(linear_fp8_act);
     RT_DEF(gemm_nvfp4_grouped);
     RT_DEF(moe_route);
     RT_DEF(moe_permute);
@@ -764,6 +808,7 @@ PYBIND11_MODULE(_rt_torch, m) {
     RT_DEF(moe_combine);
     RT_DEF(moe_experts);
     RT_DEF(index_prep);
+    RT_DEF(index_head_weights);
     RT_DEF(fp8_index);
     RT_DEF(index_topk);
     RT_DEF(mla_sparse_decode);

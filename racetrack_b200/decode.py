@@ -110,17 +110,18 @@ class DecodeLayer(RealisticLayer):
         end = start_pos + 1
         positions = torch.full((batch,), start_pos, device=normed.device, dtype=torch.int64)
         qkv = self.w_qkv_a(normed)
-        q_c, kv_c, k_pe = ops.fused_norm_rope(
+        # the new token's latent row and rope key go straight into the caches
+        q_c, _, _ = ops.fused_norm_rope(
             qkv[:, :s.q_lora], self.q_norm, qkv[:, s.q_lora:s.q_lora + s.kv_lora], self.kv_norm,
-            qkv[:, s.q_lora + s.kv_lora:], positions, eps=s.eps, rope_base=s.rope_base)
+            qkv[:, s.q_lora + s.kv_lora:], positions, eps=s.eps, rope_base=s.rope_base,
+            _into=(c.kv[:, start_pos], c.pe[:, start_pos]))
         q = self.w_q_b(q_c).view(batch, h, s.qk_dim)
         ops.fused_rope_half(q[..., s.nope:], positions, rope_base=s.rope_base, inplace=True)
-        c.kv[:, start_pos] = kv_c
-        c.pe[:, start_pos] = k_pe
         # absorbed query: q_nope . W_UK per head (deepseek.py:799)
         q_abs = ops.linear_bf16_batched(q[..., :s.nope], self.w_uk_t)                    # [B, h, kv_lora]
         picked = indexer.indexer_decode(normed, q_c, self.index_weights, c.index_k, c.index_scale,
-                                        start_pos, self.freqs, self.index_topk)
+                                        start_pos, self.freqs, self.index_topk,
+                                        positions=positions)
         latent = ops.mla_sparse_decode(q_abs, q[..., s.nope:], c.kv[:, :end], c.pe[:, :end], picked,
                                        self.softmax_scale)                                 # [B, h, kv_lora]
         heads_out = ops.linear_bf16_batched(latent, self.w_uv)                          # [B, h, v]

@@ -84,13 +84,10 @@ def indexer_forward(x: torch.Tensor, qr: torch.Tensor, w: IndexerWeights, k_cach
     q = ops.linear_bf16(qr, w.wq_b).view(s_len, w.heads, w.head_dim)
     q_fp8, q_scale = ops.index_prep(q, freqs_cis, positions=positions)
     k = ops.linear_bf16(x, w.wk).view(s_len, 1, w.head_dim)
-    k_fp8, k_scale = ops.index_prep(k, freqs_cis, positions=positions,
-                                    ln_weight=w.k_norm_weight, ln_bias=w.k_norm_bias)
-    k_cache[start_pos:end_pos] = k_fp8.view(s_len, w.head_dim)
-    k_scale_cache[start_pos:end_pos] = k_scale.view(s_len)
+    ops.index_prep(k, freqs_cis, positions=positions, ln_weight=w.k_norm_weight, ln_bias=w.k_norm_bias,
+                   _into=(k_cache[start_pos:end_pos], k_scale_cache[start_pos:end_pos]))
     # per-head weights in fp32, as the reference forms them (deepseek.py:677-678)
-    head_w = ops.linear_f32_weight(x, w.weights_proj) * w.heads ** -0.5
-    head_w = head_w * q_scale * w.head_dim ** -0.5
+    head_w = ops.index_head_weights(x, w.weights_proj, q_scale)
     scores = ops.fp8_index(q_fp8.unsqueeze(0), head_w.unsqueeze(0), k_cache[:end_pos].unsqueeze(0),
                            k_scale_cache[:end_pos].unsqueeze(0),
                            causal_offset=start_pos if causal else None)
@@ -114,12 +111,9 @@ def indexer_decode(x: torch.Tensor, qr: torch.Tensor, w: IndexerWeights, k_cache
     q = ops.linear_bf16(qr, w.wq_b).view(batch, w.heads, w.head_dim)
     q_fp8, q_scale = ops.index_prep(q, freqs_cis, positions=positions)
     k = ops.linear_bf16(x, w.wk).view(batch, 1, w.head_dim)
-    k_fp8, k_scale = ops.index_prep(k, freqs_cis, positions=positions,
-                                    ln_weight=w.k_norm_weight, ln_bias=w.k_norm_bias)
-    k_cache[:, start_pos] = k_fp8.view(batch, w.head_dim)
-    k_scale_cache[:, start_pos] = k_scale.view(batch)
-    head_w = ops.linear_f32_weight(x, w.weights_proj) * w.heads ** -0.5
-    head_w = head_w * q_scale.view(batch, w.heads) * w.head_dim ** -0.5
+    ops.index_prep(k, freqs_cis, positions=positions, ln_weight=w.k_norm_weight, ln_bias=w.k_norm_bias,
+                   _into=(k_cache[:, start_pos], k_scale_cache[:, start_pos]))
+    head_w = ops.index_head_weights(x, w.weights_proj, q_scale)
     scores = ops.fp8_index(q_fp8.view(batch, 1, w.heads, w.head_dim), head_w.view(batch, 1, w.heads),
                            k_cache[:, :end_pos], k_scale_cache[:, :end_pos])
     return ops.index_topk(scores.view(batch, end_pos), index_topk)

@@ -13,7 +13,7 @@ expert), quantised once from bf16 with the same kernel that quantises activation
 from __future__ import annotations
 
 from dataclasses import dataclass
-from typing import Optional
+from typing import Callable, Optional
 
 import torch
 
@@ -103,7 +103,8 @@ def fused_moe_experts(x: Optional[torch.Tensor], weights: torch.Tensor, indices:
                       out_dtype: torch.dtype = torch.bfloat16,
                       parts: Optional[dict] = None,
                       x_quant: Optional[tuple] = None,
-                      out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                      out: Optional[torch.Tensor] = None,
+                      _around_w13: Optional[Callable[[bool], object]] = None) -> torch.Tensor:
     """y[t] = sum over the token's routed experts owned here of w * expert(x[t]) (+ shared[t]).
 
     x [T, hidden] bf16; weights fp32 [T, k] and indices int64 [T, k] from fused_moe_route;
@@ -115,6 +116,8 @@ def fused_moe_experts(x: Optional[torch.Tensor], weights: torch.Tensor, indices:
     token-sharded layer quantise their own rows and all-gather the codes.
     A dict passed as `parts` receives the intermediates (expert offsets, permutation, the two
     tensor-wide amax values, gate_up, h and the per-pair expert outputs) for stage-wise checks.
+    `_around_w13` is called with True before and False after the first expert GEMM is enqueued (a
+    benchmark's events).
     """
     q_codes, q_sf, q_gs = x_quant if x_quant is not None else (None, None, None)
     if out_dtype not in (torch.bfloat16, torch.float32):
@@ -122,7 +125,7 @@ def fused_moe_experts(x: Optional[torch.Tensor], weights: torch.Tensor, indices:
     y, *stages = _lib.native().moe_experts(
         x, weights, indices, experts.w13_codes, experts.w13_sf, experts.w13_gs, experts.w2_codes,
         experts.w2_sf, experts.w2_gs, experts.count, experts.inter, n_experts, expert_begin, shared,
-        out_dtype == torch.float32, q_codes, q_sf, q_gs, out)
+        out_dtype == torch.float32, q_codes, q_sf, q_gs, out, _around_w13)
     if parts is not None:
         parts.update(zip(("offsets", "sorted_pairs", "pair_pos", "x_gs", "x_amax", "gate_up", "h", "h_amax",
                           "expert_out"), stages))

@@ -114,7 +114,8 @@ def _inv_freq(half: int, base: float, device: torch.device) -> torch.Tensor:
 
 
 def fused_norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, positions, *, eps: float,
-                    rope_base: float, fallback: Optional[Callable] = None):
+                    rope_base: float, fallback: Optional[Callable] = None,
+                    _into: Optional[tuple] = None):
     """(rms_norm(q_c), rms_norm(kv_c), apply_rope(k_pe)) with half-split RoPE.
 
     Contract of partitions/dsv3_2/model.py:84-99 and its call site :333-344; the three
@@ -122,7 +123,8 @@ def fused_norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, positions, *, eps: flo
     """
     del fallback
     table = _inv_freq(k_pe.shape[-1] // 2, rope_base, k_pe.device)
-    return _native().norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, positions, table, None, eps)
+    into = _into if _into is not None else (None, None)
+    return _native().norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, positions, table, None, eps, *into)
 
 
 def fused_norm_rope_interleaved(q_c, q_weight, kv_c, kv_weight, k_pe, freqs_cis, *, eps: float,
@@ -131,7 +133,7 @@ def fused_norm_rope_interleaved(q_c, q_weight, kv_c, kv_weight, k_pe, freqs_cis,
     (racetrack/models/deepseek.py:766-776). ``freqs_cis`` is the complex64
     [seqlen, rope_dim/2] slice for the tokens; rows wrap around per batch element."""
     del fallback
-    return _native().norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, None, None, freqs_cis, eps)
+    return _native().norm_rope(q_c, q_weight, kv_c, kv_weight, k_pe, None, None, freqs_cis, eps, None, None)
 
 
 def fused_rope(x: torch.Tensor, freqs_cis: torch.Tensor, *, inplace: bool = False,
@@ -332,12 +334,8 @@ _SPLIT_WEIGHTS: dict[tuple, tuple] = {}     # key -> (hi | lo halves, the weight
 _SPLIT_WEIGHTS_MAX = 256
 
 
-def linear_f32_weight(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """F.linear(x.float(), weight) for bf16 x [..., K] and an fp32 weight [N, K] -> fp32 [..., N] on
-    the tensor cores: the weight is split once into two bf16 matrices hi + lo (exact to 16
-    mantissa bits: a relative 2^-17 per weight, below the fp32 round-off of a K-long sum), both
-    multiply x with fp32 accumulation in one launch, and the two halves are added. The fp32
-    projections of the model: the indexer's weights_proj (racetrack/models/deepseek.py:677)."""
+def _linear_f32_halves(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """x [..., K] times the bf16 halves hi | lo of an fp32 weight [N, K] -> fp32 [..., 2 * N]."""
     _require_cuda(x, weight)
     _require_bf16("linear_f32_weight x", x)
     if weight.dtype != torch.float32 or weight.dim() != 2:
@@ -353,9 +351,17 @@ def linear_f32_weight(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
         while len(_SPLIT_WEIGHTS) >= _SPLIT_WEIGHTS_MAX:
             _SPLIT_WEIGHTS.pop(next(iter(_SPLIT_WEIGHTS)))
         _SPLIT_WEIGHTS[key] = entry
-    split = entry[0]
-    n = weight.shape[0]
-    both = linear_bf16(x, split, out_dtype=torch.float32)
+    return linear_bf16(x, entry[0], out_dtype=torch.float32)
+
+
+def linear_f32_weight(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """F.linear(x.float(), weight) for bf16 x [..., K] and an fp32 weight [N, K] -> fp32 [..., N] on
+    the tensor cores: the weight is split once into two bf16 matrices hi + lo (exact to 16
+    mantissa bits: a relative 2^-17 per weight, below the fp32 round-off of a K-long sum), both
+    multiply x with fp32 accumulation in one launch, and the two halves are added. The fp32
+    projections of the model: the indexer's weights_proj (racetrack/models/deepseek.py:677)."""
+    n = weight.shape[0] if weight.dim() == 2 else 0
+    both = _linear_f32_halves(x, weight)
     return both[..., :n] + both[..., n:]
 
 
@@ -416,7 +422,8 @@ def linear_fp8_act(x: torch.Tensor, w_codes: torch.Tensor, w_scales: torch.Tenso
                    out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """`linear(x, weight)` with an FP8 weight as racetrack/models/deepseek.py:343-345 runs it:
     act_quant(x) then the FP8 block-scaled GEMM."""
-    return _native().linear_fp8_act(x, w_codes, w_scales, out)
+    codes, scales = fused_act_quant(x)
+    return linear_fp8(codes, scales, w_codes, w_scales, out=out)
 
 
 def moe_tile_map(offsets: torch.Tensor, g_begin: int, g_end: int, max_tiles: int):
@@ -445,7 +452,7 @@ def gemm_nvfp4_grouped(a_codes: torch.Tensor, a_sf: torch.Tensor, a_gs: torch.Te
 
 def index_prep(x: torch.Tensor, freqs_cis: torch.Tensor, *, positions: Optional[torch.Tensor] = None,
                ln_weight: Optional[torch.Tensor] = None, ln_bias: Optional[torch.Tensor] = None,
-               eps: float = 1e-6, return_rotated: bool = False):
+               eps: float = 1e-6, return_rotated: bool = False, _into: Optional[tuple] = None):
     """The indexer's path from projected rows to FP8 in one pass (racetrack/models/deepseek.py:
     659-676): [LayerNorm for keys] -> non-interleaved RoPE on the first 64 dims -> Hadamard
     rotation -> act_quant.
@@ -453,7 +460,15 @@ def index_prep(x: torch.Tensor, freqs_cis: torch.Tensor, *, positions: Optional[
     x bf16 [S, H, 128] (H = 1 for keys); freqs_cis complex64 [table, 32]; positions int64 [S]
     (default 0..S-1). Returns (codes float8_e4m3fn [S, H, 128], scales fp32 [S, H]) and, on
     request, the rotated bf16 tensor that was quantised."""
-    return _native().index_prep(x, freqs_cis, positions, ln_weight, ln_bias, eps, return_rotated)
+    into = _into if _into is not None else (None, None)
+    return _native().index_prep(x, freqs_cis, positions, ln_weight, ln_bias, eps, return_rotated, *into)
+
+
+def index_head_weights(x: torch.Tensor, weights_proj: torch.Tensor, q_scale: torch.Tensor) -> torch.Tensor:
+    """linear(x, weights_proj) * H^-0.5 * q_scale * 128^-0.5 in fp32 (racetrack/models/deepseek.py:677-678):
+    x bf16 [S, dim], weights_proj fp32 [H, dim], q_scale fp32 [S, H] as index_prep returns it."""
+    heads = weights_proj.shape[0]
+    return _native().index_head_weights(_linear_f32_halves(x, weights_proj), q_scale, heads ** -0.5, 128 ** -0.5)
 
 
 def fp8_index(q: torch.Tensor, weights: torch.Tensor, k: torch.Tensor, k_scale: torch.Tensor, *,

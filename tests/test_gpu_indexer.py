@@ -300,3 +300,50 @@ def test_indexer_decode_equals_the_single_sequence_path():
         assert torch.equal(idx[b], one[0])
     assert torch.equal(k_cache.view(torch.uint8), k1.view(torch.uint8))
     assert torch.equal(ks_cache, s1)
+
+
+@pytest.mark.parametrize("rows,heads", [(1, 64), (13, 64), (257, 8)])
+def test_index_head_weights_equal_the_separate_operations(ops, rows, heads):
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, 256, generator=g).bfloat16().cuda()
+    w = (torch.randn(heads, 256, generator=g) * 0.05).cuda()
+    q_scale = torch.rand(rows, heads, generator=g).cuda()
+    want = ops.linear_f32_weight(x, w) * heads ** -0.5
+    want = want * q_scale * 128 ** -0.5
+    assert torch.equal(ops.index_head_weights(x, w, q_scale), want)
+
+
+@pytest.mark.parametrize("kind", ["in place", "padded rows", "bf16 scales", "odd row pitch"])
+def test_key_rows_written_into_a_cache(ops, kind):
+    """index_prep into cache rows: in place where the cache can take them, through a copy otherwise;
+    the rows around them stay."""
+    g = torch.Generator().manual_seed(5)
+    x = torch.randn(4, 1, 128, generator=g).bfloat16().cuda()
+    freqs = torch.polar(torch.ones(9, 32), torch.randn(9, 32, generator=g)).cuda()
+    pos = torch.tensor([3, 1, 8, 0], device="cuda")
+    codes, scales = ops.index_prep(x, freqs, positions=pos)
+    width = {"padded rows": 160, "odd row pitch": 130}.get(kind, 128)
+    cache = torch.zeros(4, 7, width, device="cuda").to(torch.float8_e4m3fn)
+    scale_cache = torch.zeros(4, 7, device="cuda", dtype=torch.bfloat16 if kind == "bf16 scales" else torch.float32)
+    version = cache._version
+    ops.index_prep(x, freqs, positions=pos, _into=(cache[:, 2, :128], scale_cache[:, 2]))
+    assert cache._version > version
+    assert torch.equal(cache[:, 2, :128].view(torch.uint8), codes.view(4, 128).view(torch.uint8))
+    assert torch.equal(scale_cache[:, 2], scales.view(4).to(scale_cache.dtype))
+    rest = [0, 1, 3, 4, 5, 6]
+    assert not cache[:, rest].view(torch.uint8).any() and not scale_cache[:, rest].any()
+
+
+def test_latent_rows_written_into_a_cache(ops):
+    g = torch.Generator().manual_seed(6)
+    qkv = torch.randn(5, 2112, generator=g).bfloat16().cuda()
+    ones = torch.ones(2048, device="cuda", dtype=torch.bfloat16)
+    pos = torch.full((5,), 77, device="cuda")
+    args = (qkv[:, :1536], ones[:1536], qkv[:, 1536:2048], ones[:512], qkv[:, 2048:], pos)
+    want = ops.fused_norm_rope(*args, eps=1e-6, rope_base=10000.0)
+    for kv_w, pe_w in ((512, 64), (520, 66), (513, 64)):      # the last pitch cannot be written in place
+        kv = torch.zeros(5, 3, kv_w, device="cuda", dtype=torch.bfloat16)
+        pe = torch.zeros(5, 3, pe_w, device="cuda", dtype=torch.bfloat16)
+        q, _, _ = ops.fused_norm_rope(*args, eps=1e-6, rope_base=10000.0, _into=(kv[:, 1, :512], pe[:, 1, :64]))
+        assert torch.equal(q, want[0]) and torch.equal(kv[:, 1, :512], want[1]) and torch.equal(pe[:, 1, :64], want[2])
+        assert not kv[:, [0, 2]].any() and not pe[:, [0, 2]].any() and not kv[:, 1, 512:].any() and not pe[:, 1, 64:].any()
