@@ -301,21 +301,10 @@ class PrefillStackWorkload:
 
     def _wrap_dominant(self):
         """CUDA events around every first expert GEMM (w13) of the timed region."""
-        ops, inter2 = self.ops, 2 * self.shape.moe_inter // getattr(self, "moe_tp", 1)
-        inner = ops.gemm_nvfp4_grouped
+        ops = self.ops
         wl = self
 
-        def timed(*a, **kw):
-            if wl.recording and kw.get("n") == inter2:
-                s, e = wl._event_pair()
-                s.record()
-                out = inner(*a, **kw)
-                e.record()
-                return out
-            return inner(*a, **kw)
-
         self.recording = False
-        ops.gemm_nvfp4_grouped = timed
         if self.ffn == "dense":
             # the gate-up projection [2 * 18432 / world, 7168] of the dense FFN
             rows13 = 2 * self.shape.dense_inter // self.world
@@ -334,14 +323,20 @@ class PrefillStackWorkload:
             ops.linear_fp8 = timed_linear(ops.linear_fp8, 2)      # (codes, scales, w_codes, w_scales)
             ops.linear_bf16 = timed_linear(ops.linear_bf16, 1)    # (x, weight)
         # experts that actually receive tokens (their weights are what the GEMM reads)
-        inner_permute = ops.fused_moe_permute
+        moe = self.layer_mod.moe
+        inner_experts = moe.fused_moe_experts
         self.touched = []
         self.rank_rows = []       # per recorded layer: routed rows of every rank's expert block
 
-        def permute(indices, n_experts):
-            out = inner_permute(indices, n_experts)
-            if wl.recording and len(wl.touched) < 64:
-                off = out[0]
+        def experts(*a, n_experts, parts=None, **kw):
+            if not wl.recording:
+                return inner_experts(*a, n_experts=n_experts, parts=parts, **kw)
+            s, e = wl._event_pair()
+            parts = {} if parts is None else parts
+            out = inner_experts(*a, n_experts=n_experts, parts=parts,
+                                _around_w13=lambda begin: (s if begin else e).record(), **kw)
+            if len(wl.touched) < 64:
+                off = parts["offsets"]
                 lo = wl.ep_rank * (n_experts // wl.ep_world)
                 hi = lo + n_experts // wl.ep_world
                 wl.touched.append(((off[lo + 1:hi + 1] - off[lo:hi]) > 0).sum())
@@ -349,7 +344,7 @@ class PrefillStackWorkload:
                     wl.rank_rows.append((off[1:] - off[:-1]).view(wl.ep_world, -1).sum(-1))
             return out
 
-        ops.fused_moe_permute = permute
+        moe.fused_moe_experts = experts
 
     @property
     def units_per_step(self) -> int:
@@ -579,20 +574,18 @@ class MoeLayerWorkload:
         sw13, sw2 = layer.draw_expert(s, s.n_experts, device, std=0.02)     # the shared expert
         self.sw13, self.sw2 = sw13.contiguous(), sw2.contiguous()
         self.dom_events, self.recording = [], False
-        inner = ops.gemm_nvfp4_grouped
+        inner = self.moe.fused_moe_experts
         wl = self
 
         def timed(*a, **kw):
-            if wl.recording and kw.get("n") == 2 * s.moe_inter:
-                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-                e0.record()
-                out = inner(*a, **kw)
-                e1.record()
-                wl.dom_events.append((e0, e1))
-                return out
-            return inner(*a, **kw)
+            if not wl.recording:
+                return inner(*a, **kw)
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            out = inner(*a, _around_w13=lambda begin: (e0 if begin else e1).record(), **kw)
+            wl.dom_events.append((e0, e1))
+            return out
 
-        ops.gemm_nvfp4_grouped = timed
+        self.moe.fused_moe_experts = timed
 
     @property
     def units_per_step(self) -> int:
