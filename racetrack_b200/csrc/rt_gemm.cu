@@ -744,13 +744,11 @@ __global__ void __launch_bounds__(kFThreads, 1) gemm_nvfp4_kernel(
 // token scales); the epilogue drains the accumulator into registers, releases it, and only
 // then writes: lane = weight row = output column, so one warp store covers 64 contiguous bytes
 // of one token's output row.
-// What the issuing thread does per operand stage is the pace of this kernel once the operands
-// arrive in time: a tcgen05.mma costs it about 65 cycles, a commit as much and a barrier wait
-// 100 - 250, whatever the MMA's shape (trace of the first version: two waits, four MMAs and two
-// commits per K block, 800 cycles for 540 cycles of tensor work, the same for 16-token tiles).
-// So a stage is ONE wait, eight MMAs and ONE commit: the scale loaders arrive on the same
-// "stage full" barrier as the operands, and one multicast commit per stage tells both CTAs
-// that the stage's shared memory AND its scale columns are free.
+// What the issuing thread does per operand stage matters once the operands arrive in time: ONE
+// wait, eight MMAs and ONE commit. The scale loaders arrive on the same "stage full" barrier as the
+// operands, and one multicast commit per stage tells both CTAs that the stage's shared memory AND
+// its scale columns are free. (The loop's operands in uniform registers, see elect_one: w2 of 4096
+// tokens 842 -> 638 us, of 8192 1072 -> 858.)
 // Warps (both CTAs): 0 operand producer (one elected thread), 1 tensor-memory owner and MMA
 // issuer (leader CTA, cluster rank 0) or relay (peer: tells the leader that its operands have
 // landed), 2-5 scale loaders (shared -> tensor memory), 6-13 epilogue (lane quarter w % 4,
@@ -1261,23 +1259,12 @@ __global__ void __launch_bounds__(1024) moe_tile_map_kernel(const int32_t* __res
 // Tile 128 x 256, stage = one K block: 16 KB of A + 32 KB of B, 4 stages.
 // Warps: 0 TMA producer, 1 MMA issuer, 2-9 epilogue (warp w: lane quarter w % 4, column half
 // (w - 2) / 4).
-// What holds it at about 975 cycles per K block (1.8-1.9 PFLOP/s; the four MMAs of a K block
-// take 512): the round trip of a buffer. Measured in isolation on this part: an e4m3
-// 128 x 256 x 32 MMA takes 128 cycles back to back (twice the bf16 flops per cycle); tensor-memory
-// loads and MMAs do not slow each other down (the fold alone, eight warps, 386 cycles per
-// 128 x 256 block, with or without MMAs running); one hop through an mbarrier (arrive or commit
-// -> the parked waiter runs again) costs 145-175 cycles; and four MMAs issued into an IDLE
-// tensor pipe are seen complete by a waiter 977 cycles after the first issue (about 260 cycles
-// from issue to execution, 512 of execution, the hop). With two buffers a buffer comes back after
-// issue + execution + hop + loads + hop + the issuing thread's own wait, about 1900 cycles, and
-// two K blocks fit into that. Tried and measured no faster, because none of them shortens that
-// loop: a CTA-pair variant (256 x 256 tiles, two thirds of the operand bytes per K block, one
-// wait and one multicast commit per K block), a second issuing thread (one per buffer), one
-// arrival per warp instead of per thread, polling instead of parked waits, and the issuing thread
-// looking at the next K block's barriers before its last MMA. A third buffer does not fit (512
-// tensor-memory columns), narrower buffers make the issuing thread the limit (eight MMAs per K
-// block), and 16 fold warps or a register copy of the whole buffer before the fold do not fit
-// the register file (128 accumulators per thread).
+// What holds it at about 885 cycles per K block (1.9-2.15 PFLOP/s; the four MMAs take 512): shared
+// memory, 48 KB of operands written and 48 KB read per K block at 128 bytes a cycle are 768, and the
+// fold warps' chain of wait, tensor-memory load and 128 FMAs behind it. Measured against 975 us for
+// 8192 x 7168 x 16384 on one B200: a fold that reads a quarter of the buffer 842 (the rest is not the
+// fold), four 128-column buffers 1000 (A is read twice), CTA pairs with 256 x 256 tiles 1108 (a
+// third less shared-memory traffic, but the buffer's round trip crosses CTAs), 16 fold warps 1549.
 constexpr int kQBN = 256;
 constexpr int kQBK = 128;
 constexpr int kQStages = 4;
