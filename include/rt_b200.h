@@ -437,7 +437,9 @@ int rt_gemm_bf16_batched(const void* a, const void* b, void* c, int64_t batch, i
  * ldo) as RT_BF16 (one rounding of the fp32 sum, as a single-pass GEMM does) or RT_F32.
  * The summation order is fixed, so the result is bit-reproducible from run to run and equal
  * on every rank that computes it from the same operands. splits =
- * rt_gemm_bf16_splitk_splits(m, n, k).
+ * rt_gemm_bf16_splitk_splits(m, n, k): a function of n and k alone for up to 128 rows (a row's sum does
+ * not depend on how many others are in the call), 1 for more rows, which rt_gemm_bf16 adds over the
+ * whole of K in one order whatever tiles it picks.
  * ref: racetrack/models/deepseek.py:316-345 (linear with bf16 weights -> F.linear).
  */
 int64_t rt_gemm_bf16_splitk_splits(int64_t m, int64_t n, int64_t k);

@@ -10,6 +10,8 @@
 // The accumulator is double buffered in tensor memory, so the epilogue of tile i
 // overlaps the main loop of tile i+1. Every wait is bounded (rt_tc.cuh).
 #include <algorithm>
+#include <type_traits>
+#include <utility>
 
 #include "rt_tc.cuh"
 
@@ -23,14 +25,14 @@ constexpr int kGroupM = 16;      // m-tiles walked before moving to the next n-t
 
 template <int BN>
 struct GemmCfg {
-    static constexpr int kStages = (BN == 256) ? 4 : 6;
+    static constexpr int kStages = BN == 256 ? 4 : BN == 128 ? 6 : BN == 64 ? 8 : 10;   // about 200 KB
     static constexpr uint32_t kABytes = kBM * kBK * 2;
     static constexpr uint32_t kBBytes = BN * kBK * 2;
     static constexpr uint32_t kStageBytes = kABytes + kBBytes;
     static constexpr uint32_t kBarOffset = kStages * kStageBytes;
     // full[S], empty[S], tmem_full[2], tmem_empty[2], tmem slot, abort flag
     static constexpr uint32_t kSmemBytes = kBarOffset + (2 * kStages + 4) * 8 + 16 + 1024;
-    static constexpr uint32_t kTmemCols = 2 * BN;  // 256 or 512: powers of two
+    static constexpr uint32_t kTmemCols = 2 * BN;  // 64 ... 512: powers of two
     // instruction descriptor: fp32 accumulate, bf16 x bf16, both K-major, N, M = 128
     static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) |
                                        (static_cast<uint32_t>(BN >> 3) << 17) |
@@ -1884,25 +1886,52 @@ static int launch_bf16(const void* a, const void* b, void* c, int64_t M, int64_t
     return check_launch("gemm_bf16_kernel");
 }
 
-// How many ranges the K blocks of a product with `tiles` output tiles are cut into: the count with
-// the smallest estimate of ((rounds of work items over the SMs) x (K blocks of an item, half a block
-// for the change of tile) + 4 for the first loads and the last epilogue) x (time of a K block) + the
-// pass that adds the slabs (a launch, then slab_bytes written and read per range). One item per SM
-// and round, so 56 tiles take 5 ranges (280 items, two rounds of 148), not 6 (336, a third round
-// for a quarter of the SMs). 64 x 7168 x 16384 on one B200: 52 -> 44 us, 4096 x 256 x 7168 (32 whole
-// tiles before) 47 -> 23, 2048 x 128 x 7168 28 -> 15.
-static int64_t pick_splits(int64_t tiles, int64_t num_kb, int64_t min_kb, double kb_us, double slab_bytes) {
-    const int64_t sms = sm_count();
+// How many ranges the K blocks of a product of at most 128 rows (one row of `tiles` output tiles) are
+// cut into: the count with the smallest estimate of ((rounds of work items over the SMs) x (K blocks
+// of an item, half a block for the change of tile) + 4 for the first loads and the last epilogue) x
+// (0.25 us, a K block of 64 of a 128 x 128 tile) + the pass that adds the slabs (a launch, then a
+// slab written and read per range). One item per SM and round, so 56 tiles take 5 ranges (280 items,
+// two rounds of 148), not 6 (336, a third round for a quarter of the SMs): 64 x 7168 x 16384 on one
+// B200 53 -> 44 us. The slab is estimated for kSplitRows rows whatever the call has: the cut, and with
+// it the order in which a row's products are added, depends on the weight alone, so a token has the
+// same bits in every batch of up to 128. (32: a cut that pays there costs fewer rows nothing, 13 or
+// 5 ranges of 1 x 7168 x 16384 take 42 us alike; the 3 ranges that one row's slab allows 24576 x 1536
+// take 24 us at 64 rows against 18 whole.)
+constexpr double kSplitRows = 32;
+static int64_t pick_splits(int64_t n, int64_t k) {
+    const int64_t sms = sm_count(), tiles = (n + 127) / 128, num_kb = (k + kBK - 1) / kBK;
+    const double kb_us = 0.25, slab_us = 4.0 * kSplitRows * static_cast<double>(n) / 3.0e6;
     int64_t best = 1;
     double best_us = (static_cast<double>((tiles + sms - 1) / sms) * (num_kb + 0.5) + 4) * kb_us;
-    for (int64_t s = 2; s <= num_kb / min_kb && s <= 64; ++s) {
+    for (int64_t s = 2; s <= num_kb / 4 && s <= 64; ++s) {
         const int64_t per = (num_kb + s - 1) / s;
         if ((num_kb + per - 1) / per != s) continue;             // a range would be empty
         const double us = (static_cast<double>((tiles * s + sms - 1) / sms) * (per + 0.5) + 4) * kb_us + 2.0 +
-                          s * slab_bytes / 3.0e6;
+                          s * slab_us;
         if (us < best_us) {
             best_us = us;
             best = s;
+        }
+    }
+    return best;
+}
+
+// Columns of an output tile of the single-CTA kernel: the width with the smallest product of rounds
+// over the SMs and time of a K block. Every width adds a row's products in the same order, so this
+// choice, unlike a cut of K, may depend on the number of rows: narrow tiles are what occupies the SMs
+// when a prefill meets few columns (a router, an index projection). The times, of a round with K =
+// 7168 on one B200: 47 us at 256 columns, 27 at 128, 20 at 64, 18 at 32 (a K block brings 16 KB of A
+// whatever the width). As 256-wide tiles, then by this rule: 4096 x 256 x 7168 47 -> 22 us,
+// 777 x 256 x 7168 47 -> 18.5, 777 x 2112 x 7168 49 -> 29, 2048 x 128 x 7168 41 -> 19.
+static int bf16_tile_cols(int64_t m, int64_t n) {
+    const int64_t sms = sm_count(), m_tiles = (m + kBM - 1) / kBM;
+    int best = 256;
+    double best_cost = 1e300;
+    for (const auto& [cols, cost_kb] : {std::pair<int, double>{256, 1.75}, {128, 1.0}, {64, 0.72}, {32, 0.66}}) {
+        const double cost = static_cast<double>((m_tiles * ((n + cols - 1) / cols) + sms - 1) / sms) * cost_kb;
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = cols;
         }
     }
     return best;
@@ -2381,19 +2410,18 @@ extern "C" int rt_gemm_bf16(const void* a, const void* b, void* c, int64_t m, in
         if (out_dtype == RT_F32) return tc::launch_bf16_pair<true>(a, b, c, m, n, k, lda, ldb, ldc, st);
         return tc::launch_bf16_pair<false>(a, b, c, m, n, k, lda, ldb, ldc, st);
     }
-    // a K block of a 128 x 256 tile takes 1.6 times as long as one of 128 x 128: narrow tiles where
-    // they need less than that many more rounds over the SMs (777 x 2112 x 7168: 119 tiles against
-    // 63, both one round)
-    const int64_t m_tiles = (m + 127) / 128, sms = tc::sm_count();
-    const int64_t rounds_narrow = (m_tiles * ((n + 127) / 128) + sms - 1) / sms;
-    const int64_t rounds_wide = (m_tiles * ((n + 255) / 256) + sms - 1) / sms;
-    const bool narrow = n <= 128 || 5 * rounds_narrow < 8 * rounds_wide;
-    if (out_dtype == RT_F32) {
-        if (narrow) return tc::launch_bf16<128, true>(a, b, c, m, n, k, lda, ldb, ldc, st);
-        return tc::launch_bf16<256, true>(a, b, c, m, n, k, lda, ldb, ldc, st);
+    const bool f32 = out_dtype == RT_F32;
+    auto launch = [&](auto cols) {
+        constexpr int kCols = decltype(cols)::value;
+        return f32 ? tc::launch_bf16<kCols, true>(a, b, c, m, n, k, lda, ldb, ldc, st)
+                   : tc::launch_bf16<kCols, false>(a, b, c, m, n, k, lda, ldb, ldc, st);
+    };
+    switch (tc::bf16_tile_cols(m, n)) {
+        case 32: return launch(std::integral_constant<int, 32>{});
+        case 64: return launch(std::integral_constant<int, 64>{});
+        case 128: return launch(std::integral_constant<int, 128>{});
+        default: return launch(std::integral_constant<int, 256>{});
     }
-    if (narrow) return tc::launch_bf16<128, false>(a, b, c, m, n, k, lda, ldb, ldc, st);
-    return tc::launch_bf16<256, false>(a, b, c, m, n, k, lda, ldb, ldc, st);
 }
 
 extern "C" int rt_gemm_bf16_batched(const void* a, const void* b, void* c, int64_t batch, int64_t m,
@@ -2415,9 +2443,10 @@ extern "C" int rt_gemm_bf16_batched(const void* a, const void* b, void* c, int64
 }
 
 extern "C" int64_t rt_gemm_bf16_splitk_splits(int64_t m, int64_t n, int64_t k) {
-    if (m <= 0 || n <= 0 || k <= 0 || tc::g_bf16_schedule != 0 || bf16_pair_pays(m, n, k)) return 1;
-    // a K block of 64 of a 128 x 128 tile: 0.25 us of its CTA
-    return tc::pick_splits(((m + 127) / 128) * ((n + 127) / 128), (k + 63) / 64, 4, 0.25, 4.0 * m * n);
+    // more rows than one row tile: K stays whole, so that a token's sums (a router's logits above all)
+    // do not depend on how many others are in the call; the tile width occupies the SMs instead
+    if (m <= 0 || m > 128 || n <= 0 || k <= 0 || tc::g_bf16_schedule != 0) return 1;
+    return tc::pick_splits(n, k);
 }
 
 extern "C" int rt_gemm_bf16_splitk(const void* a, const void* b, float* workspace, void* out,

@@ -308,7 +308,9 @@ def tc_error_state() -> None:
     _lib.check(_lib.load().rt_tc_error_state(), "tensor-core kernel")
 
 
-SPLITK_MAX_ROWS = 65536   # linear_bf16 never splits K for more rows than this
+# linear_bf16 cuts K for at most this many rows: one row tile, where the cut is a property of the weight
+# alone (rt_gemm_bf16_splitk_splits). 0 turns it off.
+SPLITK_MAX_ROWS = 128
 
 
 def linear_bf16(x: torch.Tensor, weight: torch.Tensor, *,

@@ -272,10 +272,11 @@ def test_linear_bf16_split_k_for_few_rows(ops, m, n, k, out_dtype):
 
 
 @pytest.mark.parametrize("m,n,k,out_dtype,splits", [
-    (777, 256, 7168, torch.float32, True),     # router logits of a prefill: 14 tiles, split
-    (2048, 128, 7168, torch.bfloat16, True),   # the indexer's key projection: one column of tiles
-    (129, 136, 1096, torch.float32, True),     # second row and column tile nearly empty, partial K block
-    (1000, 2112, 7168, torch.bfloat16, False), # narrow tiles instead of split ones
+    (777, 256, 7168, torch.float32, False),    # router logits of a prefill: tiles of 32 columns, K whole
+    (2048, 128, 7168, torch.bfloat16, False),  # the indexer's key projection: one column of 128-wide tiles
+    (129, 136, 1096, torch.float32, False),    # second row tile and last column tile nearly empty, partial K block
+    (128, 136, 1096, torch.float32, True),     # one row tile: cut along K
+    (1000, 2112, 7168, torch.bfloat16, False), # ragged last column tile
     (64, 24576, 1536, torch.bfloat16, None),   # few rows against many columns: never CTA pairs
     (3, 40, 264, torch.bfloat16, False),       # a box of 8 rows, 3 of them there
 ])
@@ -294,6 +295,36 @@ def test_linear_bf16_tile_and_split_choice(ops, m, n, k, out_dtype, splits):
     if out_dtype == torch.bfloat16:
         bound += 2.0 ** -8 * ref.abs()
     assert bool(((out.double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("n,k,out_dtype", [
+    (256, 7168, torch.float32),      # router logits: a last bit decides between experts of nearly equal score
+    (128, 7168, torch.bfloat16),     # the indexer's key projection
+    (2112, 7168, torch.bfloat16),    # qkv_a, whose rows a token-sharded layer spreads over ranks
+    (520, 1096, torch.float32),      # ragged tiles, partial K block (no CTA pairs)
+])
+def test_linear_bf16_rows_do_not_depend_on_the_call(ops, n, k, out_dtype):
+    """A row of x gives the same bits in every call of more than 128 rows, whatever tile width or
+    schedule its size selects, and in every call of up to 128 (where K is cut by n and k alone)."""
+    x = I.randn((4500, k), 900 + n).cuda()
+    w = I.randn((n, k), 901 + n, std=0.02).cuda()
+
+    def rows(m):
+        return ops.linear_bf16(x[:m], w, out_dtype=out_dtype)
+    few, many = rows(128), rows(129)
+    for m in (1, 8, 9, 13, 32, 64, 127):
+        assert torch.equal(rows(m), few[:m]), m
+    for m in (200, 512, 777, 1024, 2048, 2049, 4096, 4500):
+        assert torch.equal(rows(m)[:129], many), m
+    # the last rows of a call as well as the first
+    assert torch.equal(ops.linear_bf16(x[4000:], w, out_dtype=out_dtype), rows(4500)[4000:])
+    for schedule in (1, 2):
+        previous = ops.gemm_bf16_schedule(schedule)
+        try:
+            assert torch.equal(rows(777)[:129], many), schedule
+        finally:
+            ops.gemm_bf16_schedule(previous)
+    ops.tc_error_state()
 
 
 @pytest.mark.parametrize("m,n,k", [

@@ -248,3 +248,20 @@ def test_experts_quantise_few_rows_in_expert_order(mods, tokens):
     want = moe.fused_moe_experts(None, weights, indices, experts, n_experts=16,
                                  x_quant=(codes, sf.view(torch.uint8), gs))
     assert torch.equal(got, want)
+
+
+def test_a_token_is_routed_alike_in_calls_of_different_length(mods):
+    """The experts and weights of a token do not depend on how many tokens a prefill chunk holds."""
+    ops, _moe = mods
+    g = torch.Generator(device="cuda").manual_seed(17)
+    x = torch.empty(4096, 7168, device="cuda").normal_(generator=g).bfloat16()
+    gate = torch.empty(256, 7168, device="cuda").normal_(0.0, 0.02, generator=g).bfloat16()
+    bias = torch.empty(256, device="cuda").uniform_(-0.1, 0.1, generator=g)
+
+    def route(m):
+        logits = ops.linear_bf16(x[:m], gate, out_dtype=torch.float32)
+        return ops.fused_moe_route(logits, bias, n_groups=8, topk_groups=4, topk=8, route_scale=2.5)
+    weights, indices = route(4096)
+    for m in (200, 777, 2048):
+        w, i = route(m)
+        assert torch.equal(i, indices[:m]) and torch.equal(w, weights[:m]), m
