@@ -562,14 +562,24 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return y;
 }
 
+// max(x, c) that hands on a NaN (fmaxf would return c).
+__device__ __forceinline__ float max_nan(float x, float c) {
+    float y;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(x), "f"(c));
+    return y;
+}
+
 // 2^x of a pair for x <= 8 on the FMA pipe, two elements per instruction: x = n + f with
 // n = round(x), |f| <= 1/2, 2^f by the degree-5 minimax polynomial (Remez; relative error 2.3e-7
-// evaluated in fp32, as much as ex2.approx), 2^n by adding n to the exponent field. Inputs below
-// -125 give 0 to within 2^-125.
+// evaluated in fp32, as much as ex2.approx), times 2^n. As with ex2.approx a NaN comes out as NaN
+// and what lies below the range of an exponent, -infinity of a masked score above all, as exactly 0:
+// 2^n is a factor whose bits are those of n + 127 in the exponent field, none of them set at n = -127.
+// (Added to the exponent field of 2^f instead, n would make a finite number of a NaN and leave 2^-125
+// of a masked score.)
 __device__ __forceinline__ void ex2_poly2(uint64_t x, float& p0, float& p1) {
     float x0, x1;
     unpack_f32x2(x, x0, x1);
-    x = pack_f32x2(fmaxf(x0, -125.f), fmaxf(x1, -125.f));
+    x = pack_f32x2(max_nan(x0, -127.f), max_nan(x1, -127.f));
     const uint64_t magic = pack_f32x2(12582912.f, 12582912.f);    // 1.5 * 2^23: the integer part lands in the low bits
     const uint64_t nmagic = pack_f32x2(-12582912.f, -12582912.f);
     const uint64_t t = add_f32x2(x, magic);
@@ -581,9 +591,9 @@ __device__ __forceinline__ void ex2_poly2(uint64_t x, float& p0, float& p1) {
     p = fma_f32x2(p, f, pack_f32x2(1.00000007f, 1.00000007f));
     float t0, t1;
     unpack_f32x2(t, t0, t1);
-    unpack_f32x2(p, p0, p1);
-    p0 = __uint_as_float(__float_as_uint(p0) + (__float_as_uint(t0) << 23));
-    p1 = __uint_as_float(__float_as_uint(p1) + (__float_as_uint(t1) << 23));
+    const float n0 = __uint_as_float((__float_as_uint(t0) << 23) + 0x3f800000u);
+    const float n1 = __uint_as_float((__float_as_uint(t1) << 23) + 0x3f800000u);
+    unpack_f32x2(mul_f32x2(p, pack_f32x2(n0, n1)), p0, p1);
 }
 
 // 32 scores of one row -> 32 probabilities as 16 bf16 pairs, and their fp32 sum (in two pairs of

@@ -180,3 +180,45 @@ def test_fp8_epilogue_equals_act_quant_of_the_bf16_output(tokens, heads):
     w2 = ops.fused_act_quant(ops.attention_prefill(q2, k2, kpe[:, :32].contiguous(), v2).view(tokens, heads * 128))
     assert torch.equal(c2.view(torch.uint8), w2[0].view(torch.uint8)) and torch.equal(s2, w2[1])
     ops.tc_error_state()
+
+
+@pytest.mark.parametrize("first", [0, 32, 96, 160])
+@pytest.mark.parametrize("special", [float("nan"), float("inf"), float("-inf")])
+def test_a_special_key_at_every_column(ops, first, special):
+    """Head h has one key of infinite or NaN scores, at column first + h of its keys, so every column of
+    a 32-key group is met: as in torch, a NaN or +infinity among the scores makes the row NaN from that
+    key on, -infinity takes the key out (whatever its value), and the rows before it do not change."""
+    tokens, heads = 257, 32
+    q, kn, kp, v = (t.cuda() for t in _qkv(tokens, heads, 128, 64, 128, 300 + first))
+    q[..., 0] = 1.0                                           # the special key dim reaches every query as it is
+    at = first + torch.arange(heads, device="cuda")
+    h = torch.arange(heads, device="cuda")
+    clean = ops.attention_prefill(q, kn, kp, v)
+    kn2, v2 = kn.clone(), v.clone()
+    kn2[at, h, 0] = special
+    if special == float("-inf"):
+        v2[at, h] = 3.0e38
+    got = ops.attention_prefill(q, kn2, kp, v2)
+    ops.tc_error_state()
+    before = torch.arange(tokens, device="cuda")[:, None] < at[None, :]          # [T, H]
+    assert torch.equal(got[before], clean[before])
+    if special != float("-inf"):
+        wrong = ~got[~before].isnan().all(dim=-1)
+        assert not wrong.any(), f"{int(wrong.sum())} rows are not NaN"
+        return
+    want = _reference(q.cpu(), kn2.cpu(), kp.cpu(), v.cpu()).cuda()              # the key's value does not matter
+    row0 = (at == 0)[None, :] & (torch.arange(tokens, device="cuda") == 0)[:, None]
+    assert got[row0].isnan().all()                                               # no other key is left
+    assert rel_err(got[~before & ~row0], want[~before & ~row0]) <= 1e-2
+
+
+@pytest.mark.parametrize("tokens", [64, 128, 200, 257])
+def test_masked_keys_weigh_nothing(ops, tokens):
+    """Values of keys behind a query do not reach it, however large they are."""
+    q, kn, kp, v = (t.cuda() for t in _qkv(tokens, 2, 128, 64, 128, 400 + tokens))
+    for cut in (1, 11, 33, tokens // 2, tokens - 1):
+        small, large = v.clone(), v.clone()
+        small[cut:], large[cut:] = 0.0, 3.0e38
+        a, b = ops.attention_prefill(q, kn, kp, small), ops.attention_prefill(q, kn, kp, large)
+        assert torch.equal(a[:cut], b[:cut]), cut
+    ops.tc_error_state()
