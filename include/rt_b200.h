@@ -460,15 +460,13 @@ int rt_gemm_bf16_splitk(const void* a, const void* b, float* workspace, void* ou
 int rt_gemm_fp8(const void* a, const float* a_scales, const void* b, const float* b_scales,
                 void* c, int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb, int64_t ldc,
                 void* stream);
-/* The same with rt_gemm_fp8_workspace_bytes(m, n, k) bytes of device scratch (16-byte aligned; NULL
- * is rt_gemm_fp8): the output tiles that do not fill a round over the SMs are cut along K, their
- * fp32 partial sums go through the workspace and are added in a fixed order (run-to-run
- * bit-identical). 0 bytes: nothing is cut for this shape. */
+/* rt_gemm_fp8 for callers that reserve rt_gemm_fp8_workspace_bytes(m, n, k) bytes of device scratch: no
+ * shape needs any (0), and workspace may be NULL. Every element is one chain of sums over the K blocks
+ * in order, so a row's bits do not depend on m. */
 int64_t rt_gemm_fp8_workspace_bytes(int64_t m, int64_t n, int64_t k);
 int rt_gemm_fp8_ws(const void* a, const float* a_scales, const void* b, const float* b_scales,
                    void* c, void* workspace, int64_t m, int64_t n, int64_t k, int64_t lda,
                    int64_t ldb, int64_t ldc, void* stream);
-
 
 /*
  * Work lists of the grouped GEMM, built on the device from the per-expert row offsets

@@ -1281,28 +1281,97 @@ constexpr uint32_t kQTmemCols = 512;
 constexpr uint32_t kQIdesc = (1u << 4) | (static_cast<uint32_t>(kQBN >> 3) << 17) |
                              (static_cast<uint32_t>(kBM >> 4) << 24);
 
-// Work items: the first full_tiles output tiles whole, the tiles behind them cut along K into
-// k_splits ranges of kb_per blocks, one item each. A cut item leaves its fp32 sums in slab
-// (tile - full_tiles) * k_splits + range of the workspace (a 128 x 256 block as [64 column
-// quads][128 rows] float4, so that a warp's stores are contiguous) and fp8_tail_reduce_kernel adds
-// the ranges in order. SPLIT = false: no such tiles.
+// Work items: the first full_tiles output tiles whole, the tiles behind them cut along N into PARTS
+// pieces of 256 / PARTS columns, one item each. A piece's K blocks take 256 / PARTS columns of tensor
+// memory, so PARTS consecutive ones share a buffer (a wait, a commit and a hand-back for all of them),
+// and the fold adds them one after the other: every element is the same chain of sums, in the same
+// order, as in a whole tile, whatever the number of rows makes of the plan.
 // a_bytes: what the A box of a stage brings in (the rows there are, when fewer than 128).
 struct Fp8Item {
-    int tile, kb0, kb1;      // K blocks [kb0, kb1)
-    int slab;                // -1: a whole tile
+    int tile, part;          // part -1: the whole tile
 };
-__device__ __forceinline__ Fp8Item fp8_item(int item, int full_tiles, int k_splits, int kb_per, int num_kb) {
-    if (item < full_tiles) return {item, 0, num_kb, -1};
-    const int rel = item - full_tiles, range = rel % k_splits;
-    return {full_tiles + rel / k_splits, range * kb_per, min(num_kb, (range + 1) * kb_per), rel};
+template <int PARTS>
+__device__ __forceinline__ Fp8Item fp8_item(int item, int full_tiles) {
+    if (PARTS == 1 || item < full_tiles) return {item, -1};
+    const int rel = item - full_tiles;
+    return {full_tiles + rel / PARTS, rel % PARTS};
 }
 
-template <bool SPLIT>
+// An epilogue warp's share of a piece: half of its columns, the K blocks of a buffer one after the other.
+template <int PARTS>
+__device__ __forceinline__ bool fold_part(int part, int tn, int row, int half, int num_kb, int M, int N, int64_t ldc,
+                                          const float* as_row, const float* __restrict__ b_s,
+                                          __nv_bfloat16* __restrict__ c, uint32_t lane_base, uint32_t pfull0,
+                                          uint32_t pempty0, int& buf, uint32_t& buf_phase,
+                                          volatile int* abort_flag) {
+    constexpr int kPartN = kQBN / PARTS, kCols = kPartN / 2;            // 64 or 32 columns of a warp
+    static_assert(PARTS == 2 || PARTS == 4, "64-column halves read in one go, or 32-column ones of two K blocks");
+    const int col_base = tn * kQBN + part * kPartN + half * kCols;
+    const bool live = col_base < N;
+    const float* bs_row = b_s + static_cast<int64_t>(live ? col_base >> 7 : 0) * num_kb;
+    float acc[kCols];
+#pragma unroll
+    for (int i = 0; i < kCols; ++i) acc[i] = 0.f;
+    for (int kb0 = 0; kb0 < num_kb; kb0 += PARTS) {
+        float scale[PARTS];
+#pragma unroll
+        for (int j = 0; j < PARTS; ++j) scale[j] = kb0 + j < num_kb ? __ldg(as_row + kb0 + j) * __ldg(bs_row + kb0 + j) : 0.f;
+        if (!mbar_wait(pfull0 + 8u * buf, buf_phase, abort_flag, 24)) return false;
+        tc_fence_after();
+        const uint32_t taddr = lane_base + static_cast<uint32_t>(buf * kQBN + half * kCols);
+        // 64 columns per wait, as for a whole tile: both 32-column groups of one K block, or one of two
+        constexpr uint32_t kSecond = kCols == 64 ? 32u : static_cast<uint32_t>(kPartN);
+        constexpr int kStep = kCols == 64 ? 1 : 2;                      // K blocks per wait
+#pragma unroll
+        for (int j = 0; j < PARTS; j += kStep) {
+            uint32_t r0[32], r1[32];
+            tmem_ld_32x32(taddr + static_cast<uint32_t>(j * kPartN), r0);
+            tmem_ld_32x32(taddr + static_cast<uint32_t>(j * kPartN) + kSecond, r1);
+            tmem_ld_wait(r0);
+            tmem_ld_wait(r1);
+            if (j + kStep == PARTS) {          // every column of the buffer has been read
+                tc_fence_before();
+                mbar_arrive(pempty0 + 8u * buf);
+            }
+            if (kb0 + j < num_kb) {            // the columns of missing K blocks hold old sums
+#pragma unroll
+                for (int i = 0; i < 32; ++i) acc[i] = fmaf(__uint_as_float(r0[i]), scale[j], acc[i]);
+            }
+            if (kb0 + j + kStep - 1 < num_kb) {
+                constexpr int kAt = kCols == 64 ? 32 : 0;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) acc[kAt + i] = fmaf(__uint_as_float(r1[i]), scale[j + kStep - 1], acc[kAt + i]);
+            }
+        }
+        if (++buf == 2) {
+            buf = 0;
+            buf_phase ^= 1u;
+        }
+    }
+    if (row < M && live) {
+        __nv_bfloat16* crow = c + static_cast<int64_t>(row) * ldc + col_base;
+#pragma unroll
+        for (int v = 0; v < kCols / 8; ++v) {
+            if (col_base + v * 8 < N) {
+                float f[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) f[i] = acc[v * 8 + i];
+                *reinterpret_cast<uint4*>(crow + v * 8) = pack_bf16x8(f);
+            }
+        }
+    }
+    return true;
+}
+
+template <int PARTS>
 __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
     const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-    const float* __restrict__ a_s, const float* __restrict__ b_s, __nv_bfloat16* __restrict__ c,
-    int M, int N, int K, int64_t ldc, uint32_t a_bytes, int num_items, int full_tiles_arg, int k_splits,
-    int kb_per, float4* __restrict__ slabs) {
+    const __grid_constant__ CUtensorMap tmap_part, const float* __restrict__ a_s,
+    const float* __restrict__ b_s, __nv_bfloat16* __restrict__ c, int M, int N, int K, int64_t ldc,
+    uint32_t a_bytes, int num_items, int full_tiles) {
+    constexpr int kPartN = kQBN / PARTS;
+    constexpr uint32_t kPartIdesc = (1u << 4) | (static_cast<uint32_t>(kPartN >> 3) << 17) |
+                                    (static_cast<uint32_t>(kBM >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -1319,7 +1388,6 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
     const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
     const int num_m = (M + kBM - 1) / kBM, num_n = (N + kQBN - 1) / kQBN;
     const int num_kb = K / kQBK;
-    const int full_tiles = SPLIT ? full_tiles_arg : num_items;
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
@@ -1334,6 +1402,7 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
         fence_mbar_init();
         tma_prefetch_desc(&tmap_a);
         tma_prefetch_desc(&tmap_b);
+        if constexpr (PARTS > 1) tma_prefetch_desc(&tmap_part);
     }
     if (warp == 1) {
         tmem_alloc(slot, kQTmemCols);
@@ -1350,15 +1419,19 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
             uint32_t phase = 0;
             bool ok = true;
             for (int item = blockIdx.x; ok && item < num_items; item += gridDim.x) {
-                const Fp8Item it = fp8_item(item, full_tiles, k_splits, kb_per, num_kb);
+                const Fp8Item it = fp8_item<PARTS>(item, full_tiles);
                 int tm, tn;
                 tile_coords(it.tile, num_m, num_n, tm, tn);
-                for (int kb = it.kb0; kb < it.kb1; ++kb) {
+                const bool whole = PARTS == 1 || it.part < 0;
+                const CUtensorMap* map_b = whole ? &tmap_b : &tmap_part;
+                const uint32_t tx = a_bytes + (whole ? kQBBytes : kQBBytes / PARTS);
+                const int b_row = tn * kQBN + (whole ? 0 : it.part * kPartN);
+                for (int kb = 0; kb < num_kb; ++kb) {
                     if (!(ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, 21))) break;
                     const uint32_t sa = base + stage * kQStageBytes;
-                    mbar_arrive_expect_tx(full_bar(stage), a_bytes + kQBBytes);
+                    mbar_arrive_expect_tx(full_bar(stage), tx);
                     tma_load_2d(sa, &tmap_a, kb * kQBK, tm * kBM, full_bar(stage));
-                    tma_load_2d(sa + kQABytes, &tmap_b, kb * kQBK, tn * kQBN, full_bar(stage));
+                    tma_load_2d(sa + kQABytes, map_b, kb * kQBK, b_row, full_bar(stage));
                     if (++stage == kQStages) {
                         stage = 0;
                         phase ^= 1u;
@@ -1375,26 +1448,32 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
             uint32_t buf_phase = 0;
             bool ok = true;
             for (int item = blockIdx.x; ok && item < num_items; item += gridDim.x) {
-                const Fp8Item it = fp8_item(item, full_tiles, k_splits, kb_per, num_kb);
-                for (int kb = it.kb0; kb < it.kb1; ++kb) {
+                const bool whole = PARTS == 1 || fp8_item<PARTS>(item, full_tiles).part < 0;
+                const int per_buf = whole ? 1 : PARTS;          // K blocks that share a buffer
+                const uint32_t idesc = whole ? kQIdesc : kPartIdesc;
+                for (int kb0 = 0; ok && kb0 < num_kb; kb0 += per_buf) {
                     if (!(ok = mbar_wait(pempty_bar(buf), buf_phase ^ 1u, abort_flag, 22))) break;
-                    if (!(ok = mbar_wait(full_bar(stage), phase, abort_flag, 23))) break;
-                    tc_fence_after();
-                    const uint32_t sa = base + stage * kQStageBytes;
-                    const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * kQBN);
-                    const uint64_t adesc = smem_desc_sw128(sa);
-                    const uint64_t bdesc = smem_desc_sw128(sa + kQABytes);
+                    const int blocks = min(per_buf, num_kb - kb0);
+                    for (int i = 0; i < blocks; ++i) {
+                        if (!(ok = mbar_wait(full_bar(stage), phase, abort_flag, 23))) break;
+                        tc_fence_after();
+                        const uint32_t sa = base + stage * kQStageBytes;
+                        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * kQBN + i * kPartN);
+                        const uint64_t adesc = smem_desc_sw128(sa);
+                        const uint64_t bdesc = smem_desc_sw128(sa + kQABytes);
 #pragma unroll
-                    for (int j = 0; j < kQBK / 32; ++j) {
-                        // 32 e4m3 = 32 bytes along K: +2 in the 16-byte-unit address field
-                        mma_f8f6f4(d_tmem, adesc + 2u * j, bdesc + 2u * j, kQIdesc, j != 0 ? 1u : 0u);
+                        for (int j = 0; j < kQBK / 32; ++j) {
+                            // 32 e4m3 = 32 bytes along K: +2 in the 16-byte-unit address field
+                            mma_f8f6f4(d_tmem, adesc + 2u * j, bdesc + 2u * j, idesc, j != 0 ? 1u : 0u);
+                        }
+                        mma_commit(empty_bar(stage));   // smem stage reusable
+                        if (++stage == kQStages) {
+                            stage = 0;
+                            phase ^= 1u;
+                        }
                     }
-                    mma_commit(empty_bar(stage));   // smem stage reusable
-                    mma_commit(pfull_bar(buf));     // partial product of this K block complete
-                    if (++stage == kQStages) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
+                    if (!ok) break;
+                    mma_commit(pfull_bar(buf));     // the buffer's partial products are complete
                     if (++buf == 2) {
                         buf = 0;
                         buf_phase ^= 1u;
@@ -1411,18 +1490,26 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
         uint32_t buf_phase = 0;
         bool ok = true;
         for (int item = blockIdx.x; ok && item < num_items; item += gridDim.x) {
-            const Fp8Item it = fp8_item(item, full_tiles, k_splits, kb_per, num_kb);
+            const Fp8Item it = fp8_item<PARTS>(item, full_tiles);
             int tm, tn;
             tile_coords(it.tile, num_m, num_n, tm, tn);
             const int row = tm * kBM + quad * 32 + lane;
+            const float* as_row = a_s + static_cast<int64_t>(row < M ? row : 0) * kbs;
+            if constexpr (PARTS > 1) {
+                if (it.part >= 0) {
+                    ok = fold_part<PARTS>(it.part, tn, row, half, num_kb, M, N, ldc, as_row, b_s, c,
+                                          tmem_base + (static_cast<uint32_t>(quad * 32) << 16), pfull_bar(0),
+                                          pempty_bar(0), buf, buf_phase, abort_flag);
+                    continue;
+                }
+            }
             const int col_base = tn * kQBN + half * 128;
             const bool live = col_base < N;                       // whole half outside the matrix?
-            const float* as_row = a_s + static_cast<int64_t>(row < M ? row : 0) * kbs;
             const float* bs_row = b_s + static_cast<int64_t>(live ? col_base >> 7 : 0) * kbs;
             float acc[128];
 #pragma unroll
             for (int i = 0; i < 128; ++i) acc[i] = 0.f;
-            for (int kb = it.kb0; kb < it.kb1; ++kb) {
+            for (int kb = 0; kb < num_kb; ++kb) {
                 const float scale = __ldg(as_row + kb) * __ldg(bs_row + kb);
                 if (!(ok = mbar_wait(pfull_bar(buf), buf_phase, abort_flag, 24))) break;
                 tc_fence_after();
@@ -1456,15 +1543,6 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
                 }
             }
             if (!ok) break;
-            if (SPLIT && it.slab >= 0) {
-                if (row < M && live) {
-                    float4* dst = slabs + (static_cast<int64_t>(it.slab) * 64 + half * 32) * 128 + quad * 32 + lane;
-#pragma unroll
-                    for (int v = 0; v < 32; ++v)
-                        dst[v * 128] = make_float4(acc[4 * v], acc[4 * v + 1], acc[4 * v + 2], acc[4 * v + 3]);
-                }
-                continue;
-            }
             if (row < M && live) {
                 __nv_bfloat16* crow = c + static_cast<int64_t>(row) * ldc + col_base;
 #pragma unroll
@@ -1485,28 +1563,6 @@ __global__ void __launch_bounds__(kQThreads, 1) gemm_fp8_kernel(
         tc_fence_after();
         tmem_dealloc(tmem_base, kQTmemCols);
     }
-}
-
-// The tiles gemm_fp8_kernel<true> cut along K: c = bf16(range 0 + range 1 + ...). One CTA per 16
-// columns of a tile, one thread per row and 8 columns.
-__global__ void __launch_bounds__(256) fp8_tail_reduce_kernel(const float4* __restrict__ slabs,
-                                                              __nv_bfloat16* __restrict__ c, int M, int N,
-                                                              int64_t ldc, int full_tiles, int k_splits) {
-    const int num_m = (M + kBM - 1) / kBM, num_n = (N + kQBN - 1) / kQBN;
-    const int rel = blockIdx.x >> 4, cols = ((blockIdx.x & 15) * 2 + (threadIdx.x >> 7)) * 8;
-    int tm, tn;
-    tile_coords(full_tiles + rel, num_m, num_n, tm, tn);
-    const int row = tm * kBM + (threadIdx.x & 127), col = tn * kQBN + cols;
-    if (row >= M || col >= N) return;              // N % 8 == 0: a started vector is complete
-    const float4* src = slabs + (static_cast<int64_t>(rel) * k_splits * 64 + cols / 4) * 128 + (threadIdx.x & 127);
-    float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (int s = 0; s < k_splits; ++s, src += 64 * 128) {
-        const float4 lo = __ldg(src), hi = __ldg(src + 128);
-        f[0] += lo.x; f[1] += lo.y; f[2] += lo.z; f[3] += lo.w;
-        f[4] += hi.x; f[5] += hi.y; f[6] += hi.z; f[7] += hi.w;
-    }
-    *reinterpret_cast<uint4*>(c + static_cast<int64_t>(row) * ldc + col) = pack_bf16x8(f);
 }
 
 // ---------------------------------------------------------------------------
@@ -2104,57 +2160,59 @@ static int launch_index_score(const void* q, const float* weights, const void* k
     return check_launch("index_score_kernel");
 }
 
-// How rt_gemm_fp8_ws cuts a product: whole tiles for the full rounds over the SMs, the tiles of the
-// last, partial round along K, so that it takes a fraction of a round instead of a whole one with
-// most SMs idle (2048 x 7168: 448 tiles are three rounds of 148 and four tiles; a decode projection
-// is a partial round only). `splits` == 1: not cut, because half the SMs or more have a tile of the
-// round anyway or the ranges and the pass that adds them would cost what they save (0.5 us a K
-// block; a launch and the slabs, written and read at L2's pace).
+// How a product's tiles become work items: whole tiles for the full rounds over the SMs, the tiles of
+// the last, partial round in pieces of 128 or 64 columns where that ends the round sooner (2048 x 7168:
+// 448 tiles are three rounds of 148 and four tiles; a decode projection is a partial round only). A
+// round of halves takes 0.73 of a round of whole tiles, one of quarters 0.62 (16 KB of A come in for
+// every K block whatever the width), so quarters pay up to 37 tiles and halves up to 74. One B200, whole
+// -> cut: 13 x 7168 x 16384 59 -> 43 us, 13 x 2112 x 7168 31 -> 22, 777 x 7168 x 16384 132 -> 115,
+// 777 x 2112 x 7168 37 -> 27, 2048 x 7168 x 18432 293 -> 262, 8192 x 7168 x 16384 961 -> 941.
+// Cutting K instead shortens the round further (34, 20, 105, 30, 245 and 916 us), but by a cut that
+// follows the number of rows: a row's last bits would depend on the size of the call, and the rows of a
+// rank that holds a share of the tokens would differ from those of one that holds them all.
 struct Fp8Plan {
-    int64_t full, splits, per;
+    int64_t full;            // whole tiles
+    int parts;               // pieces of each tile behind them
 };
-static Fp8Plan fp8_plan(int64_t m, int64_t n, int64_t k) {
-    const int64_t tiles = ((m + kBM - 1) / kBM) * ((n + kQBN - 1) / kQBN), num_kb = k / kQBK, sms = sm_count();
+static Fp8Plan fp8_plan(int64_t m, int64_t n) {
+    const int64_t tiles = ((m + kBM - 1) / kBM) * ((n + kQBN - 1) / kQBN), sms = sm_count();
     const int64_t tail = tiles % sms;
-    Fp8Plan whole = {tiles, 1, num_kb};
-    if (tail == 0) return whole;
-    int64_t splits = std::min(sms / tail, num_kb / 3);
-    if (splits < 2) return whole;
-    const int64_t per = (num_kb + splits - 1) / splits;
-    splits = (num_kb + per - 1) / per;
-    const double slab_us = 2.0 * tail * splits * kBM * kQBN * 4 * std::min<int64_t>(m, kBM) / kBM / 6.0e6;
-    if (0.5 * per + 5.0 + slab_us >= 0.5 * num_kb) return whole;
-    return {tiles - tail, splits, per};
+    int parts = 1;
+    double best = tail ? 1.0 : 0.0;
+    for (const auto& [cut, cost_kb] : {std::pair<int, double>{2, 0.73}, {4, 0.62}}) {
+        const double cost = static_cast<double>((tail * cut + sms - 1) / sms) * cost_kb;
+        if (cost < best) {
+            best = cost;
+            parts = cut;
+        }
+    }
+    return {parts == 1 ? tiles : tiles - tail, parts};
 }
 
-static int launch_fp8(const void* a, const float* a_s, const void* b, const float* b_s, void* c, void* workspace,
+static int launch_fp8(const void* a, const float* a_s, const void* b, const float* b_s, void* c,
                       int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc,
                       cudaStream_t st) {
-    CUtensorMap ta, tb;
+    CUtensorMap ta, tb, tp;
     const uint32_t a_rows = a_box_rows(M);
     if (int rc = make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, a, K, M, lda, kQBK, a_rows)) return rc;
     if (int rc = make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, b, K, N, ldb, kQBK, kQBN)) return rc;
     const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + kQBN - 1) / kQBN);
-    const Fp8Plan plan = workspace ? fp8_plan(M, N, K) : Fp8Plan{tiles, 1, K / kQBK};
-    const bool split = plan.splits > 1;
-    const int64_t items = plan.full + (tiles - plan.full) * plan.splits;
-    auto kernel = split ? &gemm_fp8_kernel<true> : &gemm_fp8_kernel<false>;
+    const Fp8Plan plan = fp8_plan(M, N);
+    if (plan.parts == 1)
+        tp = tb;
+    else if (int rc = make_tmap_2d(&tp, CU_TENSOR_MAP_DATA_TYPE_UINT8, b, K, N, ldb, kQBK, kQBN / plan.parts))
+        return rc;
+    const int64_t items = plan.full + (tiles - plan.full) * plan.parts;
+    auto kernel = plan.parts == 1 ? &gemm_fp8_kernel<1> : plan.parts == 2 ? &gemm_fp8_kernel<2> : &gemm_fp8_kernel<4>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(kQSmemBytes),
                                      "rt_gemm_fp8"))
         return rc;
     const int grid = static_cast<int>(items < sm_count() ? items : sm_count());
     kernel<<<grid, kQThreads, kQSmemBytes, st>>>(
-        ta, tb, a_s, b_s, static_cast<__nv_bfloat16*>(c), static_cast<int>(M), static_cast<int>(N),
-        static_cast<int>(K), ldc, a_rows * kQBK, static_cast<int>(items), static_cast<int>(plan.full),
-        static_cast<int>(plan.splits), static_cast<int>(plan.per), static_cast<float4*>(workspace));
+        ta, tb, tp, a_s, b_s, static_cast<__nv_bfloat16*>(c), static_cast<int>(M), static_cast<int>(N),
+        static_cast<int>(K), ldc, a_rows * kQBK, static_cast<int>(items), static_cast<int>(plan.full));
     count_launch();
-    if (int rc = check_launch("gemm_fp8_kernel")) return rc;
-    if (!split) return RT_OK;
-    fp8_tail_reduce_kernel<<<static_cast<unsigned>(16 * (tiles - plan.full)), 256, 0, st>>>(
-        static_cast<const float4*>(workspace), static_cast<__nv_bfloat16*>(c), static_cast<int>(M),
-        static_cast<int>(N), ldc, static_cast<int>(plan.full), static_cast<int>(plan.splits));
-    count_launch();
-    return check_launch("fp8_tail_reduce_kernel");
+    return check_launch("gemm_fp8_kernel");
 }
 
 // Schedule of the NVFP4 GEMM: 0 = by size (CTA pairs unless the work list is too short to
@@ -2222,39 +2280,29 @@ static int launch_nvfp4_pair(const void* a_codes, const void* a_sf, const float*
 
 using namespace rt;
 
-static int gemm_fp8_checked(const void* a, const float* a_scales, const void* b, const float* b_scales, void* c,
-                            void* workspace, int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb,
-                            int64_t ldc, void* stream) {
+extern "C" int rt_gemm_fp8(const void* a, const float* a_scales, const void* b,
+                           const float* b_scales, void* c, int64_t m, int64_t n, int64_t k,
+                           int64_t lda, int64_t ldb, int64_t ldc, void* stream) {
     RT_REQUIRE(m >= 0 && n > 0 && k > 0, RT_ERR_BAD_ARG, "rt_gemm_fp8: bad shape");
     if (m == 0) return RT_OK;
     RT_REQUIRE(a && a_scales && b && b_scales && c, RT_ERR_BAD_ARG, "rt_gemm_fp8: null pointer");
     RT_REQUIRE(k % 128 == 0, RT_ERR_UNSUPPORTED, "rt_gemm_fp8: k must be a multiple of 128");
     RT_REQUIRE(n % 8 == 0 && lda % 16 == 0 && ldb % 16 == 0 && ldc % 8 == 0, RT_ERR_UNSUPPORTED,
                "rt_gemm_fp8: n %% 8, lda/ldb %% 16 and ldc %% 8 are required");
-    RT_REQUIRE(aligned16(a) && aligned16(b) && aligned16(c) && aligned16(workspace), RT_ERR_UNSUPPORTED,
+    RT_REQUIRE(aligned16(a) && aligned16(b) && aligned16(c), RT_ERR_UNSUPPORTED,
                "rt_gemm_fp8: pointers must be 16-byte aligned");
     RT_REQUIRE(m < (1LL << 31) && n < (1LL << 31) && k < (1LL << 31), RT_ERR_UNSUPPORTED,
                "rt_gemm_fp8: dimension too large");
-    return tc::launch_fp8(a, a_scales, b, b_scales, c, workspace, m, n, k, lda, ldb, ldc, as_stream(stream));
+    return tc::launch_fp8(a, a_scales, b, b_scales, c, m, n, k, lda, ldb, ldc, as_stream(stream));
 }
 
-extern "C" int rt_gemm_fp8(const void* a, const float* a_scales, const void* b, const float* b_scales, void* c,
-                           int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb, int64_t ldc, void* stream) {
-    return gemm_fp8_checked(a, a_scales, b, b_scales, c, nullptr, m, n, k, lda, ldb, ldc, stream);
-}
-
-extern "C" int64_t rt_gemm_fp8_workspace_bytes(int64_t m, int64_t n, int64_t k) {
-    if (m <= 0 || n <= 0 || k <= 0 || k % 128) return 0;
-    const tc::Fp8Plan plan = tc::fp8_plan(m, n, k);
-    if (plan.splits < 2) return 0;
-    const int64_t tiles = ((m + 127) / 128) * ((n + 255) / 256);
-    return (tiles - plan.full) * plan.splits * 128 * 256 * 4;
-}
+// Callers that reserve scratch by rt_gemm_fp8_workspace_bytes: no shape needs any.
+extern "C" int64_t rt_gemm_fp8_workspace_bytes(int64_t, int64_t, int64_t) { return 0; }
 
 extern "C" int rt_gemm_fp8_ws(const void* a, const float* a_scales, const void* b, const float* b_scales, void* c,
-                              void* workspace, int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb,
-                              int64_t ldc, void* stream) {
-    return gemm_fp8_checked(a, a_scales, b, b_scales, c, workspace, m, n, k, lda, ldb, ldc, stream);
+                              void*, int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb, int64_t ldc,
+                              void* stream) {
+    return rt_gemm_fp8(a, a_scales, b, b_scales, c, m, n, k, lda, ldb, ldc, stream);
 }
 
 static int fp8_index_checked(const void* q, const float* weights, const void* k,

@@ -24,7 +24,7 @@ using OptTensor = std::optional<Tensor>;
     X(rt_nvfp4_quant) X(rt_moe_route) X(rt_moe_permute_workspace_bytes) X(rt_moe_permute)         \
     X(rt_moe_tile_map) X(rt_moe_plan) X(rt_absmax_onto) X(rt_swiglu_absmax_rows_onto) X(rt_moe_gather_nvfp4) X(rt_moe_quant_nvfp4) X(rt_moe_combine)             \
     X(rt_gemm_bf16) X(rt_gemm_bf16_splitk_splits) X(rt_gemm_bf16_splitk) X(rt_gemm_bf16_batched)  \
-    X(rt_gemm_fp8_workspace_bytes) X(rt_gemm_fp8_ws) X(rt_gemm_nvfp4_grouped) X(rt_index_prep_into) X(rt_index_head_weights) X(rt_fp8_index_batched)              \
+    X(rt_gemm_fp8) X(rt_gemm_nvfp4_grouped) X(rt_index_prep_into) X(rt_index_head_weights) X(rt_fp8_index_batched)              \
     X(rt_index_topk) X(rt_mla_sparse_decode_splits) X(rt_mla_sparse_decode)
 
 #define RT_POINTER(name) decltype(&::name) p_##name = nullptr;
@@ -435,11 +435,8 @@ Tensor linear_fp8(const Tensor& x_codes, const Tensor& x_scales, const Tensor& w
         !same_shape(w_scales, {(n + 127) / 128, k / 128}))
         fail("linear_fp8: scales must be fp32 [M, K/128] and [ceil(N/128), K/128]");
     Tensor out = out_buffer(out_in, with_last(x_codes, n), at::kBFloat16, x_codes);
-    const int64_t m = xc.size(0), scratch = p_rt_gemm_fp8_workspace_bytes(m, n, k);
-    OptTensor workspace;
-    if (scratch > 0) workspace = empty({scratch}, at::kByte, x_codes);
-    check(p_rt_gemm_fp8_ws(xc.data_ptr(), data<float>(xs), w_codes.data_ptr(), data<float>(w_scales), out.data_ptr(),
-                           workspace ? workspace->data_ptr() : nullptr, m, n, k, k, k, n, stream()),
+    check(p_rt_gemm_fp8(xc.data_ptr(), data<float>(xs), w_codes.data_ptr(), data<float>(w_scales), out.data_ptr(),
+                        xc.size(0), n, k, k, k, n, stream()),
           "rt_gemm_fp8");
     return out;
 }

@@ -328,18 +328,18 @@ def test_linear_bf16_rows_do_not_depend_on_the_call(ops, n, k, out_dtype):
 
 
 @pytest.mark.parametrize("m,n,k", [
-    (13, 2112, 7168),       # a decode projection: nine tiles, all of them cut, the last one narrow
+    (13, 2112, 7168),       # a decode projection: nine tiles in quarters, those past column 2112 empty
     (1, 7168, 2048),        # a box of 8 rows, one of them there
-    (129, 264, 1664),       # two row and two column tiles, nearly empty, 13 K blocks
-    (2048, 7168, 2304),     # three full rounds and four tiles, cut
-    (300, 4096, 384),       # three K blocks: whole tiles
+    (129, 264, 1664),       # two row and two column tiles, nearly empty, 13 K blocks: one in the last buffer
+    (2048, 7168, 2304),     # three full rounds and four tiles, in quarters
+    (300, 4096, 384),       # 48 tiles in halves, three K blocks: one in the last buffer
+    (64, 1024, 256),        # quarters, fewer K blocks than a buffer holds
+    (777, 24576, 384),      # four full rounds and 80 tiles: whole
 ])
-def test_linear_fp8_tail_tiles_cut_along_k(ops, m, n, k):
-    """Tiles of a partial round over the SMs are summed in K ranges: against fp64 of the dequantised
+def test_linear_fp8_tail_tiles_in_pieces(ops, m, n, k):
+    """Tiles of a partial round over the SMs in pieces of their columns: against fp64 of the dequantised
     operands. Per K block of 128 the products are exact in fp32 to 128 * 2^-24 of their magnitudes,
-    the scaled sums add k / 128 + ranges roundings more, bf16 rounds once."""
-    from racetrack_b200 import _lib
-    lib = _lib.load()
+    the scaled sums add k / 128 roundings more, bf16 rounds once."""
     x = I.randn((m, k), 700 + m).cuda()
     w = I.randn((n, k), 800 + n, std=0.05).cuda()
     xc, xs = ops.fused_act_quant(x)
@@ -349,13 +349,18 @@ def test_linear_fp8_tail_tiles_cut_along_k(ops, m, n, k):
     assert torch.equal(out, ops.linear_fp8(xc, xs, wc, ws)), "must be bit-reproducible"
     a = xc.double() * xs.double().repeat_interleave(128, dim=1)
     b = wc.double() * ws.double().repeat_interleave(128, dim=0)[:n].repeat_interleave(128, dim=1)
-    bound = (256 + k // 64) * 2.0 ** -24 * (a.abs() @ b.abs().t()) + 2.0 ** -8 * (a @ b.t()).abs()
+    bound = (256 + k // 128) * 2.0 ** -24 * (a.abs() @ b.abs().t()) + 2.0 ** -8 * (a @ b.t()).abs()
     assert bool(((out.double() - a @ b.t()).abs() <= bound).all())
-    # whole tiles only: the same sums in one range
-    whole = torch.empty_like(out)
-    _lib.check(lib.rt_gemm_fp8(xc.data_ptr(), xs.data_ptr(), wc.data_ptr(), ws.data_ptr(), whole.data_ptr(), m, n,
-                               k, k, k, n, torch.cuda.current_stream().cuda_stream), "rt_gemm_fp8")
-    if int(lib.rt_gemm_fp8_workspace_bytes(m, n, k)) == 0:
-        assert torch.equal(out, whole)
-    else:
-        assert bool(((out.double() - whole.double()).abs() <= 2 * bound).all())
+
+
+def test_linear_fp8_rows_do_not_depend_on_the_call(ops):
+    """A row gives the same bits in calls of every length: whole tiles, halves and quarters of tiles
+    (at 2112 columns the last round over the SMs has 9 tiles, 27, 63, 72, 108, 144 or 28 of a third)."""
+    n, k = 2112, 1664
+    xc, xs = ops.fused_act_quant(I.randn((4500, k), 950).cuda())
+    wc, ws = ops.quantize_weight_fp8(I.randn((n, k), 951, std=0.05).cuda())
+    every = ops.linear_fp8(xc, xs, wc, ws)
+    for m in (1, 13, 64, 128, 129, 300, 777, 1024, 1500, 2048):
+        assert torch.equal(ops.linear_fp8(xc[:m], xs[:m], wc, ws), every[:m]), m
+    assert torch.equal(ops.linear_fp8(xc[4001:], xs[4001:], wc, ws), every[4001:])
+    ops.tc_error_state()
