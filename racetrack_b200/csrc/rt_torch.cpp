@@ -552,6 +552,7 @@ Tensor moe_combine(Tensor expert_out, const Tensor& pair_pos, Tensor weights, Op
     require_cuda({&expert_out, &pair_pos, &weights});
     require_bf16("fused_moe_combine", expert_out);
     const int64_t tokens = weights.size(0), topk = weights.size(1), cols = expert_out.size(-1);
+    if (pair_pos.numel() < tokens * topk) fail("fused_moe_combine: pair_pos must have a position for every weight");
     expert_out = expert_out.contiguous();
     weights = weights.to(at::kFloat).contiguous();
     if (shared) {
@@ -574,12 +575,17 @@ py::tuple moe_experts(const OptTensor& x, const Tensor& weights, const Tensor& i
                       const Tensor& w2_gs, int64_t count, int64_t inter, int64_t n_experts, int64_t expert_begin,
                       const OptTensor& shared, bool f32_out, const OptTensor& q_codes, const OptTensor& q_sf,
                       const OptTensor& q_gs, const OptTensor& out, const std::optional<py::function>& around_w13) {
-    const int64_t tokens = q_codes ? q_codes->size(0) : x->size(0);
-    const int64_t hidden = q_codes ? q_codes->size(1) * 2 : x->size(1);
-    const int64_t topk = indices.size(1), pairs = tokens * topk;
-    require_cuda({&indices});
+    if (q_codes ? !(q_sf && q_gs) : !x) fail("fused_moe_experts: x or x_quant (codes, scales, global scale) is required");
+    const Tensor& in = q_codes ? *q_codes : *x;
+    if (in.dim() != 2) fail("fused_moe_experts: x must be [T, hidden] (x_quant codes [T, hidden / 2])");
     if (indices.scalar_type() != at::kLong || indices.dim() != 2)
         fail("fused_moe_permute: indices must be a 2-D int64 tensor");
+    // the routed rows are those of indices: they name rows of x, and weights has one value for each
+    const int64_t tokens = indices.size(0), topk = indices.size(1), pairs = tokens * topk;
+    if (tokens > in.size(0) || weights.dim() != 2 || weights.size(0) > tokens || weights.size(1) != topk)
+        fail("fused_moe_experts: x, weights and indices disagree on the token count or on topk");
+    const int64_t hidden = q_codes ? in.size(1) * 2 : in.size(1);
+    require_cuda({&indices, &in});
     const Tensor idx = indices.contiguous();
     const int64_t max_tiles = (pairs + 127) / 128 + count;
     Tensor workspace = empty(
@@ -604,12 +610,11 @@ py::tuple moe_experts(const OptTensor& x, const Tensor& weights, const Tensor& i
         x_gs = *q_gs;
         std::tie(a_codes, a_sf) = moe_gather_nvfp4(*q_codes, *q_sf, sorted_pairs, topk, tile_map, tile_count, pairs);
     } else {
-        require_cuda({&*x});
         require_bf16("tensor_absmax", *x);
         if (hidden % 16 != 0) fail("tensor_absmax: last dim must be a multiple of 16");
         const Tensor x2 = rows_view(*x);
         x_amax = amax2.slice(0, 0, 1);
-        check(p_rt_absmax_onto(x2.data_ptr(), data<float>(amax2), tokens, hidden, x2.stride(0), RT_BF16, stream()),
+        check(p_rt_absmax_onto(x2.data_ptr(), data<float>(amax2), x2.size(0), hidden, x2.stride(0), RT_BF16, stream()),
               "rt_absmax_onto");
         if (pairs <= 256) {
             // few rows: quantised straight into expert order, once per pair, instead of once per token

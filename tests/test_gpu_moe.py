@@ -265,3 +265,23 @@ def test_a_token_is_routed_alike_in_calls_of_different_length(mods):
     for m in (200, 777, 2048):
         w, i = route(m)
         assert torch.equal(i, indices[:m]) and torch.equal(w, weights[:m]), m
+
+
+def test_expert_mlp_of_the_first_rows_of_a_buffer(mods):
+    """Routing of fewer rows than x has (a padded token buffer): the routed rows' outputs, those of a
+    call with these rows alone where the padding holds nothing larger."""
+    ops, moe = mods
+    tokens, hidden, inter, n_experts, topk = 200, 512, 256, 8, 2
+    x, w13, w2 = _setup(tokens, hidden, inter, n_experts, topk)[:3]
+    experts = moe.quantize_experts(w13.cuda(), w2.cuda())
+    g = torch.Generator().manual_seed(3)
+    x = x.cuda()
+    for rows in (1, 40, 150):                 # few and many pairs
+        indices = torch.randint(0, n_experts, (rows, topk), generator=g).cuda()
+        weights = torch.rand(rows, topk, generator=g).cuda()
+        padded = x.clone()
+        padded[rows:] = 0
+        want = moe.fused_moe_experts(x[:rows], weights, indices, experts, n_experts=n_experts)
+        got = moe.fused_moe_experts(padded, weights, indices, experts, n_experts=n_experts)
+        assert got.shape == (rows, hidden) and torch.equal(got, want)
+    ops.tc_error_state()

@@ -1,0 +1,46 @@
+"""Calls the tensor-level entry points refuse, by checks that come before any device is touched."""
+from __future__ import annotations
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from racetrack_b200 import moe
+
+
+def _experts(hidden=128, inter=64, count=4):
+    u8 = lambda *s: torch.zeros(*s, dtype=torch.uint8)
+    return SimpleNamespace(
+        w13_codes=u8(count * 2 * inter, hidden // 2), w13_sf=u8(count * 2 * inter * hidden // 16), w13_gs=torch.ones(count),
+        w2_codes=u8(count * hidden, inter // 2), w2_sf=u8(count * hidden * inter // 16), w2_gs=torch.ones(count),
+        count=count, inter=inter)
+
+
+def _routing(tokens, topk=2):
+    return torch.ones(tokens, topk), torch.zeros(tokens, topk, dtype=torch.int64)
+
+
+X = torch.zeros(16, 128, dtype=torch.bfloat16)
+CODES, SF, GS = torch.zeros(16, 64, dtype=torch.uint8), torch.zeros(16, 8, dtype=torch.uint8), torch.ones(1)
+
+
+@pytest.mark.parametrize("x,x_quant,rows,says", [
+    (X.view(1, 16, 128), None, 16, "x must be"),                          # a batch dimension
+    (X[0], None, 1, "x must be"),
+    (None, (CODES.view(1, 16, 64), SF, GS), 16, "x must be"),
+    (None, None, 16, "is required"),
+    (None, (CODES, None, GS), 16, "is required"),
+    (X, None, 17, "disagree"),                                            # more routed rows than x has
+])
+def test_expert_mlp_refuses_what_it_cannot_index(x, x_quant, rows, says):
+    weights, indices = _routing(rows)
+    with pytest.raises(RuntimeError, match=says):
+        moe.fused_moe_experts(x, weights, indices, _experts(), n_experts=4, x_quant=x_quant)
+
+
+def test_expert_mlp_refuses_weights_of_other_tokens():
+    weights, indices = _routing(16)
+    for bad in (_routing(17)[0], _routing(16, 3)[0], weights.view(-1)):
+        with pytest.raises(RuntimeError, match="disagree"):
+            moe.fused_moe_experts(X, bad, indices, _experts(), n_experts=4)
