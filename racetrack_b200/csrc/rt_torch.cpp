@@ -143,12 +143,22 @@ bool row_slots(const Tensor& out, int64_t rows, int64_t cols, at::ScalarType typ
            reinterpret_cast<uintptr_t>(out.data_ptr()) % align == 0;
 }
 
+// Python hands these on as they came: a None in the wrong place is refused, not dereferenced.
+void require_one_rotation(const char* who, const OptTensor& positions, const OptTensor& inv_freq,
+                          const OptTensor& freqs_cis) {
+    if (positions ? !inv_freq : !freqs_cis) fail(std::string(who) + ": positions or freqs_cis is missing");
+}
+void require_pair(const char* who, const OptTensor& first, const OptTensor& second) {
+    if (first.has_value() != second.has_value()) fail(std::string(who) + ": out must be a pair of tensors");
+}
+
 // positions + inverse frequencies (half-split pairs), or a complex table (interleaved pairs)
 std::tuple<Tensor, Tensor, Tensor> norm_rope(const Tensor& q_c, const Tensor& q_weight, const Tensor& kv_c,
                                              const Tensor& kv_weight, const Tensor& k_pe,
                                              const OptTensor& positions, const OptTensor& inv_freq,
                                              const OptTensor& freqs_cis, double eps, const OptTensor& kv_into,
                                              const OptTensor& k_into) {
+    require_one_rotation("fused_norm_rope", positions, inv_freq, freqs_cis);
     Tensor pos, table;
     int mode = RT_ROPE_INTERLEAVED;
     int64_t table_rows = 0;
@@ -198,6 +208,7 @@ std::tuple<Tensor, Tensor, Tensor> norm_rope(const Tensor& q_c, const Tensor& q_
 
 Tensor rope(const Tensor& x, const OptTensor& positions, const OptTensor& inv_freq, const OptTensor& freqs_cis,
             bool inplace) {
+    require_one_rotation("fused_rope", positions, inv_freq, freqs_cis);
     Tensor pos, table;
     int mode = RT_ROPE_INTERLEAVED;
     int64_t table_rows = 0;
@@ -246,6 +257,7 @@ Tensor swiglu(const Tensor& gate, const Tensor& up) {
 }
 
 std::tuple<Tensor, Tensor> act_quant(const Tensor& x, const OptTensor& out_codes, const OptTensor& out_scales) {
+    require_pair("fused_act_quant", out_codes, out_scales);
     require_cuda({&x});
     require_bf16("fused_act_quant", x);
     const int64_t n = x.size(-1);
@@ -310,6 +322,7 @@ int64_t sf_tiled_bytes(int64_t rows, int64_t cols) { return ((rows + 127) / 128)
 
 std::tuple<Tensor, Tensor, Tensor> nvfp4_quant(const Tensor& x, const OptTensor& up, const OptTensor& amax_in,
                                                bool tiled, const OptTensor& out_codes, const OptTensor& out_sf) {
+    require_pair("fused_nvfp4_quant", out_codes, out_sf);
     require_cuda({&x});
     require_bf16("fused_nvfp4_quant", x);
     const int64_t n = x.size(-1);
@@ -464,6 +477,7 @@ Tensor gemm_nvfp4_grouped(const Tensor& a_codes, const Tensor& a_sf, const Tenso
 std::tuple<Tensor, Tensor> moe_route(Tensor logits, OptTensor bias, int64_t n_groups, int64_t topk_groups,
                                      int64_t topk, double route_scale, int score_func, const OptTensor& out_weights,
                                      const OptTensor& out_indices) {
+    require_pair("fused_moe_route", out_weights, out_indices);
     require_cuda({&logits});
     if (logits.scalar_type() != at::kFloat || logits.dim() != 2)
         fail("fused_moe_route: logits must be a 2-D float32 tensor");

@@ -6,7 +6,7 @@ from types import SimpleNamespace
 import pytest
 import torch
 
-from racetrack_b200 import moe
+from racetrack_b200 import moe, ops
 
 
 def _experts(hidden=128, inter=64, count=4):
@@ -44,3 +44,20 @@ def test_expert_mlp_refuses_weights_of_other_tokens():
     for bad in (_routing(17)[0], _routing(16, 3)[0], weights.view(-1)):
         with pytest.raises(RuntimeError, match="disagree"):
             moe.fused_moe_experts(X, bad, indices, _experts(), n_experts=4)
+
+
+@pytest.mark.parametrize("call", [
+    lambda: ops.fused_rope_half(torch.zeros(2, 3, 64), None),
+    lambda: ops.fused_rope(torch.zeros(2, 3, 64), None),
+    lambda: ops.fused_norm_rope(X, X[0], X, X[0], X, None, eps=1e-6, rope_base=1e4),
+    lambda: ops.fused_norm_rope_interleaved(X, X[0], X, X[0], X, None, eps=1e-6),
+    lambda: ops.fused_act_quant(X, out=(X, None)),
+    lambda: ops.fused_act_quant(X, out=(None, X)),
+    lambda: ops.fused_nvfp4_quant(X, out=(X, None)),
+    lambda: ops.fused_moe_route(torch.zeros(2, 8), None, n_groups=1, topk_groups=1, topk=2, route_scale=1.0,
+                                out=(torch.zeros(2, 2), None)),
+])
+def test_a_missing_tensor_is_refused(call):
+    """A None where a tensor belongs raises; it is not dereferenced."""
+    with pytest.raises(RuntimeError, match="is missing|must be a pair"):
+        call()
