@@ -361,6 +361,7 @@ __global__ void __launch_bounds__(kActThreads) quant_nvfp4_tiles_kernel(
     const float six_gs = __fmul_rn(6.0f, gs);
     const uint32_t kt = items_per_row >> 2;
     uint8_t* sf_tile = sf + static_cast<int64_t>(tm.w) * kt * 512;
+    const bool wide = (reinterpret_cast<uintptr_t>(sf) & 15u) == 0;      // else byte by byte
     const uint32_t row0 = sub * 8u;
     const uint32_t valid = static_cast<uint32_t>(min(8, max(0, tm.z - static_cast<int>(row0))));
     for (uint32_t it = threadIdx.x; it < valid * items_per_row; it += kActThreads) {
@@ -373,22 +374,29 @@ __global__ void __launch_bounds__(kActThreads) quant_nvfp4_tiles_kernel(
         uint32_t v[8], bs;
         load_item<UP>(x, up, src_row, col, xstride, ustride, v);
         st_stream8(codes + dst_row * (cols >> 1) + (col >> 1), quant_item_nvfp4(v, gs, six_gs, bs));
+        uint8_t* sf_row = sf_tile + static_cast<int64_t>(blk >> 2) * 512 + (r_local & 31u) * 16u + (r_local >> 5) * 4u;
+        if (!wide) {
+            sf_row[blk & 3u] = static_cast<uint8_t>(bs);
+            continue;
+        }
         // four neighbouring lanes hold the four scales of one 64-column group of the row (a row has a
         // multiple of four blocks): one 4-byte store
         const uint32_t quad = 0xfu << (threadIdx.x & 28u);
         bs <<= 8 * (blk & 3u);
         bs |= __shfl_xor_sync(quad, bs, 1);
         bs |= __shfl_xor_sync(quad, bs, 2);
-        if ((blk & 3u) == 0)
-            *reinterpret_cast<uint32_t*>(sf_tile + static_cast<int64_t>(blk >> 2) * 512 + (r_local & 31u) * 16u +
-                                         (r_local >> 5) * 4u) = bs;
+        if ((blk & 3u) == 0) *reinterpret_cast<uint32_t*>(sf_row) = bs;
     }
     // rows past the tile's valid ones: zero scales. A warp per 512-byte scale tile, lane l the 16 bytes
     // of rows l, l + 32, l + 64, l + 96.
     const int lane = threadIdx.x & 31;
     for (uint32_t k = sub * (kActThreads / 32) + (threadIdx.x >> 5); k < kt; k += 16 * (kActThreads / 32)) {
-        uint32_t* dst = reinterpret_cast<uint32_t*>(sf_tile + static_cast<int64_t>(k) * 512 + lane * 16);
-        if (lane >= tm.z) {
+        uint8_t* bytes = sf_tile + static_cast<int64_t>(k) * 512 + lane * 16;
+        uint32_t* dst = reinterpret_cast<uint32_t*>(bytes);
+        if (!wide) {
+            for (int i = 0; i < 16; ++i)
+                if (lane + 32 * (i >> 2) >= tm.z) bytes[i] = 0;
+        } else if (lane >= tm.z) {
             *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
         } else {
 #pragma unroll
@@ -639,8 +647,7 @@ extern "C" int rt_moe_quant_nvfp4(const void* x, const void* up, const int32_t* 
     RT_REQUIRE(cols % 64 == 0, RT_ERR_UNSUPPORTED,
                "rt_moe_quant_nvfp4: cols must be a multiple of 64 (whole scale tiles)");
     RT_REQUIRE(x_stride % 8 == 0 && aligned16(x) && (!up || (up_stride % 8 == 0 && aligned16(up))) &&
-                   aligned16(tile_map) && (reinterpret_cast<uintptr_t>(codes) & 7u) == 0 &&
-                   aligned16(block_scales),
+                   aligned16(tile_map) && (reinterpret_cast<uintptr_t>(codes) & 7u) == 0,
                RT_ERR_UNSUPPORTED, "rt_moe_quant_nvfp4: alignment (16-byte inputs, stride %% 8)");
     RT_REQUIRE(max_tiles < (1LL << 27), RT_ERR_UNSUPPORTED, "rt_moe_quant_nvfp4: too many tiles");
     const unsigned grid = static_cast<unsigned>(max_tiles * 16);

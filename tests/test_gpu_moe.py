@@ -285,3 +285,29 @@ def test_expert_mlp_of_the_first_rows_of_a_buffer(mods):
         got = moe.fused_moe_experts(padded, weights, indices, experts, n_experts=n_experts)
         assert got.shape == (rows, hidden) and torch.equal(got, want)
     ops.tc_error_state()
+
+
+@pytest.mark.parametrize("offset", [1, 4, 8])
+@pytest.mark.parametrize("sizes", [(1, 7), (40, 0, 129), (200, 33, 96)])
+def test_block_scales_at_any_address(mods, offset, sizes):
+    """rt_moe_quant_nvfp4 writes the same codes and scales to scale buffers of any alignment."""
+    from racetrack_b200 import _lib
+    ops, _moe = mods
+    rows, cols = sum(sizes), 512
+    x = I.randn((rows, cols), 31).cuda()
+    offsets = torch.tensor([0, *torch.tensor(sizes).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
+    max_tiles = rows // 128 + len(sizes) + 1
+    tile_map, _, tile_count = ops.moe_tile_map(offsets, 0, len(sizes), max_tiles)
+    amax = ops.tensor_absmax(x)
+
+    def quantise(shift):
+        codes = torch.zeros(rows, cols // 2, dtype=torch.uint8, device="cuda")
+        sf = torch.full((max_tiles * (cols // 64) * 512 + 32,), 0xee, dtype=torch.uint8, device="cuda")
+        _lib.check(_lib.load().rt_moe_quant_nvfp4(
+            x.data_ptr(), None, None, 1, amax.data_ptr(), codes.data_ptr(), sf.data_ptr() + shift, None,
+            tile_map.data_ptr(), tile_count.data_ptr(), max_tiles, cols, x.stride(0), 0, _lib.RT_BF16,
+            torch.cuda.current_stream().cuda_stream), "rt_moe_quant_nvfp4")
+        assert (sf[:shift] == 0xee).all()
+        return codes, sf[shift:shift + max_tiles * (cols // 64) * 512]
+    want, got = quantise(0), quantise(offset)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
