@@ -584,7 +584,8 @@ Tensor moe_combine(Tensor expert_out, const Tensor& pair_pos, Tensor weights, Op
 
 // The whole routed-expert MLP (racetrack_b200/moe.py, fused_moe_experts). Returns y and, for
 // stage-wise checks, (offsets, sorted_pairs, pair_pos, x_gs, x_amax, gate_up, h, h_amax, expert_out).
-py::tuple moe_experts(const OptTensor& x, const Tensor& weights, const Tensor& indices, const Tensor& w13_codes,
+using Experts = std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor, Tensor, Tensor, Tensor, Tensor>;
+Experts moe_experts(const OptTensor& x, const Tensor& weights, const Tensor& indices, const Tensor& w13_codes,
                       const Tensor& w13_sf, const Tensor& w13_gs, const Tensor& w2_codes, const Tensor& w2_sf,
                       const Tensor& w2_gs, int64_t count, int64_t inter, int64_t n_experts, int64_t expert_begin,
                       const OptTensor& shared, bool f32_out, const OptTensor& q_codes, const OptTensor& q_sf,
@@ -644,10 +645,15 @@ py::tuple moe_experts(const OptTensor& x, const Tensor& weights, const Tensor& i
             std::tie(a_codes, a_sf) = moe_gather_nvfp4(x_codes, x_sf, sorted_pairs, topk, tile_map, tile_count, pairs);
         }
     }
-    if (around_w13) (*around_w13)(true);
+    auto around = [&](bool begin) {
+        if (!around_w13) return;
+        py::gil_scoped_acquire gil;
+        (*around_w13)(begin);
+    };
+    around(true);
     Tensor gate_up_out = gemm_nvfp4_grouped(a_codes, a_sf, x_gs, w13_codes, w13_sf, w13_gs, tile_map, tile_count,
                                             2 * inter, count, std::nullopt);
-    if (around_w13) (*around_w13)(false);
+    around(false);
     // SwiGLU once: this pass writes h and finds the tensor-wide amax its quantisation needs
     const Tensor gate = gate_up_out.slice(1, 0, inter), up = gate_up_out.slice(1, inter, 2 * inter);
     Tensor h = empty({pairs, inter}, at::kBFloat16, gate_up_out), h_amax = amax2.slice(0, 1, 2);
@@ -659,12 +665,12 @@ py::tuple moe_experts(const OptTensor& x, const Tensor& weights, const Tensor& i
     Tensor expert_out = gemm_nvfp4_grouped(h_codes, h_sf, h_gs, w2_codes, w2_sf, w2_gs, tile_map, tile_count, hidden,
                                            count, std::nullopt);
     Tensor y = moe_combine(expert_out, pair_pos, weights, shared, 0, std::nullopt, begin, end, f32_out, out);
-    return py::make_tuple(y, offsets, sorted_pairs, pair_pos, x_gs, x_amax, gate_up_out, h, h_amax, expert_out);
+    return {y, offsets, sorted_pairs, pair_pos, x_gs, x_amax, gate_up_out, h, h_amax, expert_out};
 }
 
 // ---- sparse indexer and decode attention -----------------------------------------------------------
 
-py::tuple index_prep(const Tensor& x, const Tensor& freqs_cis, const OptTensor& positions, const OptTensor& ln_weight,
+std::tuple<Tensor, Tensor, OptTensor> index_prep(const Tensor& x, const Tensor& freqs_cis, const OptTensor& positions, const OptTensor& ln_weight,
                      const OptTensor& ln_bias, double eps, bool return_rotated, const OptTensor& codes_into,
                      const OptTensor& scales_into) {
     require_cuda({&x, &freqs_cis});
@@ -700,7 +706,7 @@ py::tuple index_prep(const Tensor& x, const Tensor& freqs_cis, const OptTensor& 
         codes_into->copy_(codes.view({s_len, heads * dim}));
         scales_into->copy_(scales.view({s_len * heads}));
     }
-    return return_rotated ? py::make_tuple(codes, scales, *rotated) : py::make_tuple(codes, scales);
+    return {codes, scales, rotated};
 }
 
 Tensor index_head_weights(const Tensor& both, const Tensor& q_scale, double c1, double c2) {
@@ -800,7 +806,9 @@ PYBIND11_MODULE(_rt_torch, m) {
 #undef RT_NAME
         return names;
     });
-#define RT_DEF(name) m.def(#name, &name)
+    // Other Python threads run while a call checks, allocates and launches: a launch may block on a full
+    // queue (as behind a ctypes call, which lets go of the interpreter too).
+#define RT_DEF(name) m.def(#name, &name, py::call_guard<py::gil_scoped_release>())
     RT_DEF(residual_norm);
     RT_DEF(rms_norm);
     RT_DEF(norm_rope);

@@ -463,7 +463,8 @@ def index_prep(x: torch.Tensor, freqs_cis: torch.Tensor, *, positions: Optional[
     (default 0..S-1). Returns (codes float8_e4m3fn [S, H, 128], scales fp32 [S, H]) and, on
     request, the rotated bf16 tensor that was quantised."""
     into = _into if _into is not None else (None, None)
-    return _native().index_prep(x, freqs_cis, positions, ln_weight, ln_bias, eps, return_rotated, *into)
+    prepared = _native().index_prep(x, freqs_cis, positions, ln_weight, ln_bias, eps, return_rotated, *into)
+    return prepared if return_rotated else prepared[:2]
 
 
 def index_head_weights(x: torch.Tensor, weights_proj: torch.Tensor, q_scale: torch.Tensor) -> torch.Tensor:
