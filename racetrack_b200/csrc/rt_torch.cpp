@@ -135,9 +135,9 @@ Tensor freqs_table(const Tensor& freqs_cis, int64_t half) {
     return table.scalar_type() == at::kFloat ? table : table.to(at::kFloat);
 }
 
-// Whether `out` can take [rows, cols] of `type` rows in place (a slice of a cache).
-bool row_slots(const Tensor& out, int64_t rows, int64_t cols, at::ScalarType type, int64_t align) {
-    return out.is_cuda() && out.scalar_type() == type && out.dim() == 2 && same_shape(out, {rows, cols}) &&
+// Whether `out` can take [rows, cols] of `type` rows in place (a slice of a cache on x's device).
+bool row_slots(const Tensor& out, const Tensor& x, int64_t rows, int64_t cols, at::ScalarType type, int64_t align) {
+    return out.device() == x.device() && out.scalar_type() == type && out.dim() == 2 && same_shape(out, {rows, cols}) &&
            out.stride(1) == 1 && (rows <= 1 || out.stride(0) >= cols) &&
            out.stride(0) * out.element_size() % align == 0 &&
            reinterpret_cast<uintptr_t>(out.data_ptr()) % align == 0;
@@ -185,8 +185,8 @@ std::tuple<Tensor, Tensor, Tensor> norm_rope(const Tensor& q_c, const Tensor& q_
     if (qw.scalar_type() != kvw.scalar_type()) kvw = kvw.to(qw.scalar_type());
     Tensor q_out = empty(q_c.sizes(), at::kBFloat16, q_c);
     // into the caller's rows where they can be written as they are, else a tensor and a copy
-    const bool into = kv_into && k_into && row_slots(*kv_into, tokens, kv2.size(1), at::kBFloat16, 16) &&
-                      row_slots(*k_into, tokens, k2.size(1), at::kBFloat16, 2);
+    const bool into = kv_into && k_into && row_slots(*kv_into, q_c, tokens, kv2.size(1), at::kBFloat16, 16) &&
+                      row_slots(*k_into, q_c, tokens, k2.size(1), at::kBFloat16, 2);
     Tensor kv_out = into ? *kv_into : empty(kv_c.sizes(), at::kBFloat16, kv_c);
     Tensor k_out = into ? *k_into : empty(k_pe.sizes(), at::kBFloat16, k_pe);
     check(p_rt_norm_rope_into(q2.data_ptr(), qw.data_ptr(), kv2.data_ptr(), kvw.data_ptr(), weight_tag(qw),
@@ -683,7 +683,8 @@ std::tuple<Tensor, Tensor, OptTensor> index_prep(const Tensor& x, const Tensor& 
     if (fr.dim() < 2 || fr.size(-2) != 32 || fr.size(-1) != 2) fail("index_prep: freqs_cis must be [table, 32] complex");
     // one key per token: into the caller's cache rows where they can be written as they are
     const bool into = codes_into && scales_into && heads == 1 &&
-                      row_slots(*codes_into, s_len, dim, at::kFloat8_e4m3fn, 4) && scales_into->is_cuda() &&
+                      row_slots(*codes_into, x, s_len, dim, at::kFloat8_e4m3fn, 4) &&
+                      scales_into->device() == x.device() &&
                       scales_into->scalar_type() == at::kFloat && scales_into->dim() == 1 &&
                       scales_into->size(0) == s_len && (s_len <= 1 || scales_into->stride(0) >= 1);
     Tensor codes = into ? *codes_into : empty({s_len, heads, dim}, at::kFloat8_e4m3fn, x);

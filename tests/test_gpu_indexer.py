@@ -347,3 +347,25 @@ def test_latent_rows_written_into_a_cache(ops):
         q, _, _ = ops.fused_norm_rope(*args, eps=1e-6, rope_base=10000.0, _into=(kv[:, 1, :512], pe[:, 1, :64]))
         assert torch.equal(q, want[0]) and torch.equal(kv[:, 1, :512], want[1]) and torch.equal(pe[:, 1, :64], want[2])
         assert not kv[:, [0, 2]].any() and not pe[:, [0, 2]].any() and not kv[:, 1, 512:].any() and not pe[:, 1, 64:].any()
+
+
+@pytest.mark.parametrize("where", ["cpu", "cuda:1"])
+def test_rows_written_into_a_cache_of_another_device(ops, where):
+    """Caches that lie on another device take the rows through a copy."""
+    if torch.device(where).index and torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    g = torch.Generator().manual_seed(8)
+    x = torch.randn(4, 1, 128, generator=g).bfloat16().cuda()
+    freqs = torch.polar(torch.ones(4, 32), torch.randn(4, 32, generator=g)).cuda()
+    codes, scales = ops.index_prep(x, freqs)
+    cache = torch.zeros(4, 3, 128, device=where).to(torch.float8_e4m3fn)
+    scale_cache = torch.zeros(4, 3, device=where)
+    ops.index_prep(x, freqs, _into=(cache[:, 1], scale_cache[:, 1]))
+    assert torch.equal(cache[:, 1].view(torch.uint8).cpu(), codes.view(4, 128).view(torch.uint8).cpu())
+    assert torch.equal(scale_cache[:, 1].cpu(), scales.view(4).cpu())
+    qkv, ones, pos = x.view(4, 128), torch.ones(64, device="cuda", dtype=torch.bfloat16), torch.arange(4, device="cuda")
+    args = (qkv[:, :64], ones, qkv[:, :64], ones, qkv[:, 64:], pos)
+    _, kv, pe = ops.fused_norm_rope(*args, eps=1e-6, rope_base=1e4)
+    kv_cache, pe_cache = (torch.zeros(4, 3, 64, device=where, dtype=torch.bfloat16) for _ in range(2))
+    ops.fused_norm_rope(*args, eps=1e-6, rope_base=1e4, _into=(kv_cache[:, 1], pe_cache[:, 1]))
+    assert torch.equal(kv_cache[:, 1].cpu(), kv.cpu()) and torch.equal(pe_cache[:, 1].cpu(), pe.cpu())
