@@ -483,7 +483,7 @@ def fp8_index(q: torch.Tensor, weights: torch.Tensor, k: torch.Tensor, k_scale: 
     first N rows of longer per-sequence caches), k_scale fp32 [B, N] or [B, N, 1]; the batch
     dimension may be missing. With causal_offset = c, keys n > m + c get -inf (the mask the
     reference adds before top-k). One launch for all sequences. Returns fp32 [B, M, N]."""
-    return _native().fp8_index(q, weights, k, k_scale, causal_offset)
+    return _native().fp8_index(q, weights, k, k_scale, None if causal_offset is None else int(causal_offset))
 
 
 def index_topk(scores: torch.Tensor, topk: int) -> torch.Tensor:

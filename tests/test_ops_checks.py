@@ -61,3 +61,11 @@ def test_a_missing_tensor_is_refused(call):
     """A None where a tensor belongs raises; it is not dereferenced."""
     with pytest.raises(RuntimeError, match="is missing|must be a pair"):
         call()
+
+
+@pytest.mark.parametrize("offset", [None, 3, 3.0, torch.tensor(3.0)])
+def test_numbers_of_any_kind_are_taken(offset):
+    """A causal offset that int() takes gets past the conversion (to the check for CUDA tensors)."""
+    z = torch.zeros
+    with pytest.raises(RuntimeError, match="need CUDA"):
+        ops.fp8_index(z(1, 2, 4, 128), z(1, 2, 4), z(1, 5, 128), z(1, 5), causal_offset=offset)
