@@ -6,12 +6,15 @@ object is missing or a call returns a non-zero status, a RuntimeError is raised.
 from __future__ import annotations
 
 import ctypes
+import importlib.metadata
 import importlib.util
+import sys
 from ctypes import c_char_p, c_float, c_int, c_int64, c_void_p
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "librt_b200.so"
 TORCH_PATH = LIB_PATH.with_name("_rt_torch.so")
+TORCH_STAMP = LIB_PATH.with_name("_rt_torch.stamp")     # the torch and Python it was compiled against
 
 RT_BF16, RT_F32, RT_F16 = 0, 1, 2
 RT_ROPE_HALF, RT_ROPE_INTERLEAVED = 0, 1
@@ -108,6 +111,11 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+def torch_abi() -> str:
+    """What a compiled tensor-level module depends on besides its source."""
+    return f"torch {importlib.metadata.version('torch')} python {sys.version_info[0]}.{sys.version_info[1]}"
+
+
 _native = None
 
 
@@ -121,6 +129,9 @@ def native():
     if not TORCH_PATH.exists():
         raise RuntimeError(
             f"_rt_torch.so not found at {TORCH_PATH}; build it with `python -m racetrack_b200.build`")
+    if TORCH_STAMP.exists() and TORCH_STAMP.read_text() != torch_abi():
+        raise RuntimeError(f"_rt_torch.so was built for {TORCH_STAMP.read_text()}, this is {torch_abi()}; "
+                           "build it again with `python -m racetrack_b200.build`")
     import torch  # noqa: F401  (its libraries resolve the module's symbols)
     spec = importlib.util.spec_from_file_location("_rt_torch", TORCH_PATH)
     mod = importlib.util.module_from_spec(spec)

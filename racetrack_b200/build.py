@@ -16,11 +16,13 @@ import sys
 import sysconfig
 from pathlib import Path
 
+from . import _lib
+
 PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_DIR = PKG_DIR / "lib"
 LIB_PATH = LIB_DIR / "librt_b200.so"
-TORCH_PATH = LIB_DIR / "_rt_torch.so"
+TORCH_PATH = _lib.TORCH_PATH
 STAMP = LIB_DIR / "librt_b200.stamp"
 
 # Flags per source. The element-wise kernels are built without FMA contraction so
@@ -55,6 +57,9 @@ def _fingerprint() -> str:
                        + [PKG_DIR.parent / "include" / "rt_b200.h", Path(__file__)]):
         h.update(path.name.encode())
         h.update(path.read_bytes())
+    # _rt_torch.so is compiled against the installed torch and the running Python
+    h.update(_lib.torch_abi().encode())
+    h.update(" ".join(_torch_command()).encode())
     return h.hexdigest()
 
 
@@ -63,8 +68,8 @@ def _torch_command() -> list[str]:
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     includes = [torch_dir / "include", torch_dir / "include/torch/csrc/api/include",
                 sysconfig.get_paths()["include"], f"{cuda_home}/include"]
-    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
-            "-DTORCH_EXTENSION_NAME=_rt_torch", *[f"-I{d}" for d in includes],
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
+            "-DTORCH_EXTENSION_NAME=_rt_torch", *[f"-isystem{d}" for d in includes],
             str(CSRC / "rt_torch.cpp"), "-o", str(TORCH_PATH), f"-L{torch_dir / 'lib'}",
             "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python",
             f"-Wl,-rpath,{torch_dir / 'lib'}"]
@@ -101,6 +106,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         raise RuntimeError("librt_b200 build failed")
     link = [nvcc, "-shared", "-o", str(LIB_PATH), *objs, "-lcudart"]
     subprocess.run(link, check=True)
+    _lib.TORCH_STAMP.write_text(_lib.torch_abi())
     STAMP.write_text(fp)
     return LIB_PATH
 
