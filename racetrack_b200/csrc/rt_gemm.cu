@@ -2229,6 +2229,10 @@ static int launch_nvfp4_single(const void* a_codes, const void* a_sf, const floa
     CUtensorMap tb;
     TokenMaps ta;
     for (int b = 0; b < 5; ++b) {
+        if (b > 0 && (4 << b) >= total_rows) {          // no tile has more rows than the box before this one
+            ta.box[b] = ta.box[b - 1];
+            continue;
+        }
         if (int rc = make_tmap_2d(&ta.box[b], CU_TENSOR_MAP_DATA_TYPE_UINT8, a_codes, K / 2, total_rows,
                                   K / 2, 128, 8u << b))
             return rc;
