@@ -256,6 +256,19 @@ def test_swiglu_of_every_bf16_gate(ops):
         assert torch.equal(got.view(torch.int16)[~nan], want.view(torch.int16)[~nan]), f"up = {up}"
 
 
+def test_swiglu_of_every_bf16_gate_and_up_mantissa(ops):
+    """bf16(silu(g) * u) for every gate against all 128 mantissas of up: among them lie the products next
+    to a rounding boundary of bf16, where a last bit of the fp32 quotient shows."""
+    gate = torch.arange(-32768, 32768, device="cuda").to(torch.int16).view(torch.bfloat16)
+    up = (torch.arange(128, device="cuda").to(torch.int16) + 0x3f80).view(torch.bfloat16)       # [1, 2)
+    g, u = gate[:, None].expand(-1, 128).contiguous(), up.expand(65536, 128).contiguous()
+    want = (torch.nn.functional.silu(g.float()) * u.float()).to(torch.bfloat16)
+    got = ops.fused_swiglu(g, u)
+    nan = torch.isnan(want)
+    assert torch.equal(torch.isnan(got), nan)
+    assert torch.equal(got.view(torch.int16)[~nan], want.view(torch.int16)[~nan])
+
+
 def test_swiglu_nvfp4_quant_without_rows(ops):
     x = torch.empty(0, 256, device="cuda", dtype=torch.bfloat16)
     codes, sf, _ = ops.fused_swiglu_nvfp4_quant(x, x)
