@@ -1118,6 +1118,7 @@ extern "C" int rt_mla_sparse_decode(const void* q_abs, const void* q_pe, const v
 }
 
 extern "C" int rt_attn_prefill_schedule(int schedule) {
+    // one schedule: the setting is kept for the caller and selects nothing
     const int prev = tc::g_attn_schedule;
     if (schedule >= 0 && schedule <= 2) tc::g_attn_schedule = schedule;
     return prev;

@@ -35,20 +35,14 @@ def _reference(q, k_nope, k_pe, v):
     return ref_layer.causal_attention(q, torch.cat((k_nope, pe), dim=-1), v)
 
 
-@pytest.mark.parametrize("schedule", [1, 2])
 @pytest.mark.parametrize("tokens,heads", [(1, 1), (7, 2), (128, 1), (129, 3), (256, 2), (300, 4),
                                           (513, 2), (640, 1), (1000, 3), (1300, 2)])
-def test_mla_shape_matches_the_reference(ops, tokens, heads, schedule):
+def test_mla_shape_matches_the_reference(ops, tokens, heads):
     """The DeepSeek-V3.2 head: 128 nope + 64 shared rope dims, values of width 128; ragged
-    lengths around the 128-row tiles, the 256-row blocks of the single-CTA schedule (1) and
-    the 512-row blocks of the CTA-pair schedule (2)."""
+    lengths around the 128-row tiles and the 256-row blocks of a CTA."""
     q, kn, kp, v = _qkv(tokens, heads, 128, 64, 128, 100 + tokens)
     want = _reference(q, kn, kp, v)
-    prev = ops.attention_prefill_schedule(schedule)
-    try:
-        got = ops.attention_prefill(q.cuda(), kn.cuda(), kp.cuda(), v.cuda())
-    finally:
-        ops.attention_prefill_schedule(prev)
+    got = ops.attention_prefill(q.cuda(), kn.cuda(), kp.cuda(), v.cuda())
     ops.tc_error_state()
     assert got.shape == want.shape and got.dtype == torch.bfloat16
     assert rel_err(got, want) <= 1e-2, f"relative error {rel_err(got, want)}"
@@ -71,20 +65,14 @@ def test_other_head_shapes(ops, nope, rope, v_dim, shared):
     assert rel_err(got, want) <= 1e-2, f"relative error {rel_err(got, want)}"
 
 
-@pytest.mark.parametrize("schedule", [1, 2])
-def test_strided_views_of_projection_outputs(ops, schedule):
+def test_strided_views_of_projection_outputs(ops):
     """q a view of the q_b output, k_nope / v column slices of one kv_b output [T, H, nope + v]:
     consumed in place; a per-head rope key as well."""
-    tokens, heads = 333, 4
-    prev = ops.attention_prefill_schedule(schedule)
-    try:
-        _strided_case(ops, tokens, heads)
-        q, kn, kp, v = _qkv(700, 3, 128, 64, 128, 58, shared_pe=False)
-        got = ops.attention_prefill(q.cuda(), kn.cuda(), kp.cuda(), v.cuda())
-        ops.tc_error_state()
-        assert rel_err(got, _reference(q, kn, kp, v)) <= 1e-2
-    finally:
-        ops.attention_prefill_schedule(prev)
+    _strided_case(ops, 333, 4)
+    q, kn, kp, v = _qkv(700, 3, 128, 64, 128, 58, shared_pe=False)
+    got = ops.attention_prefill(q.cuda(), kn.cuda(), kp.cuda(), v.cuda())
+    ops.tc_error_state()
+    assert rel_err(got, _reference(q, kn, kp, v)) <= 1e-2
 
 
 def _strided_case(ops, tokens, heads):
@@ -98,18 +86,9 @@ def _strided_case(ops, tokens, heads):
     assert rel_err(got, _reference(q, kn, kp, v)) <= 1e-2
 
 
-@pytest.mark.parametrize("schedule", [1, 2])
-def test_growing_maxima_and_large_scores(ops, schedule):
+def test_growing_maxima_and_large_scores(ops):
     """Scores that grow along the sequence (the running maximum is replaced again and again,
     the accumulator rescaled) and a wide score range (exp2 underflow of the early keys)."""
-    prev = ops.attention_prefill_schedule(schedule)
-    try:
-        _growing_case(ops)
-    finally:
-        ops.attention_prefill_schedule(prev)
-
-
-def _growing_case(ops):
     tokens, heads = 640, 2
     q, kn, kp, v = _qkv(tokens, heads, 128, 64, 128, 91, scale=1.0)
     ramp = torch.linspace(0.2, 3.0, tokens).view(tokens, 1, 1)
@@ -150,10 +129,22 @@ def test_longer_sequence_many_heads_against_the_same_math_on_the_gpu(ops):
     assert rel_err(got, full) <= 1e-2
 
 
-@pytest.mark.parametrize("tokens,heads", [(300, 3), (1500, 2)])
+@pytest.mark.parametrize("schedule", [0, 1, 2])
+def test_every_setting_runs_the_one_schedule(ops, schedule):
+    q, kn, kp, v = (t.cuda() for t in _qkv(300, 2, 128, 64, 128, 61))
+    want = ops.attention_prefill(q, kn, kp, v)
+    prev = ops.attention_prefill_schedule(schedule)
+    try:
+        assert torch.equal(ops.attention_prefill(q, kn, kp, v), want)
+    finally:
+        assert ops.attention_prefill_schedule(prev) == schedule
+
+
+@pytest.mark.parametrize("tokens,heads", [(1, 2), (127, 1), (128, 2), (129, 1), (255, 1), (256, 2), (257, 1),
+                                          (300, 3), (1500, 2)])
 def test_fp8_epilogue_equals_act_quant_of_the_bf16_output(tokens, heads):
     """attention_prefill(quantized=True): the codes and scales the kernel's own epilogue writes are
-    those fused_act_quant makes of the bf16 output of the same schedule (racetrack/models/
+    those fused_act_quant makes of the bf16 output (racetrack/models/
     deepseek.py:85-107 applied to racetrack/runtime/torch_ops.py:97-110), bit for bit; other head
     shapes run the quantiser behind the kernel."""
     from racetrack_b200 import ops
@@ -161,11 +152,7 @@ def test_fp8_epilogue_equals_act_quant_of_the_bf16_output(tokens, heads):
     q = (torch.randn(tokens, heads, 192, generator=g) * 0.4).bfloat16().cuda()
     kv = (torch.randn(tokens, heads, 256, generator=g) * 0.4).bfloat16().cuda()
     kpe = (torch.randn(tokens, 64, generator=g) * 0.4).bfloat16().cuda()
-    prev = ops.attention_prefill_schedule(2)
-    try:
-        plain = ops.attention_prefill(q, kv[..., :128], kpe, kv[..., 128:])
-    finally:
-        ops.attention_prefill_schedule(prev)
+    plain = ops.attention_prefill(q, kv[..., :128], kpe, kv[..., 128:])
     want_c, want_s = ops.fused_act_quant(plain.view(tokens, heads * 128))
     codes, scales = ops.attention_prefill(q, kv[..., :128], kpe, kv[..., 128:], quantized=True)
     assert torch.equal(codes.view(torch.uint8), want_c.view(torch.uint8))
