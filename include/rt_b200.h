@@ -652,8 +652,9 @@ int rt_mla_sparse_decode(const void* q_abs, const void* q_pe, const void* kv, co
  *      racetrack/models/deepseek.py:780-792 (MHA prefill of MLA.forward).
  */
 /* Selects the schedule of rt_attn_causal_prefill for this process and returns the previous
- * setting: 0 (default), 1 or 2. One schedule is left (one CTA per 256 query rows with key tiles
- * of 128), so every setting runs it. */
+ * setting: 0 = by tokens and heads (default), 1 = one CTA per 256 query rows with key tiles of
+ * 128, 2 = CTA pairs (tcgen05 cta_group::2, 256 query rows per pair, key tiles of 256) wherever
+ * the head shape is 128 + 64 / 128. */
 int rt_attn_prefill_schedule(int schedule);
 int rt_attn_causal_prefill(const void* q, const void* k_nope, const void* k_pe, const void* v,
                            void* out, int64_t tokens, int64_t heads, int64_t nope_dim,
@@ -681,6 +682,19 @@ int rt_attn_causal_prefill_fp8(const void* q, const void* k_nope, const void* k_
                                int64_t kn_head_stride, int64_t kp_token_stride, int64_t kp_head_stride,
                                int64_t v_token_stride, int64_t v_head_stride, float softmax_scale,
                                void* stream);
+
+/*
+ * Either of the two for a rank's share of the heads of a layer: `heads` of layer_heads (>= heads). The
+ * schedule is the one a call with all of the layer's heads would take, so the share has the bits that
+ * call gives. out (bf16) or, with out == NULL, out_codes and out_scales.
+ */
+int rt_attn_causal_prefill_share(const void* q, const void* k_nope, const void* k_pe, const void* v, void* out,
+                                 void* out_codes, float* out_scales, int64_t tokens, int64_t heads,
+                                 int64_t layer_heads, int64_t nope_dim, int64_t rope_dim, int64_t v_dim,
+                                 int64_t q_token_stride, int64_t q_head_stride, int64_t kn_token_stride,
+                                 int64_t kn_head_stride, int64_t kp_token_stride, int64_t kp_head_stride,
+                                 int64_t v_token_stride, int64_t v_head_stride, int64_t o_token_stride,
+                                 int64_t o_head_stride, float softmax_scale, void* stream);
 
 /* ------------------------------------------------------------------------ */
 /* Collective steps over NVLink peer memory (one process per GPU)              */

@@ -527,11 +527,8 @@ __device__ long long g_fa_trace[10 * 64];
 #define RT_FTRACE(ev, it) do { } while (0)
 #endif
 
-// What rt_attn_prefill_schedule was last given. There is one schedule: the CTA pairs with key tiles
-// of 256 keys that used to take the MLA head shape from 1024 tokens on only paid while every MMA
-// cost its issuing thread 60 - 70 cycles (28 large MMAs per 256 keys instead of 40). With
-// the issuing loops behind elect_one() one B200 gives, pairs against this schedule: 8192 tokens x 128
-// heads 2643 / 2438 us, 4096 731 / 645, 2048 259 / 219, 1024 106 / 85, 777 97 / 71.
+// 0: by size (attn_pairs_pay), 1: the single-CTA kernel, 2: CTA pairs wherever the head shape allows
+// (rt_attn_prefill_schedule; for A/B measurements and tests).
 static int g_attn_schedule = 0;
 
 struct PrefillArgs {
@@ -600,9 +597,10 @@ __device__ __forceinline__ void ex2_poly2(uint64_t x, float& p0, float& p1) {
 // partial sums). One pair in kPolyEvery takes the polynomial, the rest the special-function unit
 // (0: none take it).
 // The softmax of a tile is a chain between two MMAs, so its instructions count although neither the
-// issue slots nor the special-function unit are full: two elements per FMA and an eighth of the
-// exponentials off the special-function unit, 4096 tokens x 128 heads 717 -> 673 us, 2048 226 -> 218
-// (one pair in 4: the same; one in 2: 731; no polynomial: 709).
+// issue slots nor the special-function unit are full: two elements per FMA. Taking an eighth of the
+// exponentials off the special-function unit is worth what two runs differ by (one B200, 128 heads,
+// one pair in 6 / none / one in 4: 8192 tokens 2452 / 2468 / 2492 us, 4096 701 / 709 / 717, 2048
+// 241 / 241 / 243).
 #ifndef RT_FA_POLY_EVERY
 #define RT_FA_POLY_EVERY 6
 #endif
@@ -968,6 +966,370 @@ __global__ void __launch_bounds__(kFThreads, 1) attn_prefill_kernel(
     }
 }
 
+// ---------------------------------------------------------------------------
+// The same attention on CTA PAIRS (tcgen05 cta_group::2) with key tiles of 256 keys, for the
+// MLA head shape (128 nope + 64 rope dims, values of 128)
+// ---------------------------------------------------------------------------
+// The kernel above gives 256 query rows to one CTA. With few heads (a rank of a tensor-parallel layer)
+// there are fewer such CTAs than SMs, or the longest of them, which walks all the keys, outlasts the
+// rest. Here a pair of CTAs covers 256 query rows of one head (128 per CTA) and walks key tiles of 256
+// keys, so the longest walk takes about half as long, on twice as many SMs:
+//   S = Q K^T     12 MMAs of 256 x 256 x 16 (each CTA brings its own 128 query rows as A and 128
+//                 of the tile's keys as B), 128 cycles of tensor core each;
+//   O += P V      16 MMAs of 256 x 128 x 16 (A = P from tensor memory, B = the values MN-major,
+//                 each CTA bringing 64 of the 128 value dims for all 256 keys), 64 cycles each;
+// Tensor memory per CTA: S 256 columns | P 128 (bf16 pairs) | O 128. P has its own columns,
+// so S(j + 1) is issued as soon as the softmax threads hold the scores of tile j in registers
+// and runs under their exponentials; O += P(j) V(j) follows when P(j) is complete. Softmax: 16
+// warps, four threads per query row with 64 scores each; the four partial maxima of a row meet
+// in shared memory as bf16. A thread writes P(j) only after O += P(j - 1) V(j - 1) has completed
+// (the same barrier tells it that O is at rest for a rescale). Shared memory per CTA: Q 48 KB,
+// two stages of its 128 keys (96 KB), two stages of its 64 value dims of 256 keys (64 KB).
+// One thread of the leader CTA (cluster rank 0) issues every MMA and commits to the barriers of
+// both CTAs; the peer's warp 1 relays "my tiles have landed" to the leader; the softmax warps of
+// both CTAs arrive on the leader's s_free and p_full. Loads never use multicast.
+constexpr uint32_t kGQOff = 0;                              // [3 chunks][128 rows][128 B]
+constexpr uint32_t kGKOff = 3 * kFChunk;                    // key stages: 2 x 3 chunks of this CTA's 128 keys
+constexpr uint32_t kGKStage = 3 * kFChunk;
+constexpr uint32_t kGVOff = kGKOff + 2 * kGKStage;          // value stages: 2 x [256 keys][64 dims]
+constexpr uint32_t kGVStage = 2 * kFChunk;
+constexpr uint32_t kGBarOff = kGVOff + 2 * kGVStage;
+constexpr int kGBars = 15;     // q_full k_full[2] v_full[2] s_done[2] pv_done[2] s_free p_full row_sync[4]
+constexpr uint32_t kGXmOff = kGBarOff + kGBars * 8 + 16;    // row maxima as bf16 [2 steps][128 rows][4]
+constexpr uint32_t kGSmemBytes = kGXmOff + 2 * 128 * 4 * 2 + 1024;
+constexpr uint32_t kGTmemP = 256, kGTmemO = 384;            // first column of P and of O
+static_assert(kGSmemBytes <= 232448, "shared memory budget");
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFThreads, 1) attn_prefill_pair_kernel(
+    const __grid_constant__ CUtensorMap tm_qn, const __grid_constant__ CUtensorMap tm_qp,
+    const __grid_constant__ CUtensorMap tm_kn, const __grid_constant__ CUtensorMap tm_kp,
+    const __grid_constant__ CUtensorMap tm_v, const PrefillArgs a) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t bars = base + kGBarOff;
+    const uint32_t q_full = bars;
+    auto k_full = [&](int st) { return bars + 8u * (1 + st); };
+    auto v_full = [&](int st) { return bars + 8u * (3 + st); };
+    auto s_done = [&](int st) { return bars + 8u * (5 + st); };     // S of a key tile complete: scores
+                                                                    // readable, its key stage free
+    auto pv_done = [&](int st) { return bars + 8u * (7 + st); };    // O += P V of a key tile complete: its
+                                                                    // value stage and P free, O at rest
+    const uint32_t s_free = bars + 8u * 9, p_full = bars + 8u * 10; // used in the leader only
+    auto row_sync = [&](int quad) { return bars + 8u * (11 + quad); };  // the four warps that share query rows
+    const uint32_t slot = bars + 8u * kGBars;
+    volatile uint32_t* slot_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + kGBarOff + 8 * kGBars);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(slot_ptr + 1);
+
+    const int warp = uniform_warp_id(), lane = threadIdx.x & 31;
+    const int rank = static_cast<int>(cluster_ctarank());
+    const int qb = static_cast<int>(gridDim.x >> 1) - 1 - static_cast<int>(blockIdx.x >> 1);   // heaviest first
+    const int h = blockIdx.y;
+    const int q0 = qb * 256;                 // first query row of the pair
+    const int n = qb + 1;                    // key tiles 0 .. qb of 256 keys; the last one is diagonal
+
+    if (threadIdx.x == 0) {
+        *abort_flag = 0;
+        const uint32_t landed = rank == 0 ? 2 : 1;          // own producer (+ the peer's relay)
+        mbar_init(q_full, landed);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(k_full(i), landed);
+            mbar_init(v_full(i), landed);
+            mbar_init(s_done(i), 1);
+            mbar_init(pv_done(i), 1);
+        }
+        mbar_init(s_free, 32);                              // lane 0 of the 16 softmax warps of both CTAs
+        mbar_init(p_full, 32);
+        for (int i = 0; i < 4; ++i) mbar_init(row_sync(i), 4);
+        fence_mbar_init();
+        // The queries and the first two key tiles are requested here, by the thread that has just
+        // initialised the barriers they complete on (this CTA's own), so that their latency runs
+        // under the tensor-memory allocation and the cluster-wide synchronisation below instead
+        // of after them: a work item lasts some tens of microseconds and there are thousands.
+        const int pe_head0 = a.pe_shared ? 0 : h;
+        mbar_arrive_expect_tx(q_full, 3 * kFChunk);
+        tma_load_4d(base + kGQOff, &tm_qn, 0, q0 + 128 * rank, 0, h, q_full);
+        tma_load_4d(base + kGQOff + 2 * kFChunk, &tm_qp, 0, q0 + 128 * rank, 0, h, q_full);
+        for (int j = 0; j < 2 && j < n; ++j) {
+            const uint32_t dst = base + kGKOff + j * kGKStage;
+            mbar_arrive_expect_tx(k_full(j), kGKStage);
+            tma_load_4d(dst, &tm_kn, 0, 256 * j + 128 * rank, 0, h, k_full(j));
+            tma_load_4d(dst + 2 * kFChunk, &tm_kp, 0, 256 * j + 128 * rank, 0, pe_head0, k_full(j));
+        }
+        tma_prefetch_desc(&tm_v);
+    }
+    if (warp == 1) {
+        tmem_alloc_pair(slot, 512);
+        tmem_relinquish_pair();
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                          // the peer's barriers exist before anyone signals them
+    tc_fence_after();
+    const uint32_t tmem_base = *slot_ptr;
+
+    // The u-th use of a two-stage barrier (key tile 2 u + st) completes its phase u.
+    if (warp == 0) {
+        if (elect_one()) {
+            const int pe_head = a.pe_shared ? 0 : h;
+            bool ok = true;
+            auto load_k = [&](int j) {                         // this CTA's 128 keys of key tile j
+                const int st = j & 1;
+                if (j >= 2 && !(ok = mbar_wait(s_done(st), ((j >> 1) & 1) ^ 1u, abort_flag, 81))) return;
+                const uint32_t dst = base + kGKOff + st * kGKStage;
+                const int row = 256 * j + 128 * rank;
+                mbar_arrive_expect_tx(k_full(st), kGKStage);
+                tma_load_4d(dst, &tm_kn, 0, row, 0, h, k_full(st));
+                tma_load_4d(dst + 2 * kFChunk, &tm_kp, 0, row, 0, pe_head, k_full(st));
+            };
+            auto load_v = [&](int j) {                         // this CTA's 64 value dims of key tile j
+                const int st = j & 1;
+                if (j >= 2 && !(ok = mbar_wait(pv_done(st), ((j >> 1) & 1) ^ 1u, abort_flag, 82))) return;
+                mbar_arrive_expect_tx(v_full(st), kGVStage);
+                tma_load_4d(base + kGVOff + st * kGVStage, &tm_v, 0, 256 * j, rank, h, v_full(st));
+            };
+            // in the order the stages become free: S(j) completes after O += P(j - 2) V(j - 2)
+            // (the queries and key tiles 0 and 1 were requested before the cluster-wide set-up)
+            for (int j = 0; ok && j < n; ++j) {
+                load_v(j);
+                if (ok && j + 2 < n) load_k(j + 2);
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (rank == 0 && elect_one()) {
+            // fp32 accumulate, bf16 x bf16, M = 256 over the pair; S: N = 256, both K-major; O: N = 128, B MN-major
+            const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (32u << 17) | (16u << 24);
+            const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (16u << 17) | (16u << 24);
+            auto issue_s = [&](int j) {
+                const uint32_t kb = base + kGKOff + (j & 1) * kGKStage;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const uint64_t adesc = smem_desc_sw128(base + kGQOff + c * kFChunk);
+                    const uint64_t bdesc = smem_desc_sw128(kb + c * kFChunk);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        mma_f16_pair(tmem_base, adesc + 2u * k, bdesc + 2u * k, idesc_s, (c | k) != 0 ? 1u : 0u);
+                }
+                mma_commit_pair_both(s_done(j & 1));
+            };
+            auto issue_pv = [&](int j) {
+                const uint32_t vb = base + kGVOff + (j & 1) * kGVStage;
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    mma_f16_ts_pair(tmem_base + kGTmemO, tmem_base + kGTmemP + 8u * k,
+                                    smem_desc_sw128_mn(vb + k * 2048, kGVStage), idesc_o, (j | k) != 0 ? 1u : 0u);
+                }
+                mma_commit_pair_both(pv_done(j & 1));
+            };
+            bool ok = mbar_wait(q_full, 0, abort_flag, 83) && mbar_wait(k_full(0), 0, abort_flag, 84);
+            if (ok) {
+                tc_fence_after();
+                issue_s(0);
+            }
+            for (int j = 0; ok && j < n; ++j) {
+                if (j + 1 < n) {
+                    RT_FTRACE(0, j);
+                    if (!(ok = mbar_wait(s_free, j & 1, abort_flag, 85))) break;
+                    if (!(ok = mbar_wait(k_full((j + 1) & 1), ((j + 1) >> 1) & 1, abort_flag, 84))) break;
+                    RT_FTRACE(1, j);
+                    tc_fence_after();
+                    issue_s(j + 1);
+                    RT_FTRACE(2, j);
+                }
+                if (!(ok = mbar_wait(p_full, j & 1, abort_flag, 86))) break;
+                RT_FTRACE(3, j);
+                if (!(ok = mbar_wait(v_full(j & 1), (j >> 1) & 1, abort_flag, 87))) break;
+                RT_FTRACE(4, j);
+                tc_fence_after();
+                issue_pv(j);
+                RT_FTRACE(5, j);
+            }
+        } else if (rank == 1 && elect_one()) {
+            // Relay: tells the leader that this CTA's tiles have landed, in the producer's order.
+            bool ok = mbar_wait(q_full, 0, abort_flag, 88);
+            if (ok) mbar_arrive_cluster(map_to_cta(q_full, 0));
+            auto relay = [&](uint32_t bar, int j) {
+                if ((ok = mbar_wait(bar, (j >> 1) & 1, abort_flag, 89))) mbar_arrive_cluster(map_to_cta(bar, 0));
+            };
+            if (ok) relay(k_full(0), 0);
+            if (ok && n > 1) relay(k_full(1), 1);
+            for (int j = 0; ok && j < n; ++j) {
+                relay(v_full(j & 1), j);
+                if (ok && j + 2 < n) relay(k_full(j & 1), j + 2);
+            }
+        }
+        __syncwarp();
+    } else {
+        const int quad = warp & 3;                            // the tensor-memory lane quarter it may touch
+        const int cq = (warp - 2) >> 2;                       // which 64 key columns of the tile
+        const int row = quad * 32 + lane;                     // query row within this CTA's tile
+        const int prow = 128 * rank + row;                    // query row within the pair's 256
+        const uint32_t row_bar = row_sync(quad);              // barrier of the four warps of these rows (a
+                                                              // bounded wait, unlike a named barrier)
+        const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
+        const uint32_t ts = tmem_base + lane_base + static_cast<uint32_t>(64 * cq);
+        const uint32_t tp = tmem_base + lane_base + kGTmemP + static_cast<uint32_t>(32 * cq);
+        const uint32_t to = tmem_base + lane_base + kGTmemO + static_cast<uint32_t>(32 * cq);
+        const uint32_t s_free_leader = map_to_cta(s_free, 0), p_leader = map_to_cta(p_full, 0);
+        const float ninf = __int_as_float(0xff800000);
+        __nv_bfloat16* xm_base = reinterpret_cast<__nv_bfloat16*>(base_ptr + kGXmOff) + row * 4;
+        float m_ref = ninf, l = 0.f;
+        bool ok = true;
+        for (int j = 0; ok && j < n; ++j) {
+            if (!(ok = mbar_wait(s_done(j & 1), (j >> 1) & 1, abort_flag, 90))) break;
+            if (threadIdx.x == 64) RT_FTRACE(6, j);
+            tc_fence_after();
+            // this thread's 64 scores in registers; then the score columns are free for the next tile
+            uint32_t r0[32], r1[32];
+            tmem_ld_32x32(ts, r0);
+            tmem_ld_32x32(ts + 32u, r1);
+            tmem_ld_wait(r0);
+            tmem_ld_wait(r1);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(s_free_leader);
+            if (threadIdx.x == 64) RT_FTRACE(7, j);
+            if (j == n - 1) {                                 // diagonal tile: keys beyond the row's own are masked
+                const int c0 = 64 * cq;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    if (c0 + i > prow) r0[i] = 0xff800000u;
+                    if (c0 + 32 + i > prow) r1[i] = 0xff800000u;
+                }
+            }
+            float mx0 = ninf, mx1 = ninf, mx2 = ninf, mx3 = ninf;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                mx0 = fmaxf(mx0, __uint_as_float(r0[i]));
+                mx1 = fmaxf(mx1, __uint_as_float(r0[16 + i]));
+                mx2 = fmaxf(mx2, __uint_as_float(r1[i]));
+                mx3 = fmaxf(mx3, __uint_as_float(r1[16 + i]));
+            }
+            // the four threads of a row exchange their maxima as bf16, so all use the same value;
+            // the slots alternate with the step, so a fast warp cannot overwrite one still being read
+            __nv_bfloat16* xm = xm_base + (j & 1) * 512;
+            xm[cq] = __float2bfloat16_rn(fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * a.scale_log2);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(row_bar);
+            if (!(ok = mbar_wait(row_bar, j & 1, abort_flag, 93))) break;
+            const uint2 all = *reinterpret_cast<const uint2*>(xm_base + (j & 1) * 512);
+            const __nv_bfloat162 p01 = *reinterpret_cast<const __nv_bfloat162*>(&all.x);
+            const __nv_bfloat162 p23 = *reinterpret_cast<const __nv_bfloat162*>(&all.y);
+            const float mt = fmaxf(fmaxf(__low2float(p01), __high2float(p01)),
+                                   fmaxf(__low2float(p23), __high2float(p23)));
+            const bool grow = mt > m_ref + 8.f;
+            const float m_new = grow ? mt : m_ref;
+            // the probabilities first, in registers: P(j - 1) still occupies the P columns
+            const uint64_t scale2 = pack_f32x2(a.scale_log2, a.scale_log2), neg_m2 = pack_f32x2(-m_new, -m_new);
+            uint64_t sums[2] = {0u, 0u};
+            uint32_t pk0[16], pk1[16];
+            softmax_chunk<RT_FA_POLY_EVERY>(r0, pk0, scale2, neg_m2, sums);
+            softmax_chunk<RT_FA_POLY_EVERY>(r1, pk1, scale2, neg_m2, sums);
+            if (threadIdx.x == 64) RT_FTRACE(8, j);
+            // P(j - 1) has been consumed and O is at rest once O += P(j - 1) V(j - 1) has completed
+            if (j > 0) {
+                if (!(ok = mbar_wait(pv_done((j - 1) & 1), ((j - 1) >> 1) & 1, abort_flag, 91))) break;
+                tc_fence_after();
+                if (__any_sync(0xffffffffu, grow)) {
+                    const float alpha = grow ? ex2_approx(m_ref - m_new) : 1.f;
+                    l *= alpha;
+#pragma unroll 1
+                    for (int c = 0; c < 4; ++c) {             // this thread's 32 output columns, 8 at a time
+                        uint32_t o[8];
+                        tmem_ld_32x8(to + 8u * c, o);
+                        tmem_ld_wait(o);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st_32x8(to + 8u * c, o);
+                    }
+                }
+            }
+            m_ref = m_new;
+            tmem_st_32x16(tp, pk0);
+            tmem_st_32x16(tp + 16u, pk1);
+            float s0, s1;
+            unpack_f32x2(add_f32x2(sums[0], sums[1]), s0, s1);
+            l += s0 + s1;
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(p_leader);
+            if (threadIdx.x == 64) RT_FTRACE(9, j);
+        }
+        if (ok && (ok = mbar_wait(pv_done((n - 1) & 1), ((n - 1) >> 1) & 1, abort_flag, 92))) {
+            tc_fence_after();
+            // the row's denominator is the sum of its four threads' partial sums: exchanged through
+            // the query tile's shared memory, which no MMA reads any more
+            float* xl = reinterpret_cast<float*>(base_ptr + kGQOff) + row * 4;
+            xl[cq] = l;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(row_bar);
+            ok = mbar_wait(row_bar, n & 1, abort_flag, 93);
+            const float4 ls = *reinterpret_cast<const float4*>(xl);
+            const float inv = 1.f / ((ls.x + ls.y) + (ls.z + ls.w));
+            const int token = q0 + prow;
+            uint32_t o[32];
+            tmem_ld_32x32(to, o);
+            tmem_ld_wait(o);
+            if (a.out_codes != nullptr) {
+                // act_quant of the bf16 output (racetrack/models/deepseek.py:85-107) without writing
+                // it: the 128 values of this row and head are one quantisation group; its amax is
+                // the maximum of the four threads' 32 values, rounded to bf16 as the tensor would be
+                float xb[32];
+                float amax = 0.f;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    xb[i] = __bfloat162float(__float2bfloat16_rn(__uint_as_float(o[i]) * inv));
+                    amax = fmaxf(amax, fabsf(xb[i]));
+                }
+                float* xa = xl + 512;                         // [128 rows][4], behind the denominators
+                xa[cq] = amax;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(row_bar);
+                ok = ok && mbar_wait(row_bar, (n + 1) & 1, abort_flag, 93);
+                const float4 am = *reinterpret_cast<const float4*>(xa);
+                amax = fmaxf(fmaxf(fmaxf(am.x, am.y), fmaxf(am.z, am.w)), 1.0e-4f);
+                const float scale = __fdiv_rn(amax, 448.0f);
+                const float rscale = __frcp_rn(scale);
+                if (ok && token < a.tokens) {
+                    uint32_t w[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        w[k] = attn_cvt_e4m3x2(div_shared(xb[4 * k], scale, rscale),
+                                               div_shared(xb[4 * k + 1], scale, rscale)) |
+                               (attn_cvt_e4m3x2(div_shared(xb[4 * k + 2], scale, rscale),
+                                                div_shared(xb[4 * k + 3], scale, rscale)) << 16);
+                    uint8_t* crow = a.out_codes + (static_cast<int64_t>(token) * a.heads + h) * 128 + 32 * cq;
+                    *reinterpret_cast<uint4*>(crow) = make_uint4(w[0], w[1], w[2], w[3]);
+                    *reinterpret_cast<uint4*>(crow + 16) = make_uint4(w[4], w[5], w[6], w[7]);
+                    if (cq == 0) a.out_scales[static_cast<int64_t>(token) * a.heads + h] = scale;
+                }
+            } else if (ok && token < a.tokens) {
+                __nv_bfloat16* orow = a.out + static_cast<int64_t>(token) * a.o_ts +
+                                      static_cast<int64_t>(h) * a.o_hs + 32 * cq;
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    uint4 w;
+                    w.x = pack_bf16x2(__uint_as_float(o[8 * v + 0]) * inv, __uint_as_float(o[8 * v + 1]) * inv);
+                    w.y = pack_bf16x2(__uint_as_float(o[8 * v + 2]) * inv, __uint_as_float(o[8 * v + 3]) * inv);
+                    w.z = pack_bf16x2(__uint_as_float(o[8 * v + 4]) * inv, __uint_as_float(o[8 * v + 5]) * inv);
+                    w.w = pack_bf16x2(__uint_as_float(o[8 * v + 6]) * inv, __uint_as_float(o[8 * v + 7]) * inv);
+                    *reinterpret_cast<uint4*>(orow + 8 * v) = w;
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();     // no CTA leaves, or frees tensor memory, while its peer may still signal it
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, 512);
+    }
+}
+
+int sm_count();                                    // rt_gemm.cu
 int make_tmap_bf16_4d(CUtensorMap* map, const void* ptr, const uint64_t dims[4], const uint64_t strides[3],
                       const uint32_t box[4]);      // rt_gemm.cu
 
@@ -976,13 +1338,13 @@ int make_tmap_bf16_4d(CUtensorMap* map, const void* ptr, const uint64_t dims[4],
 // (an SM retires about one tiled load per 500 cycles whatever its size); otherwise the row is
 // the fastest dimension and one box per chunk is issued, the part beyond dim reading as zero.
 static int make_attn_tmap(CUtensorMap* map, const void* ptr, int64_t dim, int64_t tokens, int64_t heads,
-                          int64_t ts, int64_t hs, bool* one_op) {
+                          int64_t ts, int64_t hs, bool* one_op, uint32_t box_rows = 128, uint32_t box_chunks = 0) {
     *one_op = dim % 64 == 0;
     if (*one_op) {
         const uint64_t dims[4] = {64, static_cast<uint64_t>(tokens), static_cast<uint64_t>(dim / 64),
                                   static_cast<uint64_t>(heads)};
         const uint64_t strides[3] = {static_cast<uint64_t>(ts) * 2, 128, static_cast<uint64_t>(hs) * 2};
-        const uint32_t box[4] = {64, 128, static_cast<uint32_t>(dim / 64), 1};
+        const uint32_t box[4] = {64, box_rows, box_chunks ? box_chunks : static_cast<uint32_t>(dim / 64), 1};
         return make_tmap_bf16_4d(map, ptr, dims, strides, box);
     }
     const uint64_t dims[4] = {static_cast<uint64_t>(dim), static_cast<uint64_t>(tokens), 1,
@@ -1118,7 +1480,6 @@ extern "C" int rt_mla_sparse_decode(const void* q_abs, const void* q_pe, const v
 }
 
 extern "C" int rt_attn_prefill_schedule(int schedule) {
-    // one schedule: the setting is kept for the caller and selects nothing
     const int prev = tc::g_attn_schedule;
     if (schedule >= 0 && schedule <= 2) tc::g_attn_schedule = schedule;
     return prev;
@@ -1126,7 +1487,7 @@ extern "C" int rt_attn_prefill_schedule(int schedule) {
 
 static int attn_causal_prefill(const void* q, const void* k_nope, const void* k_pe, const void* v,
                                void* out, void* out_codes, float* out_scales, int64_t tokens,
-                               int64_t heads, int64_t nope_dim, int64_t rope_dim, int64_t v_dim,
+                               int64_t heads, int64_t layer_heads, int64_t nope_dim, int64_t rope_dim, int64_t v_dim,
                                int64_t q_token_stride, int64_t q_head_stride, int64_t kn_token_stride,
                                int64_t kn_head_stride, int64_t kp_token_stride, int64_t kp_head_stride,
                                int64_t v_token_stride, int64_t v_head_stride, int64_t o_token_stride,
@@ -1141,7 +1502,7 @@ extern "C" int rt_attn_causal_prefill(const void* q, const void* k_nope, const v
                                       int64_t v_head_stride, int64_t o_token_stride,
                                       int64_t o_head_stride, float softmax_scale, void* stream) {
     RT_REQUIRE(out, RT_ERR_BAD_ARG, "rt_attn_causal_prefill: null pointer");
-    return attn_causal_prefill(q, k_nope, k_pe, v, out, nullptr, nullptr, tokens, heads, nope_dim, rope_dim,
+    return attn_causal_prefill(q, k_nope, k_pe, v, out, nullptr, nullptr, tokens, heads, heads, nope_dim, rope_dim,
                                v_dim, q_token_stride, q_head_stride, kn_token_stride, kn_head_stride,
                                kp_token_stride, kp_head_stride, v_token_stride, v_head_stride,
                                o_token_stride, o_head_stride, softmax_scale, stream);
@@ -1155,19 +1516,49 @@ extern "C" int rt_attn_causal_prefill_fp8(const void* q, const void* k_nope, con
                                           int64_t kp_token_stride, int64_t kp_head_stride,
                                           int64_t v_token_stride, int64_t v_head_stride,
                                           float softmax_scale, void* stream) {
-    RT_REQUIRE(out_codes && out_scales, RT_ERR_BAD_ARG, "rt_attn_causal_prefill_fp8: null pointer");
-    RT_REQUIRE(nope_dim == 128 && rope_dim == 64 && v_dim == 128, RT_ERR_UNSUPPORTED,
-               "rt_attn_causal_prefill_fp8: the FP8 epilogue exists for the 128 + 64 / 128 head shape");
-    RT_REQUIRE(aligned16(out_codes), RT_ERR_BAD_ARG, "rt_attn_causal_prefill_fp8: codes must be 16-byte aligned");
-    return attn_causal_prefill(q, k_nope, k_pe, v, nullptr, out_codes, out_scales, tokens, heads, nope_dim,
-                               rope_dim, v_dim, q_token_stride, q_head_stride, kn_token_stride, kn_head_stride,
-                               kp_token_stride, kp_head_stride, v_token_stride, v_head_stride, 8, 8,
-                               softmax_scale, stream);
+    return rt_attn_causal_prefill_share(q, k_nope, k_pe, v, nullptr, out_codes, out_scales, tokens, heads, heads,
+                                        nope_dim, rope_dim, v_dim, q_token_stride, q_head_stride, kn_token_stride,
+                                        kn_head_stride, kp_token_stride, kp_head_stride, v_token_stride,
+                                        v_head_stride, 8, 8, softmax_scale, stream);
+}
+
+extern "C" int rt_attn_causal_prefill_share(const void* q, const void* k_nope, const void* k_pe, const void* v,
+                                            void* out, void* out_codes, float* out_scales, int64_t tokens,
+                                            int64_t heads, int64_t layer_heads, int64_t nope_dim, int64_t rope_dim,
+                                            int64_t v_dim, int64_t q_token_stride, int64_t q_head_stride,
+                                            int64_t kn_token_stride, int64_t kn_head_stride,
+                                            int64_t kp_token_stride, int64_t kp_head_stride,
+                                            int64_t v_token_stride, int64_t v_head_stride, int64_t o_token_stride,
+                                            int64_t o_head_stride, float softmax_scale, void* stream) {
+    RT_REQUIRE(layer_heads >= heads, RT_ERR_BAD_ARG, "rt_attn_causal_prefill_share: layer_heads below heads");
+    if (out == nullptr) {
+        RT_REQUIRE(out_codes && out_scales, RT_ERR_BAD_ARG, "rt_attn_causal_prefill_fp8: null pointer");
+        RT_REQUIRE(nope_dim == 128 && rope_dim == 64 && v_dim == 128, RT_ERR_UNSUPPORTED,
+                   "rt_attn_causal_prefill_fp8: the FP8 epilogue exists for the 128 + 64 / 128 head shape");
+        RT_REQUIRE(aligned16(out_codes), RT_ERR_BAD_ARG,
+                   "rt_attn_causal_prefill_fp8: codes must be 16-byte aligned");
+    }
+    return attn_causal_prefill(q, k_nope, k_pe, v, out, out ? nullptr : out_codes, out ? nullptr : out_scales, tokens,
+                               heads, layer_heads, nope_dim, rope_dim, v_dim, q_token_stride, q_head_stride,
+                               kn_token_stride, kn_head_stride, kp_token_stride, kp_head_stride, v_token_stride,
+                               v_head_stride, o_token_stride, o_head_stride, softmax_scale, stream);
+}
+
+// Whether CTA pairs take a prefill of the 128 + 64 / 128 head shape: where every pair has its SMs at once
+// (one B200, single CTA / pairs: 16 heads x 1024 tokens 26 / 20 us, 8 x 2048 42 / 27, 32 x 512 18 / 16),
+// and from 3072 tokens on while the longest CTA takes a good part of what an SM has to do in all, its n
+// blocks of keys against heads x n x n / 2 over the SMs (16 heads x 4096 117 / 107, x 8192 329 / 305, 8 x
+// 4096 74 / 67). Elsewhere the single CTA's two query tiles in turn fill the tensor core better: 16 x
+// 2048 44 / 46, 32 x 1024 27 / 33, 64 x 4096 327 / 347, 128 x 1024 80 / 100, 128 x 8192 2336 / 2486;
+// 32 heads from 4096 tokens on are a tie.
+static bool attn_pairs_pay(int64_t tokens, int64_t heads) {
+    const int64_t blocks = (tokens + 255) / 256, sms = tc::sm_count();
+    return 2 * blocks * heads <= sms || (blocks >= 12 && 2 * blocks * heads <= 7 * sms);
 }
 
 static int attn_causal_prefill(const void* q, const void* k_nope, const void* k_pe, const void* v,
-                               void* out, void* out_codes, float* out_scales, int64_t tokens, int64_t heads, int64_t nope_dim,
-                                      int64_t rope_dim, int64_t v_dim, int64_t q_token_stride,
+                               void* out, void* out_codes, float* out_scales, int64_t tokens, int64_t heads,
+                                      int64_t layer_heads, int64_t nope_dim, int64_t rope_dim, int64_t v_dim, int64_t q_token_stride,
                                       int64_t q_head_stride, int64_t kn_token_stride,
                                       int64_t kn_head_stride, int64_t kp_token_stride,
                                       int64_t kp_head_stride, int64_t v_token_stride,
@@ -1227,6 +1618,23 @@ static int attn_causal_prefill(const void* q, const void* k_nope, const void* k_
         tm_kp = tm_kn;
     }
     a.one_op = (one[0] ? 1 : 0) | (one[1] ? 2 : 0) | (one[2] ? 4 : 0) | (one[3] ? 8 : 0) | (one[4] ? 16 : 0);
+    const bool mla_shape = nope_dim == 128 && rope_dim == 64 && v_dim == 128;
+    if (mla_shape && (tc::g_attn_schedule == 2 || (tc::g_attn_schedule == 0 && attn_pairs_pay(tokens, layer_heads)))) {
+        // the MLA head shape on CTA pairs with key tiles of 256 keys: a CTA brings 128 keys of a
+        // tile (the boxes above) and 64 of the value dims for all of its 256 keys
+        bool ignore;
+        if (int rc = tc::make_attn_tmap(&tm_v, v, v_dim, tokens, heads, v_token_stride, v_head_stride, &ignore,
+                                        256, 1))
+            return rc;
+        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&tc::attn_prefill_pair_kernel),
+                                         static_cast<int>(tc::kGSmemBytes), "rt_attn_causal_prefill"))
+            return rc;
+        dim3 pgrid(static_cast<unsigned>(2 * ((tokens + 255) / 256)), static_cast<unsigned>(heads));
+        tc::attn_prefill_pair_kernel<<<pgrid, tc::kFThreads, tc::kGSmemBytes, as_stream(stream)>>>(
+            tm_qn, tm_qp, tm_kn, tm_kp, tm_v, a);
+        count_launch();
+        return check_launch("attn_prefill_pair_kernel");
+    }
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&tc::attn_prefill_kernel),
                                      static_cast<int>(tc::kFSmemBytes), "rt_attn_causal_prefill"))
         return rc;

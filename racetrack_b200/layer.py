@@ -319,8 +319,9 @@ class RealisticLayer:
         if self.attn_core == "rt":
             kv = self.w_kv_b(kv_c).view(tokens, h, s.nope + s.v_dim)
             if quantized:
-                return ops.attention_prefill(q, kv[..., :s.nope], k_pe, kv[..., s.nope:], quantized=True, out=out)
-            local = ops.attention_prefill(q, kv[..., :s.nope], k_pe, kv[..., s.nope:])
+                return ops.attention_prefill(q, kv[..., :s.nope], k_pe, kv[..., s.nope:], quantized=True, out=out,
+                                             layer_heads=s.heads)
+            local = ops.attention_prefill(q, kv[..., :s.nope], k_pe, kv[..., s.nope:], layer_heads=s.heads)
         else:
             kv = self.w_kv_b(kv_c).view(tokens, h, s.qk_dim + s.v_dim)
             ops.head_broadcast_(kv[..., s.nope:s.qk_dim], k_pe)       # K = [k_nope | k_pe] in place

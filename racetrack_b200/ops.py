@@ -505,7 +505,8 @@ def mla_sparse_decode(q_abs: torch.Tensor, q_pe: torch.Tensor, kv_cache: torch.T
 
 def attention_prefill(q: torch.Tensor, k_nope: torch.Tensor, k_pe: Optional[torch.Tensor],
                       v: torch.Tensor, softmax_scale: Optional[float] = None, *,
-                      quantized: bool = False, out: Optional[tuple] = None):
+                      quantized: bool = False, out: Optional[tuple] = None,
+                      layer_heads: Optional[int] = None):
     """Causal attention over [tokens, heads, dim] tensors on the tensor cores
     (racetrack/runtime/torch_ops.py:97-110; the attention core of
     racetrack/realistic_bench.py:304-313): q bf16 [T, H, nope + rope]; the key of head h is
@@ -516,7 +517,10 @@ def attention_prefill(q: torch.Tensor, k_nope: torch.Tensor, k_pe: Optional[torc
     quantized=True returns act_quant of that output instead, (FP8 codes [T, H * v_dim], fp32 scales
     [T, H]), bit for bit what fused_act_quant makes of it; for the 128 + 64 / 128 head shape the
     attention kernel writes them from its own epilogue, otherwise the quantiser runs behind it.
-    ``out`` = (codes, scales) to write into (contiguous, 1-byte codes)."""
+    ``out`` = (codes, scales) to write into (contiguous, 1-byte codes).
+
+    layer_heads: the heads of the whole layer where a rank holds a share of them (default: H). The schedule
+    is the one the whole layer would take, so the share has the bits a call with every head gives."""
     _require_cuda(q, k_nope, v)
     tokens, heads, qk = q.shape
     nope = k_nope.shape[-1]
@@ -555,21 +559,21 @@ def attention_prefill(q: torch.Tensor, k_nope: torch.Tensor, k_pe: Optional[torc
                 raise RuntimeError("attention_prefill: out must be contiguous (1-byte codes [T, H*v], fp32 scales [T, H*v/128])")
         if (nope, rope, v_dim) != (128, 64, 128):
             # no fused epilogue for this head shape: the quantiser runs behind the attention kernel
-            return fused_act_quant(attention_prefill(q, k_nope, k_pe, v, softmax_scale)
+            return fused_act_quant(attention_prefill(q, k_nope, k_pe, v, softmax_scale, layer_heads=layer_heads)
                                    .view(tokens, heads * v_dim), out=out)
         if out is None:
             codes = torch.empty(tokens, heads * v_dim, dtype=torch.float8_e4m3fn, device=q.device)
             scales = torch.empty(tokens, heads, dtype=torch.float32, device=q.device)
-        _lib.check(lib.rt_attn_causal_prefill_fp8(
-            q.data_ptr(), k_nope.data_ptr(), k_pe.data_ptr(), v.data_ptr(), codes.data_ptr(),
-            scales.data_ptr(), tokens, heads, nope, rope, v_dim, q.stride(0), q.stride(1),
-            k_nope.stride(0), k_nope.stride(1), kp_ts, kp_hs, v.stride(0), v.stride(1),
+        _lib.check(lib.rt_attn_causal_prefill_share(
+            q.data_ptr(), k_nope.data_ptr(), k_pe.data_ptr(), v.data_ptr(), None, codes.data_ptr(),
+            scales.data_ptr(), tokens, heads, layer_heads or heads, nope, rope, v_dim, q.stride(0), q.stride(1),
+            k_nope.stride(0), k_nope.stride(1), kp_ts, kp_hs, v.stride(0), v.stride(1), 8, 8,
             float(softmax_scale), _stream()), "rt_attn_causal_prefill_fp8")
         return codes, scales
     out = torch.empty(tokens, heads, v_dim, dtype=torch.bfloat16, device=q.device)
-    _lib.check(lib.rt_attn_causal_prefill(
+    _lib.check(lib.rt_attn_causal_prefill_share(
         q.data_ptr(), k_nope.data_ptr(), k_pe.data_ptr() if rope else None, v.data_ptr(),
-        out.data_ptr(), tokens, heads, nope, rope, v_dim, q.stride(0), q.stride(1),
+        out.data_ptr(), None, None, tokens, heads, layer_heads or heads, nope, rope, v_dim, q.stride(0), q.stride(1),
         k_nope.stride(0), k_nope.stride(1), kp_ts, kp_hs, v.stride(0), v.stride(1),
         out.stride(0), out.stride(1), float(softmax_scale), _stream()), "rt_attn_causal_prefill")
     return out
@@ -583,8 +587,9 @@ def causal_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch
 
 
 def attention_prefill_schedule(schedule: int) -> int:
-    """Selects the schedule of attention_prefill for this process (0 default, 1, 2) and returns the
-    previous setting. One schedule is left, one CTA per 256 query rows: every setting runs it."""
+    """Selects the schedule of attention_prefill for this process (0 default = by tokens and heads,
+    1 one CTA per 256 query rows, 2 CTA pairs with key tiles of 256 where the head shape allows)
+    and returns the previous setting."""
     return int(_lib.load().rt_attn_prefill_schedule(int(schedule)))
 
 

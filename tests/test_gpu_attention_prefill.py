@@ -35,14 +35,20 @@ def _reference(q, k_nope, k_pe, v):
     return ref_layer.causal_attention(q, torch.cat((k_nope, pe), dim=-1), v)
 
 
+@pytest.mark.parametrize("schedule", [1, 2])
 @pytest.mark.parametrize("tokens,heads", [(1, 1), (7, 2), (128, 1), (129, 3), (256, 2), (300, 4),
                                           (513, 2), (640, 1), (1000, 3), (1300, 2)])
-def test_mla_shape_matches_the_reference(ops, tokens, heads):
+def test_mla_shape_matches_the_reference(ops, tokens, heads, schedule):
     """The DeepSeek-V3.2 head: 128 nope + 64 shared rope dims, values of width 128; ragged
-    lengths around the 128-row tiles and the 256-row blocks of a CTA."""
+    lengths around the 128-row tiles, the 256-row blocks of the single-CTA schedule (1) and
+    the 512-row blocks of the CTA-pair schedule (2)."""
     q, kn, kp, v = _qkv(tokens, heads, 128, 64, 128, 100 + tokens)
     want = _reference(q, kn, kp, v)
-    got = ops.attention_prefill(q.cuda(), kn.cuda(), kp.cuda(), v.cuda())
+    prev = ops.attention_prefill_schedule(schedule)
+    try:
+        got = ops.attention_prefill(q.cuda(), kn.cuda(), kp.cuda(), v.cuda())
+    finally:
+        ops.attention_prefill_schedule(prev)
     ops.tc_error_state()
     assert got.shape == want.shape and got.dtype == torch.bfloat16
     assert rel_err(got, want) <= 1e-2, f"relative error {rel_err(got, want)}"
@@ -65,14 +71,20 @@ def test_other_head_shapes(ops, nope, rope, v_dim, shared):
     assert rel_err(got, want) <= 1e-2, f"relative error {rel_err(got, want)}"
 
 
-def test_strided_views_of_projection_outputs(ops):
+@pytest.mark.parametrize("schedule", [1, 2])
+def test_strided_views_of_projection_outputs(ops, schedule):
     """q a view of the q_b output, k_nope / v column slices of one kv_b output [T, H, nope + v]:
     consumed in place; a per-head rope key as well."""
-    _strided_case(ops, 333, 4)
-    q, kn, kp, v = _qkv(700, 3, 128, 64, 128, 58, shared_pe=False)
-    got = ops.attention_prefill(q.cuda(), kn.cuda(), kp.cuda(), v.cuda())
-    ops.tc_error_state()
-    assert rel_err(got, _reference(q, kn, kp, v)) <= 1e-2
+    tokens, heads = 333, 4
+    prev = ops.attention_prefill_schedule(schedule)
+    try:
+        _strided_case(ops, tokens, heads)
+        q, kn, kp, v = _qkv(700, 3, 128, 64, 128, 58, shared_pe=False)
+        got = ops.attention_prefill(q.cuda(), kn.cuda(), kp.cuda(), v.cuda())
+        ops.tc_error_state()
+        assert rel_err(got, _reference(q, kn, kp, v)) <= 1e-2
+    finally:
+        ops.attention_prefill_schedule(prev)
 
 
 def _strided_case(ops, tokens, heads):
@@ -86,9 +98,18 @@ def _strided_case(ops, tokens, heads):
     assert rel_err(got, _reference(q, kn, kp, v)) <= 1e-2
 
 
-def test_growing_maxima_and_large_scores(ops):
+@pytest.mark.parametrize("schedule", [1, 2])
+def test_growing_maxima_and_large_scores(ops, schedule):
     """Scores that grow along the sequence (the running maximum is replaced again and again,
     the accumulator rescaled) and a wide score range (exp2 underflow of the early keys)."""
+    prev = ops.attention_prefill_schedule(schedule)
+    try:
+        _growing_case(ops)
+    finally:
+        ops.attention_prefill_schedule(prev)
+
+
+def _growing_case(ops):
     tokens, heads = 640, 2
     q, kn, kp, v = _qkv(tokens, heads, 128, 64, 128, 91, scale=1.0)
     ramp = torch.linspace(0.2, 3.0, tokens).view(tokens, 1, 1)
@@ -129,22 +150,18 @@ def test_longer_sequence_many_heads_against_the_same_math_on_the_gpu(ops):
     assert rel_err(got, full) <= 1e-2
 
 
-@pytest.mark.parametrize("schedule", [0, 1, 2])
-def test_every_setting_runs_the_one_schedule(ops, schedule):
-    q, kn, kp, v = (t.cuda() for t in _qkv(300, 2, 128, 64, 128, 61))
-    want = ops.attention_prefill(q, kn, kp, v)
-    prev = ops.attention_prefill_schedule(schedule)
-    try:
-        assert torch.equal(ops.attention_prefill(q, kn, kp, v), want)
-    finally:
-        assert ops.attention_prefill_schedule(prev) == schedule
+@pytest.fixture(params=[0, 1, 2], ids=["default", "single_cta", "cta_pairs"])
+def schedule_set(request, ops):
+    previous = ops.attention_prefill_schedule(request.param)
+    yield request.param
+    ops.attention_prefill_schedule(previous)
 
 
 @pytest.mark.parametrize("tokens,heads", [(1, 2), (127, 1), (128, 2), (129, 1), (255, 1), (256, 2), (257, 1),
                                           (300, 3), (1500, 2)])
-def test_fp8_epilogue_equals_act_quant_of_the_bf16_output(tokens, heads):
+def test_fp8_epilogue_equals_act_quant_of_the_bf16_output(schedule_set, tokens, heads):
     """attention_prefill(quantized=True): the codes and scales the kernel's own epilogue writes are
-    those fused_act_quant makes of the bf16 output (racetrack/models/
+    those fused_act_quant makes of the bf16 output of the same call (racetrack/models/
     deepseek.py:85-107 applied to racetrack/runtime/torch_ops.py:97-110), bit for bit; other head
     shapes run the quantiser behind the kernel."""
     from racetrack_b200 import ops
@@ -171,7 +188,7 @@ def test_fp8_epilogue_equals_act_quant_of_the_bf16_output(tokens, heads):
 
 @pytest.mark.parametrize("first", [0, 32, 96, 160])
 @pytest.mark.parametrize("special", [float("nan"), float("inf"), float("-inf")])
-def test_a_special_key_at_every_column(ops, first, special):
+def test_a_special_key_at_every_column(ops, schedule_set, first, special):
     """Head h has one key of infinite or NaN scores, at column first + h of its keys, so every column of
     a 32-key group is met: as in torch, a NaN or +infinity among the scores makes the row NaN from that
     key on, -infinity takes the key out (whatever its value), and the rows before it do not change."""
@@ -200,7 +217,7 @@ def test_a_special_key_at_every_column(ops, first, special):
 
 
 @pytest.mark.parametrize("tokens", [64, 128, 200, 257])
-def test_masked_keys_weigh_nothing(ops, tokens):
+def test_masked_keys_weigh_nothing(ops, schedule_set, tokens):
     """Values of keys behind a query do not reach it, however large they are."""
     q, kn, kp, v = (t.cuda() for t in _qkv(tokens, 2, 128, 64, 128, 400 + tokens))
     for cut in (1, 11, 33, tokens // 2, tokens - 1):
@@ -209,3 +226,41 @@ def test_masked_keys_weigh_nothing(ops, tokens):
         a, b = ops.attention_prefill(q, kn, kp, small), ops.attention_prefill(q, kn, kp, large)
         assert torch.equal(a[:cut], b[:cut]), cut
     ops.tc_error_state()
+
+
+@pytest.mark.parametrize("tokens,heads,share", [(1024, 64, 8), (300, 128, 4), (3100, 20, 10)])
+def test_a_share_of_the_heads_has_the_bits_of_the_whole(ops, tokens, heads, share):
+    """A rank's heads with layer_heads = all heads: the schedule, and every bit, of the call with all heads,
+    as bf16 and as FP8 codes; without it the few heads may take the other schedule (same values to bf16)."""
+    g = torch.Generator().manual_seed(tokens)
+    q, kv, kpe = ((torch.randn(*s, generator=g) * 0.4).bfloat16().cuda()
+                  for s in ((tokens, heads, 192), (tokens, heads, 256), (tokens, 64)))
+
+    def attend(lo, hi, **kw):
+        return ops.attention_prefill(q[:, lo:hi], kv[:, lo:hi, :128], kpe, kv[:, lo:hi, 128:], **kw)
+    whole = attend(0, heads)
+    codes, scales = attend(0, heads, quantized=True)
+    for lo in (0, heads - share):
+        part = attend(lo, lo + share, layer_heads=heads)
+        assert torch.equal(part, whole[:, lo:lo + share])
+        c, s = attend(lo, lo + share, layer_heads=heads, quantized=True)
+        assert torch.equal(c.view(torch.uint8), codes.view(torch.uint8)[:, lo * 128:(lo + share) * 128])
+        assert torch.equal(s, scales[:, lo:lo + share])
+        assert rel_err(attend(lo, lo + share), whole[:, lo:lo + share]) <= 1e-2
+    with pytest.raises(RuntimeError, match="layer_heads"):
+        attend(0, heads, layer_heads=heads - 1)
+    ops.tc_error_state()
+
+
+@pytest.mark.parametrize("tokens,heads", [(512, 37), (512, 36), (3072, 44), (2900, 20), (3072, 12), (4100, 30)])
+def test_both_sides_of_the_schedule_rule(ops, tokens, heads):
+    """Sizes next to the lines between the schedules: the default is one of the two, and both agree."""
+    q, kn, kp, v = (t.cuda() for t in _qkv(tokens, heads, 128, 64, 128, 500 + heads))
+    outs = []
+    for schedule in (0, 1, 2):
+        previous = ops.attention_prefill_schedule(schedule)
+        outs.append(ops.attention_prefill(q, kn, kp, v))
+        ops.attention_prefill_schedule(previous)
+    ops.tc_error_state()
+    assert torch.equal(outs[0], outs[1]) or torch.equal(outs[0], outs[2])
+    assert rel_err(outs[1], outs[2]) <= 1e-2
