@@ -2497,7 +2497,7 @@ extern "C" int rt_gemm_bf16_batched(const void* a, const void* b, void* c, int64
 extern "C" int64_t rt_gemm_bf16_splitk_splits(int64_t m, int64_t n, int64_t k) {
     // more rows than one row tile: K stays whole, so that a token's sums (a router's logits above all)
     // do not depend on how many others are in the call; the tile width occupies the SMs instead
-    if (m <= 0 || m > 128 || n <= 0 || k <= 0 || tc::g_bf16_schedule != 0) return 1;
+    if (m <= 0 || m > 128 || n <= 0 || k <= 0) return 1;
     return tc::pick_splits(n, k);
 }
 

@@ -327,6 +327,24 @@ def test_linear_bf16_rows_do_not_depend_on_the_call(ops, n, k, out_dtype):
     ops.tc_error_state()
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 2112, 7168), (64, 256, 7168), (128, 1024, 1032)])
+def test_few_rows_are_split_under_every_schedule(ops, m, n, k):
+    """The schedule setting chooses between tiles of many rows; a few-row product is cut along K whatever
+    it says, with the same bits."""
+    from racetrack_b200 import _lib
+    lib = _lib.load()
+    x, w = I.randn((m, k), 970 + m).cuda(), I.randn((n, k), 971, std=0.05).cuda()
+    splits, want = int(lib.rt_gemm_bf16_splitk_splits(m, n, k)), ops.linear_bf16(x, w)
+    assert splits > 1
+    for schedule in (1, 2):
+        previous = ops.gemm_bf16_schedule(schedule)
+        try:
+            assert int(lib.rt_gemm_bf16_splitk_splits(m, n, k)) == splits
+            assert torch.equal(ops.linear_bf16(x, w), want)
+        finally:
+            ops.gemm_bf16_schedule(previous)
+
+
 @pytest.mark.parametrize("m,n,k", [
     (13, 2112, 7168),       # a decode projection: nine tiles in quarters, those past column 2112 empty
     (1, 7168, 2048),        # a box of 8 rows, one of them there
