@@ -458,7 +458,8 @@ class RealisticLayer:
                 if self.w_o_full is not None:
                     # the heads' outputs change hands, not w_o's partial sums: 1 / world of the bytes
                     # (half of that again in FP8), and this half of the layer equals the single-GPU
-                    # evaluation bit for bit
+                    # evaluation bit for bit while a rank has more than 128 rows (linear_bf16 cuts K
+                    # for fewer)
                     if self.w_o_full.fp8:
                         self.attention_heads(px.local["qkv"], positions, quantized=True,
                                              out=(px.local["ao_codes"], px.local["ao_scales"]))
