@@ -352,6 +352,7 @@ def test_few_rows_are_split_under_every_schedule(ops, m, n, k):
     (2048, 7168, 2304),     # three full rounds and four tiles, in quarters
     (300, 4096, 384),       # 48 tiles in halves, three K blocks: one in the last buffer
     (64, 1024, 256),        # quarters, fewer K blocks than a buffer holds
+    (777, 7168, 640),       # a full round and 48 tiles in halves, five K blocks
     (777, 24576, 384),      # four full rounds and 80 tiles: whole
 ])
 def test_linear_fp8_tail_tiles_in_pieces(ops, m, n, k):

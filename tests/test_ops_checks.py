@@ -6,7 +6,7 @@ from types import SimpleNamespace
 import pytest
 import torch
 
-from racetrack_b200 import moe, ops
+from racetrack_b200 import _lib, moe, ops
 
 
 def _experts(hidden=128, inter=64, count=4):
@@ -69,3 +69,12 @@ def test_numbers_of_any_kind_are_taken(offset):
     z = torch.zeros
     with pytest.raises(RuntimeError, match="need CUDA"):
         ops.fp8_index(z(1, 2, 4, 128), z(1, 2, 4), z(1, 5, 128), z(1, 5), causal_offset=offset)
+
+
+@pytest.mark.parametrize("n,k", [(256, 7168), (2112, 7168), (7168, 16384), (1024, 2048)])
+def test_no_product_of_more_than_128_rows_is_cut_along_k(n, k):
+    """What the bit-identity of token-sharded layers rests on: a rank's rows and all rows are summed alike."""
+    lib = _lib.load()
+    for m in (129, 256, 512, 777, 8192):
+        assert lib.rt_gemm_bf16_splitk_splits(m, n, k) == 1
+        assert lib.rt_gemm_fp8_workspace_bytes(m, n, k) == 0
